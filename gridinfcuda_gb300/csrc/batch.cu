@@ -84,7 +84,7 @@ __device__ __forceinline__ SweepParams batch_params(const BatchLaunch &b, const 
 
 
 // Persistent kernel: half-sweeps it_begin..it_end-1 of every grid of one
-// label bucket (L == LM when EXACT, else L < LM; one kernel per bucket keeps
+// label bucket (L == LM when LMIN == LM, else LMIN <= L <= LM; one kernel per bucket keeps
 // the register allocation of the single-grid sweep).  Within
 // a half-sweep the tiles of all grids are independent: block k takes work-
 // list tiles k, k + gridDim.x, ... and issues the bulk load of its next tile
@@ -92,7 +92,7 @@ __device__ __forceinline__ SweepParams batch_params(const BatchLaunch &b, const 
 // binary search over the tile bases, kept in shared memory).  Between
 // half-sweeps each block waits for its own bulk stores, fences them against
 // the next half-sweep's bulk loads and meets the others at the grid barrier.
-template <int NW, int LM, bool EXACT, bool DIRECT = false>
+template <int NW, int LM, int LMIN, bool DIRECT = false>
 __global__ void __launch_bounds__(NW * 32) batch_kernel(const BatchLaunch b) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(NW * 32) batch_kernel(const BatchLaunch b) {
             tile_load<NW>(p, t - base, smem, &full_bar);
         }
         for (; t < b.total_tiles; t += gridDim.x) {
-            if (!tile_finish<float, float, LM, EXACT, NW, KIND_LINEAR, DIRECT>(
-                    p, table_consts<float, KIND_LINEAR>(p.V, EXACT ? LM : p.L), t - base, smem, &full_bar, parity))
+            if (!tile_finish<float, float, LM, LMIN, NW, KIND_LINEAR, DIRECT>(
+                    p, table_consts<float, KIND_LINEAR>(p.V, LMIN == LM ? LM : p.L), t - base, smem, &full_bar, parity))
                 return;
             const int tn = t + gridDim.x;
             if (tn < b.total_tiles) {
@@ -245,8 +245,9 @@ ginf_status bfail(ginf_status s, const std::string &msg) {
 
 }  // namespace
 
-// Grids whose label count falls in one bucket (LM = 16, 32 or 64; exact when
-// L == LM), solved by one kernel instantiation; items first..first+count-1.
+// Grids whose label count falls in one bucket (lm = 8, 16, ... 64; exact: L is
+// 16, 32 or 64), solved by one kernel instantiation; items
+// first..first+count-1.
 struct BatchGroup {
     int lm = 64;
     bool exact = true;
@@ -288,13 +289,16 @@ struct ginf_batch {
 
 namespace {
 
-int label_bucket(int L) { return L <= 16 ? 16 : (L <= 32 ? 32 : 64); }
+// Labels a grid's kernel is compiled for: L rounded up to a multiple of 8 (see
+// launch_sweep_tm).
+int label_bucket(int L) { return (L + 7) / 8 * 8; }
+bool label_exact(int L) { return L == 16 || L == 32 || L == 64; }
 
 // Groups the grids by label bucket (once, at creation).
 void make_groups(ginf_batch *b) {
     b->groups.clear();
     b->order.clear();
-    for (int lm : {16, 32, 64})
+    for (int lm = 8; lm <= 64; lm += 8)
         for (int exact = 1; exact >= 0; --exact) {
             BatchGroup grp;
             grp.lm = lm;
@@ -302,7 +306,7 @@ void make_groups(ginf_batch *b) {
             grp.first = (int)b->order.size();
             for (int i = 0; i < b->count; ++i) {
                 const int L = b->grids[i].num_labels;
-                if (label_bucket(L) != lm || (L == lm) != grp.exact) continue;
+                if (label_bucket(L) != lm || label_exact(L) != grp.exact) continue;
                 b->order.push_back(i);
                 grp.max_slot = std::max(grp.max_slot, b->fmt[i].slot_bytes);
             }
@@ -343,9 +347,9 @@ std::vector<BatchItem> make_items(ginf_batch *b, int tile_nodes) {
     return items;
 }
 
-template <int NW, int LM, bool EXACT, bool DIRECT = false>
+template <int NW, int LM, int LMIN, bool DIRECT = false>
 cudaError_t launch_batch(BatchLaunch bl, uint32_t max_slot, int num_sms, cudaStream_t s) {
-    auto kern = batch_kernel<NW, LM, EXACT, DIRECT>;
+    auto kern = batch_kernel<NW, LM, LMIN, DIRECT>;
     bl.tile_smem = (uint32_t)(((size_t)NW * 8 * max_slot + 15) / 16 * 16);
     const size_t bases_bytes = sizeof(int) * (size_t)bl.count;
     bl.bases_in_smem = bases_bytes <= 16 * 1024 ? 1 : 0;
@@ -371,26 +375,33 @@ cudaError_t launch_batch(BatchLaunch bl, uint32_t max_slot, int num_sms, cudaStr
     return cudaLaunchKernelEx(&cfg, kern, bl);
 }
 
-template <int LM, bool EXACT>
+template <int LM, int LMIN>
 cudaError_t launch_batch_nw(int tile_nodes, const BatchLaunch &bl, uint32_t max_slot, int num_sms, cudaStream_t s) {
-    if constexpr (LM == 16 && EXACT) {
+    if constexpr (LM == 16 && LMIN == LM) {
         // 64-byte messages: ordinary stores on large groups (see tile_finish).
         if (tile_nodes == 16 && bl.total_tiles >= kDirectStoreTiles)
-            return launch_batch<2, LM, EXACT, true>(bl, max_slot, num_sms, s);
+            return launch_batch<2, LM, LMIN, true>(bl, max_slot, num_sms, s);
     }
-    if (tile_nodes == 8) return launch_batch<1, LM, EXACT>(bl, max_slot, num_sms, s);
-    if (tile_nodes == 32) return launch_batch<4, LM, EXACT>(bl, max_slot, num_sms, s);
-    return launch_batch<2, LM, EXACT>(bl, max_slot, num_sms, s);
+    if (tile_nodes == 8) return launch_batch<1, LM, LMIN>(bl, max_slot, num_sms, s);
+    if (tile_nodes == 32) return launch_batch<4, LM, LMIN>(bl, max_slot, num_sms, s);
+    return launch_batch<2, LM, LMIN>(bl, max_slot, num_sms, s);
 }
 
 cudaError_t launch_group(const BatchGroup &grp, int tile_nodes, const BatchLaunch &bl, int num_sms, cudaStream_t s) {
-    switch (grp.lm * 2 + (grp.exact ? 1 : 0)) {
-        case 33: return launch_batch_nw<16, true>(tile_nodes, bl, grp.max_slot, num_sms, s);
-        case 32: return launch_batch_nw<16, false>(tile_nodes, bl, grp.max_slot, num_sms, s);
-        case 65: return launch_batch_nw<32, true>(tile_nodes, bl, grp.max_slot, num_sms, s);
-        case 64: return launch_batch_nw<32, false>(tile_nodes, bl, grp.max_slot, num_sms, s);
-        case 129: return launch_batch_nw<64, true>(tile_nodes, bl, grp.max_slot, num_sms, s);
-        default: return launch_batch_nw<64, false>(tile_nodes, bl, grp.max_slot, num_sms, s);
+    if (grp.exact) {
+        if (grp.lm == 16) return launch_batch_nw<16, 16>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        if (grp.lm == 32) return launch_batch_nw<32, 32>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        return launch_batch_nw<64, 64>(tile_nodes, bl, grp.max_slot, num_sms, s);
+    }
+    switch (grp.lm) {
+        case 8: return launch_batch_nw<8, 1>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        case 16: return launch_batch_nw<16, 9>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        case 24: return launch_batch_nw<24, 17>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        case 32: return launch_batch_nw<32, 25>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        case 40: return launch_batch_nw<40, 33>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        case 48: return launch_batch_nw<48, 41>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        case 56: return launch_batch_nw<56, 49>(tile_nodes, bl, grp.max_slot, num_sms, s);
+        default: return launch_batch_nw<64, 57>(tile_nodes, bl, grp.max_slot, num_sms, s);
     }
 }
 

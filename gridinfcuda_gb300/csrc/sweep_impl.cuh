@@ -148,13 +148,17 @@ __device__ __forceinline__ void zero_bytes(unsigned char *p, uint32_t bytes) {
     for (uint32_t o = 0; o < bytes; o += 16) *reinterpret_cast<uint4 *>(p + o) = make_uint4(0, 0, 0, 0);
 }
 
+// Label counts of a kernel: compiled for LMAX labels, it runs grids with
+// LMIN <= L <= LMAX, so labels below LMIN need no test and LMIN == LMAX makes
+// L a compile-time constant.
+//
 // val / L in T arithmetic.  With L a compile-time power of two the division is
 // a multiplication by the exact reciprocal, which rounds identically.
-template <typename T, int LMAX, bool EXACT>
+template <typename T, int LMAX, int LMIN>
 __device__ __forceinline__ T mean_of(T sum, int L) {
-    if constexpr (EXACT && (LMAX & (LMAX - 1)) == 0 && !std::is_same<T, int>::value) {
+    if constexpr (LMIN == LMAX && (LMAX & (LMAX - 1)) == 0 && !std::is_same<T, int>::value) {
         return sum * (T(1) / T(LMAX));
-    } else if constexpr (EXACT) {
+    } else if constexpr (LMIN == LMAX) {
         return div_labels(sum, LMAX);
     } else {
         return div_labels(sum, L);
@@ -168,7 +172,7 @@ __device__ __forceinline__ T mean_of(T sum, int L) {
 // label); labels are visited in increasing order, so combining the four
 // partial results by (value, label) gives the reference's first argmin
 // (strict <, bp.cc:74-80).
-template <typename T, typename M, int LMAX, bool EXACT>
+template <typename T, typename M, int LMAX, int LMIN>
 __device__ __forceinline__ void belief_part(const SweepParams &p, unsigned char *slot, int L, int dir, T &best,
                                             int &bl) {
     constexpr int B = MIO<M, T>::B;
@@ -177,7 +181,7 @@ __device__ __forceinline__ void belief_part(const SweepParams &p, unsigned char 
 #pragma unroll
     for (int j = 0; j < (NCH + 3) / 4; ++j) {
         const int c = (4 * j + dir) * B;
-        if (c < LMAX && (EXACT || c < L)) {
+        if (LMIN == LMAX ? c < LMAX : c < L) {
             T v[B], a[B];
             load_t<T, B>(slot + c * sizeof(T), v);
 #pragma unroll
@@ -190,7 +194,7 @@ __device__ __forceinline__ void belief_part(const SweepParams &p, unsigned char 
 #pragma unroll
             for (int kk = 0; kk < B; ++kk) {
                 const int i = c + kk;
-                if ((EXACT || i < L) && (bl == 0x7fffffff || v[kk] < best)) {
+                if ((LMIN == LMAX || i < L) && (bl == 0x7fffffff || v[kk] < best)) {
                     best = v[kk];
                     bl = i;
                 }
@@ -220,7 +224,7 @@ __device__ __forceinline__ void argmin_combine(T &best, int &bl) {
 // h = from - in[dir], min of h, forward and backward min-plus scans with slope
 // V(0,1), truncation at min(h) + V(0,L-1), subtraction of the mean (or the
 // minimum), written over in[dir].
-template <typename T, typename M, int LMAX, bool EXACT>
+template <typename T, typename M, int LMAX, int LMIN>
 __device__ __forceinline__ void message_linear(const SweepParams &p, unsigned char *slot, int L, int dir, T scale,
                                                T trunc) {
     constexpr int B = MIO<M, T>::B;
@@ -228,7 +232,7 @@ __device__ __forceinline__ void message_linear(const SweepParams &p, unsigned ch
     T o[LMAX];
 #pragma unroll
     for (int c = 0; c < LMAX; c += B) {
-        if (EXACT || c < L) {
+        if (c < LMIN || c < L) {
             T a[B], f[B];
             MIO<M, T>::load(md + c * sizeof(M), a);
             load_t<T, B>(slot + c * sizeof(T), f);
@@ -239,18 +243,18 @@ __device__ __forceinline__ void message_linear(const SweepParams &p, unsigned ch
     T minh = o[0];
 #pragma unroll
     for (int i = 1; i < LMAX; ++i)
-        if (EXACT || i < L) minh = rmin(minh, o[i]);
+        if (i < LMIN || i < L) minh = rmin(minh, o[i]);
 #pragma unroll
     for (int i = 1; i < LMAX; ++i)
-        if (EXACT || i < L) o[i] = rmin(o[i], o[i - 1] + scale);
+        if (i < LMIN || i < L) o[i] = rmin(o[i], o[i - 1] + scale);
 #pragma unroll
     for (int i = LMAX - 2; i >= 0; --i)
-        if (EXACT || i + 1 < L) o[i] = rmin(o[i], o[i + 1] + scale);
+        if (i + 1 < LMIN || i + 1 < L) o[i] = rmin(o[i], o[i + 1] + scale);
     minh += trunc;
     T val = T(0);
 #pragma unroll
     for (int i = 0; i < LMAX; ++i)
-        if (EXACT || i < L) {
+        if (i < LMIN || i < L) {
             o[i] = rmin(o[i], minh);
             val += o[i];
         }
@@ -258,13 +262,13 @@ __device__ __forceinline__ void message_linear(const SweepParams &p, unsigned ch
         val = o[0];
 #pragma unroll
         for (int i = 1; i < LMAX; ++i)
-            if (EXACT || i < L) val = rmin(val, o[i]);
+            if (i < LMIN || i < L) val = rmin(val, o[i]);
     } else {
-        val = mean_of<T, LMAX, EXACT>(val, L);
+        val = mean_of<T, LMAX, LMIN>(val, L);
     }
 #pragma unroll
     for (int c = 0; c < LMAX; c += B) {
-        if (EXACT || c < L) {
+        if (c < LMIN || c < L) {
             T r[B];
 #pragma unroll
             for (int k = 0; k < B; ++k) r[k] = o[c + k] - val;
@@ -405,11 +409,13 @@ __device__ __forceinline__ float window_pair(const float *h, int i, int k) {
 // Outputs c .. c + B - 1 of the windowed quadratic transform over h[0, N)
 // (padded with +inf where the caller has no labels), two at a time: the
 // sums h + V(0,k) of a pair of outputs in one f32x2 addition, their minima
-// as scalars, the shift subtracted in pairs.  Values are those of the scalar
-// form below; sum accumulates the outputs in label order.
-template <int N, int QW, int B>
+// as scalars, the shift subtracted in pairs.  Symmetric taps share their
+// cost: min(h[i-k], h[i+k]) + V(0,k) rounds exactly like the two separate
+// sums (rounding is monotone).  sum accumulates, in label order, the outputs
+// i < L (those below LMIN always are).
+template <int N, int QW, int B, int LMIN = N>
 __device__ __forceinline__ void window_outputs(const float *h, int c, const float *vtap, float cap, float shift,
-                                               float &sum, float *r) {
+                                               float &sum, float *r, int L = N) {
 #pragma unroll
     for (int k = 0; k < B; k += 2) {
         const int i = c + k;
@@ -433,8 +439,8 @@ __device__ __forceinline__ void window_outputs(const float *h, int c, const floa
                 m1 = fminf(m1, a1[k2]);
             }
         }
-        sum += m0;
-        sum += m1;
+        if (i < LMIN || i < L) sum += m0;
+        if (i + 1 < LMIN || i + 1 < L) sum += m1;
         const float2 o = sub_f32x2(m0, m1, shift, shift);
         r[k] = o.x;
         r[k + 1] = o.y;
@@ -474,20 +480,21 @@ __device__ __forceinline__ int quad_radius(const T *Vt, int L, T trunc) {
 // nondecreasing from V(0,0) and rounding is monotone), so each message is
 // rounded to the store type once; with the mean subtracted (FP32 store only)
 // the unnormalised values are stored exactly and corrected in a second pass.
-template <typename T, typename M, int LMAX, bool EXACT, int QW>
+template <typename T, typename M, int LMAX, int LMIN, int QW>
 __device__ __forceinline__ void message_quad_window(const SweepParams &p, unsigned char *slot, int L, int dir,
                                                     const T *vtap, T trunc) {
+    static_assert(std::is_same<T, float>::value, "the window form is FP32 arithmetic");
     constexpr int B = MIO<M, T>::B;
     unsigned char *md = slot + p.d_bytes + dir * p.m_bytes;
     T h[LMAX];
 #pragma unroll
     for (int c = 0; c < LMAX; c += B) {
-        if (EXACT || c < L) {
+        if (c < LMIN || c < L) {
             T a[B], f[B];
             MIO<M, T>::load(md + c * sizeof(M), a);
             load_t<T, B>(slot + c * sizeof(T), f);
 #pragma unroll
-            for (int k = 0; k < B; ++k) h[c + k] = (EXACT || c + k < L) ? f[k] - a[k] : pos_inf<T>();
+            for (int k = 0; k < B; ++k) h[c + k] = (c + k < LMIN || c + k < L) ? f[k] - a[k] : pos_inf<T>();
         } else {
 #pragma unroll
             for (int k = 0; k < B; ++k) h[c + k] = pos_inf<T>();
@@ -496,43 +503,24 @@ __device__ __forceinline__ void message_quad_window(const SweepParams &p, unsign
     T minh = h[0];
 #pragma unroll
     for (int i = 1; i < LMAX; ++i)
-        if (EXACT || i < L) minh = fminf(minh, h[i]);
+        if (i < LMIN || i < L) minh = fminf(minh, h[i]);
     const T cap = minh + trunc;
     const bool norm_min = p.norm_min != 0;
     const T shift = norm_min ? minh + vtap[0] : T(0);
     T sum = T(0);
 #pragma unroll
     for (int c = 0; c < LMAX; c += B) {
-        if constexpr (EXACT && std::is_same<T, float>::value) {
+        if (c < LMIN || c < L) {
             T r[B];
-            window_outputs<LMAX, QW, B>(h, c, vtap, cap, shift, sum, r);
-            MIO<M, T>::store(md + c * sizeof(M), r);
-        } else if (EXACT || c < L) {
-            T r[B];
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int i = c + k;
-                // Symmetric taps share their cost: min(h[i-k], h[i+k]) + V(0,k)
-                // rounds exactly like the two separate sums (rounding is monotone).
-                T m = fminf(cap, h[i] + vtap[0]);
-#pragma unroll
-                for (int k2 = 1; k2 <= QW; ++k2) {
-                    const bool lo = i - k2 >= 0, hi = i + k2 < LMAX;
-                    if (lo && hi) m = fminf(m, fminf(h[i - k2], h[i + k2]) + vtap[k2]);
-                    else if (lo) m = fminf(m, h[i - k2] + vtap[k2]);
-                    else if (hi) m = fminf(m, h[i + k2] + vtap[k2]);
-                }
-                if (EXACT || i < L) sum += m;
-                r[k] = m - shift;
-            }
+            window_outputs<LMAX, QW, B, LMIN>(h, c, vtap, cap, shift, sum, r, L);
             MIO<M, T>::store(md + c * sizeof(M), r);
         }
     }
     if (!norm_min) {
-        const T val = mean_of<T, LMAX, EXACT>(sum, L);
+        const T val = mean_of<T, LMAX, LMIN>(sum, L);
 #pragma unroll
         for (int c = 0; c < LMAX; c += B) {
-            if (EXACT || c < L) {
+            if (c < LMIN || c < L) {
                 T r[B];
                 MIO<M, T>::load(md + c * sizeof(M), r);
 #pragma unroll
@@ -616,7 +604,7 @@ __device__ void message_std_quad(const SweepParams &p, unsigned char *slot, int 
 // positive increment), so the min-normalised message is 0 at its argmin.
 // Passes beyond r get an infinite increment and change nothing.
 constexpr int kQuadPasses = 4;
-template <typename M, int LMAX, bool EXACT>
+template <typename M, int LMAX, int LMIN>
 __device__ __forceinline__ void message_quad_passes(const SweepParams &p, unsigned char *slot, int L, int dir,
                                                     const float *cpass, float trunc) {
     constexpr int B = MIO<M, float>::B;
@@ -626,15 +614,15 @@ __device__ __forceinline__ void message_quad_passes(const SweepParams &p, unsign
     float m[LMAX];
 #pragma unroll
     for (int c = 0; c < LMAX; c += B) {
-        if (EXACT || c < L) {
+        if (c < LMIN || c < L) {
             float a[B], f[B];
             MIO<M, float>::load(md + c * sizeof(M), a);
             load_t<float, B>(slot + c * sizeof(float), f);
 #pragma unroll
             for (int k = 0; k < B; k += 2) {
                 const float2 d = sub_f32x2(f[k], f[k + 1], a[k], a[k + 1]);
-                m[c + k] = (EXACT || c + k < L) ? d.x : inf;
-                m[c + k + 1] = (EXACT || c + k + 1 < L) ? d.y : inf;
+                m[c + k] = (c + k < LMIN || c + k < L) ? d.x : inf;
+                m[c + k + 1] = (c + k + 1 < LMIN || c + k + 1 < L) ? d.y : inf;
             }
         } else {
 #pragma unroll
@@ -666,7 +654,7 @@ __device__ __forceinline__ void message_quad_passes(const SweepParams &p, unsign
     }
 #pragma unroll
     for (int c = 0; c < LMAX; c += B) {
-        if (EXACT || c < L) {
+        if (c < LMIN || c < L) {
             float r[B];
 #pragma unroll
             for (int k = 0; k < B; k += 2) {
@@ -804,12 +792,12 @@ __device__ __forceinline__ void tile_load(const SweepParams &p, int t, unsigned 
 // 16-byte stores instead of one bulk copy each, which pays on large launches
 // (the copy engine's per-copy cost dominates 64-byte copies) and not on small,
 // L2-resident ones.
-template <typename T, typename M, int LMAX, bool EXACT, int NW, int KIND, bool DIRECT = false>
+template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, bool DIRECT = false>
 __device__ __forceinline__ bool tile_finish(const SweepParams &p, const TableConsts<T> &tc, int t,
                                             unsigned char *smem, uint64_t *bar, uint32_t &parity) {
     const int dir = (threadIdx.x & 31) >> 3;
     const int node = (threadIdx.x >> 5) * 8 + (threadIdx.x & 7);
-    const int L = EXACT ? LMAX : p.L;
+    const int L = LMIN == LMAX ? LMAX : p.L;
     unsigned char *slot = smem + (size_t)node * p.slot_bytes;
     const bool got = mbar_wait_bounded(bar, parity, p.status);
     parity ^= 1u;
@@ -820,32 +808,27 @@ __device__ __forceinline__ bool tile_finish(const SweepParams &p, const TableCon
     __syncwarp();
     T best = pos_inf<T>();
     int label = 0x7fffffff;
-    if (act) belief_part<T, M, LMAX, EXACT>(p, slot, L, dir, best, label);
+    if (act) belief_part<T, M, LMAX, LMIN>(p, slot, L, dir, best, label);
     argmin_combine(best, label);
     __syncwarp();
     if (act) {
         if constexpr (KIND == KIND_LINEAR) {
-            message_linear<T, M, LMAX, EXACT>(p, slot, L, dir, tc.scale, tc.trunc);
+            message_linear<T, M, LMAX, LMIN>(p, slot, L, dir, tc.scale, tc.trunc);
         } else if constexpr (KIND == KIND_QUADPASS) {
             if constexpr (std::is_same<T, float>::value && sizeof(M) == 2)
-                message_quad_passes<M, LMAX, EXACT>(p, slot, L, dir, tc.cpass, tc.trunc);
+                message_quad_passes<M, LMAX, LMIN>(p, slot, L, dir, tc.cpass, tc.trunc);
         } else if constexpr (KIND == KIND_QUAD || KIND == KIND_QUAD4) {
             constexpr int QW = KIND == KIND_QUAD4 ? kQuadWindowSmall : kQuadWindow;
-            if constexpr (sizeof(T) == 4 && !std::is_same<T, int>::value) {
-                if (tc.qr <= QW) message_quad_window<T, M, LMAX, EXACT, QW>(p, slot, L, dir, tc.vtap, tc.trunc);
-                else message_std_quad<T, M, LMAX>(p, slot, L, dir, tc.scale, tc.trunc);
-            } else {
-                message_std_quad<T, M, LMAX>(p, slot, L, dir, tc.scale, tc.trunc);
-            }
+            // Launched only when the table's truncation radius fits the window.
+            message_quad_window<T, M, LMAX, LMIN, QW>(p, slot, L, dir, tc.vtap, tc.trunc);
         } else {
-            if (p.mode == MODE_LINEAR) message_linear<T, M, LMAX, EXACT>(p, slot, L, dir, tc.scale, tc.trunc);
-            else if (p.mode == MODE_REF_MINCONV) messages_ref_minconv<T, M, LMAX>(p, slot, L, dir);
+            if (p.mode == MODE_REF_MINCONV) messages_ref_minconv<T, M, LMAX>(p, slot, L, dir);
             else if (p.mode == MODE_STD_MINCONV) message_std_minconv<T, M, LMAX>(p, slot, L, dir);
             else message_std_quad<T, M, LMAX>(p, slot, L, dir, tc.scale, tc.trunc);
         }
     }
     if constexpr (DIRECT) {
-        static_assert(EXACT && LMAX * sizeof(M) == 64, "direct stores are for 64-byte messages");
+        static_assert(LMIN == LMAX && LMAX * sizeof(M) == 64, "direct stores are for 64-byte messages");
         __syncwarp();
         if (act) {
             if (dir == 0 && p.write_labels) p.labels[(size_t)y * p.W + x] = label;
@@ -878,17 +861,17 @@ __device__ __forceinline__ bool tile_finish(const SweepParams &p, const TableCon
 }
 
 // ---------------------------------------------------------------------------
-// Split kernel: FP32 records, L = 128, truncated quadratic with the windowed
-// transform (window radius QW).  A lane holding a whole 128-label message
-// needs ~235 registers, which leaves 8 warps per SM and the kernel
+// Split kernel: FP32 records, 64 < L <= LMAX <= 128, truncated quadratic with
+// the windowed transform (window radius QW).  A lane holding a whole 128-label
+// message needs ~235 registers, which leaves 8 warps per SM and the kernel
 // latency-bound; here two warps serve each group of eight nodes and a lane
-// (k, dir) of warp 2g + hf computes labels [64 hf, 64 hf + 64) of node
-// g * 8 + k's message towards dir, with h read over that range plus a QW-label
-// halo.  Results are bit-identical to message_quad_window:
+// (k, dir) of warp 2g + hf computes labels [HL hf, HL hf + HL), HL = LMAX / 2,
+// of node g * 8 + k's message towards dir, with h read over that range plus a
+// QW-label halo.  Results are bit-identical to message_quad_window:
 //   - min(h) is the fminf of the two halves' minima (fminf is exact);
 //   - each output value is the same expression over the same h values (h is
 //     +inf outside [0, L), as the single-lane form's missing taps);
-//   - the mean's sum stays sequential in label order: half 0 sums its 64
+//   - the mean's sum stays sequential in label order: half 0 sums its HL
 //     outputs from zero, half 1 continues from that partial sum;
 //   - the argmin combines the halves' first minima by (value, label).
 // Shared words exchanged between the two warps of a group.
@@ -901,14 +884,17 @@ struct SplitXch {
     int label[NW][8];        // and its first label
 };
 
-// Belief over labels [base, base + 64) of one node by its four lanes of one
-// warp (chunks base + 4 (4 j + dir)); see belief_part.
-__device__ __forceinline__ void belief_half(const SweepParams &p, unsigned char *slot, int dir, int base, float &best,
-                                            int &bl) {
+// Belief over labels [base, base + HL) below L of one node by its four lanes
+// of one warp (chunks base + 4 (4 j + dir)); see belief_part.
+template <int HL, bool FULL>
+__device__ __forceinline__ void belief_half(const SweepParams &p, unsigned char *slot, int L, int dir, int base,
+                                            float &best, int &bl) {
     const unsigned char *mb = slot + p.d_bytes;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < (HL / 4 + 3) / 4; ++j) {
         const int c = base + (4 * j + dir) * 4;
+        if (HL % 16 != 0 && 4 * j + dir >= HL / 4) break;
+        if (!FULL && c >= L) break;
         float v[4], a[4];
         load_t<float, 4>(slot + c * sizeof(float), v);
 #pragma unroll
@@ -920,7 +906,7 @@ __device__ __forceinline__ void belief_half(const SweepParams &p, unsigned char 
         store_t<float, 4>(slot + c * sizeof(float), v);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-            if (bl == 0x7fffffff || v[kk] < best) {
+            if ((FULL || c + kk < L) && (bl == 0x7fffffff || v[kk] < best)) {
                 best = v[kk];
                 bl = c + kk;
             }
@@ -931,30 +917,34 @@ __device__ __forceinline__ void belief_half(const SweepParams &p, unsigned char 
 // One tile of the split kernel (8 * NW / 2 nodes).  Block barriers: after the
 // beliefs (the halo of h reads the other half's), after h is loaded (the
 // outgoing messages overwrite the incoming slots), after half 0's partial
-// sum, and after half 1's mean.  Each half bulk-stores its own 256 bytes.
-template <int NW, int QW>
+// sum, and after half 1's mean.  Each half bulk-stores its own labels.
+template <int LMAX, int LMIN, int NW, int QW>
 __device__ __forceinline__ bool tile_finish_split(const SweepParams &p, const TableConsts<float> &tc, int t,
                                                   unsigned char *smem, uint64_t *bar, uint32_t &parity,
                                                   SplitXch<NW> &xs) {
-    constexpr int L = 128, HL = 64, NH = HL + 2 * QW;
-    static_assert(QW % 4 == 0, "the halo is whole 16-byte chunks");
+    constexpr int HL = LMAX / 2, NH = HL + 2 * QW;
+    static_assert(QW % 4 == 0 && HL % 8 == 0, "halves and halo are whole 16-byte chunks");
+    static_assert(LMIN >= HL + QW, "half 0 and its trailing halo lie below every L");
+    const int L = LMIN == LMAX ? LMAX : p.L;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hf = w & 1, g = w >> 1;
     const int dir = lane >> 3, k = lane & 7;
     const int base = hf * HL;
     unsigned char *slot = smem + (size_t)(g * 8 + k) * p.slot_bytes;
     unsigned char *md = slot + p.d_bytes + dir * p.m_bytes;
+    const uint32_t half_bytes =
+        LMIN == LMAX || hf == 0 ? HL * (uint32_t)sizeof(float) : p.m_bytes - HL * (uint32_t)sizeof(float);
     const bool got = mbar_wait_bounded(bar, parity, p.status);
     parity ^= 1u;
     if (!__syncthreads_and(got)) return false;
     int x, y;
     const bool act = tile_node<NW, 2>(p, t, x, y);
     // Each half zeroes, then sums, only its own labels of the incoming slots.
-    if (act && ((zero_mask(p, x, y) >> dir) & 1u)) zero_bytes(md + base * sizeof(float), HL * sizeof(float));
+    if (act && ((zero_mask(p, x, y) >> dir) & 1u)) zero_bytes(md + base * sizeof(float), half_bytes);
     __syncwarp();
     float best = pos_inf<float>();
     int label = 0x7fffffff;
-    if (act) belief_half(p, slot, dir, base, best, label);
+    if (act) belief_half<HL, LMIN == LMAX>(p, slot, L, dir, base, best, label);
     argmin_combine(best, label);
     if (dir == 0) {
         xs.best[w][k] = best;
@@ -973,14 +963,17 @@ __device__ __forceinline__ bool tile_finish_split(const SweepParams &p, const Ta
         for (int c = 0; c < NH; c += 4) {
             // Chunk labels base - QW + c .. +3: below 0 only for half 0's
             // leading halo, at or above L only for half 1's trailing halo.
-            const bool in = (c >= QW || hf == 1) && (c < HL + QW || hf == 0);
+            // Labels from LMIN on (half 1 only) exist where they are below L.
+            const int u0 = HL - QW + c;  // half 1's first label of the chunk
+            const bool in = (c >= QW || hf == 1) && (c < HL + QW || hf == 0) && (hf == 0 || u0 < LMIN || u0 < L);
             if (in) {
                 const int j0 = base - QW + c;
                 float a[4], f[4];
                 MIO<float, float>::load(md + j0 * sizeof(float), a);
                 load_t<float, 4>(slot + j0 * sizeof(float), f);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) h[c + kk] = f[kk] - a[kk];
+                for (int kk = 0; kk < 4; ++kk)
+                    h[c + kk] = (hf == 0 || u0 + kk < LMIN || u0 + kk < L) ? f[kk] - a[kk] : pos_inf<float>();
             } else {
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) h[c + kk] = pos_inf<float>();
@@ -1005,6 +998,7 @@ __device__ __forceinline__ bool tile_finish_split(const SweepParams &p, const Ta
         for (int c = 0; c < HL; c += 4) {
             // h[QW .. QW + HL) are this half's labels; the halo (+inf off the
             // grid of labels) lies on both sides, so no output is at an end.
+            if (!(hf == 0 || HL + c < LMIN || HL + c < L)) break;
             float r[4];
             window_outputs<NH, QW, 4>(h, c + QW, tc.vtap, cap, shift, sum, r);
             MIO<float, float>::store(mh + c * sizeof(float), r);
@@ -1017,18 +1011,21 @@ __device__ __forceinline__ bool tile_finish_split(const SweepParams &p, const Ta
             float s = xs.sum[g][lane];
 #pragma unroll
             for (int c = 0; c < HL; c += 4) {
+                if (!(HL + c < LMIN || HL + c < L)) break;
                 float r[4];
                 MIO<float, float>::load(mh + c * sizeof(float), r);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) s += r[kk];
+                for (int kk = 0; kk < 4; ++kk)
+                    if (HL + c + kk < LMIN || HL + c + kk < L) s += r[kk];
             }
-            xs.mean[g][lane] = mean_of<float, L, true>(s, L);
+            xs.mean[g][lane] = mean_of<float, LMAX, LMIN>(s, L);
         }
         __syncthreads();
         if (act) {
             const float val = xs.mean[g][lane];
 #pragma unroll
             for (int c = 0; c < HL; c += 4) {
+                if (!(hf == 0 || HL + c < LMIN || HL + c < L)) break;
                 float r[4];
                 MIO<float, float>::load(mh + c * sizeof(float), r);
 #pragma unroll
@@ -1043,7 +1040,7 @@ __device__ __forceinline__ bool tile_finish_split(const SweepParams &p, const Ta
         if (hf == 0 && dir == 0 && p.write_labels) p.labels[(size_t)y * p.W + x] = label;
         const int qx = x + dir_dx(dir), qy = y + dir_dy(dir);
         unsigned char *dst = p.rec + ((size_t)qy * p.W + qx) * p.rec_bytes + p.d_bytes + opp_dir(dir) * p.m_bytes;
-        bulk_store(dst + base * sizeof(float), mh, HL * sizeof(float));
+        bulk_store(dst + base * sizeof(float), mh, half_bytes);
         bulk_commit();
         bulk_wait_read_all();
     }
@@ -1051,14 +1048,14 @@ __device__ __forceinline__ bool tile_finish_split(const SweepParams &p, const Ta
     return true;
 }
 
-template <int NW, int QW>
+template <int LMAX, int LMIN, int NW, int QW>
 __global__ void __launch_bounds__(NW * 32, 5) sweep_kernel_split(const SweepParams p) {
     static_assert(NW % 2 == 0, "warps come in pairs");
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
     __shared__ SplitXch<NW> xs;
     launch_dependents();
-    const TableConsts<float> tc = table_consts<float, KIND_QUAD>(p.V, 128);
+    const TableConsts<float> tc = table_consts<float, KIND_QUAD>(p.V, LMIN == LMAX ? LMAX : p.L);
     if (threadIdx.x == 0) {
         mbar_init(&full_bar, NW * 32);
         fence_barrier_init();
@@ -1069,7 +1066,7 @@ __global__ void __launch_bounds__(NW * 32, 5) sweep_kernel_split(const SweepPara
     if (t < p.num_tiles) tile_load<NW, 2>(p, t, smem, &full_bar);
     uint32_t parity = 0;
     for (; t < p.num_tiles; t += gridDim.x) {
-        if (!tile_finish_split<NW, QW>(p, tc, t, smem, &full_bar, parity, xs)) return;
+        if (!tile_finish_split<LMAX, LMIN, NW, QW>(p, tc, t, smem, &full_bar, parity, xs)) return;
         const int tn = t + gridDim.x;
         if (tn < p.num_tiles) tile_load<NW, 2>(p, tn, smem, &full_bar);
     }
@@ -1078,14 +1075,14 @@ __global__ void __launch_bounds__(NW * 32, 5) sweep_kernel_split(const SweepPara
 
 // One checkerboard half-sweep of one level: blocks take tiles in turn, each
 // issuing the copies of its next tile as soon as the current one is done.
-template <typename T, typename M, int LMAX, bool EXACT, int NW, int KIND, bool DIRECT>
+template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, bool DIRECT>
 __device__ __forceinline__ void sweep_body(const SweepParams &p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
     // The next half-sweep may be launched now; its blocks take SM slots as
     // these retire and wait below before touching any record.
     launch_dependents();
-    const TableConsts<T> tc = table_consts<T, KIND>(p.V, EXACT ? LMAX : p.L);
+    const TableConsts<T> tc = table_consts<T, KIND>(p.V, LMIN == LMAX ? LMAX : p.L);
     if (threadIdx.x == 0) {
         mbar_init(&full_bar, NW * 32);
         fence_barrier_init();
@@ -1097,16 +1094,16 @@ __device__ __forceinline__ void sweep_body(const SweepParams &p) {
     if (t < p.num_tiles) tile_load<NW>(p, t, smem, &full_bar);
     uint32_t parity = 0;
     for (; t < p.num_tiles; t += gridDim.x) {
-        if (!tile_finish<T, M, LMAX, EXACT, NW, KIND, DIRECT>(p, tc, t, smem, &full_bar, parity)) return;
+        if (!tile_finish<T, M, LMAX, LMIN, NW, KIND, DIRECT>(p, tc, t, smem, &full_bar, parity)) return;
         const int tn = t + gridDim.x;
         if (tn < p.num_tiles) tile_load<NW>(p, tn, smem, &full_bar);
     }
     bulk_wait_all();
 }
 
-template <typename T, typename M, int LMAX, bool EXACT, int NW, int KIND, bool DIRECT = false>
+template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, bool DIRECT = false>
 __global__ void __launch_bounds__(NW * 32) sweep_kernel(const SweepParams p) {
-    sweep_body<T, M, LMAX, EXACT, NW, KIND, DIRECT>(p);
+    sweep_body<T, M, LMAX, LMIN, NW, KIND, DIRECT>(p);
 }
 
 // The same kernel with room for MINB blocks per SM in the register
@@ -1114,9 +1111,9 @@ __global__ void __launch_bounds__(NW * 32) sweep_kernel(const SweepParams p) {
 // six (168 registers): their packed window form would otherwise take every
 // register.  (Any explicit bound, even one block, changes the allocation, so
 // the other kernels have none.)
-template <typename T, typename M, int LMAX, bool EXACT, int NW, int KIND, int MINB>
+template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, int MINB>
 __global__ void __launch_bounds__(NW * 32, MINB) sweep_kernel_bounded(const SweepParams p) {
-    sweep_body<T, M, LMAX, EXACT, NW, KIND, false>(p);
+    sweep_body<T, M, LMAX, LMIN, NW, KIND, false>(p);
 }
 
 // Per-kernel launch state (one per kernel instantiation, in static storage).
@@ -1162,76 +1159,133 @@ cudaError_t launch_tiles(K kern, LaunchCache &lc_state, int NW, int nodes, const
     return cudaLaunchKernelEx(&lc, kern, p);
 }
 
-template <typename T, typename M, int LMAX, bool EXACT, int NW, int KIND, bool DIRECT = false>
+template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, bool DIRECT = false>
 cudaError_t launch_one(const SweepParams &params, uint32_t slot_bytes, cudaStream_t s, int num_sms) {
     static LaunchCache cache;
     if constexpr ((KIND == KIND_QUAD || KIND == KIND_QUAD4 || KIND == KIND_QUADPASS) && sizeof(M) == 2 &&
                   LMAX == 128 && !DIRECT) {
-        return launch_tiles(sweep_kernel_bounded<T, M, LMAX, EXACT, NW, KIND, 6>, cache, NW, NW * 8, params,
+        return launch_tiles(sweep_kernel_bounded<T, M, LMAX, LMIN, NW, KIND, 6>, cache, NW, NW * 8, params,
                             slot_bytes, s, num_sms);
     } else {
-        return launch_tiles(sweep_kernel<T, M, LMAX, EXACT, NW, KIND, DIRECT>, cache, NW, NW * 8, params, slot_bytes,
+        return launch_tiles(sweep_kernel<T, M, LMAX, LMIN, NW, KIND, DIRECT>, cache, NW, NW * 8, params, slot_bytes,
                             s, num_sms);
     }
 }
 
-template <int NW, int QW>
+template <int LMAX, int LMIN, int NW, int QW>
 cudaError_t launch_split(const SweepParams &params, uint32_t slot_bytes, cudaStream_t s, int num_sms) {
     static LaunchCache cache;
-    return launch_tiles(sweep_kernel_split<NW, QW>, cache, NW, NW / 2 * 8, params, slot_bytes, s, num_sms);
+    return launch_tiles(sweep_kernel_split<LMAX, LMIN, NW, QW>, cache, NW, NW / 2 * 8, params, slot_bytes, s,
+                        num_sms);
 }
 
+// The min-convolution rules and the lower envelope: one kernel per power of
+// two, labels tested against the run-time L.
 template <typename T, typename M, int LM>
+cudaError_t launch_general(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
+    return launch_one<T, M, LM, 1, 2, KIND_GENERAL>(p, f.slot_bytes, s, num_sms);
+}
+
+// Half-sweeps of grids with LO <= f.L <= LM labels.  Label counts that are a
+// power of two run kernels with L a compile-time constant.
+template <typename T, typename M, int LM, int LO>
 cudaError_t launch_variant(const RecordFormat &f, const SweepConfig &cfg, const SweepParams &p, cudaStream_t s,
                            int num_sms) {
-    const bool exact = f.L == LM;
+    constexpr bool kPow2 = (LM & (LM - 1)) == 0 && LM >= 16;
+    constexpr bool kF32 = std::is_same<T, float>::value;
+    const bool exact = kPow2 && f.L == LM;
     if (p.mode == MODE_STD_QUAD) {
         // The host measured the truncation radius (quad_radius_host); radius-4
         // windows run the cheaper 9-tap kernel.
-        if constexpr (std::is_same<T, float>::value && std::is_same<M, float>::value && LM == 128) {
-            // FP32 records at L = 128: two warps per eight nodes (register relief).
-            if (exact && p.quad_radius <= kQuadWindowSmall) return launch_split<4, 4>(p, f.slot_bytes, s, num_sms);
-            if (exact && p.quad_radius <= kQuadWindow) return launch_split<4, 8>(p, f.slot_bytes, s, num_sms);
-        }
-        if constexpr (std::is_same<T, float>::value && sizeof(M) == 2) {
-            // FP16 store and an exactly quadratic table: the pass form.
-            if (p.quad_exact && p.quad_radius <= kQuadPasses) {
-                if (exact) return launch_one<T, M, LM, true, 2, KIND_QUADPASS>(p, f.slot_bytes, s, num_sms);
-                return launch_one<T, M, LM, false, 2, KIND_QUADPASS>(p, f.slot_bytes, s, num_sms);
+        if constexpr (kF32 && std::is_same<M, float>::value && LM > 64) {
+            // FP32 records above 64 labels: two warps per eight nodes (register relief).
+            if (p.quad_radius <= kQuadWindowSmall) {
+                if constexpr (kPow2)
+                    if (exact) return launch_split<LM, LM, 4, 4>(p, f.slot_bytes, s, num_sms);
+                return launch_split<LM, LO, 4, 4>(p, f.slot_bytes, s, num_sms);
+            }
+            if (p.quad_radius <= kQuadWindow) {
+                if constexpr (kPow2)
+                    if (exact) return launch_split<LM, LM, 4, 8>(p, f.slot_bytes, s, num_sms);
+                return launch_split<LM, LO, 4, 8>(p, f.slot_bytes, s, num_sms);
+            }
+        } else {
+            if constexpr (kF32 && sizeof(M) == 2) {
+                // FP16 store and an exactly quadratic table: the pass form.
+                if (p.quad_exact && p.quad_radius <= kQuadPasses) {
+                    if constexpr (kPow2)
+                        if (exact) return launch_one<T, M, LM, LM, 2, KIND_QUADPASS>(p, f.slot_bytes, s, num_sms);
+                    return launch_one<T, M, LM, LO, 2, KIND_QUADPASS>(p, f.slot_bytes, s, num_sms);
+                }
+            }
+            if constexpr (kF32) {
+                if (p.quad_radius <= kQuadWindowSmall) {
+                    if constexpr (kPow2)
+                        if (exact) return launch_one<T, M, LM, LM, 2, KIND_QUAD4>(p, f.slot_bytes, s, num_sms);
+                    return launch_one<T, M, LM, LO, 2, KIND_QUAD4>(p, f.slot_bytes, s, num_sms);
+                }
+                if (p.quad_radius <= kQuadWindow) {
+                    if constexpr (kPow2)
+                        if (exact) return launch_one<T, M, LM, LM, 2, KIND_QUAD>(p, f.slot_bytes, s, num_sms);
+                    return launch_one<T, M, LM, LO, 2, KIND_QUAD>(p, f.slot_bytes, s, num_sms);
+                }
             }
         }
-        if (p.quad_radius <= kQuadWindowSmall) {
-            if (exact) return launch_one<T, M, LM, true, 2, KIND_QUAD4>(p, f.slot_bytes, s, num_sms);
-            return launch_one<T, M, LM, false, 2, KIND_QUAD4>(p, f.slot_bytes, s, num_sms);
-        }
-        if (exact) return launch_one<T, M, LM, true, 2, KIND_QUAD>(p, f.slot_bytes, s, num_sms);
-        return launch_one<T, M, LM, false, 2, KIND_QUAD>(p, f.slot_bytes, s, num_sms);
     }
-    if (p.mode != MODE_LINEAR) return launch_one<T, M, LM, false, 2, KIND_GENERAL>(p, f.slot_bytes, s, num_sms);
-    if (!exact) return launch_one<T, M, LM, false, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
-    if constexpr (std::is_same<T, float>::value) {
-        if (cfg.nt == 8) return launch_one<T, M, LM, true, 1, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
-        if (cfg.nt == 32) return launch_one<T, M, LM, true, 4, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
-        if constexpr (LM * sizeof(M) == 64) {
-            const int n1 = p.W >= 3 ? (p.W - 3) / 2 + 1 : 0;
-            const long tiles = p.H >= 3 ? (long)(p.H - 2) * ((n1 + 15) / 16) : 0;
-            if (tiles >= kDirectStoreTiles)
-                return launch_one<T, M, LM, true, 2, KIND_LINEAR, true>(p, f.slot_bytes, s, num_sms);
+    if (p.mode != MODE_LINEAR) {
+        if (f.L <= 16) return launch_general<T, M, 16>(f, p, s, num_sms);
+        if (f.L <= 32) return launch_general<T, M, 32>(f, p, s, num_sms);
+        if (f.L <= 64) return launch_general<T, M, 64>(f, p, s, num_sms);
+        return launch_general<T, M, 128>(f, p, s, num_sms);
+    }
+    if constexpr (kPow2) {
+        if (exact) {
+            if constexpr (kF32) {
+                if (cfg.nt == 8) return launch_one<T, M, LM, LM, 1, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
+                if (cfg.nt == 32) return launch_one<T, M, LM, LM, 4, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
+                if constexpr (LM * sizeof(M) == 64) {
+                    const int n1 = p.W >= 3 ? (p.W - 3) / 2 + 1 : 0;
+                    const long tiles = p.H >= 3 ? (long)(p.H - 2) * ((n1 + 15) / 16) : 0;
+                    if (tiles >= kDirectStoreTiles)
+                        return launch_one<T, M, LM, LM, 2, KIND_LINEAR, true>(p, f.slot_bytes, s, num_sms);
+                }
+            }
+            return launch_one<T, M, LM, LM, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
         }
     }
-    return launch_one<T, M, LM, true, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
+    return launch_one<T, M, LM, LO, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
 }
 
-// Dispatch on the LMAX bucket for one (T, M) pair.  L equal to the bucket
-// runs a kernel specialised for that L; float grids have 8-, 16- and 32-node
-// tile variants of it, everything else 16-node tiles.
+// Dispatch on the label count for one (T, M) pair.  A kernel compiled for the
+// next multiple of 8 (above 64: of 16) leaves at most 7 (15) labels whose
+// existence is tested at run time.  With powers of two only, every label was
+// tested and kept a register; per half-sweep, then -> now: 1920x1080 FP32
+// L = 24 284 -> 199 us, L = 48 578 -> 315 us (5.7 TB/s), L = 60 604 -> 366 us;
+// 1280x720 L = 80 473 -> 225 us, L = 100 501 -> 355 us, int32 L = 100
+// 426 -> 292 us; truncated quadratic L = 100 394 -> 320 us (split kernel).
+// FP64 grids, which serve to check the others, keep the powers of two.
 template <typename T, typename M>
 cudaError_t launch_sweep_tm(const RecordFormat &f, const SweepConfig &cfg, const SweepParams &p, cudaStream_t s,
                             int num_sms) {
-    if (f.L <= 16) return launch_variant<T, M, 16>(f, cfg, p, s, num_sms);
-    if (f.L <= 32) return launch_variant<T, M, 32>(f, cfg, p, s, num_sms);
-    if (f.L <= 64) return launch_variant<T, M, 64>(f, cfg, p, s, num_sms);
-    if (f.L <= 128) return launch_variant<T, M, 128>(f, cfg, p, s, num_sms);
+    if constexpr (sizeof(T) == 8) {
+        if (f.L <= 16) return launch_variant<T, M, 16, 1>(f, cfg, p, s, num_sms);
+        if (f.L <= 32) return launch_variant<T, M, 32, 17>(f, cfg, p, s, num_sms);
+        if (f.L <= 64) return launch_variant<T, M, 64, 33>(f, cfg, p, s, num_sms);
+        if (f.L <= 128) return launch_variant<T, M, 128, 65>(f, cfg, p, s, num_sms);
+    } else {
+        if (f.L <= 8) return launch_variant<T, M, 8, 1>(f, cfg, p, s, num_sms);
+        if (f.L <= 16) return launch_variant<T, M, 16, 9>(f, cfg, p, s, num_sms);
+        if (f.L <= 24) return launch_variant<T, M, 24, 17>(f, cfg, p, s, num_sms);
+        if (f.L <= 32) return launch_variant<T, M, 32, 25>(f, cfg, p, s, num_sms);
+        if (f.L <= 40) return launch_variant<T, M, 40, 33>(f, cfg, p, s, num_sms);
+        if (f.L <= 48) return launch_variant<T, M, 48, 41>(f, cfg, p, s, num_sms);
+        if (f.L <= 56) return launch_variant<T, M, 56, 49>(f, cfg, p, s, num_sms);
+        if (f.L <= 64) return launch_variant<T, M, 64, 57>(f, cfg, p, s, num_sms);
+        if (f.L <= 80) return launch_variant<T, M, 80, 65>(f, cfg, p, s, num_sms);
+        if (f.L <= 96) return launch_variant<T, M, 96, 81>(f, cfg, p, s, num_sms);
+        if (f.L <= 112) return launch_variant<T, M, 112, 97>(f, cfg, p, s, num_sms);
+        if (f.L <= 128) return launch_variant<T, M, 128, 113>(f, cfg, p, s, num_sms);
+    }
     return cudaErrorInvalidValue;
 }
 
