@@ -822,9 +822,11 @@ __device__ __forceinline__ bool tile_finish(const SweepParams &p, const TableCon
             // Launched only when the table's truncation radius fits the window.
             message_quad_window<T, M, LMAX, LMIN, QW>(p, slot, L, dir, tc.vtap, tc.trunc);
         } else {
-            if (p.mode == MODE_REF_MINCONV) messages_ref_minconv<T, M, LMAX>(p, slot, L, dir);
-            else if (p.mode == MODE_STD_MINCONV) message_std_minconv<T, M, LMAX>(p, slot, L, dir);
-            else message_std_quad<T, M, LMAX>(p, slot, L, dir, tc.scale, tc.trunc);
+            if constexpr (sizeof(T) == 8) {
+                if (p.mode == MODE_REF_MINCONV) messages_ref_minconv<T, M, LMAX>(p, slot, L, dir);
+                if (p.mode == MODE_STD_MINCONV) message_std_minconv<T, M, LMAX>(p, slot, L, dir);
+            }
+            if (p.mode == MODE_STD_QUAD) message_std_quad<T, M, LMAX>(p, slot, L, dir, tc.scale, tc.trunc);
         }
     }
     if constexpr (DIRECT) {
@@ -1124,17 +1126,17 @@ struct LaunchCache {
 
 // Launches one half-sweep kernel over tiles of `nodes` nodes, NW warps per
 // block, one block per resident slot of every SM (fewer if there are fewer
-// tiles).
+// tiles); extra_smem bytes follow the nodes' slots in shared memory.
 template <typename K>
 cudaError_t launch_tiles(K kern, LaunchCache &lc_state, int NW, int nodes, const SweepParams &params,
-                         uint32_t slot_bytes, cudaStream_t s, int num_sms) {
+                         uint32_t slot_bytes, cudaStream_t s, int num_sms, size_t extra_smem = 0) {
     // The tiling follows the variant actually launched.
     SweepParams p = params;
     const int n1 = p.W >= 3 ? (p.W - 3) / 2 + 1 : 0;
     p.tiles_per_row = (n1 + nodes - 1) / nodes;
     p.num_tiles = p.H >= 3 ? (p.H - 2) * p.tiles_per_row : 0;
     if (p.num_tiles <= 0) return cudaSuccess;
-    const size_t smem = (size_t)nodes * slot_bytes;
+    const size_t smem = (size_t)nodes * slot_bytes + extra_smem;
     cudaError_t e = lc_state.smem.ensure(kern, smem);
     if (e != cudaSuccess) return e;
     int occ = 0;
@@ -1179,8 +1181,12 @@ cudaError_t launch_split(const SweepParams &params, uint32_t slot_bytes, cudaStr
                         num_sms);
 }
 
-// The min-convolution rules and the lower envelope: one kernel per power of
-// two, labels tested against the run-time L.
+// Min-convolutions with 4-byte arithmetic (sweep_table.cuh).
+template <typename T, typename M>
+cudaError_t launch_table(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms);
+
+// The lower envelope, and FP64 min-convolutions: one kernel per power of two,
+// labels tested against the run-time L.
 template <typename T, typename M, int LM>
 cudaError_t launch_general(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
     return launch_one<T, M, LM, 1, 2, KIND_GENERAL>(p, f.slot_bytes, s, num_sms);
@@ -1232,11 +1238,18 @@ cudaError_t launch_variant(const RecordFormat &f, const SweepConfig &cfg, const 
             }
         }
     }
+    if constexpr (sizeof(T) == 4) {
+        if (p.mode == MODE_REF_MINCONV || p.mode == MODE_STD_MINCONV) return launch_table<T, M>(f, p, s, num_sms);
+    }
     if (p.mode != MODE_LINEAR) {
-        if (f.L <= 16) return launch_general<T, M, 16>(f, p, s, num_sms);
-        if (f.L <= 32) return launch_general<T, M, 32>(f, p, s, num_sms);
-        if (f.L <= 64) return launch_general<T, M, 64>(f, p, s, num_sms);
-        return launch_general<T, M, 128>(f, p, s, num_sms);
+        if constexpr (std::is_same<T, int>::value) {
+            return cudaErrorInvalidValue;  // int32 grids have no lower envelope
+        } else {
+            if (f.L <= 16) return launch_general<T, M, 16>(f, p, s, num_sms);
+            if (f.L <= 32) return launch_general<T, M, 32>(f, p, s, num_sms);
+            if (f.L <= 64) return launch_general<T, M, 64>(f, p, s, num_sms);
+            return launch_general<T, M, 128>(f, p, s, num_sms);
+        }
     }
     if constexpr (kPow2) {
         if (exact) {
