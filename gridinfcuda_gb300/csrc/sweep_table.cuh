@@ -9,21 +9,27 @@
 //               message, then the mean (or the minimum) subtracted
 //
 // A min-convolution is a matrix product over (min, +): V (L x L) times the
-// tile's L x 16 (reference) or L x 64 (standard) vectors.  A block of 128
-// threads holds V in shared memory for all its tiles (16 nodes each) and gives
+// tile's L x 16 (reference) or L x 64 (standard) vectors.  A block
+// holds V in shared memory for all its tiles (16 nodes each) and gives
 // every thread TI outputs of TN vectors in registers, so that four steps of j
-// read TI floats of V and four of each vector from shared memory for
-// 4 TI TN additions and minima.  Additions go two outputs to an instruction
-// (add.rn.f32x2, rounded as the scalar one) and minima two steps of j to one
-// (three-input minimum).  TI and TN follow L so that the 128 threads have one
+// read 4 TI entries of V and four of each vector from shared memory for
+// 4 TI TN additions and minima.  Additions and minima go two steps of j to an
+// instruction (add.rn.f32x2, rounded as the scalar one; three-input minimum).  TI and TN follow L so that the block's threads have one
 // group of outputs each or nearly so (launch_table).  The lane-per-message
 // form this replaces read V through the cache once per addition and kept the
 // standard rule's vectors in local memory.
 //
-// Bound: HBM (36 B per updated node and label) for the reference rule and up
-// to about 64 labels of the standard rule, then the instruction issue rate.
-// Measured, 640x480 FP32, us per half-sweep, before -> now:
-//   TABLE_MEASURED
+// Bound: HBM (36 B per updated node and label) for the reference rule up to
+// about 32 labels; above that the latency of a tile's phases with the few
+// blocks that the table leaves room for, and for the standard rule the issue
+// rate (at L = 64, 13 T additions and minima a second).  Measured, 640x480
+// FP32, us per half-sweep, lane-per-message form -> this one:
+//   L           16         32         64          128
+//   reference   52 -> 24   146 -> 37  727 -> 85   - -> 256
+//   standard    127 -> 39  697 -> 75  3866 -> 200 - -> 720
+// Also measured for the standard rule at L = 64: four warps of 8 x 4 outputs
+// 237, two of 8 x 8 with the additions paired along i 197 (the reference rule,
+// whose vectors need no subtraction, is faster paired along j).
 //
 // Exactness.  The reference takes (a < b) ? a : b in order of j.  On operands
 // that are neither NaN nor a zero of either sign against the other, the
@@ -39,8 +45,7 @@
 
 namespace ginf_gpu {
 
-constexpr int kTableWarps = 4, kTableSplit = 2, kTableNodes = kTableWarps / kTableSplit * 8;
-constexpr int kTableThreads = kTableWarps * 32;
+constexpr int kTableNodes = 16;  // nodes per tile
 constexpr float kTableBig = 1e38f;
 constexpr int kTableMaxGroups = 16;  // output groups per vector: Lp / TI
 
@@ -58,42 +63,37 @@ __device__ __forceinline__ void load4(const unsigned char *p, T *o) {
         MIO<M, T>::load(p, o);
     }
 }
+// Two consecutive elements.
 template <typename M, typename T>
-__device__ __forceinline__ void store4(unsigned char *p, const T *o) {
+__device__ __forceinline__ void store2(unsigned char *p, T a, T b) {
     if constexpr (sizeof(M) == 2) {
-        const __half2 a = __floats2half2_rn(o[0], o[1]), b = __floats2half2_rn(o[2], o[3]);
-        *reinterpret_cast<uint2 *>(p) =
-            make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        const __half2 h = __floats2half2_rn(a, b);
+        *reinterpret_cast<uint32_t *>(p) = *reinterpret_cast<const uint32_t *>(&h);
+    } else if constexpr (std::is_same<T, int>::value) {
+        *reinterpret_cast<int2 *>(p) = make_int2(a, b);
     } else {
-        MIO<M, T>::store(p, o);
+        *reinterpret_cast<float2 *>(p) = make_float2(a, b);
     }
 }
 
-// acc(i) = min(acc(i), v0(i) + h0, v1(i) + h1) for TI outputs.
-template <int TI>
-__device__ __forceinline__ void table_step2(float *acc, const float *v0, float h0, const float *v1, float h1) {
-#pragma unroll
-    for (int i = 0; i < TI; i += 2) {
-        const float2 a = add_f32x2(v0[i], v0[i + 1], h0, h0), b = add_f32x2(v1[i], v1[i + 1], h1, h1);
-        acc[i] = min3_f32(acc[i], a.x, b.x);
-        acc[i + 1] = min3_f32(acc[i + 1], a.y, b.y);
-    }
+// Steps j and j + 1 of one output: acc = min(acc, v0 + h0, v1 + h1).
+__device__ __forceinline__ float table_step(float acc, float v0, float v1, float h0, float h1) {
+    const float2 t = add_f32x2(v0, v1, h0, h1);
+    return min3_f32(acc, t.x, t.y);
 }
-template <int TI>
-__device__ __forceinline__ void table_step2(int *acc, const int *v0, int h0, const int *v1, int h1) {
-#pragma unroll
-    for (int i = 0; i < TI; ++i) acc[i] = min(min(acc[i], v0[i] + h0), v1[i] + h1);
+__device__ __forceinline__ int table_step(int acc, int v0, int v1, int h0, int h1) {
+    return min(min(acc, v0 + h0), v1 + h1);
 }
-template <int TI>
-__device__ __forceinline__ void table_step1(float *acc, const float *v, float h) {
-#pragma unroll
-    for (int i = 0; i < TI; ++i) acc[i] = fminf(acc[i], v[i] + h);
+__device__ __forceinline__ void sub4(float *h, const float *a) {
+    const float2 x = sub_f32x2(h[0], h[1], a[0], a[1]), y = sub_f32x2(h[2], h[3], a[2], a[3]);
+    h[0] = x.x; h[1] = x.y; h[2] = y.x; h[3] = y.y;
 }
-template <int TI>
-__device__ __forceinline__ void table_step1(int *acc, const int *v, int h) {
+__device__ __forceinline__ void sub4(int *h, const int *a) {
 #pragma unroll
-    for (int i = 0; i < TI; ++i) acc[i] = min(acc[i], v[i] + h);
+    for (int k = 0; k < 4; ++k) h[k] -= a[k];
 }
+__device__ __forceinline__ float table_min(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ int table_min(int a, int b) { return min(a, b); }
 
 // The belief of one node by its four lanes, as belief_part, noting values the
 // fast form does not cover.
@@ -130,97 +130,112 @@ __device__ __forceinline__ void table_belief(const SweepParams &p, unsigned char
     }
 }
 
-// The tile's min-convolutions, fast form.  Vs is V with rows of Lp outputs
-// (Vs[j * Lp + i] = V(i, j)).  Vector m is node m (reference: the output goes
-// to the node's first message slot) or message (node m / 4, direction m % 4)
-// (standard: in place, which is why a round's reads end before its writes).
+// The tile's min-convolutions, fast form.  Vs holds V with the steps of j in
+// pairs: V(i, j) at ((j / 2) Lp + i) 2 + j % 2, so that a 16-byte load brings
+// two outputs' entries for j and j + 1, each pair an operand of one packed
+// addition with the pair h(j), h(j + 1) as it lies in the node's slot.  Vector
+// m is node m (reference: the output goes to the node's first message slot) or
+// message (node m / 4, direction m % 4) (standard: in place, which is why the
+// block's reads end before its writes).  Thread (ig, mb / TN) has the outputs
+// 2 (ig + c groups), + 1, c < TI / 2, of the vectors mb .. mb + TN - 1: eight
+// neighbouring threads read 128 consecutive bytes of V.
 template <typename T, typename M, bool STD, int TI, int TN>
 __device__ __forceinline__ void table_convolve(const SweepParams &p, const T *Vs, unsigned char *smem, int L,
                                                T (*mins)[kTableMaxGroups]) {
     constexpr int NV = STD ? 4 * kTableNodes : kTableNodes;
     const int groups = p.Lp / TI;
-    const int per_round = kTableThreads / groups;
-    const int ig = (int)threadIdx.x % groups, mine = (int)threadIdx.x / groups;
-    for (int m0 = 0; m0 < NV; m0 += per_round * TN) {
-        const int mb = m0 + mine * TN;
-        const bool on = mine < per_round && mb < NV;
-        T acc[TN][TI];
-        if (on) {
-            const unsigned char *sl[TN], *in[TN];
+    const int ig = (int)threadIdx.x % groups, mb = (int)threadIdx.x / groups * TN;
+    const bool on = mb < NV;
+    T acc[TN][TI];
+    if (on) {
+        const unsigned char *sl[TN], *in[TN];
 #pragma unroll
-            for (int u = 0; u < TN; ++u) {
-                sl[u] = smem + (size_t)(STD ? (mb + u) / 4 : mb + u) * p.slot_bytes;
-                in[u] = sl[u] + p.d_bytes + (STD ? (mb + u) % 4 : 0) * p.m_bytes;
+        for (int u = 0; u < TN; ++u) {
+            sl[u] = smem + (size_t)(STD ? (mb + u) / 4 : mb + u) * p.slot_bytes;
+            in[u] = sl[u] + p.d_bytes + (STD ? (mb + u) % 4 : 0) * p.m_bytes;
+#pragma unroll
+            for (int i = 0; i < TI; ++i) acc[u][i] = pos_inf<T>();
+        }
+        const unsigned char *vp = reinterpret_cast<const unsigned char *>(Vs + ig * 4);
+        const int row = 2 * p.Lp * (int)sizeof(T), chunk = 4 * groups * (int)sizeof(T);
+        // h(j .. j + 3) of vector u.
+        auto load_h = [&](int u, int j, T *h) {
+            load_t<T, 4>(sl[u] + j * sizeof(T), h);
+            if constexpr (STD) {
+                T a[4];
+                load4<M, T>(in[u] + j * sizeof(M), a);
+                sub4(h, a);
             }
+        };
+        // Four steps of j at a time; the reference rule's loop has registers to
+        // spare for loads ahead (L = 128: 313 us at one step per pass, 280 at four).
+        const int L4 = L & ~3;
+#pragma unroll(STD ? 1 : 4)
+        for (int j = 0; j < L4; j += 4) {
+            T h[TN][4];
 #pragma unroll
-            for (int u = 0; u < TN; ++u)
+            for (int u = 0; u < TN; ++u) load_h(u, j, h[u]);
 #pragma unroll
-                for (int i = 0; i < TI; ++i) acc[u][i] = pos_inf<T>();
-            const T *vp = Vs + ig * TI;
-            // Four steps of j; rows past L are never read.
-#pragma unroll 1
-            for (int j = 0; j < L; j += 4) {
-                T h[TN][4];
+            for (int k = 0; k < 4; k += 2) {
 #pragma unroll
-                for (int u = 0; u < TN; ++u) {
-                    load_t<T, 4>(sl[u] + j * sizeof(T), h[u]);
-                    if constexpr (STD) {
-                        T a[4];
-                        load4<M, T>(in[u] + j * sizeof(M), a);
+                for (int c = 0; c < TI / 2; ++c) {
+                    T v[4];
+                    load_t<T, 4>(vp + c * chunk, v);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) h[u][k] = h[u][k] - a[k];
+                    for (int u = 0; u < TN; ++u) {
+                        acc[u][2 * c] = table_step(acc[u][2 * c], v[0], v[1], h[u][k], h[u][k + 1]);
+                        acc[u][2 * c + 1] = table_step(acc[u][2 * c + 1], v[2], v[3], h[u][k], h[u][k + 1]);
                     }
                 }
+                vp += row;
+            }
+        }
+        if (L4 < L) {  // one to three steps more
 #pragma unroll
-                for (int k = 0; k < 4; k += 2) {
-                    T v0[TI], v1[TI];
-                    if (j + k + 1 < L) {
-                        load_t<T, TI>(reinterpret_cast<const unsigned char *>(vp + (size_t)(j + k) * p.Lp), v0);
-                        load_t<T, TI>(reinterpret_cast<const unsigned char *>(vp + (size_t)(j + k + 1) * p.Lp), v1);
+            for (int u = 0; u < TN; ++u) {
+                T h[4];
+                load_h(u, L4, h);
 #pragma unroll
-                        for (int u = 0; u < TN; ++u) table_step2<TI>(acc[u], v0, h[u][k], v1, h[u][k + 1]);
-                    } else if (j + k < L) {
-                        load_t<T, TI>(reinterpret_cast<const unsigned char *>(vp + (size_t)(j + k) * p.Lp), v0);
+                for (int k = 0; k < 3; ++k) {
+                    if (L4 + k < L) {
 #pragma unroll
-                        for (int u = 0; u < TN; ++u) table_step1<TI>(acc[u], v0, h[u][k]);
+                        for (int c = 0; c < TI / 2; ++c) {
+                            const T *v = reinterpret_cast<const T *>(vp + (k / 2) * row + c * chunk) + (k & 1);
+                            acc[u][2 * c] = table_min(acc[u][2 * c], v[0] + h[k]);
+                            acc[u][2 * c + 1] = table_min(acc[u][2 * c + 1], v[2] + h[k]);
+                        }
                     }
                 }
             }
         }
         if constexpr (STD && sizeof(M) == 2) {
             // FP16 messages leave rounded once, the minimum already subtracted.
-            if (on) {
-#pragma unroll
-                for (int u = 0; u < TN; ++u) {
-                    T m = pos_inf<T>();
-#pragma unroll
-                    for (int i = 0; i < TI; ++i)
-                        if (ig * TI + i < L) m = fminf(m, acc[u][i]);
-                    mins[mb + u][ig] = m;
-                }
-            }
-        }
-        if constexpr (STD) __syncthreads();
-        if (on) {
 #pragma unroll
             for (int u = 0; u < TN; ++u) {
-                T shift = T(0);
-                if constexpr (STD && sizeof(M) == 2) {
-                    shift = mins[mb + u][0];
-                    for (int g = 1; g < groups; ++g) shift = fminf(shift, mins[mb + u][g]);
-                }
-                unsigned char *out = smem + (size_t)(STD ? (mb + u) / 4 : mb + u) * p.slot_bytes + p.d_bytes +
-                                     (STD ? (mb + u) % 4 : 0) * p.m_bytes + (size_t)ig * TI * sizeof(M);
+                T m = pos_inf<T>();
 #pragma unroll
-                for (int i = 0; i < TI; i += 4) {
-                    T r[4];
+                for (int i = 0; i < TI; ++i)
+                    if ((ig + i / 2 * groups) * 2 + i % 2 < L) m = fminf(m, acc[u][i]);
+                mins[mb + u][ig] = m;
+            }
+        }
+    }
+    if constexpr (STD) __syncthreads();
+    if (on) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        r[k] = ig * TI + i + k < L ? acc[u][i + k] : T(0);
-                        if constexpr (STD && sizeof(M) == 2) r[k] = ig * TI + i + k < L ? r[k] - shift : T(0);
-                    }
-                    store4<M, T>(out + i * sizeof(M), r);
-                }
+        for (int u = 0; u < TN; ++u) {
+            T shift = T(0);
+            if constexpr (STD && sizeof(M) == 2) {
+                shift = mins[mb + u][0];
+                for (int g = 1; g < groups; ++g) shift = fminf(shift, mins[mb + u][g]);
+            }
+            unsigned char *out = smem + (size_t)(STD ? (mb + u) / 4 : mb + u) * p.slot_bytes + p.d_bytes +
+                                 (STD ? (mb + u) % 4 : 0) * p.m_bytes;
+#pragma unroll
+            for (int c = 0; c < TI / 2; ++c) {
+                const int i0 = (ig + c * groups) * 2;
+                store2<M, T>(out + i0 * sizeof(M), i0 < L ? acc[u][2 * c] - shift : T(0),
+                             i0 + 1 < L ? acc[u][2 * c + 1] - shift : T(0));
             }
         }
     }
@@ -260,12 +275,20 @@ __device__ __forceinline__ void table_normalise(unsigned char *md, int L, int no
     }
 }
 
-// One half-sweep.  Warps come in pairs over eight nodes: the first of a pair
-// issues the copies and does what is done once a lane (k, dir) -- beliefs,
-// normalisation, stores -- and all four convolve.
-template <typename T, typename M, bool STD, int TI, int TN>
-__global__ void __launch_bounds__(kTableThreads) sweep_kernel_table(const SweepParams p) {
-    constexpr int NW = kTableWarps, SPL = kTableSplit;
+// Blocks per SM the registers are allocated for: what shared memory holds at
+// the kernel's largest L, or what keeps the accumulators out of local memory.
+constexpr int table_blocks(bool std_rule, int spl, int outputs) {
+    if (spl == 2) return 2;
+    if (!std_rule) return outputs == 4 ? 18 : (outputs == 8 ? 15 : 6);
+    return outputs == 8 ? 14 : (outputs == 16 ? 10 : (outputs == 32 ? 8 : 6));
+}
+
+// One half-sweep.  SPL warps serve eight nodes: the first of them issues the
+// copies and does what is done once a lane (k, dir) -- beliefs, normalisation,
+// stores -- and all convolve.
+template <typename T, typename M, bool STD, int SPL, int TI, int TN>
+__global__ void __launch_bounds__(64 * SPL, table_blocks(STD, SPL, TI * TN)) sweep_kernel_table(const SweepParams p) {
+    constexpr int NW = 2 * SPL;
     constexpr bool kF32 = std::is_same<T, float>::value;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
@@ -274,13 +297,23 @@ __global__ void __launch_bounds__(kTableThreads) sweep_kernel_table(const SweepP
     const int L = p.L;
     T *Vs = reinterpret_cast<T *>(smem + (size_t)kTableNodes * p.slot_bytes);
     int odd_table = 0;
-    for (int e = threadIdx.x; e < L * p.Lp; e += blockDim.x) {
-        const int j = e / p.Lp, i = e - j * p.Lp;
-        const T v = i < L ? __ldg(static_cast<const T *>(p.V) + i + (size_t)L * j) : T(0);
-        Vs[e] = v;
-        if constexpr (kF32)
-            if (!(v > -pos_inf<float>()) || __float_as_uint(v) == 0x80000000u) odd_table = 1;
-    }
+    // Warp w stages the rows w, w + NW, ..., eight of them in flight.
+    for (int j0 = (int)(threadIdx.x >> 5); j0 < L; j0 += 8 * NW)
+        for (int i = (int)(threadIdx.x & 31); i < p.Lp; i += 32) {
+            T v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int j = j0 + q * NW;
+                v[q] = j < L && i < L ? __ldg(static_cast<const T *>(p.V) + i + (size_t)L * j) : T(0);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int j = j0 + q * NW;
+                if (j < L) Vs[((j >> 1) * p.Lp + i) * 2 + (j & 1)] = v[q];
+                if constexpr (kF32)
+                    if (!(v[q] > -pos_inf<float>()) || __float_as_uint(v[q]) == 0x80000000u) odd_table = 1;
+            }
+        }
     if (threadIdx.x == 0) {
         mbar_init(&full_bar, NW * 32);
         fence_barrier_init();
@@ -341,28 +374,30 @@ __global__ void __launch_bounds__(kTableThreads) sweep_kernel_table(const SweepP
     bulk_wait_all();
 }
 
-template <typename T, typename M, bool STD, int TI, int TN>
+template <typename T, typename M, bool STD, int SPL, int TI, int TN>
 cudaError_t launch_table_t(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
     static LaunchCache cache;
-    return launch_tiles(sweep_kernel_table<T, M, STD, TI, TN>, cache, kTableWarps, kTableNodes, p, f.slot_bytes, s,
-                        num_sms, (size_t)f.L * f.Lp * sizeof(T));
+    return launch_tiles(sweep_kernel_table<T, M, STD, SPL, TI, TN>, cache, 2 * SPL, kTableNodes, p, f.slot_bytes, s,
+                        num_sms, (size_t)(f.L + 1) / 2 * 2 * f.Lp * sizeof(T));
 }
 
-// Outputs per thread: 128 threads cover L / TI groups of 16 / TN (reference)
-// or 64 / TN (standard) vectors in one round at the powers of two; between
-// them some threads idle or a second round runs.
+// Threads and outputs per thread: Lp / TI groups times 16 / TN (reference) or
+// 64 / TN (standard) vector groups fill the block's 64 (128 above 64 labels)
+// threads at the powers of two and leave some idle between them.  The largest
+// TI x TN that fills the block reads the least shared memory per addition.
 template <typename T, typename M>
 cudaError_t launch_table(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
     if (p.mode == MODE_REF_MINCONV) {
-        if (f.L <= 32) return launch_table_t<T, M, false, 4, 1>(f, p, s, num_sms);
-        if (f.L <= 64) return launch_table_t<T, M, false, 4, 2>(f, p, s, num_sms);
-        return launch_table_t<T, M, false, 4, 4>(f, p, s, num_sms);
+        if (f.L <= 16) return launch_table_t<T, M, false, 1, 4, 1>(f, p, s, num_sms);
+        if (f.L <= 32) return launch_table_t<T, M, false, 1, 4, 2>(f, p, s, num_sms);
+        if (f.L <= 64) return launch_table_t<T, M, false, 1, 4, 4>(f, p, s, num_sms);
+        return launch_table_t<T, M, false, 2, 4, 4>(f, p, s, num_sms);
     }
-    if (f.L <= 8) return launch_table_t<T, M, true, 4, 1>(f, p, s, num_sms);
-    if (f.L <= 24) return launch_table_t<T, M, true, 4, 2>(f, p, s, num_sms);
-    if (f.L <= 32) return launch_table_t<T, M, true, 4, 4>(f, p, s, num_sms);
-    if (f.L <= 64) return launch_table_t<T, M, true, 8, 4>(f, p, s, num_sms);
-    return launch_table_t<T, M, true, 8, 8>(f, p, s, num_sms);
+    if (f.L <= 8) return launch_table_t<T, M, true, 1, 8, 1>(f, p, s, num_sms);
+    if (f.L <= 16) return launch_table_t<T, M, true, 1, 8, 2>(f, p, s, num_sms);
+    if (f.L <= 32) return launch_table_t<T, M, true, 1, 8, 4>(f, p, s, num_sms);
+    if (f.L <= 64) return launch_table_t<T, M, true, 1, 8, 8>(f, p, s, num_sms);
+    return launch_table_t<T, M, true, 2, 8, 8>(f, p, s, num_sms);
 }
 
 }  // namespace ginf_gpu
