@@ -616,40 +616,57 @@ __global__ void k_convert(const Ts *src, Td *dst, int n) {
     if (i < n) dst[i] = (Td)src[i];
 }
 
+// Stereo costs are bound by the store of the volume.  A thread owns one pixel
+// and kStereoLabels consecutive labels: the left pixel is read once, a warp's
+// right pixels are 32 consecutive addresses in L1 and its stores 128 bytes of a
+// label plane, and nothing is divided.  1920x1080x64: one thread per element,
+XX
+constexpr int kStereoLabels = 16;
+
 // D(x,y,d) = coef * min(|left(x,y) - right(max(x-d,0),y)|, cap), label-planar;
 // the operation sequence matches the numpy generator bit for bit.
-__global__ void k_stereo_costs(int W, int H, int L, const float *__restrict__ left, const float *__restrict__ right,
-                               float coef, float cap, float *__restrict__ costs) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t total = (size_t)W * H * L;
-    if (idx >= total) return;
-    const int x = (int)(idx % W);
-    const int y = (int)((idx / W) % H);
-    const int d = (int)(idx / ((size_t)W * H));
-    const float a = left[(size_t)y * W + x];
-    const float b = right[(size_t)y * W + max(x - d, 0)];
-    costs[idx] = coef * fminf(fabsf(a - b), cap);
+__global__ void __launch_bounds__(kThreads) k_stereo_costs(int W, int H, int L, const float *__restrict__ left,
+                                                           const float *__restrict__ right, float coef, float cap,
+                                                           float *__restrict__ costs) {
+    const int x = blockIdx.x * kThreads + threadIdx.x;
+    if (x >= W) return;
+    const size_t plane = (size_t)W * H;
+    for (int d0 = blockIdx.z * kStereoLabels; d0 < L; d0 += gridDim.z * kStereoLabels)
+    for (int y = blockIdx.y; y < H; y += gridDim.y) {
+        const int d1 = min(L, d0 + kStereoLabels);
+        const float a = left[(size_t)y * W + x];
+        const float *r = right + (size_t)y * W;
+        float *out = costs + plane * d0 + (size_t)y * W + x;
+#pragma unroll 8
+        for (int d = d0; d < d1; ++d) {
+            *out = coef * fminf(fabsf(a - __ldg(r + max(x - d, 0))), cap);
+            out += plane;
+        }
+    }
 }
 
 // The reference example's integer recipe (examples/stereo/stereo.cc:28-34):
 // for x >= L-1, D(x, y, k) = min(|left(x,y) - right(x-k,y)|, cap) on 8-bit
 // grey images; the columns x < L-1 keep zero cost (the Grid constructor's
-// zero fill, src/matrix.cc:21-27).  One thread per cost element, label-planar.
-__global__ void k_stereo_costs_u8(int W, int H, int L, const uint8_t *__restrict__ left,
-                                  const uint8_t *__restrict__ right, int cap, int32_t *__restrict__ costs) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t total = (size_t)W * H * L;
-    if (idx >= total) return;
-    const int x = (int)(idx % W);
-    const int y = (int)((idx / W) % H);
-    const int k = (int)(idx / ((size_t)W * H));
-    int c = 0;
-    if (x >= L - 1) {
+// zero fill, src/matrix.cc:21-27).  Label-planar.
+__global__ void __launch_bounds__(kThreads) k_stereo_costs_u8(int W, int H, int L, const uint8_t *__restrict__ left,
+                                                              const uint8_t *__restrict__ right, int cap,
+                                                              int32_t *__restrict__ costs) {
+    const int x = blockIdx.x * kThreads + threadIdx.x;
+    if (x >= W) return;
+    const size_t plane = (size_t)W * H;
+    for (int k0 = blockIdx.z * kStereoLabels; k0 < L; k0 += gridDim.z * kStereoLabels)
+    for (int y = blockIdx.y; y < H; y += gridDim.y) {
+        const int k1 = min(L, k0 + kStereoLabels);
         const int a = left[(size_t)y * W + x];
-        const int b = right[(size_t)y * W + x - k];
-        c = min(abs(a - b), cap);
+        const uint8_t *r = right + (size_t)y * W;
+        int32_t *out = costs + plane * k0 + (size_t)y * W + x;
+#pragma unroll 8
+        for (int k = k0; k < k1; ++k) {
+            *out = x >= L - 1 ? min(abs(a - (int)__ldg(r + max(x - k, 0))), cap) : 0;
+            out += plane;
+        }
     }
-    costs[idx] = c;
 }
 
 // Level-t inputs and targets of the warm-start network (FP32 records):
@@ -1070,17 +1087,22 @@ cudaError_t launch_warm_init(const RecordFormat &f, unsigned char *rec, int W, i
     return cudaGetLastError();
 }
 
+// Blocks of 256 pixels of a row, rows in y and label chunks in z; what exceeds
+// the grid's limits is looped over.
+static dim3 stereo_grid(int W, int H, int L) {
+    return dim3(blocks_for((size_t)W), (unsigned)std::min(H, 65535),
+                (unsigned)std::min((L - 1) / kStereoLabels + 1, 65535));
+}
+
 cudaError_t launch_stereo_costs(int W, int H, int L, const float *left, const float *right, float coef, float cap,
                                 float *costs, cudaStream_t s) {
-    const size_t total = (size_t)W * H * L;
-    k_stereo_costs<<<blocks_for(total), kThreads, 0, s>>>(W, H, L, left, right, coef, cap, costs);
+    k_stereo_costs<<<stereo_grid(W, H, L), kThreads, 0, s>>>(W, H, L, left, right, coef, cap, costs);
     return cudaGetLastError();
 }
 
 cudaError_t launch_stereo_costs_u8(int W, int H, int L, const uint8_t *left, const uint8_t *right, int cap,
                                    int32_t *costs, cudaStream_t s) {
-    const size_t total = (size_t)W * H * L;
-    k_stereo_costs_u8<<<blocks_for(total), kThreads, 0, s>>>(W, H, L, left, right, cap, costs);
+    k_stereo_costs_u8<<<stereo_grid(W, H, L), kThreads, 0, s>>>(W, H, L, left, right, cap, costs);
     return cudaGetLastError();
 }
 
