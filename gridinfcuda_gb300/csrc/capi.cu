@@ -326,6 +326,7 @@ struct Call {
     ginf_stats *stats;
     int64_t launches = 0;
     int64_t h2d = 0, d2h = 0;
+    bool keep_msgs = false;  // the level-0 messages are read after the last half-sweep
     void ev(int i) {
         if (stats) cudaEventRecord(ws->ev[i], r.stream);
     }
@@ -473,10 +474,11 @@ ginf_status table_radius(Call &c, Prepared &P, int &radius, int &exact) {
 }
 
 // Bytes a half-sweep must move through HBM: per updated node its costs and
-// four incoming messages in, four outgoing messages out.
-int64_t sweep_alg_bytes(const RecordFormat &f, const Level &lv) {
+// four incoming messages in, four outgoing messages out (no messages out when
+// only labels are wanted).
+int64_t sweep_alg_bytes(const RecordFormat &f, const Level &lv, bool labels_only = false) {
     const int64_t nodes = (int64_t)(lv.W - 2) * (lv.H - 2) / 2;
-    return nodes * ((int64_t)f.d_bytes + 8 * (int64_t)f.m_bytes);
+    return nodes * ((int64_t)f.d_bytes + (labels_only ? 4 : 8) * (int64_t)f.m_bytes);
 }
 
 // The HBP level loop on prepared records, levels `from` down to `to`:
@@ -568,11 +570,15 @@ ginf_status run_levels(Call &c, Prepared &P, int iters, int64_t &nli, int from, 
             p.iter = it;
             p.read_mode = it == 0 ? first : RD_OWN;
             p.write_labels = (t == 0 && stale && it >= iters - 2) ? 1 : 0;
-            GINF_CK(launch_sweep(f, c.r.cfg, p, s, c.ws->num_sms));
+            // The solve's last half-sweep only gives labels, unless its
+            // messages are handed on.
+            const bool labels_only = t == 0 && stale && it == iters - 1 && p.read_mode == RD_OWN && !c.keep_msgs;
+            if (labels_only) GINF_CK(launch_sweep_labels(f, p, s));
+            else GINF_CK(launch_sweep(f, c.r.cfg, p, s, c.ws->num_sms));
             ++c.launches;
             if (t == 0 && c.stats) {
                 ++c.stats->level0_sweep_launches;
-                c.stats->level0_alg_bytes += sweep_alg_bytes(f, lv);
+                c.stats->level0_alg_bytes += sweep_alg_bytes(f, lv, labels_only);
             }
         }
         if (nlaunch > 0) {
@@ -868,6 +874,7 @@ ginf_status ginf_decode_hbp(ginf_workspace *wsp, const ginf_grid *grid, int32_t 
     // so the untouched border goes back unchanged.
     GINF_TRY(prepare(c, P, num_levels, false, nullptr, host ? nullptr : labels));
     int64_t nli = 0;
+    c.keep_msgs = opt && opt->msgs_out;
     GINF_TRY(run_bp(c, P, iters_per_level, nli));
     c.ev(EV_ICM);
     c.ev(EV_ENERGY);
@@ -1061,6 +1068,7 @@ ginf_status ginf_solve(ginf_workspace *wsp, const ginf_grid *grid, int32_t num_l
     // The caller's labels seed the device copy: ICM reads the border labels.
     GINF_TRY(prepare(c, P, num_levels, true, host ? labels : nullptr, host ? nullptr : labels));
     int64_t nli = 0;
+    c.keep_msgs = opt && opt->msgs_out;
     GINF_TRY(run_bp(c, P, iters_per_level, nli));
     GINF_TRY(run_icm_sync(c, P, icm_iters));
     c.ev(EV_ICM);
@@ -1105,6 +1113,7 @@ ginf_status ginf_hbp_level_state(ginf_workspace *wsp, const ginf_grid *grid, int
     GINF_TRY(prepare(c, P, num_levels, false, nullptr, nullptr));
     const Level &lt = P.lv[level];
     const float scale = (float)(1u << (2 * level));
+    c.keep_msgs = true;  // the targets are made of messages
     if (x_out) GINF_CK(launch_level_x(P.f, P.rec + lt.off, lt.W, lt.H, scale, x_out, c.r.stream));
     if (beliefs_out) {
         int64_t nli = 0;

@@ -115,13 +115,14 @@ inline int current_device() {
 
 // The dynamic shared memory a kernel may use: raised on a device, under a
 // lock and only ever upward, the first time a launch needs more than the
-// default 48 KB or than allowed so far.
+// default or than allowed so far.
 struct SmemLimit {
+    static constexpr size_t kDefaultSmem = 40 * 1024;  // the default 48 KB less static shared memory
     std::atomic<size_t> allowed[kMaxDevices];
     std::mutex lock;
     template <typename K>
     cudaError_t ensure(K kern, size_t bytes) {
-        if (bytes <= 48 * 1024) return cudaSuccess;
+        if (bytes <= kDefaultSmem) return cudaSuccess;
         std::atomic<size_t> &a = allowed[current_device()];
         if (bytes <= a.load(std::memory_order_acquire)) return cudaSuccess;
         std::lock_guard<std::mutex> g(lock);
@@ -160,6 +161,10 @@ struct SweepConfig {
 // Launch one half-sweep; returns the kernel launch error.
 cudaError_t launch_sweep(const RecordFormat &f, const SweepConfig &cfg, SweepParams p, cudaStream_t s,
                          int num_sms);
+// Labels only of one half-sweep (RD_OWN): the argmin of each updated node's
+// belief, no messages.  For the last half-sweep when nothing reads its
+// messages; the records keep those of the one before.
+cudaError_t launch_sweep_labels(const RecordFormat &f, const SweepParams &p, cudaStream_t s);
 // Launches of 64-byte-message kernels (L = 16, FP32) with at least this many
 // 16-node tiles store their messages with ordinary stores (see tile_finish).
 constexpr long kDirectStoreTiles = 16384;

@@ -172,7 +172,10 @@ extern "C" ginf_status ginf_decode_bp_noalloc(const ginf_grid *grid, int32_t num
             p.iter = it;
             p.read_mode = (it == 0 && fused) ? RD_ZERO : RD_OWN;
             p.write_labels = it >= num_iters - 2 ? 1 : 0;
-            if ((e = launch_sweep(f, cfg, p, s, ds.num_sms)) != cudaSuccess) return cuda_error(e, "half-sweep");
+            // The last half-sweep only gives labels.
+            e = it == num_iters - 1 && p.read_mode == RD_OWN ? launch_sweep_labels(f, p, s)
+                                                             : launch_sweep(f, cfg, p, s, ds.num_sms);
+            if (e != cudaSuccess) return cuda_error(e, "half-sweep");
         }
     }
     int st_host = 0;
