@@ -311,6 +311,8 @@ struct Prepared {
     int32_t *lab = nullptr;        // device labels (caller's or a copy)
     int32_t *lab2 = nullptr;       // second label buffer (ICM ping-pong)
     uint8_t *chg = nullptr;        // ICM change flags, two W*H byte maps (ping-pong)
+    uint32_t *boxes = nullptr;     // raster ICM's mailboxes
+    size_t box_bytes = 0;
     double *partials = nullptr;    // energy partials, status word follows
     int num_partials = 0;
     int *status = nullptr;
@@ -367,6 +369,8 @@ ginf_status prepare(Call &c, Prepared &P, int levels, bool want_lab2, const int3
     const size_t id_lab = (labels_dev == nullptr) ? a.add(lab_bytes) : 0;
     const size_t id_lab2 = want_lab2 ? a.add(lab_bytes) : 0;
     const size_t id_chg = want_lab2 ? a.add(2 * (size_t)W * H) : 0;
+    P.box_bytes = !bp && !want_lab2 ? 2 * sizeof(uint32_t) * (size_t)icm_raster_strips(H) * W : 0;
+    const size_t id_box = P.box_bytes ? a.add(P.box_bytes) : 0;
     const size_t id_part = a.add(sizeof(double) * (P.num_partials + 1) + 64);
     GINF_TRY(ws_reserve(c.ws, a.total()));
     unsigned char *base = c.ws->arena;
@@ -376,6 +380,7 @@ ginf_status prepare(Call &c, Prepared &P, int levels, bool want_lab2, const int3
     P.lab = labels_dev ? labels_dev : reinterpret_cast<int32_t *>(a.ptr(base, id_lab));
     P.lab2 = want_lab2 ? reinterpret_cast<int32_t *>(a.ptr(base, id_lab2)) : nullptr;
     P.chg = want_lab2 ? a.ptr(base, id_chg) : nullptr;
+    P.boxes = P.box_bytes ? reinterpret_cast<uint32_t *>(a.ptr(base, id_box)) : nullptr;
     P.partials = reinterpret_cast<double *>(a.ptr(base, id_part));
     P.status = reinterpret_cast<int *>(P.partials + P.num_partials);
     P.energy = P.partials + P.num_partials + 1;
@@ -656,6 +661,15 @@ ginf_status run_icm_sync(Call &c, Prepared &P, int iters) {
 ginf_status run_icm_async(Call &c, Prepared &P, int iters) {
     const int W = c.g->width, H = c.g->height;
     if (iters <= 0 || W < 3 || H < 3) return GINF_OK;
+    GINF_CK(cudaMemsetAsync(P.boxes, 0, P.box_bytes, c.r.stream));
+    bool done = false;
+    GINF_CK(launch_icm_raster(P.f, P.rec, W, H, P.Vt, P.lab, iters, P.boxes, P.status, c.r.stream, c.ws->num_sms,
+                              done));
+    if (done) {
+        ++c.launches;
+        return GINF_OK;
+    }
+    // More labels or rows than that kernel takes: one launch per diagonal.
     for (int it = 0; it < iters; ++it)
         for (int diag = 2; diag <= (W - 2) + (H - 2); ++diag) {
             GINF_CK(launch_icm_async_diag(P.f, P.rec, W, H, P.Vt, P.lab, diag, P.status, c.r.stream));

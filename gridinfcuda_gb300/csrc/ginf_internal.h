@@ -192,6 +192,13 @@ cudaError_t launch_icm_sync(const RecordFormat &f, const unsigned char *rec, int
                             int *status, cudaStream_t s);
 cudaError_t launch_icm_async_diag(const RecordFormat &f, const unsigned char *rec, int W, int H, const void *V,
                                   int32_t *labels, int diag, int *status, cudaStream_t s);
+// All iterations of raster-order ICM in one launch (icm_raster.cu).  boxes
+// holds 2 * icm_raster_strips(H) * W zeroed words.  done = false when the
+// label count or the grid's height is beyond it and nothing was launched.
+int icm_raster_strips(int H);
+cudaError_t launch_icm_raster(const RecordFormat &f, const unsigned char *rec, int W, int H, const void *V,
+                              int32_t *labels, int iters, uint32_t *boxes, int *status, cudaStream_t s, int num_sms,
+                              bool &done);
 // Energy with costs addressed as base + node*node_stride + label*label_stride
 // (elements of the compute type): records (rec_bytes/t_size, 1) or the
 // caller's label-planar array (1, W*H).  partials holds num_partials doubles.
