@@ -20,14 +20,20 @@
 // iteration t below.  All strips must be resident (cooperative launch); every
 // poll is bounded.
 //
-// Bound: the latency of a step -- a shuffle, two table rows from shared memory,
+// Bound: the latency of a step -- a shuffle, a table row from shared memory,
 // the additions, the argmin over eight lanes -- times the columns and
-// iterations, plus the strips' lags.  One launch per anti-diagonal, as before,
-// paid a launch for each: 640x480x32, five iterations, RASTER_MEASURED
+// iterations, plus the strips' lags (2.8 us each).  640x480x32 int32: 0.24 us a
+// step; five iterations 1.18 ms, against 23.0 ms with one launch per
+// anti-diagonal (5590 of them) and 1.98 ms with stores per step and the general
+// argmin (205 instructions a step on one warp, ncu).
 //
-// The sum's order, the lanes' partition of the labels and their combine are
-// icm_node's, so labels agree with the other ICM kernels whatever the costs.
+// The sum's order is the reference's and ties go to the lowest label.  Chunks
+// whose costs hold a NaN or a value near -infinity, and tables that do, take
+// icm_node's own partition and combine (raster_node_any), so that labels agree
+// with the other ICM kernels whatever the costs.
 #include <algorithm>
+
+#include <type_traits>
 
 #include "ginf_internal.h"
 #include "ptx.cuh"
@@ -52,7 +58,7 @@ template <typename T>
 struct Vec {
     static constexpr int E = 16 / sizeof(T);
     alignas(16) T v[E];
-    __device__ __forceinline__ void load(const T *p) {
+    __device__ __forceinline__ void load(const void *p) {
         *reinterpret_cast<uint4 *>(v) = *reinterpret_cast<const uint4 *>(p);
     }
     __device__ __forceinline__ void add(const Vec &o) {
@@ -60,6 +66,67 @@ struct Vec {
         for (int k = 0; k < E; ++k) v[k] += o.v[k];
     }
 };
+
+// Values above every cost, and below which a cost leaves the fast form: a sum
+// of five that are not below it is neither NaN nor -infinity.
+template <typename T>
+__device__ __forceinline__ T top_cost();
+template <>
+__device__ __forceinline__ float top_cost<float>() { return __int_as_float(0x7f800000); }
+template <>
+__device__ __forceinline__ double top_cost<double>() { return __longlong_as_double(0x7ff0000000000000ll); }
+template <>
+__device__ __forceinline__ int top_cost<int>() { return 0x7fffffff; }
+__device__ __forceinline__ bool odd_cost(float v) { return !(v > -1e37f); }
+__device__ __forceinline__ bool odd_cost(double v) { return !(v > -1e300); }
+__device__ __forceinline__ bool odd_cost(int) { return false; }
+
+// (value, label) of the smaller: the lower label of equal values.
+template <typename T>
+__device__ __forceinline__ void take_less(T &best, int &bl, T ob, int ol) {
+    const bool take = ob < best || (ob == best && ol < bl);
+    best = take ? ob : best;
+    bl = take ? ol : bl;
+}
+
+// One node's label by its eight lanes, as icm_node<T, 8> of aux_kernels.cu,
+// for any costs: the four table rows at the byte offsets fs, fe, fn, fw of Vs.
+template <typename T>
+__device__ int raster_node_any(const T *D, const unsigned char *Vs, int fs, int fe, int fn, int fw, int L, int g) {
+    constexpr int E = Vec<T>::E;
+    T best = T(0);
+    int bl = 0x7fffffff;
+    for (int l = g * E; l < L; l += 8 * E) {
+        Vec<T> c, w;
+        c.load(D + l);
+        const unsigned char *v = Vs + (size_t)l * sizeof(T);
+        w.load(v + fs);
+        c.add(w);
+        w.load(v + fe);
+        c.add(w);
+        w.load(v + fn);
+        c.add(w);
+        w.load(v + fw);
+        c.add(w);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            if (l + e < L && (bl == 0x7fffffff || c.v[e] < best)) {
+                best = c.v[e];
+                bl = l + e;
+            }
+        }
+    }
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) {
+        const T ob = __shfl_xor_sync(~0u, best, off);
+        const int ol = __shfl_xor_sync(~0u, bl, off);
+        if (ol != 0x7fffffff && (bl == 0x7fffffff || ob < best || (!(best < ob) && ol < bl))) {
+            best = ob;
+            bl = ol;
+        }
+    }
+    return bl;
+}
 
 // top / bot: mailboxes [strips][W] of each strip's first / last row, zeroed.
 // NQ: 16-byte label chunks per lane.
@@ -71,78 +138,93 @@ __global__ void __launch_bounds__(32)
     constexpr int E = Vec<T>::E;
     T *Vs = reinterpret_cast<T *>(raster_smem);  // Vs[f * Lp + l] = V(l, f)
     const int lane = threadIdx.x, r = lane >> 3, g = lane & 7;
+    bool odd_table = false;
     for (int l = lane; l < Lp; l += 32)
         for (int f0 = 0; f0 < L; f0 += 8) {
             T v[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) v[q] = l < L && f0 + q < L ? V[l + (size_t)L * (f0 + q)] : T(0);
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
+            for (int q = 0; q < 8; ++q) {
                 if (f0 + q < L) Vs[(f0 + q) * Lp + l] = v[q];
+                odd_table |= odd_cost(v[q]);
+            }
         }
+    odd_table = __any_sync(~0u, odd_table);
     __syncwarp();
     const int strip = blockIdx.x;
     const int y = 1 + kRows * strip + r;
-    const bool row = y <= H - 2;
+    const int cols = y <= H - 2 ? W - 2 : 0;  // of this lane's row
     const bool first = strip == 0, last = strip == (int)gridDim.x - 1;
     const size_t yw = (size_t)min(y, H - 2) * W;
-    const uint32_t *north = bot + (size_t)(first ? 0 : strip - 1) * W;
-    const uint32_t *south = top + (size_t)(last ? 0 : strip + 1) * W;
-    uint32_t *my_top = top + (size_t)strip * W, *my_bot = bot + (size_t)strip * W;
+    const int row_bytes = Lp * (int)sizeof(T);  // a table row
     // Where this lane's neighbour words come from: lanes 0-3 of a row hold the
     // south labels of a chunk's steps, lanes 4-7 the east ones; lanes 0-3 of
-    // the first row also the north ones.
+    // the first row also the north ones.  They are kept as the byte offsets of
+    // the labels' table rows.
     const bool south_box = g < kChunk && r == kRows - 1 && !last;
     const bool north_lane = r == 0 && g < kChunk;
     const bool north_box = north_lane && !first;
+    const bool out_top = north_lane && !first, out_bot = south_box;  // lanes that publish
     const int steps = (W - 2) + (kRows - 1);
+    // This lane's column of chunk 0, less one, and what it reads and writes there.
+    const int u0 = (g & (kChunk - 1)) - r;
+    const int32_t *east_or_south = lab + yw + 1 + u0 + (g >= kChunk ? 1 : W);
+    const int32_t *above = lab + yw + 1 + u0 - W;
+    const uint32_t *south = top + (size_t)(last ? 0 : strip + 1) * W + 1 + u0;
+    const uint32_t *north = bot + (size_t)(first ? 0 : strip - 1) * W + 1 + u0;
+    int32_t *mine = lab + yw + 1 + u0;
+    uint32_t *box = (r == 0 ? top : bot) + (size_t)strip * W + 1 + u0;
+    const unsigned char *costs = rec + (yw + 1 - r) * rec_bytes + g * 16;
     bool bad = false;
-    auto checked = [&](int f) {
+    auto offset = [&](int f) {  // of a label's table row
         if (f < 0 || f >= L) {
             bad = true;
-            return 0;
+            f = 0;
         }
-        return f;
+        return f * row_bytes;
     };
 
     for (int t = 0; t < iters; ++t) {
         __syncwarp();  // the previous iteration's labels, written by other lanes
         const uint32_t tag_s = (uint32_t)t & 0xffffu, tag_n = (uint32_t)(t + 1) & 0xffffu;
         const bool wait_s = south_box && t > 0;
-        int cur = row ? checked(__ldcg(lab + yw)) : 0;  // the west border's label
+        int cur = cols ? offset(__ldcg(lab + yw)) : 0;  // the west border's label
         uint32_t a = 0, b = 0, an = 0, bn = 0;          // neighbour words of this chunk and the next
         Vec<T> d[kChunk][NQ], dn[kChunk][NQ];
-        // Column of this lane's word and whether its step exists.
-        auto column = [&](int k) { return 1 + k * kChunk + (g & (kChunk - 1)) - r; };
-        auto exists = [&](int x) { return row && x >= 1 && x <= W - 2; };
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+#pragma unroll
+                for (int e = 0; e < E; ++e) d[j][q].v[e] = dn[j][q].v[e] = T(0);
+        // Words and costs of the chunk that starts k steps in.
         auto request = [&](int k, uint32_t &wa, uint32_t &wb, Vec<T>(&c)[kChunk][NQ]) {
-            const int x = column(k);
-            wa = wb = 0;
-            if (exists(x)) {
-                if (g >= kChunk) wa = (uint32_t)__ldcg(lab + yw + x + 1);
-                else if (wait_s) wa = ld_relaxed(south + x);
-                else wa = (uint32_t)__ldcg(lab + yw + W + x);
-                if (north_lane) wb = north_box ? ld_relaxed(north + x) : (uint32_t)__ldcg(lab + yw - W + x);
+            if ((unsigned)(u0 + k) < (unsigned)cols) {
+                wa = wait_s ? ld_relaxed(south + k) : (uint32_t)__ldcg(east_or_south + k);
+                if (north_lane) wb = north_box ? ld_relaxed(north + k) : (uint32_t)__ldcg(above + k);
             }
+            const unsigned char *p = costs + (ptrdiff_t)k * rec_bytes;
 #pragma unroll
             for (int j = 0; j < kChunk; ++j) {
-                const int xj = 1 + k * kChunk + j - r;
+                if ((unsigned)(k + j - r) < (unsigned)cols) {
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const int l = (g + 8 * q) * E;
-                    if (exists(xj) && l < L)
-                        c[j][q].load(reinterpret_cast<const T *>(rec + (yw + xj) * rec_bytes) + l);
+                    for (int q = 0; q < NQ; ++q)
+                        if ((g + 8 * q) * E < L) c[j][q].load(p + q * 128);
                 }
+                p += rec_bytes;
             }
         };
-        // Polls until this chunk's words carry their tags, then strips them.
-        auto arrive = [&](int k, uint32_t &wa, uint32_t &wb) {
-            const int x = column(k);
-            const bool ws = wait_s && exists(x), wn = north_box && exists(x);
+        // Polls until this chunk's words carry their tags, then makes them
+        // offsets; the costs have arrived too and are looked over.
+        bool slow = odd_table;
+        auto arrive = [&](int k, uint32_t &wa, uint32_t &wb, const Vec<T>(&c)[kChunk][NQ]) {
+            const bool in = (unsigned)(u0 + k) < (unsigned)cols;
+            const bool ws = wait_s && in, wn = north_box && in;
             uint64_t t0 = 0;
             for (uint32_t n = 1; !__all_sync(~0u, (!ws || wa >> 16 == tag_s) && (!wn || wb >> 16 == tag_n)); ++n) {
-                if (ws && wa >> 16 != tag_s) wa = ld_relaxed(south + x);
-                if (wn && wb >> 16 != tag_n) wb = ld_relaxed(north + x);
+                if (ws && wa >> 16 != tag_s) wa = ld_relaxed(south + k);
+                if (wn && wb >> 16 != tag_n) wb = ld_relaxed(north + k);
                 if ((n & 255u) == 0) {
                     const uint64_t now = __shfl_sync(~0u, global_timer_ns(), 0);
                     if (t0 == 0) t0 = now;
@@ -154,72 +236,100 @@ __global__ void __launch_bounds__(32)
             }
             if (ws) wa &= 0xffffu;
             if (wn) wb &= 0xffffu;
-            if (exists(x)) {
-                wa = (uint32_t)checked((int)wa);
-                if (north_lane) wb = (uint32_t)checked((int)wb);
+            if (in) {
+                wa = (uint32_t)offset((int)wa);
+                if (north_lane) wb = (uint32_t)offset((int)wb);
+            } else {
+                wa = wb = 0;
+            }
+            if constexpr (sizeof(T) == 8 || std::is_same<T, float>::value) {
+                bool odd = odd_table;
+#pragma unroll
+                for (int j = 0; j < kChunk; ++j)
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q)
+#pragma unroll
+                        for (int e = 0; e < E; ++e) odd |= odd_cost(c[j][q].v[e]);
+                slow = __any_sync(~0u, odd);
             }
             return true;
         };
         request(0, a, b, d);
-        if (!arrive(0, a, b)) return;
-        for (int k = 0; k * kChunk < steps; ++k) {
-            const bool more = (k + 1) * kChunk < steps;
-            if (more) request(k + 1, an, bn, dn);
+        if (!arrive(0, a, b, d)) return;
+        for (int k = 0; k < steps; k += kChunk) {
+            const bool more = k + kChunk < steps;
+            if (more) request(k + kChunk, an, bn, dn);
+            int found = 0;  // this lane's step's label
 #pragma unroll
             for (int j = 0; j < kChunk; ++j) {
-                const int x = 1 + k * kChunk + j - r;
                 const int fs = __shfl_sync(~0u, (int)a, (lane & ~7) + j);
                 const int fe = __shfl_sync(~0u, (int)a, (lane & ~7) + kChunk + j);
                 const int f0 = __shfl_sync(~0u, (int)b, j);
                 const int up = __shfl_up_sync(~0u, cur, 8);
                 const int fn = r == 0 ? f0 : up;
-                const bool act = exists(x);
-                T best = T(0);
-                int bl = 0x7fffffff;
-                if (act) {
+                const bool act = (unsigned)(k + j - r) < (unsigned)cols;
+                int bl;
+                if (slow) {
+                    // Inactive rows read some record of the grid.
+                    const size_t node = yw + (act ? 1 + k + j - r : 1);
+                    bl = raster_node_any(reinterpret_cast<const T *>(rec + node * rec_bytes), raster_smem, fs, fe, fn,
+                                         cur, L, g);
+                } else {
+                    T best = top_cost<T>();
+                    bl = 0x7fffffff;
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
                         const int l = (g + 8 * q) * E;
-                        if (l < L) {
-                            Vec<T> c = d[j][q], vs, ve, vn, vw;
-                            vs.load(Vs + fs * Lp + l);
-                            ve.load(Vs + fe * Lp + l);
-                            vn.load(Vs + fn * Lp + l);
-                            vw.load(Vs + cur * Lp + l);
-                            c.add(vs);
-                            c.add(ve);
-                            c.add(vn);
-                            c.add(vw);
+                        const unsigned char *v = raster_smem + l * (int)sizeof(T);
+                        if (NQ == 1 || l < L) {
+                            Vec<T> c = d[j][q], w;
+                            w.load(v + fs);
+                            c.add(w);
+                            w.load(v + fe);
+                            c.add(w);
+                            w.load(v + fn);
+                            c.add(w);
+                            w.load(v + cur);
+                            c.add(w);
 #pragma unroll
-                            for (int e = 0; e < E; ++e) {
-                                if (l + e < L && (bl == 0x7fffffff || c.v[e] < best)) {
-                                    best = c.v[e];
-                                    bl = l + e;
+                            for (int e = 0; e < E; ++e)
+                                if (l + e >= L) c.v[e] = top_cost<T>();
+                            // The first minimum of the chunk, in pairs.
+                            int m[E];
+#pragma unroll
+                            for (int e = 0; e < E; ++e) m[e] = l + e;
+#pragma unroll
+                            for (int w2 = 1; w2 < E; w2 *= 2)
+#pragma unroll
+                                for (int e = 0; e + w2 < E; e += 2 * w2) {
+                                    const bool right = c.v[e + w2] < c.v[e];
+                                    c.v[e] = right ? c.v[e + w2] : c.v[e];
+                                    m[e] = right ? m[e + w2] : m[e];
                                 }
+                            if (q == 0) {
+                                best = c.v[0];
+                                bl = m[0];
+                            } else if (c.v[0] < best) {
+                                best = c.v[0];
+                                bl = m[0];
                             }
                         }
                     }
-                }
 #pragma unroll
-                for (int off = 1; off < 8; off <<= 1) {
-                    const T ob = __shfl_xor_sync(~0u, best, off);
-                    const int ol = __shfl_xor_sync(~0u, bl, off);
-                    if (ol != 0x7fffffff && (bl == 0x7fffffff || ob < best || (!(best < ob) && ol < bl))) {
-                        best = ob;
-                        bl = ol;
-                    }
+                    for (int off = 1; off < 8; off <<= 1)
+                        take_less(best, bl, __shfl_xor_sync(~0u, best, off), __shfl_xor_sync(~0u, bl, off));
                 }
-                if (act) {
-                    cur = bl;
-                    if (g == 0) {
-                        lab[yw + x] = bl;
-                        if (r == 0 && !first) st_relaxed(my_top + x, tag_n << 16 | (uint32_t)bl);
-                        if (r == kRows - 1 && !last) st_relaxed(my_bot + x, tag_n << 16 | (uint32_t)bl);
-                    }
-                }
+                if (act) cur = bl * row_bytes;
+                if ((g & (kChunk - 1)) == j) found = bl;
+            }
+            // The chunk's labels: into the labelling and, for the strips' outer
+            // rows, the mailboxes.
+            if (g < kChunk && (unsigned)(u0 + k) < (unsigned)cols) {
+                mine[k] = found;
+                if (out_top || out_bot) st_relaxed(box + k, tag_n << 16 | (uint32_t)found);
             }
             if (more) {
-                if (!arrive(k + 1, an, bn)) return;
+                if (!arrive(k + kChunk, an, bn, dn)) return;
                 a = an;
                 b = bn;
 #pragma unroll
@@ -240,7 +350,7 @@ cudaError_t launch_raster_t(const RecordFormat &f, const unsigned char *rec, int
     static OccupancyMemo memo;
     auto kern = k_icm_raster<T, NQ>;
     const int strips = icm_raster_strips(H);
-    const size_t smem = (size_t)f.L * f.Lp * sizeof(T);
+    const size_t smem = (size_t)f.L * f.Lp * sizeof(T) + 128;  // lanes beyond L read past the last row
     cudaError_t e = limit.ensure(kern, smem);
     if (e != cudaSuccess) return e;
     int occ = 0;

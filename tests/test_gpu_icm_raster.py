@@ -48,3 +48,22 @@ def test_bad_labels_are_reported(ginf):
         with pytest.raises(ginf.GinfError) as e:
             ginf.decode_icm(P.D, P.V, P.model, init, 2, asynchronous=True)
         assert e.value.status == ginf.ERR_INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("where", ["cost inf", "cost -inf", "table inf", "table -inf", "cost -0"])
+def test_extreme_costs(ginf, orc, where):
+    """Infinite costs and table entries (no sum is NaN) and signed zeros: -inf
+    leaves the kernel's fast form for the chunks that hold it."""
+    for L in (7, 32, 70):
+        P = synth.random_problem(37, 21, L, L)
+        D, V = np.round(P.D).astype(np.float32), P.V.copy()
+        value = np.float32({"inf": np.inf, "-inf": -np.inf, "-0": -0.0}[where.split()[1]])
+        if where.startswith("cost"):
+            D[::3, 2::5, 1::4] = value
+            if value == np.inf:
+                D[:, 4, 6] = value  # a node with no finite label
+        else:
+            V[3 + L * 2] = value
+        init = np.random.RandomState(L).randint(0, L, (21, 37)).astype(np.int32)
+        want = orc.icm(D, V, init, 3, asynchronous=True)
+        assert np.array_equal(ginf.decode_icm(D, V, synth.EXPLICIT, init, 3, asynchronous=True), want), L
