@@ -1,6 +1,6 @@
 // Explicit instantiation of the half-sweep launchers for T = float, M = float
 // (one translation unit per type pair so the build compiles them in parallel).
-#include "sweep_impl.cuh"
+#include "sweep_warp.cuh"
 
 namespace ginf_gpu {
 template cudaError_t launch_sweep_tm<float, float>(const RecordFormat &, const SweepConfig &, const SweepParams &,

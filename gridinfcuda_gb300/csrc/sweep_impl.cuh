@@ -1126,10 +1126,12 @@ struct LaunchCache {
 
 // Launches one half-sweep kernel over tiles of `nodes` nodes, NW warps per
 // block, one block per resident slot of every SM (fewer if there are fewer
-// tiles); extra_smem bytes follow the nodes' slots in shared memory.
+// tiles, block_tiles of which a block takes at a time); extra_smem bytes
+// follow the nodes' slots in shared memory.
 template <typename K>
 cudaError_t launch_tiles(K kern, LaunchCache &lc_state, int NW, int nodes, const SweepParams &params,
-                         uint32_t slot_bytes, cudaStream_t s, int num_sms, size_t extra_smem = 0) {
+                         uint32_t slot_bytes, cudaStream_t s, int num_sms, size_t extra_smem = 0,
+                         int block_tiles = 1) {
     // The tiling follows the variant actually launched.
     SweepParams p = params;
     const int n1 = p.W >= 3 ? (p.W - 3) / 2 + 1 : 0;
@@ -1144,7 +1146,8 @@ cudaError_t launch_tiles(K kern, LaunchCache &lc_state, int NW, int nodes, const
     if (e != cudaSuccess) return e;
     if (occ < 1) return cudaErrorInvalidConfiguration;
     int grid = occ * num_sms;
-    if (grid > p.num_tiles) grid = p.num_tiles;
+    const int need = (p.num_tiles + block_tiles - 1) / block_tiles;
+    if (grid > need) grid = need;
     // Programmatic stream serialisation: this launch may begin while the
     // previous kernel of the stream finishes (the kernel waits for it before
     // reading records).
@@ -1180,6 +1183,11 @@ cudaError_t launch_split(const SweepParams &params, uint32_t slot_bytes, cudaStr
     return launch_tiles(sweep_kernel_split<LMAX, LMIN, NW, QW>, cache, NW, NW / 2 * 8, params, slot_bytes, s,
                         num_sms);
 }
+
+// Truncated-linear / Potts half-sweeps of few labels (sweep_warp.cuh).
+constexpr int kWarpTileLabels = 32;
+template <typename T, int LM, int LO>
+cudaError_t launch_warp_tiles(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms);
 
 // Min-convolutions with 4-byte arithmetic (sweep_table.cuh).
 template <typename T, typename M>
@@ -1251,22 +1259,28 @@ cudaError_t launch_variant(const RecordFormat &f, const SweepConfig &cfg, const 
             return launch_general<T, M, 128>(f, p, s, num_sms);
         }
     }
-    if constexpr (kPow2) {
-        if (exact) {
-            if constexpr (kF32) {
-                if (cfg.nt == 8) return launch_one<T, M, LM, LM, 1, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
-                if (cfg.nt == 32) return launch_one<T, M, LM, LM, 4, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
-                if constexpr (LM * sizeof(M) == 64) {
-                    const int n1 = p.W >= 3 ? (p.W - 3) / 2 + 1 : 0;
-                    const long tiles = p.H >= 3 ? (long)(p.H - 2) * ((n1 + 15) / 16) : 0;
-                    if (tiles >= kDirectStoreTiles)
-                        return launch_one<T, M, LM, LM, 2, KIND_LINEAR, true>(p, f.slot_bytes, s, num_sms);
+    if constexpr (sizeof(T) == 4 && std::is_same<T, M>::value && LM <= kWarpTileLabels) {
+        if constexpr (kPow2)
+            if (exact) return launch_warp_tiles<T, LM, LM>(f, p, s, num_sms);
+        return launch_warp_tiles<T, LM, LO>(f, p, s, num_sms);
+    } else {
+        if constexpr (kPow2) {
+            if (exact) {
+                if constexpr (kF32) {
+                    if (cfg.nt == 8) return launch_one<T, M, LM, LM, 1, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
+                    if (cfg.nt == 32) return launch_one<T, M, LM, LM, 4, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
+                    if constexpr (LM * sizeof(M) == 64) {
+                        const int n1 = p.W >= 3 ? (p.W - 3) / 2 + 1 : 0;
+                        const long tiles = p.H >= 3 ? (long)(p.H - 2) * ((n1 + 15) / 16) : 0;
+                        if (tiles >= kDirectStoreTiles)
+                            return launch_one<T, M, LM, LM, 2, KIND_LINEAR, true>(p, f.slot_bytes, s, num_sms);
+                    }
                 }
+                return launch_one<T, M, LM, LM, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
             }
-            return launch_one<T, M, LM, LM, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
         }
+        return launch_one<T, M, LM, LO, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
     }
-    return launch_one<T, M, LM, LO, 2, KIND_LINEAR>(p, f.slot_bytes, s, num_sms);
 }
 
 // Dispatch on the label count for one (T, M) pair.  A kernel compiled for the
