@@ -1,8 +1,10 @@
-// batch.cu -- many independent grids solved together: one persistent,
-// cooperative launch walks a work list of (grid, tile) entries for each
-// half-sweep, with a bounded grid barrier between half-sweeps; the whole
-// solve (layout transforms, initialisation, the persistent launches) is
-// captured once into a CUDA graph and replayed.  The tile shape and the
+// batch.cu -- many independent grids solved together: one persistent launch
+// per label bucket walks a work list of (grid, tile) entries, for one
+// half-sweep (the buckets then are parallel branches, each launch starting as
+// the one before it drains) or cooperatively for several with a bounded grid
+// barrier between them; the whole solve (layout transforms, initialisation,
+// the persistent launches, the labels of the last half-sweep) is captured
+// once into a CUDA graph and replayed.  The tile shape and the
 // number of half-sweeps per persistent launch come from an autotuner that
 // times the candidates on the batch itself and caches the winner per mix of
 // (grid-size class, label count) buckets in a JSON file.
@@ -22,7 +24,8 @@
 #include <vector>
 
 #include "ginf_gb300.h"
-#include "sweep_impl.cuh"
+#include "sweep_labels.cuh"
+#include "sweep_warp.cuh"
 
 namespace ginf_gpu {
 
@@ -92,7 +95,7 @@ __device__ __forceinline__ SweepParams batch_params(const BatchLaunch &b, const 
 // binary search over the tile bases, kept in shared memory).  Between
 // half-sweeps each block waits for its own bulk stores, fences them against
 // the next half-sweep's bulk loads and meets the others at the grid barrier.
-template <int NW, int LM, int LMIN, bool DIRECT = false>
+template <int NW, int LM, int LMIN>
 __global__ void __launch_bounds__(NW * 32) batch_kernel(const BatchLaunch b) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
@@ -106,6 +109,9 @@ __global__ void __launch_bounds__(NW * 32) batch_kernel(const BatchLaunch b) {
     __syncthreads();
     const int *bases = b.bases_in_smem ? bases_s : nullptr;
     uint32_t parity = 0;
+    // A launch of one half-sweep starts while the one before it drains.
+    launch_dependents();
+    grid_dependency_wait();
     for (int it = b.it_begin; it < b.it_end; ++it) {
         int t = blockIdx.x;
         SweepParams p{};
@@ -117,7 +123,7 @@ __global__ void __launch_bounds__(NW * 32) batch_kernel(const BatchLaunch b) {
             tile_load<NW>(p, t - base, smem, &full_bar);
         }
         for (; t < b.total_tiles; t += gridDim.x) {
-            if (!tile_finish<float, float, LM, LMIN, NW, KIND_LINEAR, DIRECT>(
+            if (!tile_finish<float, float, LM, LMIN, NW, KIND_LINEAR>(
                     p, table_consts<float, KIND_LINEAR>(p.V, LMIN == LM ? LM : p.L), t - base, smem, &full_bar, parity))
                 return;
             const int tn = t + gridDim.x;
@@ -134,6 +140,57 @@ __global__ void __launch_bounds__(NW * 32) batch_kernel(const BatchLaunch b) {
             if (!grid_barrier(b.barrier, gridDim.x, b.status)) return;
             fence_proxy_async_global();
         }
+    }
+}
+
+// The same for label counts of the warp half-sweep (sweep_warp.cuh): each warp
+// takes tiles of eight nodes on its own.
+template <int LM, int LMIN>
+__global__ void __launch_bounds__(kWarpTileWarps * 32) batch_kernel_warp(const BatchLaunch b) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    int *bases_s = reinterpret_cast<int *>(smem + b.tile_smem);
+    if (b.bases_in_smem)
+        for (int i = threadIdx.x; i < b.count; i += blockDim.x) bases_s[i] = b.items[i].tile_base;
+    __syncthreads();
+    const int *bases = b.bases_in_smem ? bases_s : nullptr;
+    const int warp = threadIdx.x >> 5;
+    launch_dependents();
+    grid_dependency_wait();
+    for (int it = b.it_begin; it < b.it_end; ++it) {
+        for (int t = blockIdx.x * kWarpTileWarps + warp; t < b.total_tiles; t += gridDim.x * kWarpTileWarps) {
+            const BatchItem &g = b.items[batch_item_of(b, bases, t)];
+            const SweepParams p = batch_params(b, g, it);
+            warp_tile<float, LM, LMIN>(p, table_consts<float, KIND_LINEAR>(p.V, LMIN == LM ? LM : p.L),
+                                       t - g.tile_base, smem + (size_t)warp * 8 * p.slot_bytes);
+        }
+        if (it + 1 < b.it_end && !grid_barrier(b.barrier, gridDim.x, b.status)) return;
+    }
+}
+
+// The last half-sweep, labels only (sweep_labels.cu): a warp per eight nodes,
+// `wpt` of them per work-list tile.
+constexpr int kBatchLabelWarps = 8;
+__global__ void __launch_bounds__(kBatchLabelWarps * 32) batch_labels(const BatchLaunch b, int wpt) {
+    launch_dependents();
+    grid_dependency_wait();
+    const int lane = threadIdx.x & 31;
+    const long warps = (long)gridDim.x * kBatchLabelWarps, total = (long)b.total_tiles * wpt;
+    for (long w = (long)blockIdx.x * kBatchLabelWarps + (threadIdx.x >> 5); w < total; w += warps) {
+        const int t = (int)(w / wpt);
+        const BatchItem &g = b.items[batch_item_of(b, nullptr, t)];
+        const SweepParams p = batch_params(b, g, b.it_begin);
+        const int lt = t - g.tile_base;
+        const int y = 1 + lt / p.tiles_per_row;
+        const int node = ((lt % p.tiles_per_row) * wpt + (int)(w % wpt)) * 8 + lane / 4;
+        const int x = ((y + p.iter) & 1) + 1 + 2 * node;
+        const bool act = x <= p.W - 2;
+        float best = pos_inf<float>();
+        int label = 0x7fffffff;
+        if (act)
+            label_part<float, float>(p.rec + ((size_t)y * p.W + x) * p.rec_bytes, p, zero_mask(p, x, y), 0, p.L,
+                                     lane & 3, best, label);
+        combine4(best, label);
+        if (act && (lane & 3) == 0) p.labels[(size_t)y * p.W + x] = label;
     }
 }
 
@@ -276,6 +333,8 @@ struct ginf_batch {
     TuneChoice choice;
     int launches_per_run = 0;
     cudaStream_t cap_stream = nullptr;
+    std::vector<cudaStream_t> branches;  // one per group but the first, for the capture
+    cudaEvent_t fork = nullptr, join = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -315,12 +374,16 @@ void make_groups(ginf_batch *b) {
         }
 }
 
+// Nodes per work-list tile: the warp half-sweep's eight, else the plan's.
+int group_tile_nodes(const BatchGroup &grp, int tile_nodes) { return grp.lm <= kWarpTileLabels ? 8 : tile_nodes; }
+
 // Items for a given tile size (8 * NW nodes), in group order, with tile
 // bases counted from each group's start; copied to the device.
 std::vector<BatchItem> make_items(ginf_batch *b, int tile_nodes) {
     std::vector<BatchItem> items(b->count);
     for (auto &grp : b->groups) {
         grp.total_tiles = 0;
+        const int nt = group_tile_nodes(grp, tile_nodes);
         for (int k = grp.first; k < grp.first + grp.count; ++k) {
             const int i = b->order[k];
             const ginf_grid &g = b->grids[i];
@@ -338,7 +401,7 @@ std::vector<BatchItem> make_items(ginf_batch *b, int tile_nodes) {
             it.m_bytes = f.m_bytes;
             it.slot_bytes = f.slot_bytes;
             const int n1 = g.width >= 3 ? (g.width - 3) / 2 + 1 : 0;
-            it.tiles_per_row = (n1 + tile_nodes - 1) / tile_nodes;
+            it.tiles_per_row = (n1 + nt - 1) / nt;
             it.num_tiles = (g.width >= 3 && g.height >= 3) ? (g.height - 2) * it.tiles_per_row : 0;
             it.tile_base = grp.total_tiles;
             grp.total_tiles += it.num_tiles;
@@ -347,44 +410,61 @@ std::vector<BatchItem> make_items(ginf_batch *b, int tile_nodes) {
     return items;
 }
 
-template <int NW, int LM, int LMIN, bool DIRECT = false>
-cudaError_t launch_batch(BatchLaunch bl, uint32_t max_slot, int num_sms, cudaStream_t s) {
-    auto kern = batch_kernel<NW, LM, LMIN, DIRECT>;
-    bl.tile_smem = (uint32_t)(((size_t)NW * 8 * max_slot + 15) / 16 * 16);
+// Launches one batch kernel: cooperatively when it runs several half-sweeps
+// (its blocks meet at a grid barrier), else so that it may start while the
+// launch before it drains.
+template <typename K>
+cudaError_t launch_batch(K kern, LaunchCache &cache, BatchLaunch bl, int warps, size_t slots, uint32_t max_slot,
+                         int block_tiles, int num_sms, cudaStream_t s) {
+    bl.tile_smem = (uint32_t)((slots * max_slot + 15) / 16 * 16);
     const size_t bases_bytes = sizeof(int) * (size_t)bl.count;
     bl.bases_in_smem = bases_bytes <= 16 * 1024 ? 1 : 0;
     const size_t smem = bl.tile_smem + (bl.bases_in_smem ? bases_bytes : 0);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cache.smem.ensure(kern, smem);
     if (e != cudaSuccess) return e;
     int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, NW * 32, smem);
+    e = cache.occ.blocks(kern, warps * 32, smem, occ);
     if (e != cudaSuccess) return e;
     if (occ < 1) return cudaErrorInvalidConfiguration;
+    const bool one = bl.it_end - bl.it_begin == 1;
+    const int need = std::max(1, (bl.total_tiles + block_tiles - 1) / block_tiles);
     int grid = occ * num_sms;
-    if (grid > bl.total_tiles && bl.it_end - bl.it_begin == 1) grid = std::max(1, bl.total_tiles);
+    if (grid > need && one) grid = need;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NW * 32);
+    cfg.blockDim = dim3(warps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
+    if (one) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    }
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, bl);
 }
 
+template <int NW, int LM, int LMIN>
+cudaError_t launch_batch_tiles(const BatchLaunch &bl, uint32_t max_slot, int num_sms, cudaStream_t s) {
+    static LaunchCache cache;
+    return launch_batch(batch_kernel<NW, LM, LMIN>, cache, bl, NW, NW * 8, max_slot, 1, num_sms, s);
+}
+
 template <int LM, int LMIN>
 cudaError_t launch_batch_nw(int tile_nodes, const BatchLaunch &bl, uint32_t max_slot, int num_sms, cudaStream_t s) {
-    if constexpr (LM == 16 && LMIN == LM) {
-        // 64-byte messages: ordinary stores on large groups (see tile_finish).
-        if (tile_nodes == 16 && bl.total_tiles >= kDirectStoreTiles)
-            return launch_batch<2, LM, LMIN, true>(bl, max_slot, num_sms, s);
+    if constexpr (LM <= kWarpTileLabels) {
+        static LaunchCache cache;
+        return launch_batch(batch_kernel_warp<LM, LMIN>, cache, bl, kWarpTileWarps, kWarpTileWarps * 8, max_slot,
+                            kWarpTileWarps, num_sms, s);
+    } else {
+        if (tile_nodes == 8) return launch_batch_tiles<1, LM, LMIN>(bl, max_slot, num_sms, s);
+        if (tile_nodes == 32) return launch_batch_tiles<4, LM, LMIN>(bl, max_slot, num_sms, s);
+        return launch_batch_tiles<2, LM, LMIN>(bl, max_slot, num_sms, s);
     }
-    if (tile_nodes == 8) return launch_batch<1, LM, LMIN>(bl, max_slot, num_sms, s);
-    if (tile_nodes == 32) return launch_batch<4, LM, LMIN>(bl, max_slot, num_sms, s);
-    return launch_batch<2, LM, LMIN>(bl, max_slot, num_sms, s);
 }
 
 cudaError_t launch_group(const BatchGroup &grp, int tile_nodes, const BatchLaunch &bl, int num_sms, cudaStream_t s) {
@@ -405,45 +485,81 @@ cudaError_t launch_group(const BatchGroup &grp, int tile_nodes, const BatchLaunc
     }
 }
 
+// The labels-only half-sweep bl.it_begin of a group.
+cudaError_t launch_group_labels(const BatchGroup &grp, int tile_nodes, const BatchLaunch &bl, int num_sms,
+                                cudaStream_t s) {
+    const int wpt = group_tile_nodes(grp, tile_nodes) / 8;
+    const long blocks = ((long)bl.total_tiles * wpt + kBatchLabelWarps - 1) / kBatchLabelWarps;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min<long>(blocks, (long)num_sms * 8));
+    cfg.blockDim = dim3(kBatchLabelWarps * 32);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, batch_labels, bl, wpt);
+}
+
 // Records the whole batch solve on stream s: layout transforms, start-up
 // initialisation, counters, then per label group its persistent launches.
 ginf_status record_solve(ginf_batch *b, const TuneChoice &c, cudaStream_t s, int &launches) {
     launches = 0;
     make_items(b, c.tile_nodes);  // the device copy was made before the capture
     const bool fused = b->iters >= 2;
-    for (int i = 0; i < b->count; ++i) {
-        const ginf_grid &g = b->grids[i];
-        GINF_BCK(launch_costs_to_records(b->fmt[i], CT_F32, g.data_costs, g.width, g.height, b->rec[i], s));
-        ++launches;
-        if (!fused) {
-            GINF_BCK(launch_init_messages(b->fmt[i], b->rec[i], g.width, g.height, nullptr, 0, 0, s));
-            GINF_BCK(launch_fill_interior(b->labels[i], g.width, g.height, 0, s));
-            launches += 2;
-        }
-    }
     GINF_BCK(cudaMemsetAsync(b->barrier, 0, 2 * sizeof(unsigned int), s));
     GINF_BCK(cudaMemsetAsync(b->status, 0, sizeof(int), s));
-    if (b->iters == 0) return GINF_OK;
     const int spl = c.sweeps_per_launch <= 0 ? b->iters : std::min(c.sweeps_per_launch, b->iters);
+    // With one half-sweep per launch the groups are independent branches of the
+    // graph: one group's blocks fill the SMs that another's last wave leaves
+    // idle (twelve grids of four label counts, 30 half-sweeps: 13.78 -> 13.04 ms;
+    // five small ones 0.88 -> 0.71 ms).  Several half-sweeps per launch need the whole device to themselves
+    // (and share the barrier), so those launches stay in line.
+    const bool branch = spl <= 1 && b->groups.size() > 1;
+    if (branch) GINF_BCK(cudaEventRecord(b->fork, s));
+    size_t gi = 0;
     for (const BatchGroup &grp : b->groups) {
-        if (grp.total_tiles == 0) continue;
-        for (int it0 = 0; it0 < b->iters; it0 += spl) {
-            BatchLaunch bl{};
-            bl.items = b->items_dev + grp.first;
-            bl.count = grp.count;
-            bl.total_tiles = grp.total_tiles;
-            bl.it_begin = it0;
-            bl.it_end = std::min(b->iters, it0 + spl);
-            bl.iters = b->iters;
-            bl.first_mode = fused ? RD_ZERO : RD_OWN;
-            bl.barrier = b->barrier;
-            bl.status = b->status;
-            const cudaError_t e = launch_group(grp, c.tile_nodes, bl, b->num_sms, s);
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                return bfail(GINF_ERR_CUDA, std::string("persistent batch launch: ") + cudaGetErrorString(e));
-            }
+        const cudaStream_t gs = branch && gi > 0 ? b->branches[gi - 1] : s;
+        ++gi;
+        if (gs != s) GINF_BCK(cudaStreamWaitEvent(gs, b->fork, 0));
+        for (int k = grp.first; k < grp.first + grp.count; ++k) {
+            const int i = b->order[k];
+            const ginf_grid &g = b->grids[i];
+            GINF_BCK(launch_costs_to_records(b->fmt[i], CT_F32, g.data_costs, g.width, g.height, b->rec[i], gs));
             ++launches;
+            if (!fused) {
+                GINF_BCK(launch_init_messages(b->fmt[i], b->rec[i], g.width, g.height, nullptr, 0, 0, gs));
+                GINF_BCK(launch_fill_interior(b->labels[i], g.width, g.height, 0, gs));
+                launches += 2;
+            }
+        }
+        if (grp.total_tiles > 0) {
+            // The last half-sweep only gives labels; it is a launch of its own.
+            const int full = b->iters > 1 ? b->iters - 1 : b->iters;
+            for (int it0 = 0; it0 < b->iters; it0 = it0 < full ? std::min(full, it0 + std::max(spl, 1)) : b->iters) {
+                BatchLaunch bl{};
+                bl.items = b->items_dev + grp.first;
+                bl.count = grp.count;
+                bl.total_tiles = grp.total_tiles;
+                bl.it_begin = it0;
+                bl.it_end = it0 < full ? std::min(full, it0 + spl) : b->iters;
+                bl.iters = b->iters;
+                bl.first_mode = fused ? RD_ZERO : RD_OWN;
+                bl.barrier = b->barrier;
+                bl.status = b->status;
+                const cudaError_t e = it0 < full ? launch_group(grp, c.tile_nodes, bl, b->num_sms, gs)
+                                                 : launch_group_labels(grp, c.tile_nodes, bl, b->num_sms, gs);
+                if (e != cudaSuccess) {
+                    cudaGetLastError();
+                    return bfail(GINF_ERR_CUDA, std::string("batch half-sweep launch: ") + cudaGetErrorString(e));
+                }
+                ++launches;
+            }
+        }
+        if (gs != s) {
+            GINF_BCK(cudaEventRecord(b->join, gs));
+            GINF_BCK(cudaStreamWaitEvent(s, b->join, 0));
         }
     }
     return GINF_OK;
@@ -605,6 +721,19 @@ ginf_status ginf_batch_create(ginf_batch **out, const ginf_grid *grids, int32_t 
         cudaGetLastError();
         st = bfail(GINF_ERR_CUDA, "batch set-up failed");
     }
+    if (st == GINF_OK && b->groups.size() > 1) {
+        bool ok = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess &&
+                  cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) == cudaSuccess;
+        for (size_t g = 1; ok && g < b->groups.size(); ++g) {
+            cudaStream_t br = nullptr;
+            ok = cudaStreamCreateWithFlags(&br, cudaStreamNonBlocking) == cudaSuccess;
+            if (ok) b->branches.push_back(br);
+        }
+        if (!ok) {
+            cudaGetLastError();
+            st = bfail(GINF_ERR_CUDA, "batch set-up failed");
+        }
+    }
     if (st == GINF_OK) {
         TuneChoice c;
         const std::string sig = signature(b->grids, iters);
@@ -756,6 +885,9 @@ ginf_status ginf_batch_destroy(ginf_batch *b) {
     drop_graph(b);
     if (b->arena) cudaFree(b->arena);
     if (b->status_host) cudaFreeHost(b->status_host);
+    for (cudaStream_t br : b->branches) cudaStreamDestroy(br);
+    if (b->fork) cudaEventDestroy(b->fork);
+    if (b->join) cudaEventDestroy(b->join);
     if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);

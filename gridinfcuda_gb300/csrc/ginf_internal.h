@@ -165,7 +165,7 @@ cudaError_t launch_sweep(const RecordFormat &f, const SweepConfig &cfg, SweepPar
 // belief, no messages.  For the last half-sweep when nothing reads its
 // messages; the records keep those of the one before.
 cudaError_t launch_sweep_labels(const RecordFormat &f, const SweepParams &p, cudaStream_t s);
-// Launches of 64-byte-message kernels (L = 16, FP32) with at least this many
+// Launches of 64-byte-message kernels (L = 32, FP16) with at least this many
 // 16-node tiles store their messages with ordinary stores (see tile_finish).
 constexpr long kDirectStoreTiles = 16384;
 
