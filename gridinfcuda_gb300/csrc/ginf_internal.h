@@ -231,6 +231,9 @@ struct AlphaBetaParams {
     int *status;
 };
 cudaError_t launch_alpha_beta(const AlphaBetaParams &p, cudaStream_t s);
+// The same on one thread-block cluster (graphcut_cluster.cu); done = false when
+// the grid does not fit and nothing was launched.
+cudaError_t launch_alpha_beta_cluster(const AlphaBetaParams &p, cudaStream_t s, bool &done);
 
 // Sets the message ginf_last_error() returns on this host thread.
 void set_last_error(const char *msg);

@@ -445,6 +445,10 @@ __global__ void __launch_bounds__(kThreadsAB, 1) k_alpha_beta(const AlphaBetaPar
 }  // namespace
 
 cudaError_t launch_alpha_beta(const AlphaBetaParams &p, cudaStream_t s) {
+    // Grids whose state fits a cluster's shared memory.
+    bool done = false;
+    const cudaError_t e = launch_alpha_beta_cluster(p, s, done);
+    if (done || e != cudaSuccess) return e;
     k_alpha_beta<<<1, kThreadsAB, 0, s>>>(p);
     return cudaGetLastError();
 }
