@@ -26,8 +26,8 @@
 // writer at a time, and heights change only in the order above.
 //
 // The global relabel and the final reachability are level-synchronous searches
-// over the band's rows with one cluster barrier per level; the few per-pair
-// reductions ride on such barriers.  Every wait inside a round is bounded; one
+// on bit sets, 32 nodes to a word and a word to a thread, with one cluster
+// barrier per level; the few per-pair reductions ride on such barriers.  Every wait inside a round is bounded; one
 // that runs out is recorded and the round ends with all CTAs.
 //
 // Bound: the latency of a wavefront step (shared-memory loads, a handful of
@@ -58,21 +58,27 @@ struct Head {
 
 // Offsets of the arrays in dynamic shared memory; R rows per band, row pitch P.
 struct Layout {
-    uint32_t box_n, box_s, ghost_s, ex, ht, res, f, reach, bytes;
-    __host__ __device__ Layout(int R, int P) {
-        const uint32_t n = (uint32_t)R * P;
+    // masks: [6][R][words]; front: [2][R + 2][words].
+    uint32_t box_n, box_s, ghost_s, masks, front, ex, ht, res, f, bytes;
+    __host__ __device__ Layout(int R, int P, int words) {
+        const uint32_t n = (uint32_t)R * P, w = 4u * words;
         box_n = 512;
         box_s = box_n + 8u * P;
         ghost_s = box_s + 8u * P;
-        ex = ghost_s + 4u * P;
+        masks = ghost_s + 4u * P;
+        front = masks + 6u * R * w;
+        ex = front + 2u * (R + 2) * w;
         ht = ex + 4u * n;
         res = ht + 4u * n;
         f = res + 5u * 4u * n;
-        reach = f + n;
-        bytes = (reach + n + 15u) / 16u * 16u;
+        bytes = (f + n + 15u) / 16u * 16u;
     }
 };
 static_assert(sizeof(Head) <= 512, "header");
+
+// Node sets as 32-column words per row: which nodes have residue in direction
+// d (0 .. 3), which a search has not reached, which of them reach the sink.
+enum { kMaskOpen = 4, kMaskReach = 5 };
 
 // Row pitch: even, so that a diagonal's nodes (stride P - 1 words) lie in
 // distinct banks.
@@ -117,7 +123,9 @@ struct Band {
     unsigned char *sm;
     Head *hd;
     int *ex, *ht, *res[5];
-    uint8_t *f, *reach;
+    uint8_t *f;
+    int words;  // per row
+    uint32_t *masks;
     Layout lay;
     uint32_t base, base_up, base_down;  // shared-memory addresses: own, neighbours'
     int parity;
@@ -160,19 +168,20 @@ __device__ __forceinline__ int block_sum_cl(Band &b, int v) {
 // b.rows the band below's first.
 template <bool FLOW>
 __device__ __forceinline__ int label_at(const Band &b, int r, int x, int alpha, int beta) {
-    int f, reach = 0;
+    int f;
+    uint32_t reach = 0;
+    const uint32_t reach_off = b.lay.masks + 4u * (uint32_t)(kMaskReach * b.R * b.words + (x >> 5));
     if (r < 0) {
-        const uint32_t i = (uint32_t)((b.R - 1) * b.P + x);
-        f = dsmem_u8(b.base_up + b.lay.f + i);
-        if (FLOW) reach = dsmem_u8(b.base_up + b.lay.reach + i);
+        f = dsmem_u8(b.base_up + b.lay.f + (uint32_t)((b.R - 1) * b.P + x));
+        if (FLOW) reach = (uint32_t)dsmem_i32(b.base_up + reach_off + 4u * (uint32_t)((b.R - 1) * b.words));
     } else if (r >= b.rows) {
         f = dsmem_u8(b.base_down + b.lay.f + x);
-        if (FLOW) reach = dsmem_u8(b.base_down + b.lay.reach + x);
+        if (FLOW) reach = (uint32_t)dsmem_i32(b.base_down + reach_off);
     } else {
         f = b.f[r * b.P + x];
-        if (FLOW) reach = b.reach[r * b.P + x];
+        if (FLOW) reach = b.masks[(kMaskReach * b.R + r) * b.words + (x >> 5)];
     }
-    if (FLOW && (f == alpha || f == beta)) f = reach ? alpha : beta;
+    if (FLOW && (f == alpha || f == beta)) f = (reach >> (x & 31)) & 1u ? alpha : beta;
     return f;
 }
 
@@ -192,114 +201,105 @@ __device__ __forceinline__ int band_energy(const AlphaBetaParams &p, Band &b, in
     return block_sum_cl(b, acc);
 }
 
-// Pulls one search level into the nodes not yet reached: node (r, x) joins
-// when a neighbour of `level` (LEVELS) or any reached one is at the other end
-// of a non-zero residue.  REACH searches the reach bytes, else the heights
-// (negative while unreached).
-template <bool REACH>
-__device__ __forceinline__ int search_value(const Band &b, int r, int x) {
-    const uint32_t off = REACH ? b.lay.reach : b.lay.ht;
-    const int size = REACH ? 1 : 4;
-    uint32_t a;
-    if (r < 0) a = b.base_up + off + (uint32_t)((b.R - 1) * b.P + x) * size;
-    else if (r >= b.rows) a = b.base_down + off + (uint32_t)x * size;
-    else return REACH ? b.reach[r * b.P + x] : b.ht[r * b.P + x];
-    return REACH ? dsmem_u8(a) : dsmem_i32(a);
+// Breadth-first search from the nodes with sink residue over residual edges,
+// on the node sets: a word's owner thread takes the nodes of its 32 columns
+// that have residue towards a frontier node.  One level is a few shared-memory
+// words, bit operations and a cluster barrier; the edge rows' frontiers go to
+// the neighbours' copies before it.
+// LEVELS: the distances go into the heights (1 at the start nodes), as
+// graphCutGlobalRelabel's (graphcut.cc:91-140).  Leaves the unreached nodes in
+// kMaskOpen and the reached ones in kMaskReach.
+template <bool LEVELS>
+__device__ __forceinline__ void sink_search_cl(Band &b) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int words = b.words, per_mask = b.R * words;
+    uint32_t *front = reinterpret_cast<uint32_t *>(b.sm + b.lay.front);
+    const int fsize = (b.R + 2) * words;
+    for (int q = warp; q < b.rows * words; q += kThreadsCl / 32) {
+        const int r = q / words, c = q - r * words;
+        const int x = c * 32 + lane, i = r * b.P + x;
+        const bool in = x < b.W;
+        uint32_t m[5];
+#pragma unroll
+        for (int d = 0; d < 5; ++d) m[d] = __ballot_sync(~0u, in && b.res[d][i] != 0);
+        const uint32_t all = __ballot_sync(~0u, in);
+        if (LEVELS && in && ((m[4] >> lane) & 1u)) b.ht[i] = 1;
+        if (lane == 0) {
+            // Residues that point off the grid (none in the reference) lead nowhere.
+            const int y = b.y0 + r;
+            b.masks[q] = y + 1 < b.H ? m[0] : 0u;
+            b.masks[per_mask + q] = c == words - 1 ? m[1] & ~(1u << ((b.W - 1) & 31)) : m[1];
+            b.masks[2 * per_mask + q] = y > 0 ? m[2] : 0u;
+            b.masks[3 * per_mask + q] = c == 0 ? m[3] & ~1u : m[3];
+            b.masks[kMaskOpen * per_mask + q] = all & ~m[4];
+            b.masks[kMaskReach * per_mask + q] = m[4];
+            front[words + q] = m[4];
+        }
+    }
+    __syncthreads();
+    const int q = threadIdx.x;
+    const bool own = q < b.rows * words;
+    const int r = own ? q / words : 0, c = own ? q - r * words : 0;
+    uint32_t open = 0, mask[4] = {0u, 0u, 0u, 0u}, reach = 0;
+    if (own) {
+#pragma unroll
+        for (int d = 0; d < 4; ++d) mask[d] = b.masks[d * per_mask + q];
+        open = b.masks[kMaskOpen * per_mask + q];
+        reach = b.masks[kMaskReach * per_mask + q];
+    }
+    const bool send_up = own && r == 0 && b.up, send_down = own && r == b.rows - 1 && b.down;
+    // The neighbours' copies of this word: row R + 1 of the band above (a full
+    // band), row 0 of the band below.
+    const uint32_t to_up = b.base_up + b.lay.front + 4u * (uint32_t)((b.R + 1) * words + c);
+    const uint32_t to_down = b.base_down + b.lay.front + 4u * (uint32_t)c;
+    uint32_t mine = reach;
+    int cur = 0;
+    for (int level = 1;; ++level) {
+        if (send_up) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to_up + 4u * cur * fsize), "r"(mine) : "memory");
+        if (send_down)
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to_down + 4u * cur * fsize), "r"(mine) : "memory");
+        if (!cl_exchange<false>(b, __syncthreads_or(mine != 0))) break;
+        mine = 0;
+        if (own && open) {
+            const uint32_t *fr = front + cur * fsize + (r + 1) * words + c;
+            const uint32_t f = fr[0];
+            const uint32_t left = c > 0 ? fr[-1] >> 31 : 0u, right = c < words - 1 ? fr[1] << 31 : 0u;
+            mine = open & ((mask[0] & fr[words]) | (mask[2] & fr[-words]) | (mask[1] & ((f >> 1) | right)) |
+                           (mask[3] & ((f << 1) | left)));
+            open &= ~mine;
+            reach |= mine;
+            if (LEVELS)
+                for (uint32_t m = mine; m; m &= m - 1) b.ht[r * b.P + c * 32 + __ffs(m) - 1] = level + 1;
+        }
+        cur ^= 1;
+        if (own) front[cur * fsize + (r + 1) * words + c] = mine;
+    }
+    if (own) {
+        b.masks[kMaskOpen * per_mask + q] = open;
+        b.masks[kMaskReach * per_mask + q] = reach;
+    }
 }
 
-// Breadth-first distances to the sink over residual edges, in the heights
-// (graphCutGlobalRelabel, graphcut.cc:91-140): 1 at the nodes with sink
-// residue; the nodes that reach none keep max(height, N + 2).
+// graphCutGlobalRelabel: the distances; the nodes that reach no sink keep
+// max(height, N + 2).
 __device__ __forceinline__ void global_relabel(Band &b) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // Column chunks that still hold unreached nodes, one mask per row of this
-    // warp (chunks from 31 on share a bit).
-    uint32_t todo[2] = {0u, 0u};
-    int q = 0;
-    for (int r = warp; r < b.rows; r += kThreadsCl / 32, ++q)
-        for (int x = lane; x - lane < b.W; x += 32) {
-            const bool in = x < b.W;
-            const int i = r * b.P + x;
-            bool open = false;
-            if (in) {
-                open = b.res[4][i] == 0;
-                b.ht[i] = open ? b.ht[i] | (int)0x80000000 : 1;
-            }
-            if (__any_sync(~0u, open)) todo[q & 1] |= 1u << min(x >> 5, 31);
-        }
-    cluster_sync();
-    for (int level = 1;; ++level) {
-        bool changed = false;
-        q = 0;
-        for (int r = warp; r < b.rows; r += kThreadsCl / 32, ++q) {
-            uint32_t m = todo[q & 1], keep = 0u;
-            while (m) {
-                const int c = __ffs(m) - 1;
-                m &= m - 1;
-                for (int x0 = c * 32; x0 < b.W && (c == 31 || x0 == c * 32); x0 += 32) {
-                    const int x = x0 + lane, i = r * b.P + x;
-                    bool open = x < b.W && b.ht[i] < 0;
-                    if (open) {
-                        const int y = b.y0 + r;
-                        bool hit = b.res[1][i] && x + 1 < b.W && b.ht[i + 1] == level;
-                        hit = hit || (b.res[3][i] && x > 0 && b.ht[i - 1] == level);
-                        if (!hit && b.res[0][i] && y + 1 < b.H) hit = search_value<false>(b, r + 1, x) == level;
-                        if (!hit && b.res[2][i] && y > 0) hit = search_value<false>(b, r - 1, x) == level;
-                        if (hit) {
-                            b.ht[i] = level + 1;
-                            changed = true;
-                            open = false;
-                        }
-                    }
-                    if (__any_sync(~0u, open)) keep |= 1u << c;
-                }
-            }
-            todo[q & 1] = keep;
-        }
-        if (!cl_exchange<false>(b, __syncthreads_or(changed))) break;
-    }
+    sink_search_cl<true>(b);
+    cluster_sync();  // the band below's unreached nodes
+    const int open_row = kMaskOpen * b.R * b.words;
     AB_FOR_NODES(r, x) {
-        const int i = r * b.P + x, h = b.ht[i];
-        if (h < 0) b.ht[i] = max(h & 0x7fffffff, b.NP2);
+        const int i = r * b.P + x;
+        if ((b.masks[open_row + r * b.words + (x >> 5)] >> (x & 31)) & 1u) b.ht[i] = max(b.ht[i], b.NP2);
     }
     // The band below's first-row heights, for sweep 0 (the later sweeps get
-    // them by word): converted here too, since it may not have been yet, and
+    // them by word): raised here too, since they may not have been yet, and
     // stable until this band's words of sweep 1.
     if (b.down) {
         int *ghost = reinterpret_cast<int *>(b.sm + b.lay.ghost_s);
         for (int x = threadIdx.x; x < b.W; x += kThreadsCl) {
             const int h = dsmem_i32(b.base_down + b.lay.ht + 4u * x);
-            ghost[x] = h < 0 ? max(h & 0x7fffffff, b.NP2) : h;
+            const uint32_t o = (uint32_t)dsmem_i32(b.base_down + b.lay.masks + 4u * (uint32_t)(open_row + (x >> 5)));
+            ghost[x] = (o >> (x & 31)) & 1u ? max(h, b.NP2) : h;
         }
-    }
-}
-
-// Nodes that reach the sink over residual edges, into reach.
-__device__ __forceinline__ void reachability(Band &b) {
-    AB_FOR_NODES(r, x) b.reach[r * b.P + x] = b.res[4][r * b.P + x] ? 1 : 0;
-    cluster_sync();
-    for (;;) {
-        // Within the band to a fixed point, then once more with what the
-        // neighbours found.
-        bool any = false;
-        for (;;) {
-            bool changed = false;
-            AB_FOR_NODES(r, x) {
-                const int i = r * b.P + x, y = b.y0 + r;
-                if (b.reach[i]) continue;
-                bool hit = b.res[1][i] && x + 1 < b.W && b.reach[i + 1];
-                hit = hit || (b.res[3][i] && x > 0 && b.reach[i - 1]);
-                if (!hit && b.res[0][i] && y + 1 < b.H) hit = search_value<true>(b, r + 1, x) != 0;
-                if (!hit && b.res[2][i] && y > 0) hit = search_value<true>(b, r - 1, x) != 0;
-                if (hit) {
-                    b.reach[i] = 1;
-                    changed = true;
-                }
-            }
-            if (!__syncthreads_or(changed)) break;
-            any = true;
-        }
-        if (!cl_exchange<false>(b, any)) break;
     }
 }
 
@@ -446,7 +446,8 @@ __global__ void __launch_bounds__(kThreadsCl, 1) k_alpha_beta_cluster(const Alph
     extern __shared__ __align__(16) unsigned char ab_smem[];
     const int P = pitch_of(p.W);
     Band b{p.W, p.H, p.L, p.W * p.H, p.W * p.H + 2, 0, 0, 0, 0, P, R, false, false, ab_smem,
-           reinterpret_cast<Head *>(ab_smem), nullptr, nullptr, {}, nullptr, nullptr, Layout(R, P), 0, 0, 0, 0};
+           reinterpret_cast<Head *>(ab_smem), nullptr, nullptr, {}, nullptr, (p.W + 31) / 32, nullptr,
+           Layout(R, P, (p.W + 31) / 32), 0, 0, 0, 0};
     b.C = (int)gridDim.x;
     b.rank = (int)cluster_rank();
     b.y0 = b.rank * R;
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(kThreadsCl, 1) k_alpha_beta_cluster(const Alph
     b.ht = reinterpret_cast<int *>(ab_smem + b.lay.ht);
     for (int d = 0; d < 5; ++d) b.res[d] = reinterpret_cast<int *>(ab_smem + b.lay.res) + (size_t)d * R * P;
     b.f = ab_smem + b.lay.f;
-    b.reach = ab_smem + b.lay.reach;
+    b.masks = reinterpret_cast<uint32_t *>(ab_smem + b.lay.masks);
     b.base = smem_addr(ab_smem);
     b.base_up = dsmem_addr(b.base, b.rank > 0 ? b.rank - 1 : 0);
     b.base_down = dsmem_addr(b.base, b.rank + 1 < b.C ? b.rank + 1 : b.rank);
@@ -540,15 +541,13 @@ __global__ void __launch_bounds__(kThreadsCl, 1) k_alpha_beta_cluster(const Alph
                     __syncthreads();
                 }
                 if (stop) break;
-                reachability(b);
+                sink_search_cl<false>(b);
+                cluster_sync();  // the neighbours' reached nodes
                 const int cost = cl_exchange<true>(b, band_energy<true>(p, b, alpha, beta));
                 if (cost < min_cost) {
                     min_cost = cost;
                     success = true;
-                    AB_FOR_NODES(r, x) {
-                        const int i = r * P + x;
-                        if (b.f[i] == alpha || b.f[i] == beta) b.f[i] = b.reach[i] ? alpha : beta;
-                    }
+                    AB_FOR_NODES(r, x) b.f[r * P + x] = (uint8_t)label_at<true>(b, r, x, alpha, beta);
                 }
                 cluster_sync();  // the next pair reads the neighbours' labels
             }
@@ -572,11 +571,14 @@ cudaError_t launch_alpha_beta_cluster(const AlphaBetaParams &p, cudaStream_t s, 
     // The fewest bands (a power of two) of at most 32 rows that fit: every
     // further band adds its lag to a sweep.
     int C = 1, R = p.H;
-    while (C <= kMaxBands && ((R = (p.H + C - 1) / C) > kMaxRows || Layout(R, pitch_of(p.W)).bytes > (uint32_t)most)) C *= 2;
+    const int words = (p.W + 31) / 32;
+    while (C <= kMaxBands && ((R = (p.H + C - 1) / C) > kMaxRows || R * words > kThreadsCl ||
+                              Layout(R, pitch_of(p.W), words).bytes > (uint32_t)most))
+        C *= 2;
     if (C > kMaxBands) return cudaSuccess;
     auto kern = k_alpha_beta_cluster;
     static SmemLimit limit;
-    const size_t smem = Layout(R, pitch_of(p.W)).bytes;
+    const size_t smem = Layout(R, pitch_of(p.W), words).bytes;
     e = limit.ensure(kern, smem);
     if (e != cudaSuccess) return e;
     if (C > 8) {
