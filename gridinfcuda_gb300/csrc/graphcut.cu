@@ -17,6 +17,9 @@
 // next -- the excess, heights and residues of nodes outside the current
 // partition -- lives in device memory and is carried the same way.
 //
+// Grids whose state fits the shared memory of a thread-block cluster run in
+// graphcut_cluster.cu; this file is the form for the others.
+//
 // A pair's work is a chain of dependent sweeps (a round is one global
 // relabel and ten push and relabel wavefronts of W + H - 1 diagonals each),
 // so one CTA of 1024 threads runs the whole solve, every pair and iteration,

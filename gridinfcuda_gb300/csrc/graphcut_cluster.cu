@@ -30,9 +30,15 @@
 // barrier per level; the few per-pair reductions ride on such barriers.  Every wait inside a round is bounded; one
 // that runs out is recorded and the round ends with all CTAs.
 //
-// Bound: the latency of a wavefront step (shared-memory loads, a handful of
-// dependent operations, a progress counter) and the searches' barriers.
-// AB_MEASURED
+// Bound: the latency of a wavefront step with twenty warps on the SM (about
+// 800 cycles, eight per instruction; 400 steps a band, then the bands' lags:
+// 0.33 ms a round of twenty sweeps at 384x288, 16 bands) and the searches'
+// barriers.  384x288x16, one pass from the BP labels, three seeds: 787, - and -
+// ms with one CTA in global memory, 187, 87 and 138 ms here with searches that
+// walked the unreached nodes, 91, 63 and 90 ms with bit sets, 80, 55 and 79 ms
+// with the short step.  Also measured: four diagonals between two waits 137 ms
+// (the lags grow by more than the waits cost), flows formed branch-free and
+// applied by predicated additions 99 ms, no fences in a step 3 % less.
 #include <cstdint>
 
 #include "ginf_internal.h"
@@ -47,7 +53,7 @@ constexpr int kThreadsCl = kSweeps * 32;
 constexpr int kMaxBands = 16;  // largest cluster
 constexpr int kMaxRows = 32;   // rows per band: a lane each
 constexpr uint64_t kAlphaBetaLimitNs = 60ull * 1000000000ull;
-constexpr int kTagBits = 14, kHeightBits = 18;
+constexpr int kHeightBits = 18;  // of a word's upper half; the sweep's number in the other 14
 
 struct Head {
     int red[32];
@@ -84,22 +90,6 @@ enum { kMaskOpen = 4, kMaskReach = 5 };
 // distinct banks.
 __host__ __device__ inline int pitch_of(int W) { return (W + 1) & ~1; }
 
-__device__ __forceinline__ uint64_t make_word(int tag, int height, int flow) {
-    return ((uint64_t)(uint32_t)(tag & ((1 << kTagBits) - 1)) << 50) | ((uint64_t)(uint32_t)height << 32) |
-           (uint64_t)(uint32_t)flow;
-}
-__device__ __forceinline__ int word_tag(uint64_t w) { return (int)(w >> 50); }
-__device__ __forceinline__ int word_height(uint64_t w) { return (int)((w >> 32) & ((1u << kHeightBits) - 1)); }
-__device__ __forceinline__ int word_flow(uint64_t w) { return (int)(uint32_t)w; }
-
-__device__ __forceinline__ uint64_t box_load(uint32_t addr) {
-    uint64_t v;
-    asm volatile("ld.relaxed.cluster.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ void box_store(uint32_t addr, uint64_t v) {
-    asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
-}
 __device__ __forceinline__ int dsmem_i32(uint32_t addr) {
     int v;
     asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -303,142 +293,147 @@ __device__ __forceinline__ void global_relabel(Band &b) {
     }
 }
 
-// Sweep j of a round (even: pushes, graphcut.cc:143-177; odd: relabels,
-// :180-195) over the band's diagonals by one warp.  first_tag numbers the
-// round's sweep 0.
+// Called now and then by a waiting warp: false when the wait, or another of
+// this CTA, has taken too long.
+__device__ __noinline__ bool sweep_patience(Band &b, uint32_t n, int *status) {
+    volatile int *give_up = &b.hd->give_up;
+    // 2^25 polls of at least 60 cycles each are more than a second.
+    if (n >= (1u << 25) && !*give_up) {
+        if ((threadIdx.x & 31) == 0) atomicOr(status, DEV_ERR_TIMEOUT);
+        *give_up = 1;
+    }
+    return __all_sync(~0u, *give_up == 0);
+}
+
+// Flow fl from node i over its residue r at res_i into node q.
+__device__ __forceinline__ void push_to(int fl, int r, int *res_i, int *ex_q, int *res_q) {
+    *res_i = r - fl;
+    atomicAdd(ex_q, fl);
+    *res_q += fl;
+}
+
+// Sweep j of a round (pushes, graphcut.cc:143-177, or relabels, :180-195) over
+// the band's diagonals by one warp.  first_tag numbers the round's sweep 0.
+//
+// A step's latency is the sweeps' rate, and with twenty warps on the SM an
+// instruction of it costs about eight cycles, so what every step does is kept
+// short: a lane meets at most one neighbouring band (bands have two rows or
+// more), with one word in and one out; progress counters end at a value that
+// needs no comparison with the last diagonal.
+constexpr int kSweepDone = 0x3fffffff;
+template <bool PUSH>
 __device__ __forceinline__ void sweep(Band &b, int j, int first_tag, int *status) {
     if (b.rows == 0) return;
-    const int lane = threadIdx.x & 31;
-    const int klast = b.y0 + b.rows - 1 + b.W - 1;
-    const bool row = lane < b.rows;
+    const int lane = threadIdx.x & 31, W = b.W, P = b.P, NP2 = b.NP2;
+    const int steps = b.rows - 1 + W;
+    const int cols = lane < b.rows ? W : 0;
     const bool top = lane == 0 && b.up, bottom = lane == b.rows - 1 && b.down;
-    const int tag_n = (first_tag + j) & ((1 << kTagBits) - 1), tag_s = (first_tag + j - 1) & ((1 << kTagBits) - 1);
-    const bool push = (j & 1) == 0;
-    volatile int *prog = b.hd->prog;
-    const int *ghost = reinterpret_cast<const int *>(b.sm + b.lay.ghost_s);
-    int seen = j > 0 ? -1 : 0x7fffffff;
-    for (int k = b.y0; k <= klast; ++k) {
-        const int x = k - b.y0 - lane;
-        const bool in = row && x >= 0 && x < b.W;
-        const int i = lane * b.P + x;
-        const bool wait_n = in && top, wait_s = in && bottom && j > 0;
-        const int need = min(k + 1, klast);
-        uint64_t wn = 0, ws = 0;
-        bool ok_n = !wait_n, ok_s = !wait_s;
-        uint64_t t0 = 0;
+    const bool edge_n = b.y0 + lane == 0, edge_s = b.y0 + lane + 1 >= b.H;  // the grid's
+    const bool edge = top || bottom, recv = top || (bottom && j > 0);
+    // The neighbour's words of this sweep (above) or the last one (below), the
+    // band's own of this sweep; a word's upper half is tag and height.
+    const uint32_t tag = (uint32_t)(first_tag + j) << kHeightBits;
+    const uint32_t want = top ? tag : (uint32_t)(first_tag + j - 1) << kHeightBits;
+    uint32_t box = b.base + (top ? b.lay.box_n : b.lay.box_s) - 8u * lane;
+    uint32_t out = (top ? b.base_up + b.lay.box_s : b.base_down + b.lay.box_n) - 8u * lane;
+    volatile int *before = &b.hd->prog[j > 0 ? j - 1 : 0], *mine = &b.hd->prog[j];
+    const int *ghost = reinterpret_cast<const int *>(b.sm + b.lay.ghost_s) - lane;
+    int *ex = b.ex + lane * P - lane, *ht = b.ht + lane * P - lane;
+    const int array = b.R * P;  // from one residue array to the next
+    int *res = b.res[0] + lane * P - lane;
+    int seen = j > 0 ? -1 : kSweepDone;
+    // Step k is diagonal y0 + k: column k - lane of each row.
+    for (int k = 0; k < steps; ++k) {
+        const bool in = (unsigned)(k - lane) < (unsigned)cols;
+        uint32_t w_hi = 0, w_lo = 0;
+        bool ok = !(in && recv);
         for (uint32_t n = 1;; ++n) {
-            if (seen < need) seen = prog[j - 1];
-            if (!ok_n) {
-                wn = box_load(b.base + b.lay.box_n + 8u * x);
-                ok_n = word_tag(wn) == tag_n;
+            if (seen <= k) seen = *before;
+            if (!ok) {
+                asm volatile("ld.relaxed.cluster.shared::cluster.v2.u32 {%0, %1}, [%2];"
+                             : "=r"(w_lo), "=r"(w_hi)
+                             : "r"(box + 8u * k)
+                             : "memory");
+                ok = (w_hi ^ want) < (1u << kHeightBits);
             }
-            if (!ok_s) {
-                ws = box_load(b.base + b.lay.box_s + 8u * x);
-                ok_s = word_tag(ws) == tag_s;
-            }
-            if (__all_sync(~0u, seen >= need && ok_n && ok_s)) break;
-            if ((n & 1023u) == 0) {
-                const uint64_t now = __shfl_sync(~0u, global_timer_ns(), 0);
-                if (t0 == 0) t0 = now;
-                const bool late = now - t0 > kWaitLimitNs;
-                if (__any_sync(~0u, late || *(volatile int *)&b.hd->give_up)) {
-                    if (late && lane == 0) atomicOr(status, DEV_ERR_TIMEOUT);
-                    *(volatile int *)&b.hd->give_up = 1;
-                    break;
-                }
-            }
+            if (__all_sync(~0u, ok && seen > k)) break;
+            if ((n & 4095u) == 0 && !sweep_patience(b, n, status)) break;
         }
         __threadfence_block();
-        int flow_n = 0, flow_s = 0, h = 0;
+        int e = 0, h = 0;
         if (in) {
-            int e = b.ex[i];
-            const int e_was = e;
-            h = b.ht[i];
-            if (wait_n && word_flow(wn)) {
-                e += word_flow(wn);
-                b.res[2][i] += word_flow(wn);
-            }
-            if (wait_s && word_flow(ws)) {
-                e += word_flow(ws);
-                b.res[0][i] += word_flow(ws);
-            }
-            if (e && h < b.NP2) {
-                const int hs = bottom ? (j > 0 ? word_height(ws) : ghost[x]) : (b.y0 + lane + 1 < b.H ? b.ht[i + b.P] : 0);
-                const int hn = top ? word_height(wn) : (b.y0 + lane > 0 ? b.ht[i - b.P] : 0);
-                const int he = x + 1 < b.W ? b.ht[i + 1] : 0, hw = x > 0 ? b.ht[i - 1] : 0;
-                const int rs = b.res[4][i], r0 = b.res[0][i], r1 = b.res[1][i], r2 = b.res[2][i], r3 = b.res[3][i];
-                if (push) {
-                    if (rs && h == 1) {
-                        const int fl = min(rs, e);
-                        e -= fl;
-                        b.res[4][i] = rs - fl;
-                    }
-                    // Directions in order S, E, N, W; a zero flow changes nothing.
-                    if (r0 && h == hs + 1) {
-                        const int fl = min(r0, e);
-                        if (fl) {
-                            e -= fl;
-                            b.res[0][i] = r0 - fl;
-                            if (bottom) {
-                                flow_s = fl;
-                            } else {
-                                atomicAdd(&b.ex[i + b.P], fl);
-                                b.res[2][i + b.P] += fl;
-                            }
-                        }
-                    }
-                    if (r1 && h == he + 1) {
-                        const int fl = min(r1, e);
-                        if (fl) {
-                            e -= fl;
-                            b.res[1][i] = r1 - fl;
-                            atomicAdd(&b.ex[i + 1], fl);
-                            b.res[3][i + 1] += fl;
-                        }
-                    }
-                    if (r2 && h == hn + 1) {
-                        const int fl = min(r2, e);
-                        if (fl) {
-                            e -= fl;
-                            b.res[2][i] = r2 - fl;
-                            if (top) {
-                                flow_n = fl;
-                            } else {
-                                atomicAdd(&b.ex[i - b.P], fl);
-                                b.res[0][i - b.P] += fl;
-                            }
-                        }
-                    }
-                    if (r3 && h == hw + 1) {
-                        const int fl = min(r3, e);
-                        if (fl) {
-                            e -= fl;
-                            b.res[3][i] = r3 - fl;
-                            atomicAdd(&b.ex[i - 1], fl);
-                            b.res[1][i - 1] += fl;
-                        }
-                    }
-                } else {
-                    if (rs) {
-                        h = 1;
-                    } else {
-                        int mh = b.NP2;
-                        if (r0) mh = min(mh, hs);
-                        if (r1) mh = min(mh, he);
-                        if (r2) mh = min(mh, hn);
-                        if (r3) mh = min(mh, hw);
-                        h = mh + 1;
-                    }
-                    b.ht[i] = h;
-                }
-            }
-            if (e != e_was) b.ex[i] = e;
-            if (top) box_store(b.base_up + b.lay.box_s + 8u * x, make_word(tag_n, h, flow_n));
-            if (bottom) box_store(b.base_down + b.lay.box_n + 8u * x, make_word(tag_n, h, flow_s));
+            e = ex[k];
+            h = ht[k];
         }
+        const int e_was = e;
+        if (w_lo) {  // flow over the band's edge
+            e += (int)w_lo;
+            res[(top ? 2 : 0) * array + k] += (int)w_lo;
+        }
+        int flow = 0;
+        if (e && h < NP2) {
+            const int h_word = (int)(w_hi & ((1u << kHeightBits) - 1));
+            const int hs = bottom ? (j > 0 ? h_word : ghost[k]) : (edge_s ? 0 : ht[k + P]);
+            const int hn = top ? h_word : (edge_n ? 0 : ht[k - P]);
+            const int he = k - lane + 1 < W ? ht[k + 1] : 0, hw = k > lane ? ht[k - 1] : 0;
+            int *r = res + k, *x = ex + k;
+            const int rs = r[4 * array], r0 = r[0], r1 = r[array], r2 = r[2 * array], r3 = r[3 * array];
+            if (PUSH) {
+                if (rs && h == 1) {
+                    const int fl = min(rs, e);
+                    e -= fl;
+                    r[4 * array] = rs - fl;
+                }
+                // Directions in order S, E, N, W; a zero flow changes nothing,
+                // and a flow over the band's edge goes by word.
+                if (r0 && h == hs + 1) {
+                    const int fl = min(r0, e);
+                    e -= fl;
+                    if (bottom) {
+                        r[0] = r0 - fl;
+                        flow = fl;
+                    } else if (fl) {
+                        push_to(fl, r0, r, x + P, r + 2 * array + P);
+                    }
+                }
+                if (r1 && h == he + 1) {
+                    const int fl = min(r1, e);
+                    e -= fl;
+                    if (fl) push_to(fl, r1, r + array, x + 1, r + 3 * array + 1);
+                }
+                if (r2 && h == hn + 1) {
+                    const int fl = min(r2, e);
+                    e -= fl;
+                    if (top) {
+                        r[2 * array] = r2 - fl;
+                        flow = fl;
+                    } else if (fl) {
+                        push_to(fl, r2, r + 2 * array, x - P, r - P);
+                    }
+                }
+                if (r3 && h == hw + 1) {
+                    const int fl = min(r3, e);
+                    e -= fl;
+                    if (fl) push_to(fl, r3, r + 3 * array, x - 1, r + array - 1);
+                }
+            } else {
+                int mh = NP2;
+                if (r0) mh = min(mh, hs);
+                if (r1) mh = min(mh, he);
+                if (r2) mh = min(mh, hn);
+                if (r3) mh = min(mh, hw);
+                h = rs ? 1 : mh + 1;
+                ht[k] = h;
+            }
+        }
+        if (e != e_was) ex[k] = e;
+        if (in && edge)
+            asm volatile("st.relaxed.cluster.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(out + 8u * k), "r"(flow),
+                         "r"(tag | (uint32_t)h)
+                         : "memory");
         __threadfence_block();
         __syncwarp();
-        if (lane == 0) prog[j] = k;
+        if (lane == 0) *mine = k == steps - 1 ? kSweepDone : k;
     }
 }
 
@@ -536,7 +531,8 @@ __global__ void __launch_bounds__(kThreadsCl, 1) k_alpha_beta_cluster(const Alph
                     global_relabel(b);
                     if (threadIdx.x < kSweeps) b.hd->prog[threadIdx.x] = -1;
                     __syncthreads();
-                    sweep(b, threadIdx.x >> 5, tag, p.status);
+                    if ((threadIdx.x >> 5) & 1) sweep<false>(b, threadIdx.x >> 5, tag, p.status);
+                    else sweep<true>(b, threadIdx.x >> 5, tag, p.status);
                     tag += kSweeps;
                     __syncthreads();
                 }
@@ -575,7 +571,7 @@ cudaError_t launch_alpha_beta_cluster(const AlphaBetaParams &p, cudaStream_t s, 
     while (C <= kMaxBands && ((R = (p.H + C - 1) / C) > kMaxRows || R * words > kThreadsCl ||
                               Layout(R, pitch_of(p.W), words).bytes > (uint32_t)most))
         C *= 2;
-    if (C > kMaxBands) return cudaSuccess;
+    if (C > kMaxBands || (C > 1 && R < 2)) return cudaSuccess;
     auto kern = k_alpha_beta_cluster;
     static SmemLimit limit;
     const size_t smem = Layout(R, pitch_of(p.W), words).bytes;
