@@ -56,12 +56,27 @@ struct ConvTcParams {
     const float *bias;       // COUT, or null
     const float *res;        // FP32 residual [pixel][COUT] added after the activation, or null
     void *out;               // [pixel][COUT], FP32 or BF16
+    const __nv_bfloat16 *act;  // EPI_MASK: the activations whose ReLU the gradient passes
+    const float *target;       // EPI_LOSS: [pixel][COUT]
+    float scale;               // EPI_LOSS: 2 / elements
+    float *bias_part;          // EPI_MASK, EPI_LOSS: [CTA][COUT] sums of the gradient written
+    double *loss_part;         // EPI_LOSS: [CTA] sums of squared differences
     int n, h, w;             // images, rows, columns
     int bands, chunks, rows_per_chunk, items;
     int *status;
 };
 
 namespace {
+
+// What the epilogue makes of the convolution.
+enum {
+    EPI_STORE = 0,  // + bias, ReLU or residual; stored
+    EPI_MASK = 1,   // a data gradient through the ReLU below: zero where that activation is not
+                    // positive, stored as BF16, its sum per channel being the bias gradient
+    EPI_LOSS = 2    // the last layer in training: + bias + residual, the difference to the target,
+                    // its square's sum (the loss) and 2 / n times itself as BF16 (the output gradient),
+                    // whose sum per channel is the bias gradient
+};
 
 constexpr int kTileM = 128;            // pixels per tile (MMA M)
 constexpr int kSlab = kTileM + 2;      // pixels per row copy: the band and one either side
@@ -179,11 +194,25 @@ __device__ __forceinline__ uint32_t acc_col(uint32_t t) {
     return (uint32_t)(ACC - 1 - (int)(t % ACC)) * COUT;
 }
 
-template <int CIN, int COUT, bool RELU, bool OUT_F32, int RING>
+// a + b as the unevaluated pair (s, e) (Knuth's TwoSum).
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
+    s = __fadd_rn(a, b);
+    const float bb = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
+__device__ __forceinline__ uint2 pack_bf16x4(const float *v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    return make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+}
+
+// OUT_F32: FP32 results are staged (and stored, with EPI_STORE).
+template <int CIN, int COUT, bool RELU, bool OUT_F32, int RING, int EPI = EPI_STORE>
 __global__ void __launch_bounds__(kThreadsTc, 2)
     k_conv_tc(const __grid_constant__ CUtensorMap rows_map, const ConvTcParams p) {
     using Lay = TcLayout<CIN, COUT, OUT_F32, RING>;
     static_assert((CIN == 16 || CIN == 32 || CIN == 64) && COUT % 16 == 0 && COUT <= 256, "tile shape");
+    static_assert(EPI == EPI_STORE || (OUT_F32 && !RELU), "the gradients are formed from FP32 rows");
     extern __shared__ __align__(1024) unsigned char sm[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(sm + Lay::kBars);
     uint64_t *full = bars, *empty = bars + RING, *acc_full = bars + 2 * RING, *acc_empty = acc_full + Lay::kAcc,
@@ -322,6 +351,9 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         // Epilogue: warp w reads lanes 32w..32w+31 of the accumulator.
         uint32_t tile = 0;
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+        // EPI_MASK, EPI_LOSS: this lane's four channels (chunk lane % kChunksOut
+        // of a pixel, the same in every pass) and its squares as a float pair.
+        float bsum[4] = {0.f, 0.f, 0.f, 0.f}, loss_hi = 0.f, loss_lo = 0.f;
         // The tensor-memory loads are warp-collective: every decision to stop
         // is taken by the whole warp.
         for (int it = blockIdx.x; it < p.items && !__any_sync(~0u, *abort_flag); it += gridDim.x) {
@@ -374,6 +406,65 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 uint4 *o = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(p.out) + pix * Lay::kOutBytes);
                 const uint4 *rs = OUT_F32 && p.res ? reinterpret_cast<const uint4 *>(p.res + pix * COUT) : nullptr;
                 const int nq = valid * Lay::kChunksOut;
+                if constexpr (EPI != EPI_STORE) {
+                    // Passes in groups whose loads are all in flight at once;
+                    // a row's sums first, then the running ones.
+                    constexpr int kGroup = Lay::kChunksOut < 8 ? Lay::kChunksOut : 8;
+                    float rsum[4] = {0.f, 0.f, 0.f, 0.f};
+                    uint2 *g = reinterpret_cast<uint2 *>(static_cast<__nv_bfloat16 *>(p.out) + pix * COUT);
+                    const uint2 *act = EPI == EPI_MASK ? reinterpret_cast<const uint2 *>(p.act + pix * COUT) : nullptr;
+                    const float4 *res = EPI == EPI_LOSS ? reinterpret_cast<const float4 *>(p.res + pix * COUT) : nullptr;
+                    const float4 *tgt = EPI == EPI_LOSS ? reinterpret_cast<const float4 *>(p.target + pix * COUT) : nullptr;
+#pragma unroll
+                    for (int i0 = 0; i0 < Lay::kChunksOut; i0 += kGroup) {
+                        uint2 av[kGroup];
+                        float4 xv[kGroup], tv[kGroup];
+#pragma unroll
+                        for (int i = 0; i < kGroup; ++i) {
+                            const int q = lane + 32 * (i0 + i);
+                            if (q < nq) {
+                                if (EPI == EPI_MASK) av[i] = act[q];
+                                if (EPI == EPI_LOSS) {
+                                    xv[i] = res[q];
+                                    tv[i] = tgt[q];
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < kGroup; ++i) {
+                            const int q = lane + 32 * (i0 + i);
+                            if (q < nq) {
+                                const float4 f = *reinterpret_cast<const float4 *>(
+                                    stage + (q / Lay::kChunksOut) * Lay::kStagePitch + (q % Lay::kChunksOut) * 16);
+                                float o[4] = {f.x, f.y, f.z, f.w};
+                                if (EPI == EPI_MASK) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) {
+                                        const uint32_t w2 = k < 2 ? av[i].x : av[i].y;
+                                        const uint16_t bits = (uint16_t)(w2 >> (16 * (k & 1)));
+                                        if (!(__bfloat162float(__ushort_as_bfloat16(bits)) > 0.f)) o[k] = 0.f;
+                                    }
+                                } else {
+                                    const float4 a = xv[i], b = tv[i];
+                                    const float d[4] = {(f.x + a.x) - b.x, (f.y + a.y) - b.y, (f.z + a.z) - b.z,
+                                                        (f.w + a.w) - b.w};
+                                    float s, e;
+                                    two_sum(loss_hi, d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + d[3] * d[3], s, e);
+                                    two_sum(s, __fadd_rn(e, loss_lo), loss_hi, loss_lo);
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) o[k] = p.scale * d[k];
+                                }
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) rsum[k] += o[k];
+                                g[q] = pack_bf16x4(o);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) bsum[k] += rsum[k];
+                    __syncwarp();
+                    continue;
+                }
                 uint4 r[Lay::kChunksOut];  // all residual loads in flight before the first store
                 if (OUT_F32 && rs) {
 #pragma unroll
@@ -394,6 +485,40 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                     o[q] = val;
                 }
                 __syncwarp();
+            }
+        }
+        if constexpr (EPI != EPI_STORE) {
+            // The CTA's sums, in a fixed order: lanes of one channel chunk, then
+            // the four warps.
+#pragma unroll
+            for (int off = Lay::kChunksOut; off < 32; off <<= 1)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) bsum[k] += __shfl_xor_sync(~0u, bsum[k], off);
+            float *red = reinterpret_cast<float *>(stage);
+            if (lane < Lay::kChunksOut)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) red[4 * lane + k] = bsum[k];
+            double *lred = reinterpret_cast<double *>(stage + COUT * 4);
+            if (EPI == EPI_LOSS) {
+                double l = (double)loss_hi + (double)loss_lo;
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(~0u, l, off);
+                if (lane == 0) *lred = l;
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");  // the epilogue's four warps
+            constexpr int kWarpStage = 32 * Lay::kStagePitch;
+            if (threadIdx.x < COUT) {
+                float t = 0.f;
+#pragma unroll
+                for (int w = 0; w < 4; ++w)
+                    t += reinterpret_cast<const float *>(sm + Lay::kStage + w * kWarpStage)[threadIdx.x];
+                p.bias_part[(size_t)blockIdx.x * COUT + threadIdx.x] = t;
+            }
+            if (EPI == EPI_LOSS && threadIdx.x == 0) {
+                double t = 0.0;
+                for (int w = 0; w < 4; ++w)
+                    t += *reinterpret_cast<const double *>(sm + Lay::kStage + w * kWarpStage + COUT * 4);
+                p.loss_part[blockIdx.x] = t;
             }
         }
     }
@@ -493,8 +618,9 @@ bool plan_items(int n, int h, int w, int slots, ItemPlan &pl) {
     return true;
 }
 
-template <int CIN, int COUT, bool RELU, bool OUT_F32>
-cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t s) {
+// parts (may be null): the CTAs launched, each with its partial sums.
+template <int CIN, int COUT, bool RELU, bool OUT_F32, int EPI = EPI_STORE>
+cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t s, int *parts = nullptr) {
     // The deepest ring of row buffers (3 to 8) that leaves room for two CTAs
     // per SM (228 KB of shared memory, 1 KB of it reserved per CTA).
     constexpr int kBudget = 113 * 1024;
@@ -505,7 +631,7 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
     // At least 80 KB, so that no more than two CTAs share an SM's 512
     // tensor-memory columns (a third would wait in its allocation).
     constexpr int kSmem = Lay::kBytes < 80 * 1024 ? 80 * 1024 : Lay::kBytes;
-    auto kern = k_conv_tc<CIN, COUT, RELU, OUT_F32, RING>;
+    auto kern = k_conv_tc<CIN, COUT, RELU, OUT_F32, RING, EPI>;
     static TcKernelSetup setup;
     cudaError_t attr_err = setup.ensure(kern, kSmem);
     if (attr_err != cudaSuccess) return attr_err;
@@ -521,6 +647,7 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
     p.rows_per_chunk = pl.rows_per_chunk;
     p.chunks = pl.chunks;
     p.items = pl.items;
+    if (parts) *parts = pl.grid;
     kern<<<pl.grid, kThreadsTc, kSmem, s>>>(map, p);
     return cudaGetLastError();
 }
@@ -766,8 +893,10 @@ cudaError_t launch_wgrad_tc(const __nv_bfloat16 *dout, const __nv_bfloat16 *in, 
 }  // namespace
 
 // 3x3 convolution of NHWC BF16 input with weights [COUT][9][CIN] on the
-// tcgen05 path; cudaErrorInvalidValue for a channel pair it is not built for.
-cudaError_t conv_fwd_tc(int cin, int cout, bool relu, bool out_f32, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
+// tcgen05 path: hidden layers (cout 32, ReLU, BF16 out) and the last layer
+// (cin 32, FP32 out, + res); cudaErrorInvalidValue for a channel pair it is
+// not built for.
+cudaError_t conv_fwd_tc(int cin, int cout, bool relu, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
                         const float *bias, int nimg, int h, int wd, void *out, const float *res, int *status,
                         cudaStream_t s) {
     if (((uintptr_t)in | (uintptr_t)w | (uintptr_t)out | (uintptr_t)res) & 15) return cudaErrorMisalignedAddress;
@@ -780,18 +909,65 @@ cudaError_t conv_fwd_tc(int cin, int cout, bool relu, bool out_f32, const __nv_b
     p.h = h;
     p.w = wd;
     p.status = status;
-#define GINF_TC_CASE(CI, CO)                                                                    \
-    if (cin == CI && cout == CO) {                                                              \
-        if (out_f32) return relu ? cudaErrorInvalidValue : launch_conv_tc<CI, CO, false, true>(in, p, s); \
-        return relu ? launch_conv_tc<CI, CO, true, false>(in, p, s)                             \
-                    : launch_conv_tc<CI, CO, false, false>(in, p, s);                           \
+    if (relu) {
+        if (cout != 32) return cudaErrorInvalidValue;
+        if (cin == 16) return launch_conv_tc<16, 32, true, false>(in, p, s);
+        if (cin == 32) return launch_conv_tc<32, 32, true, false>(in, p, s);
+        if (cin == 64) return launch_conv_tc<64, 32, true, false>(in, p, s);
+        return cudaErrorInvalidValue;
     }
-    GINF_TC_CASE(16, 32)
-    GINF_TC_CASE(32, 32)
-    GINF_TC_CASE(64, 32)
-    GINF_TC_CASE(32, 16)
-    GINF_TC_CASE(32, 64)
-#undef GINF_TC_CASE
+    if (cin != 32) return cudaErrorInvalidValue;
+    if (cout == 16) return launch_conv_tc<32, 16, false, true>(in, p, s);
+    if (cout == 32) return launch_conv_tc<32, 32, false, true>(in, p, s);
+    if (cout == 64) return launch_conv_tc<32, 64, false, true>(in, p, s);
+    return cudaErrorInvalidValue;
+}
+
+// The last layer in training (32 -> cout): grad = BF16 of 2 / n (y - target)
+// with y = conv + bias + x, per-CTA sums of it per channel in bias_part
+// ([parts][cout]) and of the squared differences in loss_part ([parts]).
+cudaError_t conv_loss_tc(int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias, int nimg, int h,
+                         int wd, const float *x, const float *target, float scale, __nv_bfloat16 *grad,
+                         float *bias_part, double *loss_part, int *parts, int *status, cudaStream_t s) {
+    if (((uintptr_t)in | (uintptr_t)w | (uintptr_t)x | (uintptr_t)target | (uintptr_t)grad) & 15)
+        return cudaErrorMisalignedAddress;
+    ConvTcParams p{};
+    p.wt = w;
+    p.bias = bias;
+    p.res = x;
+    p.target = target;
+    p.scale = scale;
+    p.out = grad;
+    p.bias_part = bias_part;
+    p.loss_part = loss_part;
+    p.n = nimg;
+    p.h = h;
+    p.w = wd;
+    p.status = status;
+    if (cout == 16) return launch_conv_tc<32, 16, false, true, EPI_LOSS>(in, p, s, parts);
+    if (cout == 32) return launch_conv_tc<32, 32, false, true, EPI_LOSS>(in, p, s, parts);
+    if (cout == 64) return launch_conv_tc<32, 64, false, true, EPI_LOSS>(in, p, s, parts);
+    return cudaErrorInvalidValue;
+}
+
+// Data gradient (cin channels of output gradient -> 32) with flipped weights,
+// through the ReLU that made act: grad as BF16 and its per-CTA sums per channel.
+cudaError_t conv_dgrad_tc(int cin, const __nv_bfloat16 *in, const __nv_bfloat16 *w, int nimg, int h, int wd,
+                          const __nv_bfloat16 *act, __nv_bfloat16 *grad, float *bias_part, int *parts, int *status,
+                          cudaStream_t s) {
+    if (((uintptr_t)in | (uintptr_t)w | (uintptr_t)act | (uintptr_t)grad) & 15) return cudaErrorMisalignedAddress;
+    ConvTcParams p{};
+    p.wt = w;
+    p.act = act;
+    p.out = grad;
+    p.bias_part = bias_part;
+    p.n = nimg;
+    p.h = h;
+    p.w = wd;
+    p.status = status;
+    if (cin == 16) return launch_conv_tc<16, 32, false, true, EPI_MASK>(in, p, s, parts);
+    if (cin == 32) return launch_conv_tc<32, 32, false, true, EPI_MASK>(in, p, s, parts);
+    if (cin == 64) return launch_conv_tc<64, 32, false, true, EPI_MASK>(in, p, s, parts);
     return cudaErrorInvalidValue;
 }
 

@@ -28,9 +28,15 @@
 
 namespace ginf_gpu {
 
-cudaError_t conv_fwd_tc(int cin, int cout, bool relu, bool out_f32, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
+cudaError_t conv_fwd_tc(int cin, int cout, bool relu, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
                         const float *bias, int nimg, int h, int wd, void *out, const float *res, int *status,
                         cudaStream_t s);
+cudaError_t conv_loss_tc(int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias, int nimg, int h,
+                         int wd, const float *x, const float *target, float scale, __nv_bfloat16 *grad,
+                         float *bias_part, double *loss_part, int *parts, int *status, cudaStream_t s);
+cudaError_t conv_dgrad_tc(int cin, const __nv_bfloat16 *in, const __nv_bfloat16 *w, int nimg, int h, int wd,
+                          const __nv_bfloat16 *act, __nv_bfloat16 *grad, float *bias_part, int *parts, int *status,
+                          cudaStream_t s);
 cudaError_t conv_wgrad_tc(int cin, int cout, const __nv_bfloat16 *dout, const __nv_bfloat16 *in, int nimg, int h,
                           int wd, float *partials, int max_parts, int *parts, int *status, cudaStream_t s);
 
@@ -49,46 +55,42 @@ struct Geo {
     int n, h, w;  // images, rows, columns
 };
 
-// Pixels per bias-gradient partial sum, added in a fixed order by
-// k_reduce_partials.
-constexpr int kChunk = 1024;
-
-// Bias gradient partials: sum over a chunk of pixels of g[p][c] (FP32).
-// 256 threads = 256 / C groups of C channels (C divides 256); group k sums
-// the chunk's pixels k, k + groups, ..., then the groups are added in order.
-__global__ void __launch_bounds__(256) k_bias_partials(const float *__restrict__ g, int npix, int C,
-                                                        float *__restrict__ partials) {
-    __shared__ float red[256];
-    const int groups = (int)blockDim.x / C, c = (int)threadIdx.x % C, grp = (int)threadIdx.x / C;
-    const int pbeg = blockIdx.x * kChunk, pend = min(npix, pbeg + kChunk);
+// A layer's gradients from the per-CTA partial sums: out[i] = sum over k of
+// w_part[k][i] for the nw weights, then the nb biases (which follow them in
+// the parameter vector) from b_part.  Eight threads per output take every
+// eighth partial, 32 neighbouring outputs reading one 128-byte line, and are
+// added in a fixed order.  One thread per output, in order, was a chain of
+// 304 (bias: 768) loads on a few blocks: 16 and 28 us a layer at 16x256x192x64,
+// now about 6 us a layer.
+constexpr int kSlices = 8;
+__global__ void __launch_bounds__(256) k_reduce_grads(const float *__restrict__ w_part, int w_parts, int nw,
+                                                       const float *__restrict__ b_part, int b_parts, int nb,
+                                                       float *__restrict__ out) {
+    __shared__ float red[kSlices][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     float s = 0.f;
-#pragma unroll 8
-    for (int p = pbeg + grp; p < pend; p += groups) s += g[(size_t)p * C + c];
-    red[threadIdx.x] = s;
+    if (i < nw + nb) {
+        const bool bias = i >= nw;
+        const float *p = bias ? b_part + (i - nw) : w_part + i;
+        const int n = bias ? nb : nw, parts = bias ? b_parts : w_parts;
+        int k = slice;
+        for (; k + 7 * kSlices < parts; k += 8 * kSlices) {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = p[(size_t)(k + j * kSlices) * n];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s += v[j];
+        }
+        for (; k < parts; k += kSlices) s += p[(size_t)k * n];
+    }
+    red[slice][lane] = s;
     __syncthreads();
-    if ((int)threadIdx.x < C) {
-        float tot = 0.f;
-        for (int k = 0; k < groups; ++k) tot += red[k * C + threadIdx.x];
-        partials[(size_t)blockIdx.x * C + threadIdx.x] = tot;
-    }
-}
-
-// out[i] = sum over chunks k of partials[k][i], in chunk order; eight
-// partials loaded ahead of their additions.
-__global__ void k_reduce_partials(const float *__restrict__ partials, int chunks, int n, float *__restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float s = 0.f;
-    int k = 0;
-    for (; k + 8 <= chunks; k += 8) {
-        float v[8];
+    if (slice == 0 && i < nw + nb) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = partials[(size_t)(k + j) * n + i];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s += v[j];
+        for (int q = 1; q < kSlices; ++q) s += red[q][lane];
+        out[i] = s;
     }
-    for (; k < chunks; ++k) s += partials[(size_t)k * n + i];
-    out[i] = s;
 }
 
 // Flipped, transposed weights for the data gradient:
@@ -122,37 +124,6 @@ void f32_to_bf16(const float *a, __nv_bfloat16 *b, size_t n, cudaStream_t s) {
     k_f32_to_bf16<<<(unsigned)(blocks < 1 ? 1 : (blocks > 4096 ? 4096 : blocks)), kThreads, 0, s>>>(a, b, n);
 }
 
-// Loss = mean((y - t)^2) (per-block double partials), dy = 2 (y - t) / n.
-// Four values per thread and step (16-byte accesses) when the buffers are
-// 16-byte aligned; each four squares are summed in FP32 before the FP64
-// accumulation (a quarter of the FP64 additions).
-__global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, size_t n, float *__restrict__ dy,
-                      double *__restrict__ partials) {
-    double s = 0.0;
-    const float scale = 2.f / (float)n;
-    const size_t n4 = (((uintptr_t)y | (uintptr_t)t | (uintptr_t)dy) & 15) == 0 ? n / 4 : 0;
-    const size_t stride = (size_t)gridDim.x * blockDim.x, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t i = t0; i < n4; i += stride) {
-        const float4 a = reinterpret_cast<const float4 *>(y)[i], b = reinterpret_cast<const float4 *>(t)[i];
-        const float d0 = a.x - b.x, d1 = a.y - b.y, d2 = a.z - b.z, d3 = a.w - b.w;
-        reinterpret_cast<float4 *>(dy)[i] = make_float4(scale * d0, scale * d1, scale * d2, scale * d3);
-        s += (double)(d0 * d0 + d1 * d1 + d2 * d2 + d3 * d3);
-    }
-    for (size_t i = n4 * 4 + t0; i < n; i += stride) {
-        const float d = y[i] - t[i];
-        s += (double)d * d;
-        dy[i] = scale * d;
-    }
-    __shared__ double red[kThreads];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = kThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partials[blockIdx.x] = red[0];
-}
-
 // One warp: lane l sums p[l], p[l + 32], ..., then the lanes combine in a
 // fixed shuffle order (lane 0's total is the result).
 __global__ void k_sum_double(const double *p, int n, double denom, float *out) {
@@ -160,39 +131,6 @@ __global__ void k_sum_double(const double *p, int n, double denom, float *out) {
     for (int i = threadIdx.x; i < n; i += 32) s += p[i];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (threadIdx.x == 0) *out = (float)(s / denom);
-}
-
-// g = grad of a ReLU output times (activation > 0), FP32 and a BF16 copy.
-__global__ void k_relu_bwd(const float *__restrict__ grad, const __nv_bfloat16 *__restrict__ act, size_t n,
-                           float *__restrict__ g, __nv_bfloat16 *__restrict__ gb) {
-    // Eight values per thread (16-byte accesses) when every buffer is
-    // 16-byte aligned, grid-stride, scalar tail.
-    const size_t n8 = (((uintptr_t)grad | (uintptr_t)act | (uintptr_t)g | (uintptr_t)gb) & 15) == 0 ? n / 8 : 0;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t i = t; i < n8; i += stride) {
-        const float4 g0 = reinterpret_cast<const float4 *>(grad)[2 * i], g1 = reinterpret_cast<const float4 *>(grad)[2 * i + 1];
-        const uint4 a = reinterpret_cast<const uint4 *>(act)[i];
-        const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint16_t bits = (uint16_t)(aw[j / 2] >> (16 * (j & 1)));
-            o[j] = __bfloat162float(__ushort_as_bfloat16(bits)) > 0.f ? gv[j] : 0.f;
-        }
-        reinterpret_cast<float4 *>(g)[2 * i] = make_float4(o[0], o[1], o[2], o[3]);
-        reinterpret_cast<float4 *>(g)[2 * i + 1] = make_float4(o[4], o[5], o[6], o[7]);
-        reinterpret_cast<uint4 *>(gb)[i] = make_uint4(pack_bf16(__float2bfloat16_rn(o[0]), __float2bfloat16_rn(o[1])),
-                                                      pack_bf16(__float2bfloat16_rn(o[2]), __float2bfloat16_rn(o[3])),
-                                                      pack_bf16(__float2bfloat16_rn(o[4]), __float2bfloat16_rn(o[5])),
-                                                      pack_bf16(__float2bfloat16_rn(o[6]), __float2bfloat16_rn(o[7])));
-    }
-    for (size_t i = n8 * 8 + t; i < n; i += stride) {
-        const float v = __bfloat162float(act[i]) > 0.f ? grad[i] : 0.f;
-        g[i] = v;
-        gb[i] = __float2bfloat16_rn(v);
-    }
 }
 
 // Adam (bias-corrected) on FP32 master weights, refreshing the BF16 copy.
@@ -251,12 +189,10 @@ struct ginf_warmnet {
     size_t cap_pix = 0;
     __nv_bfloat16 *a[4] = {};  // a[0] = x (L ch), a[1..3] hidden
     float *y = nullptr;        // output (L ch)
-    float *gy = nullptr;       // dLoss/dy
-    float *g32 = nullptr;      // FP32 gradient scratch (max channels)
-    float *gtmp = nullptr;     // data gradient before the ReLU mask
-    __nv_bfloat16 *gb = nullptr;
+    __nv_bfloat16 *gb[2] = {};  // output gradients of one layer and the next (max channels)
     __nv_bfloat16 *wflip = nullptr;
-    float *partials = nullptr;
+    float *partials = nullptr;   // weight-gradient partial sums, one per CTA (two per SM)
+    float *bias_part = nullptr;  // bias-gradient partial sums
     size_t cap_partials = 0;
     double *loss_part = nullptr;
     float *loss_dev = nullptr;
@@ -331,102 +267,88 @@ ginf_status ensure_batch(ginf_warmnet *n, size_t pix) {
     if (pix <= n->cap_pix) return GINF_OK;
     for (int l = 0; l < 4; ++l) cudaFree(n->a[l]);
     cudaFree(n->y);
-    cudaFree(n->gy);
-    cudaFree(n->g32);
-    cudaFree(n->gtmp);
-    cudaFree(n->gb);
+    cudaFree(n->gb[0]);
+    cudaFree(n->gb[1]);
     const size_t cmax = (size_t)std::max(n->L, n->hidden);
     GINF_WCK(cudaMalloc(&n->a[0], pix * n->L * sizeof(__nv_bfloat16)));
     for (int l = 1; l < 4; ++l) GINF_WCK(cudaMalloc(&n->a[l], pix * n->hidden * sizeof(__nv_bfloat16)));
     GINF_WCK(cudaMalloc(&n->y, pix * n->L * sizeof(float)));
-    GINF_WCK(cudaMalloc(&n->gy, pix * n->L * sizeof(float)));
-    GINF_WCK(cudaMalloc(&n->g32, pix * cmax * sizeof(float)));
-    GINF_WCK(cudaMalloc(&n->gtmp, pix * cmax * sizeof(float)));
-    GINF_WCK(cudaMalloc(&n->gb, pix * cmax * sizeof(__nv_bfloat16)));
+    for (int k = 0; k < 2; ++k) GINF_WCK(cudaMalloc(&n->gb[k], pix * cmax * sizeof(__nv_bfloat16)));
     n->cap_pix = pix;
-    // Partial sums: one per bias chunk of pixels, and one per CTA of the
-    // weight gradient (up to two per SM).
-    const size_t chunks = (pix + kChunk - 1) / kChunk;
+    // Partial sums: one per CTA of a gradient kernel (up to two per SM).
     int sms = 0;
     GINF_WCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device));
-    size_t need = chunks * cmax;
+    size_t need = 0;
     for (int l = 0; l < 4; ++l) need = std::max(need, (size_t)2 * sms * n->cout[l] * 9 * n->cin[l]);
     if (need > n->cap_partials) {
         cudaFree(n->partials);
+        cudaFree(n->bias_part);
         GINF_WCK(cudaMalloc(&n->partials, need * sizeof(float)));
+        GINF_WCK(cudaMalloc(&n->bias_part, (size_t)2 * sms * cmax * sizeof(float)));
         n->cap_partials = need;
     }
     return GINF_OK;
 }
 
-// 3x3 convolution on the tcgen05 path for the supported (cin, cout) pairs.
-cudaError_t conv_fwd(int cin, int cout, bool relu, bool out_f32, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
-                     const float *bias, Geo g, void *out, const float *res, int *status, cudaStream_t s) {
-    return conv_fwd_tc(cin, cout, relu, out_f32, in, w, bias, g.n, g.h, g.w, out, res, status, s);
-}
-
-// Weight gradient on the tcgen05 path: per-CTA partial sums, then their sum
-// in CTA order (deterministic).
-cudaError_t conv_wgrad(int cin, int cout, const __nv_bfloat16 *dout, const __nv_bfloat16 *in, Geo g, float *part,
-                       size_t part_cap, float *dw, int *status, cudaStream_t s) {
-    const size_t nw = (size_t)cout * 9 * cin;
-    const size_t cap = part_cap / nw;
-    int parts = 0;
-    cudaError_t e = conv_wgrad_tc(cin, cout, dout, in, g.n, g.h, g.w, part, cap > 0x7fffffff ? 0x7fffffff : (int)cap,
-                                  &parts, status, s);
-    if (e != cudaSuccess) return e;
-    k_reduce_partials<<<nblocks(nw), kThreads, 0, s>>>(part, parts, (int)nw, dw);
-    return cudaGetLastError();
-}
-
-// y = x + net(x) into y_out (the network's own buffer when null); the last
-// layer reads x itself as its residual.
-ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStream_t s, float *y_out = nullptr) {
+// The hidden layers, from the BF16 of x.
+ginf_status forward_hidden(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStream_t s) {
     const size_t pix = (size_t)g.n * g.h * g.w;
     ginf_status st = ensure_batch(n, pix);
     if (st != GINF_OK) return st;
     f32_to_bf16(x, n->a[0], pix * n->L, s);
     GINF_WCK(cudaGetLastError());
     for (int l = 0; l < 3; ++l)
-        GINF_WCK(conv_fwd(n->cin[l], n->cout[l], true, false, n->a[l], n->wbf + n->woff[l], n->params + n->boff[l], g,
-                          n->a[l + 1], nullptr, status, s));
-    GINF_WCK(conv_fwd(n->cin[3], n->cout[3], false, true, n->a[3], n->wbf + n->woff[3], n->params + n->boff[3], g,
-                      y_out ? y_out : n->y, x, status, s));
+        GINF_WCK(conv_fwd_tc(n->cin[l], n->cout[l], true, n->a[l], n->wbf + n->woff[l], n->params + n->boff[l], g.n, g.h,
+                             g.w, n->a[l + 1], nullptr, status, s));
     return GINF_OK;
 }
 
-// Loss and every parameter gradient (into n->grads) for one batch.
-ginf_status backward(ginf_warmnet *n, const float *target, Geo g, cudaStream_t s) {
-    const size_t pix = (size_t)g.n * g.h * g.w;
-    const size_t ny = pix * n->L;
-    int blocks = (int)std::min<size_t>(1024, nblocks(ny));
-    k_mse<<<blocks, kThreads, 0, s>>>(n->y, target, ny, n->gy, n->loss_part);
-    k_sum_double<<<1, 32, 0, s>>>(n->loss_part, blocks, (double)ny, n->loss_dev);
+// y = x + net(x) into y_out (the network's own buffer when null); the last
+// layer reads x itself as its residual.
+ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStream_t s, float *y_out = nullptr) {
+    ginf_status st = forward_hidden(n, x, g, status, s);
+    if (st != GINF_OK) return st;
+    GINF_WCK(conv_fwd_tc(n->cin[3], n->cout[3], false, n->a[3], n->wbf + n->woff[3], n->params + n->boff[3], g.n, g.h,
+                         g.w, y_out ? y_out : n->y, x, status, s));
+    return GINF_OK;
+}
+
+// Loss and every parameter gradient (into n->grads) for one batch.  The last
+// layer's output stays in its kernel: the loss, the BF16 output gradient and
+// its bias sums leave from the epilogue, and each data gradient passes its
+// ReLU and leaves bias sums the same way, so no FP32 gradient is written.
+// 16x256x192x64: 1334 us a call with separate loss, conversion, ReLU and bias
+// kernels, 941 us so.
+ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo g, cudaStream_t s) {
+    ginf_status st = forward_hidden(n, x, g, n->status, s);
+    if (st != GINF_OK) return st;
+    const size_t ny = (size_t)g.n * g.h * g.w * n->L;
+    if ((uintptr_t)target & 15) {  // the kernel reads it 16 bytes at a time
+        GINF_WCK(cudaMemcpyAsync(n->y, target, ny * sizeof(float), cudaMemcpyDeviceToDevice, s));
+        target = n->y;
+    }
+    int bias_parts = 0;
+    GINF_WCK(conv_loss_tc(n->L, n->a[3], n->wbf + n->woff[3], n->params + n->boff[3], g.n, g.h, g.w, x, target,
+                          2.f / (float)ny, n->gb[0], n->bias_part, n->loss_part, &bias_parts, n->status, s));
+    k_sum_double<<<1, 32, 0, s>>>(n->loss_part, bias_parts, (double)ny, n->loss_dev);
     GINF_WCK(cudaGetLastError());
-    const int chunks = (int)((pix + kChunk - 1) / kChunk);
-    // Layer 4 (linear output): g = dy.
-    const float *gl = n->gy;
-    f32_to_bf16(n->gy, n->gb, ny, s);
-    GINF_WCK(cudaGetLastError());
+    int cur = 0;
     for (int l = 3; l >= 0; --l) {
-        const int ci = n->cin[l], co = n->cout[l];
-        // bias gradient
-        k_bias_partials<<<chunks, 256, 0, s>>>(gl, (int)pix, co, n->partials);
-        k_reduce_partials<<<nblocks(co), kThreads, 0, s>>>(n->partials, chunks, co, n->grads + n->boff[l]);
+        const int ci = n->cin[l], co = n->cout[l], nw = co * 9 * ci;
+        int w_parts = 0;
+        GINF_WCK(conv_wgrad_tc(ci, co, n->gb[cur], n->a[l], g.n, g.h, g.w, n->partials, (int)(n->cap_partials / nw),
+                               &w_parts, n->status, s));
+        k_reduce_grads<<<(nw + co + 31) / 32, 256, 0, s>>>(n->partials, w_parts, nw, n->bias_part, bias_parts, co,
+                                                           n->grads + n->woff[l]);
         GINF_WCK(cudaGetLastError());
-        // weight gradient
-        GINF_WCK(conv_wgrad(ci, co, n->gb, n->a[l], g, n->partials, n->cap_partials, n->grads + n->woff[l], n->status,
-                            s));
         if (l == 0) break;
-        // data gradient: conv of the (BF16) output gradient with the flipped weights
-        k_flip_weights<<<nblocks((size_t)ci * 9 * co), kThreads, 0, s>>>(n->wbf + n->woff[l], ci, co, n->wflip);
+        // Data gradient: conv of the output gradient with the flipped weights,
+        // through the ReLU of layer l-1's output.
+        k_flip_weights<<<nblocks((size_t)nw), kThreads, 0, s>>>(n->wbf + n->woff[l], ci, co, n->wflip);
         GINF_WCK(cudaGetLastError());
-        GINF_WCK(conv_fwd(co, ci, false, true, n->gb, n->wflip, nullptr, g, n->gtmp, nullptr, n->status, s));
-        // through the ReLU of layer l-1's output
-        k_relu_bwd<<<(unsigned)std::min<size_t>(4096, std::max<size_t>(1, nblocks(pix * ci / 8))), kThreads, 0, s>>>(
-            n->gtmp, n->a[l], pix * ci, n->g32, n->gb);
-        GINF_WCK(cudaGetLastError());
-        gl = n->g32;
+        GINF_WCK(conv_dgrad_tc(co, n->gb[cur], n->wflip, g.n, g.h, g.w, n->a[l], n->gb[cur ^ 1], n->bias_part,
+                               &bias_parts, n->status, s));
+        cur ^= 1;
     }
     return GINF_OK;
 }
@@ -519,11 +441,10 @@ ginf_status ginf_warmnet_destroy(ginf_warmnet *n) {
     cudaFree(n->wflip);
     for (int l = 0; l < 4; ++l) cudaFree(n->a[l]);
     cudaFree(n->y);
-    cudaFree(n->gy);
-    cudaFree(n->g32);
-    cudaFree(n->gtmp);
-    cudaFree(n->gb);
+    cudaFree(n->gb[0]);
+    cudaFree(n->gb[1]);
     cudaFree(n->partials);
+    cudaFree(n->bias_part);
     cudaFree(n->loss_part);
     cudaFree(n->loss_dev);
     cudaFree(n->status);
@@ -569,8 +490,7 @@ ginf_status ginf_warmnet_gradients(ginf_warmnet *n, const float *x, const float 
     if (st != GINF_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Geo g{nimg, h, w};
-    if ((st = forward(n, x, g, n->status, s)) != GINF_OK) return st;
-    if ((st = backward(n, target, g, s)) != GINF_OK) return st;
+    if ((st = gradients(n, x, target, g, s)) != GINF_OK) return st;
     if (loss) GINF_WCK(cudaMemcpyAsync(loss, n->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, s));
     if (grads_host)
         GINF_WCK(cudaMemcpyAsync(grads_host, n->grads, n->nparams * sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -585,8 +505,7 @@ ginf_status ginf_warmnet_train_step(ginf_warmnet *n, const float *x, const float
     if (st != GINF_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Geo g{nimg, h, w};
-    if ((st = forward(n, x, g, n->status, s)) != GINF_OK) return st;
-    if ((st = backward(n, target, g, s)) != GINF_OK) return st;
+    if ((st = gradients(n, x, target, g, s)) != GINF_OK) return st;
     n->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)n->step), c2 = 1.f - std::pow(b2, (float)n->step);

@@ -303,3 +303,60 @@ def test_forward_in_place(ginf):
         z = x.clone()
         ginf.check(ginf.lib().ginf_warmnet_forward(net.handle, z.data_ptr(), 2, 40, 150, z.data_ptr(), None))
     assert torch.equal(y, z)
+
+
+@pytest.mark.parametrize("L,shape", [(16, (1, 9, 7)), (32, (2, 5, 131)), (64, (3, 33, 129)), (64, (1, 1, 1))])
+def test_gradients_at_ragged_sizes_vs_torch_float64(ginf, L, shape):
+    """Loss and gradients where bands end inside a warp or a warp lies beyond
+    the image, against PyTorch float64 with the network's BF16 rounding points
+    (within 5e-3, norm-relative, as the oracle's check), and the same from a
+    target that is not 16-byte aligned."""
+    import torch
+    n, h, w = shape
+    g = torch.Generator(device="cuda").manual_seed(L + w)
+    x = torch.rand((n, h, w, L), generator=g, device="cuda")
+    buf = torch.empty(x.numel() + 1, device="cuda")
+    target = x + 0.5 * torch.randn(x.shape, generator=g, device="cuda")
+    with ginf.WarmNet(L, 32, seed=3) as net:
+        loss, grads = net.gradients(x, target)
+        params = net.get_params()
+        odd = buf[1:].view(x.shape)
+        odd.copy_(target)
+        loss2, grads2 = net.gradients(x, odd)
+    assert loss2 == loss and np.array_equal(grads2, grads)
+
+    def bf(a):
+        return a.to(torch.bfloat16).to(torch.float64)
+
+    def conv(a, wt):
+        return torch.nn.functional.conv2d(a.permute(0, 3, 1, 2), wt.permute(0, 3, 1, 2), padding=1).permute(0, 2, 3, 1)
+
+    chans = [L, 32, 32, 32, L]
+    ws, bs, off = [], [], 0
+    for k in range(4):
+        c = chans[k + 1] * 9 * chans[k]
+        ws.append(bf(torch.from_numpy(params[off:off + c]).cuda()).view(chans[k + 1], 3, 3, chans[k]))
+        bs.append(torch.from_numpy(params[off + c:off + c + chans[k + 1]]).cuda().double())
+        off += c + chans[k + 1]
+    acts = [bf(x)]
+    for k in range(3):
+        acts.append(bf(torch.relu(conv(acts[-1], ws[k]) + bs[k])))
+    d = conv(acts[3], ws[3]) + bs[3] + x.double() - target.double()
+    want_loss = float((d ** 2).mean())
+    grad = 2.0 / d.numel() * d
+    parts = []
+    for k in (3, 2, 1, 0):
+        gb = bf(grad)
+        a = acts[k].permute(0, 3, 1, 2)
+        dw = torch.nn.grad.conv2d_weight(a, (chans[k + 1], chans[k], 3, 3), gb.permute(0, 3, 1, 2), padding=1)
+        parts.insert(0, torch.cat([dw.permute(0, 2, 3, 1).reshape(-1), grad.sum((0, 1, 2))]))
+        if k:
+            back = torch.nn.functional.conv_transpose2d(gb.permute(0, 3, 1, 2), ws[k].permute(0, 3, 1, 2), padding=1)
+            grad = back.permute(0, 2, 3, 1) * (acts[k] > 0)
+    want = torch.cat(parts).cpu().numpy()
+    assert abs(loss - want_loss) <= 1e-5 * want_loss
+    off = 0
+    for k in range(4):
+        for c in (chans[k + 1] * 9 * chans[k], chans[k + 1]):
+            assert _rel(grads[off:off + c], want[off:off + c]) < 5e-3, (k, c)
+            off += c
