@@ -659,10 +659,18 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
 // buffers the forward pass uses: A = input rows, M = taps x CIN, where one
 // M = 128 tile holds 128 / CIN taps of one row offset dy as MN atoms one
 // pixel apart (LBO = a pixel's bytes; the taps past dx = +1 are computed and
-// dropped); B = the output-gradient row [128 pixels][COUT], N = COUT.  Each
-// CTA accumulates in tensor memory over all of its rows (K steps of 16
-// pixels) and writes one partial sum; the caller adds the partials in a
-// fixed order, so the result is deterministic.
+// dropped); B = the three output-gradient rows r - 1, r, r + 1 that input row
+// r meets (dy = 2, 1, 0), adjacent in the ring of row buffers and so the MN
+// atoms of one operand (LBO = a row buffer), N = 3 COUT: one MMA serves the
+// three row offsets and reads A once for them.  Where the ring wraps the run
+// splits in two.  Each CTA accumulates in tensor memory over all of its rows
+// (K steps of 16 pixels) and writes one partial sum; the caller adds the
+// partials in a fixed order, so the result is deterministic.
+//
+// Bound: the shared-memory reads of the operands (4 KB of A and COUT x 96
+// bytes of B an MMA).  16x256x192, us a layer (32 -> 64, 32 -> 32, 64 -> 32
+// channels): one MMA per row offset 59, 57, 90; now 46, 35,
+// 56.
 
 struct WgradParams {
     float *partials;  // [CTA][COUT][9][CIN]
@@ -740,7 +748,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
     }
     __syncthreads();
     // Items as in the forward pass: a 128-pixel band of one image, a chunk of
-    // its rows.
+    // its rows.  Step i of an item is input row r = y0 - 1 + i.
     ConvTcParams ip{};
     ip.n = p.n;
     ip.h = p.h;
@@ -752,27 +760,26 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
     if (warp == kCopyWarp) {
         if (lane == 0) {
             uint32_t li = 0, lo = 0;  // input rows, output-gradient rows issued
-            auto in_row = [&](int r, const Item &t) {
-                const int slot = (int)(li % RING);
-                if (!mbar_wait_bounded(&in_empty[slot], ((li / RING) & 1u) ^ 1u, p.status)) return false;
-                mbar_arrive_expect_tx(&in_full[slot], Lay::kInCopy);
-                tma_load_row(smem_addr(sm + Lay::kIn + slot * Lay::kInRow), &in_map, t.x0 - 1, r, t.img, &in_full[slot]);
-                ++li;
-                return true;
-            };
-            auto out_row = [&](int r, const Item &t) {
-                const int slot = (int)(lo % RING);
-                if (!mbar_wait_bounded(&out_empty[slot], ((lo / RING) & 1u) ^ 1u, p.status)) return false;
-                mbar_arrive_expect_tx(&out_full[slot], Lay::kOutCopy);
-                tma_load_row(smem_addr(sm + Lay::kOut + slot * Lay::kOutRow), &out_map, t.x0, r, t.img, &out_full[slot]);
-                ++lo;
-                return true;
-            };
             bool ok = true;
             for (int it = blockIdx.x; it < p.items && ok && !*abort_flag; it += gridDim.x) {
                 const Item t = item_of(ip, it);
-                ok = in_row(t.y0 - 1, t) && in_row(t.y0, t);
-                for (int j = 0; j < t.rows && ok; ++j) ok = in_row(t.y0 + j + 1, t) && out_row(t.y0 + j, t);
+                for (int i = 0; i < t.rows + 2; ++i) {
+                    int slot = (int)(li % RING);
+                    ok = mbar_wait_bounded(&in_empty[slot], ((li / RING) & 1u) ^ 1u, p.status);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(&in_full[slot], Lay::kInCopy);
+                    tma_load_row(smem_addr(sm + Lay::kIn + slot * Lay::kInRow), &in_map, t.x0 - 1, t.y0 - 1 + i, t.img,
+                                 &in_full[slot]);
+                    ++li;
+                    if (i >= t.rows) continue;
+                    slot = (int)(lo % RING);
+                    ok = mbar_wait_bounded(&out_empty[slot], ((lo / RING) & 1u) ^ 1u, p.status);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(&out_full[slot], Lay::kOutCopy);
+                    tma_load_row(smem_addr(sm + Lay::kOut + slot * Lay::kOutRow), &out_map, t.x0, t.y0 + i, t.img,
+                                 &out_full[slot]);
+                    ++lo;
+                }
             }
             if (!ok) *abort_flag = 1;
             for (uint32_t q = li > RING ? li - RING : 0; q < li; ++q)
@@ -783,25 +790,33 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         __syncwarp();
     } else if (warp == kMmaWarp) {
         if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc_bf16_mn(COUT);
             const uint32_t ibase = smem_addr(sm + Lay::kIn), obase = smem_addr(sm + Lay::kOut);
-            uint32_t li = 0, lo = 0;
-            bool ok = true, fresh = true;
+            uint32_t li = 0, lo = 0;  // input row of the step, first output-gradient row of the item
+            bool ok = true, first_item = true;
             for (int it = blockIdx.x; it < p.items && ok && !*abort_flag; it += gridDim.x) {
                 const Item t = item_of(ip, it);
-                const uint32_t base = li;
-                for (int j = 0; j < t.rows && ok; ++j, ++lo) {
-                    // Input rows y - 1, y, y + 1 of output-gradient row y = y0 + j.
-                    for (uint32_t q = j == 0 ? base : base + j + 2; q <= base + j + 2 && ok; ++q)
-                        ok = mbar_wait_bounded(&in_full[q % RING], (q / RING) & 1u, p.status);
-                    if (ok) ok = mbar_wait_bounded(&out_full[lo % RING], (lo / RING) & 1u, p.status);
+                for (int i = 0; i < t.rows + 2 && ok; ++i, ++li) {
+                    ok = mbar_wait_bounded(&in_full[li % RING], (li / RING) & 1u, p.status);
+                    if (ok && i < t.rows)
+                        ok = mbar_wait_bounded(&out_full[(lo + i) % RING], ((lo + i) / RING) & 1u, p.status);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint64_t b0 = smem_desc(obase + (lo % RING) * Lay::kOutRow, 16, 8 * Lay::kOutPix, Lay::kSwOut);
-#pragma unroll
-                    for (int dy = 0; dy < 3; ++dy) {
-                        const uint64_t a0 = smem_desc(ibase + ((base + j + dy) % RING) * Lay::kInRow, Lay::kInPix,
-                                                      8 * Lay::kInPix, Lay::kSwIn);
+                    // Blocks b: output-gradient row y0 + i - 2 + b, dy = 2 - b,
+                    // accumulator columns b * COUT on.
+                    const int blo = i < 2 ? 2 - i : 0, bhi = t.rows + 1 - i < 2 ? t.rows + 1 - i : 2;
+                    const uint64_t a0 = smem_desc(ibase + (li % RING) * Lay::kInRow, Lay::kInPix, 8 * Lay::kInPix,
+                                                  Lay::kSwIn);
+                    // Runs of adjacent row buffers; a block's first use starts
+                    // its accumulator, in a run of its own.
+                    const bool fresh = first_item && i < 3;
+                    for (int b = blo; b <= bhi;) {
+                        const uint32_t slot = (lo + i - 2 + b) % RING;
+                        const bool start = fresh && b == blo;
+                        int n = start ? 1 : bhi - b + 1;
+                        if ((int)slot + n > RING) n = RING - (int)slot;
+                        const uint64_t b0 = smem_desc(obase + slot * Lay::kOutRow, Lay::kOutRow, 8 * Lay::kOutPix,
+                                                      Lay::kSwOut);
+                        const uint32_t idesc = instr_desc_bf16_mn(n * COUT);
 #pragma unroll
                         for (int mt = 0; mt < Lay::kMT; ++mt)
 #pragma unroll
@@ -810,26 +825,22 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                                 // mt * kTaps pixels in, K step ks 16 pixels on.
                                 const uint64_t ao = (uint64_t)((mt * Lay::kTaps + 16 * ks) * Lay::kInPix >> 4);
                                 const uint64_t bo = (uint64_t)(16 * ks * Lay::kOutPix >> 4);
-                                umma_bf16(tmem + (dy * Lay::kMT + mt) * COUT, a0 + ao, b0 + bo, idesc,
-                                          fresh && ks == 0 ? 0u : 1u);
+                                umma_bf16(tmem + (mt * 3 + b) * COUT, a0 + ao, b0 + bo, idesc, start && ks == 0 ? 0u : 1u);
                             }
+                        b += n;
                     }
-                    fresh = false;
-                    umma_commit(&out_empty[lo % RING]);
-                    umma_commit(&in_empty[(base + j) % RING]);
-                    if (j == t.rows - 1) {
-                        umma_commit(&in_empty[(base + j + 1) % RING]);
-                        umma_commit(&in_empty[(base + j + 2) % RING]);
-                    }
+                    umma_commit(&in_empty[li % RING]);
+                    if (blo == 0) umma_commit(&out_empty[(lo + i - 2) % RING]);  // its last use
                 }
-                li = base + t.rows + 2;
+                first_item = false;
+                lo += t.rows;
             }
             if (!ok) *abort_flag = 1;
             umma_commit(done);
         }
         __syncwarp();
     } else {
-        // Epilogue, once: accumulator (dy, mt), lane m = 32 * warp + lane is
+        // Epilogue, once: accumulator (mt, dy), lane m = 32 * warp + lane is
         // tap dx = mt * kTaps + m / CIN, channel m % CIN.
         const bool ok = __all_sync(~0u, mbar_wait_bounded(done, 0, p.status));
         if (ok && !__any_sync(~0u, *abort_flag)) {
@@ -838,7 +849,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
             float *part = p.partials + (size_t)blockIdx.x * COUT * 9 * CIN;
 #pragma unroll 1
             for (int a = 0; a < Lay::kAcc; ++a) {
-                const int dy = a / Lay::kMT, dx = (a % Lay::kMT) * Lay::kTaps + m / CIN;
+                const int dy = 2 - a % 3, dx = (a / 3) * Lay::kTaps + m / CIN;
                 float v[COUT];
 #pragma unroll
                 for (int c = 0; c < COUT; c += 16)
