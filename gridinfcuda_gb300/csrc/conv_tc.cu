@@ -28,16 +28,21 @@
 // tensor-memory slots (adjacent unless the ring wraps, when the run splits in
 // two), and the first block into a fresh slot overwrites it.
 //
-// Roles (192 threads): warp 4 lane 0 issues the row copies into a ring of
-// RING buffers; warp 5 lane 0 issues, per input row, 3 * CIN / 16 steps of
-// one or two MMAs (descriptors formed once per row, compile-time step
-// offsets) and commits them to mbarriers (a row buffer is free after its own
-// MMAs; an output row's accumulator is full after input row r + 1); warps 0-3
-// read the accumulator back (warp w owns lanes 32w..32w+31, i.e. pixels 32w..
-// of the tile), add the bias, apply ReLU, stage the warp's 32 pixels in
-// shared memory and store them 512 bytes per instruction, adding the
-// residual in that pass.  Every wait is bounded (DEV_ERR_TIMEOUT in the
-// status word), and the tensor memory is released on every path.
+// Roles (10 warps; 6 at 16 output channels): 8 (4) warps read the accumulator
+// back (warp w owns lanes 32 (w % 4) .. + 31, i.e. those pixels of the tile,
+// and half of 32 or more output channels), add the bias, apply ReLU, stage
+// the 32 pixels in shared memory and store them 512 bytes per instruction,
+// adding the residual in that pass; of the next warp lane 0 issues the row
+// copies into a ring of RING buffers; of the last, lane 0 issues, per input
+// row, 3 * CIN / 16 steps of one or two MMAs (descriptors formed once per
+// row, compile-time step offsets) and commits them to mbarriers (a row buffer
+// is free after its own MMAs; an output row's accumulator is full after input
+// row r + 1).  The epilogues' latencies (tensor memory, staging, the residual
+// and target loads) bound the larger layers, hence two warps on each quarter
+// of the lanes: at 16x256x192x64 the loss layer 178 -> 155 us, the data
+// gradients 66 / 59 / 58 -> 63 / 54 / 54, the others equal; loads of the loss
+// in groups of four passes, eight spill.
+// Every wait is bounded (DEV_ERR_TIMEOUT in the status word), and the tensor memory is released on every path.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -80,7 +85,7 @@ enum {
 
 constexpr int kTileM = 128;            // pixels per tile (MMA M)
 constexpr int kSlab = kTileM + 2;      // pixels per row copy: the band and one either side
-constexpr int kThreadsTc = 192;        // warps 0-3 epilogue, 4 copies, 5 MMA
+constexpr int kThreadsTc = 192;        // weight gradient: warps 0-3 epilogue, 4 copies, 5 MMA
 constexpr int kCopyWarp = 4, kMmaWarp = 5;
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
@@ -161,8 +166,15 @@ __device__ __forceinline__ Item item_of(const ConvTcParams &p, int it) {
     return r;
 }
 
+// Epilogue warps of a convolution: two per 32 tensor-memory lanes, each with
+// half the channels, where half is a tensor-memory load (16 columns) or more.
+constexpr int epi_warps(int cout) { return cout >= 32 ? 8 : 4; }
+
 template <int CIN, int COUT, bool OUT_F32, int RING>
 struct TcLayout {
+    static constexpr int kEpi = epi_warps(COUT);
+    static constexpr int kThreads = (kEpi + 2) * 32;  // + copies, MMA
+    static constexpr int kCols4 = COUT * 4 / kEpi;    // channels per epilogue warp
     static constexpr int kChunks = CIN / 8;
     static constexpr int kPixBytes = CIN * 2;                          // one pixel: one swizzle row
     static constexpr uint32_t kSwizzle = CIN == 64 ? 2 : (CIN == 32 ? 4 : 6);
@@ -172,11 +184,11 @@ struct TcLayout {
     static constexpr int kRows = 0;
     static constexpr int kW = kRows + RING * kRowBytes;
     static constexpr int kBias = kW + kWBytes;
-    static constexpr int kOutBytes = COUT * (OUT_F32 ? 4 : 2);  // one pixel's outputs
+    static constexpr int kOutBytes = kCols4 * (OUT_F32 ? 4 : 2);  // one pixel's outputs of one warp
     static constexpr int kChunksOut = kOutBytes / 16;
     static constexpr int kStagePitch = kOutBytes + 16;
-    static constexpr int kStage = (kBias + COUT * 4 + 15) / 16 * 16;  // 4 warps x 32 pixel rows
-    static constexpr int kBars = kStage + 4 * 32 * kStagePitch;
+    static constexpr int kStage = (kBias + COUT * 4 + 15) / 16 * 16;  // epilogue warps x 32 pixel rows
+    static constexpr int kBars = kStage + kEpi * 32 * kStagePitch;
     static constexpr int kAcc = COUT == 64 ? 4 : 8;  // accumulator slots in tensor memory
     static constexpr int kNumBars = 2 * RING + 2 * kAcc + 1;  // full, empty, acc_full, acc_empty, done
     static constexpr int kTmemSlot = kBars + kNumBars * 8;
@@ -208,7 +220,7 @@ __device__ __forceinline__ uint2 pack_bf16x4(const float *v) {
 
 // OUT_F32: FP32 results are staged (and stored, with EPI_STORE).
 template <int CIN, int COUT, bool RELU, bool OUT_F32, int RING, int EPI = EPI_STORE>
-__global__ void __launch_bounds__(kThreadsTc, 2)
+__global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
     k_conv_tc(const __grid_constant__ CUtensorMap rows_map, const ConvTcParams p) {
     using Lay = TcLayout<CIN, COUT, OUT_F32, RING>;
     static_assert((CIN == 16 || CIN == 32 || CIN == 64) && COUT % 16 == 0 && COUT <= 256, "tile shape");
@@ -221,7 +233,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
     volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Lay::kAbort);
     float *bias = reinterpret_cast<float *>(sm + Lay::kBias);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char *stage = sm + Lay::kStage + (warp & 3) * 32 * Lay::kStagePitch;
+    unsigned char *stage = sm + Lay::kStage + warp * 32 * Lay::kStagePitch;  // epilogue warps only
 
     // Weights into [dx][chunk][j * COUT + co][8 channels]: for one column
     // offset dx the three row offsets dy = j - 1 stacked along N, so one MMA
@@ -240,7 +252,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         }
         for (int i = 0; i < Lay::kAcc; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], 4 * 32);
+            mbar_init(&acc_empty[i], Lay::kEpi * 32);
         }
         mbar_init(done, 1);
         *abort_flag = 0;
@@ -263,7 +275,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
     }
     __syncthreads();
 
-    if (warp == kCopyWarp) {
+    if (warp == Lay::kEpi) {
         if (lane == 0) {
             uint32_t ld = 0;
             for (int it = blockIdx.x; it < p.items && !*abort_flag; it += gridDim.x) {
@@ -284,7 +296,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 mbar_wait_bounded(&full[q % RING], (q / RING) & 1u, nullptr);
         }
         __syncwarp();
-    } else if (warp == kMmaWarp) {
+    } else if (warp == Lay::kEpi + 1) {
         if (lane == 0) {
             constexpr int ACC = Lay::kAcc;
             const uint32_t rbase = smem_addr(sm + Lay::kRows);
@@ -348,9 +360,12 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         }
         __syncwarp();
     } else {
-        // Epilogue: warp w reads lanes 32w..32w+31 of the accumulator.
+        // Epilogue: warp w reads lanes 32 (w % 4) .. + 31 of the accumulator,
+        // channels c0 .. c0 + CW - 1.
+        constexpr int CW = Lay::kCols4;
+        const int quarter = warp & 3, c0 = (warp >> 2) * CW;
         uint32_t tile = 0;
-        const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         // EPI_MASK, EPI_LOSS: this lane's four channels (chunk lane % kChunksOut
         // of a pixel, the same in every pass) and its squares as a float pair.
         float bsum[4] = {0.f, 0.f, 0.f, 0.f}, loss_hi = 0.f, loss_lo = 0.f;
@@ -365,15 +380,15 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                     break;
                 }
                 tc_fence_after();
-                float v[COUT];
+                float v[CW];
 #pragma unroll
-                for (int c = 0; c < COUT; c += 16)
-                    tmem_load16(tmem + lane_base + acc_col<COUT, Lay::kAcc>(tile) + c, v + c);
+                for (int c = 0; c < CW; c += 16)
+                    tmem_load16(tmem + lane_base + acc_col<COUT, Lay::kAcc>(tile) + c0 + c, v + c);
                 tc_fence_before();
                 mbar_arrive(&acc_empty[acc]);
 #pragma unroll
-                for (int c = 0; c < COUT; ++c) {
-                    v[c] += bias[c];
+                for (int c = 0; c < CW; ++c) {
+                    v[c] += bias[c0 + c];
                     if (RELU) v[c] = fmaxf(v[c], 0.f);
                 }
                 // This lane's pixel into the warp's staging rows (a pitch of
@@ -400,21 +415,27 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 // ... then the warp's 32 pixels, contiguous in the output,
                 // written 512 bytes per instruction (the residual read the
                 // same way).
-                const int x = t.x0 + warp * 32;
+                const int x = t.x0 + quarter * 32;
                 const int valid = p.w - x < 32 ? p.w - x : 32;
                 const size_t pix = ((size_t)t.img * p.h + t.y0 + j) * p.w + x;
-                uint4 *o = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(p.out) + pix * Lay::kOutBytes);
-                const uint4 *rs = OUT_F32 && p.res ? reinterpret_cast<const uint4 *>(p.res + pix * COUT) : nullptr;
+                // 16-byte chunk q of the warp's block: pixel q / kChunksOut,
+                // chunk q % kChunksOut of its channels, at(q) in the tensor.
+                constexpr int kPixChunks = Lay::kChunksOut * Lay::kEpi / 4;  // of a whole pixel
+                auto at = [&](int q) { return (q / Lay::kChunksOut) * kPixChunks + q % Lay::kChunksOut; };
+                const size_t first = pix * COUT + c0;
+                uint4 *o = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(p.out) + first * (OUT_F32 ? 4 : 2));
+                const uint4 *rs = OUT_F32 && p.res ? reinterpret_cast<const uint4 *>(p.res + first) : nullptr;
                 const int nq = valid * Lay::kChunksOut;
                 if constexpr (EPI != EPI_STORE) {
                     // Passes in groups whose loads are all in flight at once;
                     // a row's sums first, then the running ones.
-                    constexpr int kGroup = Lay::kChunksOut < 8 ? Lay::kChunksOut : 8;
+                    constexpr int kMost = EPI == EPI_LOSS ? 4 : 8;
+                    constexpr int kGroup = Lay::kChunksOut < kMost ? Lay::kChunksOut : kMost;
                     float rsum[4] = {0.f, 0.f, 0.f, 0.f};
-                    uint2 *g = reinterpret_cast<uint2 *>(static_cast<__nv_bfloat16 *>(p.out) + pix * COUT);
-                    const uint2 *act = EPI == EPI_MASK ? reinterpret_cast<const uint2 *>(p.act + pix * COUT) : nullptr;
-                    const float4 *res = EPI == EPI_LOSS ? reinterpret_cast<const float4 *>(p.res + pix * COUT) : nullptr;
-                    const float4 *tgt = EPI == EPI_LOSS ? reinterpret_cast<const float4 *>(p.target + pix * COUT) : nullptr;
+                    uint2 *g = reinterpret_cast<uint2 *>(static_cast<__nv_bfloat16 *>(p.out) + first);
+                    const uint2 *act = EPI == EPI_MASK ? reinterpret_cast<const uint2 *>(p.act + first) : nullptr;
+                    const float4 *res = EPI == EPI_LOSS ? reinterpret_cast<const float4 *>(p.res + first) : nullptr;
+                    const float4 *tgt = EPI == EPI_LOSS ? reinterpret_cast<const float4 *>(p.target + first) : nullptr;
 #pragma unroll
                     for (int i0 = 0; i0 < Lay::kChunksOut; i0 += kGroup) {
                         uint2 av[kGroup];
@@ -423,10 +444,10 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                         for (int i = 0; i < kGroup; ++i) {
                             const int q = lane + 32 * (i0 + i);
                             if (q < nq) {
-                                if (EPI == EPI_MASK) av[i] = act[q];
+                                if (EPI == EPI_MASK) av[i] = act[at(q)];
                                 if (EPI == EPI_LOSS) {
-                                    xv[i] = res[q];
-                                    tv[i] = tgt[q];
+                                    xv[i] = res[at(q)];
+                                    tv[i] = tgt[at(q)];
                                 }
                             }
                         }
@@ -456,7 +477,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                                 }
 #pragma unroll
                                 for (int k = 0; k < 4; ++k) rsum[k] += o[k];
-                                g[q] = pack_bf16x4(o);
+                                g[at(q)] = pack_bf16x4(o);
                             }
                         }
                     }
@@ -469,7 +490,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 if (OUT_F32 && rs) {
 #pragma unroll
                     for (int i = 0; i < Lay::kChunksOut; ++i)
-                        if (lane + 32 * i < nq) r[i] = rs[lane + 32 * i];
+                        if (lane + 32 * i < nq) r[i] = rs[at(lane + 32 * i)];
                 }
 #pragma unroll
                 for (int i = 0; i < Lay::kChunksOut; ++i) {
@@ -482,14 +503,14 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                                          __float_as_uint(__uint_as_float(val.y) + __uint_as_float(r[i].y)),
                                          __float_as_uint(__uint_as_float(val.z) + __uint_as_float(r[i].z)),
                                          __float_as_uint(__uint_as_float(val.w) + __uint_as_float(r[i].w)));
-                    o[q] = val;
+                    o[at(q)] = val;
                 }
                 __syncwarp();
             }
         }
         if constexpr (EPI != EPI_STORE) {
             // The CTA's sums, in a fixed order: lanes of one channel chunk, then
-            // the four warps.
+            // the warps of the same channels.
 #pragma unroll
             for (int off = Lay::kChunksOut; off < 32; off <<= 1)
 #pragma unroll
@@ -498,26 +519,26 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
             if (lane < Lay::kChunksOut)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) red[4 * lane + k] = bsum[k];
-            double *lred = reinterpret_cast<double *>(stage + COUT * 4);
+            double *lred = reinterpret_cast<double *>(stage + CW * 4);
             if (EPI == EPI_LOSS) {
                 double l = (double)loss_hi + (double)loss_lo;
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(~0u, l, off);
                 if (lane == 0) *lred = l;
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");  // the epilogue's four warps
+            asm volatile("bar.sync 1, %0;" ::"n"(Lay::kEpi * 32) : "memory");  // the epilogue's warps
             constexpr int kWarpStage = 32 * Lay::kStagePitch;
             if (threadIdx.x < COUT) {
                 float t = 0.f;
 #pragma unroll
                 for (int w = 0; w < 4; ++w)
-                    t += reinterpret_cast<const float *>(sm + Lay::kStage + w * kWarpStage)[threadIdx.x];
+                    t += reinterpret_cast<const float *>(sm + Lay::kStage + (threadIdx.x / CW * 4 + w) * kWarpStage)[threadIdx.x % CW];
                 p.bias_part[(size_t)blockIdx.x * COUT + threadIdx.x] = t;
             }
             if (EPI == EPI_LOSS && threadIdx.x == 0) {
                 double t = 0.0;
-                for (int w = 0; w < 4; ++w)
-                    t += *reinterpret_cast<const double *>(sm + Lay::kStage + w * kWarpStage + COUT * 4);
+                for (int w = 0; w < Lay::kEpi; ++w)
+                    t += *reinterpret_cast<const double *>(sm + Lay::kStage + w * kWarpStage + CW * 4);
                 p.loss_part[blockIdx.x] = t;
             }
         }
@@ -648,7 +669,7 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
     p.chunks = pl.chunks;
     p.items = pl.items;
     if (parts) *parts = pl.grid;
-    kern<<<pl.grid, kThreadsTc, kSmem, s>>>(map, p);
+    kern<<<pl.grid, Lay::kThreads, kSmem, s>>>(map, p);
     return cudaGetLastError();
 }
 
@@ -669,8 +690,7 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
 //
 // Bound: the shared-memory reads of the operands (4 KB of A and COUT x 96
 // bytes of B an MMA).  16x256x192, us a layer (32 -> 64, 32 -> 32, 64 -> 32
-// channels): one MMA per row offset 59, 57, 90; now 46, 35,
-// 56.
+// channels): one MMA per row offset 59, 57, 90; now 46, 35, 56.
 
 struct WgradParams {
     float *partials;  // [CTA][COUT][9][CIN]

@@ -318,7 +318,7 @@ ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStr
 // its bias sums leave from the epilogue, and each data gradient passes its
 // ReLU and leaves bias sums the same way, so no FP32 gradient is written.
 // 16x256x192x64: 1334 us a call with separate loss, conversion, ReLU and bias
-// kernels, 941 us so.
+// kernels, 941 us so (816 with the later changes in conv_tc.cu).
 ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo g, cudaStream_t s) {
     ginf_status st = forward_hidden(n, x, g, n->status, s);
     if (st != GINF_OK) return st;
