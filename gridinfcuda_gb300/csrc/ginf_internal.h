@@ -133,6 +133,24 @@ struct SmemLimit {
     }
 };
 
+// Launches a kernel with programmatic stream serialisation: it may begin
+// while the kernel before it in the stream still runs, and waits for that one
+// in grid_dependency_wait().
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Resident blocks per SM of a kernel at a given dynamic shared memory size:
 // the last answer per device, kept as one word (size + 1 in the high half,
 // blocks in the low half) so readers never see a torn pair.

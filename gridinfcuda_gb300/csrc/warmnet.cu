@@ -25,6 +25,7 @@
 
 #include "ginf_gb300.h"
 #include "ginf_internal.h"
+#include "ptx.cuh"
 
 namespace ginf_gpu {
 
@@ -62,12 +63,27 @@ struct Geo {
 // added in a fixed order.  One thread per output, in order, was a chain of
 // 304 (bias: 768) loads on a few blocks: 16 and 28 us a layer at 16x256x192x64,
 // now about 6 us a layer.
+//
+// With loss_part, one more block (its warp 0) sums the loss: lane l takes
+// loss_part[l], loss_part[l + 32], ..., then the lanes combine in a fixed
+// order.
 constexpr int kSlices = 8;
 __global__ void __launch_bounds__(256) k_reduce_grads(const float *__restrict__ w_part, int w_parts, int nw,
                                                        const float *__restrict__ b_part, int b_parts, int nb,
-                                                       float *__restrict__ out) {
+                                                       float *__restrict__ out, const double *loss_part,
+                                                       double denom, float *loss) {
     __shared__ float red[kSlices][32];
     const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    grid_dependency_wait();
+    launch_dependents();
+    if (loss_part && blockIdx.x == gridDim.x - 1) {
+        if (slice != 0) return;
+        double s = 0.0;
+        for (int i = lane; i < b_parts; i += 32) s += loss_part[i];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) *loss = (float)(s / denom);
+        return;
+    }
     const int i = blockIdx.x * 32 + lane;
     float s = 0.f;
     if (i < nw + nb) {
@@ -93,15 +109,6 @@ __global__ void __launch_bounds__(256) k_reduce_grads(const float *__restrict__ 
     }
 }
 
-// Flipped, transposed weights for the data gradient:
-// wf[ci][tap'][co] = w[co][8 - tap'][ci].
-__global__ void k_flip_weights(const __nv_bfloat16 *__restrict__ w, int cin, int cout, __nv_bfloat16 *__restrict__ wf) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cin * 9 * cout) return;
-    const int co = i % cout, tap = (i / cout) % 9, ci = i / (cout * 9);
-    wf[i] = w[((size_t)co * 9 + (8 - tap)) * cin + ci];
-}
-
 // Round to BF16, eight values per thread (two 16-byte loads, one 16-byte
 // store) when both buffers are 16-byte aligned, grid-stride, scalar tail.
 __global__ void k_f32_to_bf16(const float *__restrict__ a, __nv_bfloat16 *__restrict__ b, size_t n) {
@@ -122,15 +129,6 @@ __global__ void k_f32_to_bf16(const float *__restrict__ a, __nv_bfloat16 *__rest
 void f32_to_bf16(const float *a, __nv_bfloat16 *b, size_t n, cudaStream_t s) {
     const size_t blocks = (n / 8 + kThreads - 1) / kThreads;
     k_f32_to_bf16<<<(unsigned)(blocks < 1 ? 1 : (blocks > 4096 ? 4096 : blocks)), kThreads, 0, s>>>(a, b, n);
-}
-
-// One warp: lane l sums p[l], p[l + 32], ..., then the lanes combine in a
-// fixed shuffle order (lane 0's total is the result).
-__global__ void k_sum_double(const double *p, int n, double denom, float *out) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += 32) s += p[i];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) *out = (float)(s / denom);
 }
 
 // Adam (bias-corrected) on FP32 master weights, refreshing the BF16 copy.
@@ -190,13 +188,18 @@ struct ginf_warmnet {
     __nv_bfloat16 *a[4] = {};  // a[0] = x (L ch), a[1..3] hidden
     float *y = nullptr;        // output (L ch)
     __nv_bfloat16 *gb[2] = {};  // output gradients of one layer and the next (max channels)
-    __nv_bfloat16 *wflip = nullptr;
     float *partials = nullptr;   // weight-gradient partial sums, one per CTA (two per SM)
     float *bias_part = nullptr;  // bias-gradient partial sums
     size_t cap_partials = 0;
     double *loss_part = nullptr;
-    float *loss_dev = nullptr;
-    int *status = nullptr;  // device word: DEV_ERR_* from the convolution kernels' bounded waits
+    // The loss and the status word (DEV_ERR_* from the convolution kernels'
+    // bounded waits) on the device, and where one copy leaves both on the host.
+    struct Report {
+        float loss;
+        int status;
+    };
+    Report *report = nullptr, *report_host = nullptr;
+    int *status = nullptr;  // &report->status
 };
 
 namespace {
@@ -238,20 +241,22 @@ ginf_status alloc_params(ginf_warmnet *n) {
     GINF_WCK(cudaMemset(n->adam_m, 0, n->nparams * sizeof(float)));
     GINF_WCK(cudaMemset(n->adam_v, 0, n->nparams * sizeof(float)));
     GINF_WCK(cudaMemset(n->grads, 0, n->nparams * sizeof(float)));
-    size_t wf = 0;
-    for (int l = 0; l < 4; ++l) wf = std::max(wf, (size_t)n->cout[l] * 9 * n->cin[l]);
-    GINF_WCK(cudaMalloc(&n->wflip, wf * sizeof(__nv_bfloat16)));
     GINF_WCK(cudaMalloc(&n->loss_part, 1024 * sizeof(double)));
-    GINF_WCK(cudaMalloc(&n->loss_dev, sizeof(float)));
-    GINF_WCK(cudaMalloc(&n->status, sizeof(int)));
-    GINF_WCK(cudaMemset(n->status, 0, sizeof(int)));
+    GINF_WCK(cudaMalloc(&n->report, sizeof(ginf_warmnet::Report)));
+    GINF_WCK(cudaMemset(n->report, 0, sizeof(ginf_warmnet::Report)));
+    GINF_WCK(cudaMallocHost(&n->report_host, sizeof(ginf_warmnet::Report)));
+    n->status = &n->report->status;
     return GINF_OK;
 }
 
-// After a synchronisation: a wait in a convolution kernel that ran out.
-ginf_status check_status(ginf_warmnet *n) {
-    int st = 0;
-    GINF_WCK(cudaMemcpy(&st, n->status, sizeof(int), cudaMemcpyDeviceToHost));
+// The end of a call: the loss (when asked for) and the status word in one
+// copy ahead of the synchronisation, then a wait in a convolution kernel that
+// ran out.
+ginf_status finish(ginf_warmnet *n, float *loss, cudaStream_t s) {
+    GINF_WCK(cudaMemcpyAsync(n->report_host, n->report, sizeof(ginf_warmnet::Report), cudaMemcpyDeviceToHost, s));
+    GINF_WCK(cudaStreamSynchronize(s));
+    if (loss) *loss = n->report_host->loss;
+    const int st = n->report_host->status;
     if (st == 0) return GINF_OK;
     GINF_WCK(cudaMemset(n->status, 0, sizeof(int)));
     return wfail(GINF_ERR_TIMEOUT, "warm-start convolution: a device wait ran out (status " + std::to_string(st) + ")");
@@ -318,35 +323,34 @@ ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStr
 // its bias sums leave from the epilogue, and each data gradient passes its
 // ReLU and leaves bias sums the same way, so no FP32 gradient is written.
 // 16x256x192x64: 1334 us a call with separate loss, conversion, ReLU and bias
-// kernels, 941 us so (816 with the later changes in conv_tc.cu).
+// kernels, 941 us so; with the later changes in conv_tc.cu 816, with the
+// programmatic launches, the weights flipped as the data gradient loads them
+// and one copy for loss and status 746.
 ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo g, cudaStream_t s) {
-    ginf_status st = forward_hidden(n, x, g, n->status, s);
+    const size_t pix = (size_t)g.n * g.h * g.w, ny = pix * n->L;
+    ginf_status st = ensure_batch(n, pix);
     if (st != GINF_OK) return st;
-    const size_t ny = (size_t)g.n * g.h * g.w * n->L;
     if ((uintptr_t)target & 15) {  // the kernel reads it 16 bytes at a time
         GINF_WCK(cudaMemcpyAsync(n->y, target, ny * sizeof(float), cudaMemcpyDeviceToDevice, s));
         target = n->y;
     }
+    if ((st = forward_hidden(n, x, g, n->status, s)) != GINF_OK) return st;
     int bias_parts = 0;
     GINF_WCK(conv_loss_tc(n->L, n->a[3], n->wbf + n->woff[3], n->params + n->boff[3], g.n, g.h, g.w, x, target,
                           2.f / (float)ny, n->gb[0], n->bias_part, n->loss_part, &bias_parts, n->status, s));
-    k_sum_double<<<1, 32, 0, s>>>(n->loss_part, bias_parts, (double)ny, n->loss_dev);
-    GINF_WCK(cudaGetLastError());
     int cur = 0;
     for (int l = 3; l >= 0; --l) {
         const int ci = n->cin[l], co = n->cout[l], nw = co * 9 * ci;
         int w_parts = 0;
         GINF_WCK(conv_wgrad_tc(ci, co, n->gb[cur], n->a[l], g.n, g.h, g.w, n->partials, (int)(n->cap_partials / nw),
                                &w_parts, n->status, s));
-        k_reduce_grads<<<(nw + co + 31) / 32, 256, 0, s>>>(n->partials, w_parts, nw, n->bias_part, bias_parts, co,
-                                                           n->grads + n->woff[l]);
-        GINF_WCK(cudaGetLastError());
+        const bool last = l == 3;  // with the loss
+        GINF_WCK(launch_after(k_reduce_grads, (nw + co + 31) / 32 + last, 256, 0, s, n->partials, w_parts, nw,
+                              n->bias_part, bias_parts, co, n->grads + n->woff[l], last ? n->loss_part : nullptr,
+                              (double)ny, &n->report->loss));
         if (l == 0) break;
-        // Data gradient: conv of the output gradient with the flipped weights,
-        // through the ReLU of layer l-1's output.
-        k_flip_weights<<<nblocks((size_t)nw), kThreads, 0, s>>>(n->wbf + n->woff[l], ci, co, n->wflip);
-        GINF_WCK(cudaGetLastError());
-        GINF_WCK(conv_dgrad_tc(co, n->gb[cur], n->wflip, g.n, g.h, g.w, n->a[l], n->gb[cur ^ 1], n->bias_part,
+        // Data gradient, through the ReLU of layer l-1's output.
+        GINF_WCK(conv_dgrad_tc(co, n->gb[cur], n->wbf + n->woff[l], g.n, g.h, g.w, n->a[l], n->gb[cur ^ 1], n->bias_part,
                                &bias_parts, n->status, s));
         cur ^= 1;
     }
@@ -438,7 +442,6 @@ ginf_status ginf_warmnet_destroy(ginf_warmnet *n) {
     cudaFree(n->adam_v);
     cudaFree(n->grads);
     cudaFree(n->wbf);
-    cudaFree(n->wflip);
     for (int l = 0; l < 4; ++l) cudaFree(n->a[l]);
     cudaFree(n->y);
     cudaFree(n->gb[0]);
@@ -446,8 +449,8 @@ ginf_status ginf_warmnet_destroy(ginf_warmnet *n) {
     cudaFree(n->partials);
     cudaFree(n->bias_part);
     cudaFree(n->loss_part);
-    cudaFree(n->loss_dev);
-    cudaFree(n->status);
+    cudaFree(n->report);
+    cudaFreeHost(n->report_host);
     delete n;
     return GINF_OK;
 }
@@ -479,8 +482,7 @@ ginf_status ginf_warmnet_forward(ginf_warmnet *n, const float *x, int32_t nimg, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     ginf_status st = warmnet_forward_into(n, x, nimg, h, w, out, s);
     if (st != GINF_OK) return st;
-    GINF_WCK(cudaStreamSynchronize(s));
-    return check_status(n);
+    return finish(n, nullptr, s);
 }
 
 ginf_status ginf_warmnet_gradients(ginf_warmnet *n, const float *x, const float *target, int32_t nimg, int32_t h,
@@ -491,11 +493,9 @@ ginf_status ginf_warmnet_gradients(ginf_warmnet *n, const float *x, const float 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Geo g{nimg, h, w};
     if ((st = gradients(n, x, target, g, s)) != GINF_OK) return st;
-    if (loss) GINF_WCK(cudaMemcpyAsync(loss, n->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, s));
     if (grads_host)
         GINF_WCK(cudaMemcpyAsync(grads_host, n->grads, n->nparams * sizeof(float), cudaMemcpyDeviceToHost, s));
-    GINF_WCK(cudaStreamSynchronize(s));
-    return check_status(n);
+    return finish(n, loss, s);
 }
 
 ginf_status ginf_warmnet_train_step(ginf_warmnet *n, const float *x, const float *target, int32_t nimg, int32_t h,
@@ -512,9 +512,7 @@ ginf_status ginf_warmnet_train_step(ginf_warmnet *n, const float *x, const float
     k_adam<<<nblocks(n->nparams), kThreads, 0, s>>>(n->params, n->grads, n->adam_m, n->adam_v, (int)n->nparams, lr,
                                                     b1, b2, 1e-8f, c1, c2, n->wbf);
     GINF_WCK(cudaGetLastError());
-    if (loss) GINF_WCK(cudaMemcpyAsync(loss, n->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, s));
-    GINF_WCK(cudaStreamSynchronize(s));
-    return check_status(n);
+    return finish(n, loss, s);
 }
 
 // Checkpoint: magic "GINFWNET", u32 version, u32 L, u32 hidden, i64 Adam step,
