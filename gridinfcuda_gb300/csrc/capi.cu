@@ -1230,7 +1230,7 @@ static ginf_status decode_hbp_seeded(ginf_workspace *wsp, const ginf_grid *grid,
         ++c.launches;
         if (net) {
             if ((st = warmnet_forward(net, x, 1, lt.H, lt.W, &y, P.status, s)) != GINF_OK) break;
-            c.launches += 5;
+            c.launches += 4;
         }
         // Seeded path: level-t messages from the prediction, its own sweeps,
         // then the finer levels.

@@ -28,22 +28,24 @@
 // tensor-memory slots (adjacent unless the ring wraps, when the run splits in
 // two), and the first block into a fresh slot overwrites it.
 //
-// Roles (10 warps; 6 at 16 output channels): 8 (4) warps read the accumulator
-// back (warp w owns lanes 32 (w % 4) .. + 31, i.e. those pixels of the tile,
-// and half of 32 or more output channels), add the bias, apply ReLU, stage
-// the 32 pixels in shared memory and store them 512 bytes per instruction,
-// adding the residual in that pass; of the next warp lane 0 issues the row
-// copies into a ring of RING buffers; of the last, lane 0 issues, per input
-// row, 3 * CIN / 16 steps of one or two MMAs (descriptors formed once per
-// row, compile-time step offsets) and commits them to mbarriers (a row buffer
-// is free after its own MMAs; an output row's accumulator is full after input
-// row r + 1).  The epilogues' latencies (tensor memory, staging, the residual
-// and target loads) bound the larger layers, hence two warps on each quarter
-// of the lanes: at 16x256x192x64 the loss layer 178 -> 155 us, the data
-// gradients 66 / 59 / 58 -> 63 / 54 / 54, the others equal; loads of the loss
-// in groups of four passes, eight spill.  Every wait is bounded
-// (DEV_ERR_TIMEOUT in the status word), and the tensor memory is released on
-// every path.
+// Roles (10 warps): 8 warps read the accumulators back (warp w owns lanes
+// 32 (w % 4) .. + 31, i.e. those pixels of the tile; the warps of one lane
+// quarter share out the channels, 16 or more each, or take tiles in turn),
+// add the bias, apply ReLU, stage the 32 pixels in shared memory and store
+// them, adding the residual in that pass; of the next warp lane 0 issues the
+// row copies into a ring of RING buffers; of the last, lane 0 issues, per
+// input row, 3 * CIN / 16 steps of one or two MMAs (descriptors formed once
+// per row, compile-time step offsets) and commits them to mbarriers (a row
+// buffer is free after its own MMAs; an output row's accumulator is full
+// after input row r + 1).  Loads of the loss go out in groups of four passes,
+// eight spill.  Every wait is bounded (DEV_ERR_TIMEOUT in the status word),
+// and the tensor memory is released on every path.
+//
+// The first layer reads x in FP32: eight warps take the copying warp's place,
+// round the rows on their way into the buffers and, in training, store the
+// rounding for the weight gradient.  A conversion kernel before a layer that
+// read its output moved x's BF16 through memory twice: 26 + 33 us of a
+// 960x540x64 forward pass, now 43 (180 -> 169 us the call).
 //
 // Programmatic launches: each kernel sets up (barriers, tensor memory, its
 // weights) beside the tail of the one before it and waits before it touches
@@ -72,6 +74,8 @@ struct ConvTcParams {
     const float *bias;       // COUT, or null
     const float *res;        // FP32 residual [pixel][COUT] added after the activation, or null
     void *out;               // [pixel][COUT], FP32 or BF16
+    const float *x;          // IN_F32: the input, [pixel][CIN]
+    __nv_bfloat16 *x_bf16;   // IN_F32: its BF16 rounding, or null
     const __nv_bfloat16 *act;  // EPI_MASK: the activations whose ReLU the gradient passes
     const float *target;       // EPI_LOSS: [pixel][COUT]
     float scale;               // EPI_LOSS: 2 / elements
@@ -177,15 +181,22 @@ __device__ __forceinline__ Item item_of(const ConvTcParams &p, int it) {
     return r;
 }
 
-// Epilogue warps of a convolution: two per 32 tensor-memory lanes, each with
-// half the channels, where half is a tensor-memory load (16 columns) or more.
-constexpr int epi_warps(int cout) { return cout >= 32 ? 8 : 4; }
+// Warps of a convolution: epilogue, row copies, MMA.  With FP32 input eight
+// warps round the rows on their way to shared memory, and the epilogue has
+// four: eight there 176 us against 169 for a 960x540x64 forward pass (the
+// others: four 543, eight 525, sixteen 542 us at 16x256x192x64 gradients).
+constexpr int epi_warps(bool in_f32) { return in_f32 ? 4 : 8; }
+constexpr int copy_warps(bool in_f32) { return in_f32 ? 8 : 1; }
+constexpr int conv_threads(bool in_f32) { return (epi_warps(in_f32) + copy_warps(in_f32) + 1) * 32; }
 
-template <int CIN, int COUT, bool OUT_F32, int RING>
+template <int CIN, int COUT, bool OUT_F32, int RING, bool IN_F32>
 struct TcLayout {
-    static constexpr int kEpi = epi_warps(COUT);
-    static constexpr int kThreads = (kEpi + 2) * 32;  // + copies, MMA
-    static constexpr int kCols4 = COUT * 4 / kEpi;    // channels per epilogue warp
+    static constexpr int kEpi = epi_warps(IN_F32), kCopy = copy_warps(IN_F32);
+    static constexpr int kThreads = conv_threads(IN_F32);  // epilogue, copies, MMA
+    static constexpr int kCW = COUT * 4 / kEpi > 16 ? COUT * 4 / kEpi : 16;  // channels per epilogue warp
+    static constexpr int kTileWarps = COUT / kCW * 4;    // epilogue warps of a tile
+    static constexpr int kTeams = kEpi / kTileWarps;     // tiles are taken in turn by as many teams of warps
+    static_assert(kEpi % kTileWarps == 0, "whole teams");
     static constexpr int kChunks = CIN / 8;
     static constexpr int kPixBytes = CIN * 2;                          // one pixel: one swizzle row
     static constexpr uint32_t kSwizzle = CIN == 64 ? 2 : (CIN == 32 ? 4 : 6);
@@ -195,7 +206,7 @@ struct TcLayout {
     static constexpr int kRows = 0;
     static constexpr int kW = kRows + RING * kRowBytes;
     static constexpr int kBias = kW + kWBytes;
-    static constexpr int kOutBytes = kCols4 * (OUT_F32 ? 4 : 2);  // one pixel's outputs of one warp
+    static constexpr int kOutBytes = kCW * (OUT_F32 ? 4 : 2);  // one pixel's outputs of one warp
     static constexpr int kChunksOut = kOutBytes / 16;
     static constexpr int kStagePitch = kOutBytes + 16;
     static constexpr int kStage = (kBias + COUT * 4 + 15) / 16 * 16;  // epilogue warps x 32 pixel rows
@@ -230,10 +241,12 @@ __device__ __forceinline__ uint2 pack_bf16x4(const float *v) {
 }
 
 // OUT_F32: FP32 results are staged (and stored, with EPI_STORE).
-template <int CIN, int COUT, bool RELU, bool OUT_F32, int RING, int EPI = EPI_STORE>
-__global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
+// IN_F32: the input is FP32; warps round its rows to BF16 on the way into the
+// row buffers (no map).
+template <int CIN, int COUT, bool RELU, bool OUT_F32, int RING, int EPI, bool IN_F32>
+__global__ void __launch_bounds__(conv_threads(IN_F32), 2)
     k_conv_tc(const __grid_constant__ CUtensorMap rows_map, const ConvTcParams p) {
-    using Lay = TcLayout<CIN, COUT, OUT_F32, RING>;
+    using Lay = TcLayout<CIN, COUT, OUT_F32, RING, IN_F32>;
     static_assert((CIN == 16 || CIN == 32 || CIN == 64) && COUT % 16 == 0 && COUT <= 256, "tile shape");
     static_assert(EPI == EPI_STORE || (OUT_F32 && !RELU), "the gradients are formed from FP32 rows");
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -268,12 +281,12 @@ __global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
     for (int c = threadIdx.x; c < COUT; c += blockDim.x) bias[c] = p.bias ? p.bias[c] : 0.f;
     if (threadIdx.x == 0) {
         for (int i = 0; i < RING; ++i) {
-            mbar_init(&full[i], 1);
+            mbar_init(&full[i], IN_F32 ? Lay::kCopy * 32 : 1);
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < Lay::kAcc; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], Lay::kEpi * 32);
+            mbar_init(&acc_empty[i], Lay::kTileWarps * 32);
         }
         mbar_init(done, 1);
         *abort_flag = 0;
@@ -298,7 +311,61 @@ __global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
     grid_dependency_wait();
     launch_dependents();
 
-    if (warp == Lay::kEpi) {
+    if (IN_F32 && warp >= Lay::kEpi && warp < Lay::kEpi + Lay::kCopy) {
+        // Rows through registers: quad q of the row is channels 4 (q % kQuads)
+        // on of pixel q / kQuads, 8 bytes of the buffer, where the copy's
+        // swizzle would put them (address bits 4-6 xor bits 7-9, as many as a
+        // swizzle row's chunks take).  All of a thread's loads are in flight
+        // at once, ahead of the wait for the buffer.
+        constexpr int kCopyThreads = Lay::kCopy * 32, kQuads = CIN / 4, kRowQuads = kSlab * kQuads;
+        constexpr int kEach = (kRowQuads + kCopyThreads - 1) / kCopyThreads;
+        constexpr int kAhead = 1;  // rows the L2 prefetch runs ahead
+        const int t0 = threadIdx.x - Lay::kEpi * 32;
+        uint32_t ld = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < p.items && ok && !__any_sync(~0u, *abort_flag); it += gridDim.x) {
+            const Item t = item_of(p, it);
+            for (int r = t.y0 - 1; r <= t.y0 + t.rows; ++r, ++ld) {
+                const int ra = r + kAhead;
+                if (t0 == 0 && ra >= 0 && ra < p.h && ra <= t.y0 + t.rows) {
+                    const int xl = t.x0 > 0 ? t.x0 - 1 : 0, xr = t.x0 + kTileM + 1 < p.w ? t.x0 + kTileM + 1 : p.w;
+                    bulk_prefetch_l2(p.x + (((size_t)t.img * p.h + ra) * p.w + xl) * CIN, (uint32_t)((xr - xl) * CIN * 4));
+                }
+                // Quads of the row inside the image: [qlo, qhi).
+                const int left = t.x0 == 0 ? kQuads : 0, right = (p.w - t.x0 + 1) * kQuads;
+                const int qlo = r >= 0 && r < p.h ? left : kRowQuads, qhi = right < kRowQuads ? right : kRowQuads;
+                const ptrdiff_t row = (((ptrdiff_t)t.img * p.h + r) * p.w + t.x0 - 1) * CIN;  // of quad 0
+                float4 v[kEach];
+#pragma unroll
+                for (int i = 0; i < kEach; ++i) {
+                    const int q = t0 + i * kCopyThreads;
+                    v[i] = q >= qlo && q < qhi ? *reinterpret_cast<const float4 *>(p.x + row + 4 * q)
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                const int slot = (int)(ld % RING);
+                ok = __all_sync(~0u, mbar_wait_bounded(&empty[slot], ((ld / RING) & 1u) ^ 1u, p.status));
+                if (!ok) {
+                    *abort_flag = 1;
+                    break;
+                }
+                // The rounding kept: the band's own pixels of the strip's own rows, each once.
+                const bool keep = p.x_bf16 && r >= t.y0 && r < t.y0 + t.rows;
+                const int khi = qhi < (kTileM + 1) * kQuads ? qhi : (kTileM + 1) * kQuads;
+#pragma unroll
+                for (int i = 0; i < kEach; ++i) {
+                    const int q = t0 + i * kCopyThreads;
+                    if (q >= kRowQuads) break;
+                    const uint2 b = pack_bf16x4(&v[i].x);
+                    uint32_t at = (uint32_t)q * 8;
+                    at ^= ((at >> 7) & (Lay::kChunks - 1)) << 4;
+                    *reinterpret_cast<uint2 *>(sm + Lay::kRows + slot * Lay::kRowBytes + at) = b;
+                    if (keep && q >= kQuads && q < khi) *reinterpret_cast<uint2 *>(p.x_bf16 + row + 4 * q) = b;
+                }
+                fence_proxy_async_shared();  // written by threads, read by the tensor cores
+                mbar_arrive(&full[slot]);
+            }
+        }
+    } else if (warp == Lay::kEpi) {
         if (lane == 0) {
             uint32_t ld = 0;
             for (int it = blockIdx.x; it < p.items && !*abort_flag; it += gridDim.x) {
@@ -319,7 +386,7 @@ __global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
                 mbar_wait_bounded(&full[q % RING], (q / RING) & 1u, nullptr);
         }
         __syncwarp();
-    } else if (warp == Lay::kEpi + 1) {
+    } else if (warp == Lay::kEpi + Lay::kCopy) {
         if (lane == 0) {
             constexpr int ACC = Lay::kAcc;
             const uint32_t rbase = smem_addr(sm + Lay::kRows);
@@ -385,8 +452,9 @@ __global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
     } else {
         // Epilogue: warp w reads lanes 32 (w % 4) .. + 31 of the accumulator,
         // channels c0 .. c0 + CW - 1.
-        constexpr int CW = Lay::kCols4;
-        const int quarter = warp & 3, c0 = (warp >> 2) * CW;
+        constexpr int CW = Lay::kCW;
+        const int quarter = warp & 3, c0 = warp % Lay::kTileWarps / 4 * CW;
+        const uint32_t team = warp / Lay::kTileWarps;
         uint32_t tile = 0;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         // EPI_MASK, EPI_LOSS: this lane's four channels (chunk lane % kChunksOut
@@ -397,6 +465,7 @@ __global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
         for (int it = blockIdx.x; it < p.items && !__any_sync(~0u, *abort_flag); it += gridDim.x) {
             const Item t = item_of(p, it);
             for (int j = 0; j < t.rows; ++j, ++tile) {
+                if (Lay::kTeams > 1 && tile % Lay::kTeams != team) continue;
                 const uint32_t acc = tile % Lay::kAcc;
                 if (!__all_sync(~0u, mbar_wait_bounded(&acc_full[acc], (tile / Lay::kAcc) & 1u, p.status))) {
                     *abort_flag = 1;
@@ -443,7 +512,7 @@ __global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
                 const size_t pix = ((size_t)t.img * p.h + t.y0 + j) * p.w + x;
                 // 16-byte chunk q of the warp's block: pixel q / kChunksOut,
                 // chunk q % kChunksOut of its channels, at(q) in the tensor.
-                constexpr int kPixChunks = Lay::kChunksOut * Lay::kEpi / 4;  // of a whole pixel
+                constexpr int kPixChunks = Lay::kChunksOut * (COUT / CW);  // of a whole pixel
                 auto at = [&](int q) { return (q / Lay::kChunksOut) * kPixChunks + q % Lay::kChunksOut; };
                 const size_t first = pix * COUT + c0;
                 uint4 *o = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(p.out) + first * (OUT_F32 ? 4 : 2));
@@ -554,8 +623,9 @@ __global__ void __launch_bounds__((epi_warps(COUT) + 2) * 32, 2)
             if (threadIdx.x < COUT) {
                 float t = 0.f;
 #pragma unroll
-                for (int w = 0; w < 4; ++w)
-                    t += reinterpret_cast<const float *>(sm + Lay::kStage + (threadIdx.x / CW * 4 + w) * kWarpStage)[threadIdx.x % CW];
+                for (int w = 0; w < 4 * Lay::kTeams; ++w)
+                    t += reinterpret_cast<const float *>(sm + Lay::kStage + (w / 4 * Lay::kTileWarps + threadIdx.x / CW * 4 + w % 4) *
+                                                             kWarpStage)[threadIdx.x % CW];
                 p.bias_part[(size_t)blockIdx.x * COUT + threadIdx.x] = t;
             }
             if (EPI == EPI_LOSS && threadIdx.x == 0) {
@@ -674,25 +744,27 @@ bool plan_items(int n, int h, int w, int slots, ItemPlan &pl) {
 }
 
 // parts (may be null): the CTAs launched, each with its partial sums.
-template <int CIN, int COUT, bool RELU, bool OUT_F32, int EPI = EPI_STORE>
+template <int CIN, int COUT, bool RELU, bool OUT_F32, int EPI = EPI_STORE, bool IN_F32 = false>
 cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t s, int *parts = nullptr) {
     // The deepest ring of row buffers (3 to 8) that leaves room for two CTAs
     // per SM (228 KB of shared memory, 1 KB of it reserved per CTA).
     constexpr int kBudget = 113 * 1024;
-    constexpr int kFixed = TcLayout<CIN, COUT, OUT_F32, 8>::kBytes - 8 * TcLayout<CIN, COUT, OUT_F32, 8>::kRowBytes;
-    constexpr int kFit = (kBudget - kFixed) / TcLayout<CIN, COUT, OUT_F32, 8>::kRowBytes;
+    constexpr int kFixed = TcLayout<CIN, COUT, OUT_F32, 8, IN_F32>::kBytes - 8 * TcLayout<CIN, COUT, OUT_F32, 8, IN_F32>::kRowBytes;
+    constexpr int kFit = (kBudget - kFixed) / TcLayout<CIN, COUT, OUT_F32, 8, IN_F32>::kRowBytes;
     constexpr int RING = kFit < 3 ? 3 : (kFit > 8 ? 8 : kFit);
-    using Lay = TcLayout<CIN, COUT, OUT_F32, RING>;
+    using Lay = TcLayout<CIN, COUT, OUT_F32, RING, IN_F32>;
     // At least 80 KB, so that no more than two CTAs share an SM's 512
     // tensor-memory columns (a third would wait in its allocation).
     constexpr int kSmem = Lay::kBytes < 80 * 1024 ? 80 * 1024 : Lay::kBytes;
-    auto kern = k_conv_tc<CIN, COUT, RELU, OUT_F32, RING, EPI>;
+    auto kern = k_conv_tc<CIN, COUT, RELU, OUT_F32, RING, EPI, IN_F32>;
     static TcKernelSetup setup;
     cudaError_t attr_err = setup.ensure(kern, kSmem);
     if (attr_err != cudaSuccess) return attr_err;
-    alignas(64) CUtensorMap map;
-    if (!tensor_map_encoder()) return cudaErrorNotSupported;
-    if (!encode_rows_map(&map, in, CIN, p.n, p.h, p.w, kSlab)) return cudaErrorInvalidValue;
+    alignas(64) CUtensorMap map{};
+    if constexpr (!IN_F32) {
+        if (!tensor_map_encoder()) return cudaErrorNotSupported;
+        if (!encode_rows_map(&map, in, CIN, p.n, p.h, p.w, kSlab)) return cudaErrorInvalidValue;
+    }
     int slots = 0;
     cudaError_t e = cta_slots(kSmem, &slots);
     if (e != cudaSuccess) return e;
@@ -703,6 +775,10 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
     p.chunks = pl.chunks;
     p.items = pl.items;
     if (parts) *parts = pl.grid;
+    if constexpr (IN_F32) {  // the first of a call: nothing before it may be unfinished
+        kern<<<pl.grid, Lay::kThreads, kSmem, s>>>(map, p);
+        return cudaGetLastError();
+    }
     return launch_after(kern, pl.grid, Lay::kThreads, kSmem, s, map, p);
 }
 
@@ -975,16 +1051,34 @@ cudaError_t conv_fwd_tc(int cin, int cout, bool relu, const __nv_bfloat16 *in, c
     p.w = wd;
     p.status = status;
     if (relu) {
-        if (cout != 32) return cudaErrorInvalidValue;
-        if (cin == 16) return launch_conv_tc<16, 32, true, false>(in, p, s);
-        if (cin == 32) return launch_conv_tc<32, 32, true, false>(in, p, s);
-        if (cin == 64) return launch_conv_tc<64, 32, true, false>(in, p, s);
-        return cudaErrorInvalidValue;
+        if (cin != 32 || cout != 32) return cudaErrorInvalidValue;
+        return launch_conv_tc<32, 32, true, false>(in, p, s);
     }
     if (cin != 32) return cudaErrorInvalidValue;
     if (cout == 16) return launch_conv_tc<32, 16, false, true>(in, p, s);
     if (cout == 32) return launch_conv_tc<32, 32, false, true>(in, p, s);
     if (cout == 64) return launch_conv_tc<32, 64, false, true>(in, p, s);
+    return cudaErrorInvalidValue;
+}
+
+// The first layer (cin -> 32, ReLU, BF16 out) from the FP32 x, whose BF16
+// rounding goes to x_bf16 unless that is null.
+cudaError_t conv_first_tc(int cin, const float *x, __nv_bfloat16 *x_bf16, const __nv_bfloat16 *w, const float *bias,
+                          int nimg, int h, int wd, __nv_bfloat16 *out, int *status, cudaStream_t s) {
+    if (((uintptr_t)x | (uintptr_t)x_bf16 | (uintptr_t)w | (uintptr_t)out) & 15) return cudaErrorMisalignedAddress;
+    ConvTcParams p{};
+    p.wt = w;
+    p.bias = bias;
+    p.x = x;
+    p.x_bf16 = x_bf16;
+    p.out = out;
+    p.n = nimg;
+    p.h = h;
+    p.w = wd;
+    p.status = status;
+    if (cin == 16) return launch_conv_tc<16, 32, true, false, EPI_STORE, true>(nullptr, p, s);
+    if (cin == 32) return launch_conv_tc<32, 32, true, false, EPI_STORE, true>(nullptr, p, s);
+    if (cin == 64) return launch_conv_tc<64, 32, true, false, EPI_STORE, true>(nullptr, p, s);
     return cudaErrorInvalidValue;
 }
 

@@ -113,6 +113,12 @@ __device__ __forceinline__ void fence_proxy_async_global() {
     asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
+// Bulk prefetch of global memory into L2: gsrc 16-byte aligned, bytes a
+// multiple of 16, all of it inside an allocation.
+__device__ __forceinline__ void bulk_prefetch_l2(const void *gsrc, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gsrc), "r"(bytes) : "memory");
+}
+
 // Programmatic dependent launch: the next kernel in the stream (launched
 // with programmatic stream serialisation) may start now; it waits in
 // grid_dependency_wait() until this grid has completed and its memory

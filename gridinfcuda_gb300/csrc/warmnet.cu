@@ -29,6 +29,8 @@
 
 namespace ginf_gpu {
 
+cudaError_t conv_first_tc(int cin, const float *x, __nv_bfloat16 *x_bf16, const __nv_bfloat16 *w, const float *bias,
+                          int nimg, int h, int wd, __nv_bfloat16 *out, int *status, cudaStream_t s);
 cudaError_t conv_fwd_tc(int cin, int cout, bool relu, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
                         const float *bias, int nimg, int h, int wd, void *out, const float *res, int *status,
                         cudaStream_t s);
@@ -295,14 +297,15 @@ ginf_status ensure_batch(ginf_warmnet *n, size_t pix) {
     return GINF_OK;
 }
 
-// The hidden layers, from the BF16 of x.
-ginf_status forward_hidden(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStream_t s) {
+// The hidden layers, from x; its BF16 rounding into a[0] when `keep` asks for
+// it (the first weight gradient reads it).
+ginf_status forward_hidden(ginf_warmnet *n, const float *x, Geo g, bool keep, int *status, cudaStream_t s) {
     const size_t pix = (size_t)g.n * g.h * g.w;
     ginf_status st = ensure_batch(n, pix);
     if (st != GINF_OK) return st;
-    f32_to_bf16(x, n->a[0], pix * n->L, s);
-    GINF_WCK(cudaGetLastError());
-    for (int l = 0; l < 3; ++l)
+    GINF_WCK(conv_first_tc(n->L, x, keep ? n->a[0] : nullptr, n->wbf + n->woff[0], n->params + n->boff[0], g.n, g.h,
+                           g.w, n->a[1], status, s));
+    for (int l = 1; l < 3; ++l)
         GINF_WCK(conv_fwd_tc(n->cin[l], n->cout[l], true, n->a[l], n->wbf + n->woff[l], n->params + n->boff[l], g.n, g.h,
                              g.w, n->a[l + 1], nullptr, status, s));
     return GINF_OK;
@@ -311,7 +314,7 @@ ginf_status forward_hidden(ginf_warmnet *n, const float *x, Geo g, int *status, 
 // y = x + net(x) into y_out (the network's own buffer when null); the last
 // layer reads x itself as its residual.
 ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStream_t s, float *y_out = nullptr) {
-    ginf_status st = forward_hidden(n, x, g, status, s);
+    ginf_status st = forward_hidden(n, x, g, false, status, s);
     if (st != GINF_OK) return st;
     GINF_WCK(conv_fwd_tc(n->cin[3], n->cout[3], false, n->a[3], n->wbf + n->woff[3], n->params + n->boff[3], g.n, g.h,
                          g.w, y_out ? y_out : n->y, x, status, s));
@@ -325,7 +328,8 @@ ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStr
 // 16x256x192x64: 1334 us a call with separate loss, conversion, ReLU and bias
 // kernels, 941 us so; with the later changes in conv_tc.cu 816, with the
 // programmatic launches, the weights flipped as the data gradient loads them
-// and one copy for loss and status 746, with evenly filled CTAs 536.
+// and one copy for loss and status 746, with evenly filled CTAs 536, with the
+// conversion of x inside the first layer 526.
 ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo g, cudaStream_t s) {
     const size_t pix = (size_t)g.n * g.h * g.w, ny = pix * n->L;
     ginf_status st = ensure_batch(n, pix);
@@ -334,7 +338,7 @@ ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo 
         GINF_WCK(cudaMemcpyAsync(n->y, target, ny * sizeof(float), cudaMemcpyDeviceToDevice, s));
         target = n->y;
     }
-    if ((st = forward_hidden(n, x, g, n->status, s)) != GINF_OK) return st;
+    if ((st = forward_hidden(n, x, g, true, n->status, s)) != GINF_OK) return st;
     int bias_parts = 0;
     GINF_WCK(conv_loss_tc(n->L, n->a[3], n->wbf + n->woff[3], n->params + n->boff[3], g.n, g.h, g.w, x, target,
                           2.f / (float)ny, n->gb[0], n->bias_part, n->loss_part, &bias_parts, n->status, s));
