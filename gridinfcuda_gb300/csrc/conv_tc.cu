@@ -45,7 +45,7 @@
 // round the rows on their way into the buffers and, in training, store the
 // rounding for the weight gradient.  A conversion kernel before a layer that
 // read its output moved x's BF16 through memory twice: 26 + 33 us of a
-// 960x540x64 forward pass, now 43 (180 -> 169 us the call).
+// 960x540x64 forward pass, now 42 (180 -> 169 us the call).
 //
 // Programmatic launches: each kernel sets up (barriers, tensor memory, its
 // weights) beside the tail of the one before it and waits before it touches
@@ -268,7 +268,8 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
         uint4 q;
         if constexpr (EPI == EPI_MASK) {
             uint32_t w2[4];
-            const uint16_t *wt = reinterpret_cast<const uint16_t *>(p.wt) + ((size_t)c8 * 72 + 8 - j * 3 - dx) * COUT + co;
+            const uint16_t *wt =
+                reinterpret_cast<const uint16_t *>(p.wt) + ((size_t)c8 * 72 + 8 - j * 3 - dx) * COUT + co;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
                 w2[k] = (uint32_t)wt[2 * k * 9 * COUT] | ((uint32_t)wt[(2 * k + 1) * 9 * COUT] << 16);
@@ -329,7 +330,8 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                 const int ra = r + kAhead;
                 if (t0 == 0 && ra >= 0 && ra < p.h && ra <= t.y0 + t.rows) {
                     const int xl = t.x0 > 0 ? t.x0 - 1 : 0, xr = t.x0 + kTileM + 1 < p.w ? t.x0 + kTileM + 1 : p.w;
-                    bulk_prefetch_l2(p.x + (((size_t)t.img * p.h + ra) * p.w + xl) * CIN, (uint32_t)((xr - xl) * CIN * 4));
+                    bulk_prefetch_l2(p.x + (((size_t)t.img * p.h + ra) * p.w + xl) * CIN,
+                                     (uint32_t)((xr - xl) * CIN * 4));
                 }
                 // Quads of the row inside the image: [qlo, qhi).
                 const int left = t.x0 == 0 ? kQuads : 0, right = (p.w - t.x0 + 1) * kQuads;
@@ -387,41 +389,46 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
         }
         __syncwarp();
     } else if (warp == Lay::kEpi + Lay::kCopy) {
-        if (lane == 0) {
-            constexpr int ACC = Lay::kAcc;
-            const uint32_t rbase = smem_addr(sm + Lay::kRows);
-            // Weights: [dx][chunk][3 * COUT rows][16 B], K-adjacent chunks 3 * COUT * 16 bytes apart.
-            const uint64_t bdesc = smem_desc(smem_addr(sm + Lay::kW), 3 * COUT * 16, 128);
-            uint32_t ld = 0, tile = 0;
-            bool ok = true;
-            for (int it = blockIdx.x; it < p.items && ok && !*abort_flag; it += gridDim.x) {
-                const Item t = item_of(p, it);
-                // Input row r = y0 - 1 + i feeds output rows y = r + 1 - j
-                // (dy = j - 1), j in [jlo, jhi] within the strip; output row
-                // y0 + m is tile `tile + m`.
-                for (int i = 0; i < t.rows + 2 && ok; ++i, ++ld) {
-                    const int jlo = i - (t.rows - 1) > 0 ? i - (t.rows - 1) : 0, jhi = i < 2 ? i : 2;
-                    ok = mbar_wait_bounded(&full[ld % RING], (ld / RING) & 1u, p.status);
-                    // Block j = 0 starts row y0 + i's accumulator: its slot must be read out.
-                    if (ok && jlo == 0) {
-                        const uint32_t tn = tile + i;
-                        ok = mbar_wait_bounded(&acc_empty[tn % ACC], ((tn / ACC) & 1u) ^ 1u, p.status);
-                    }
-                    if (!ok) break;
-                    tc_fence_after();
-                    // The blocks j in [jlo, jhi] as at most two runs with
-                    // adjacent accumulators (the ring wraps at most once),
-                    // fixed for the row; every step then issues one MMA per
-                    // run, its descriptors the row's plus constant offsets.
-                    int k0 = jlo;
-                    while (k0 < jhi && (tile + i - k0) % ACC != 0) ++k0;
-                    const int n0 = k0 - jlo + 1, n1 = jhi - k0;  // blocks in run 0, run 1
-                    const uint32_t d0 = tmem + acc_col<COUT, ACC>(tile + i - jlo);
-                    const uint32_t d1 = tmem + acc_col<COUT, ACC>(tile + i - k0 - 1);
-                    const uint32_t i0 = instr_desc_bf16(n0 * COUT), i1 = instr_desc_bf16(n1 > 0 ? n1 * COUT : 16);
-                    const uint64_t a0 = smem_desc(rbase + (ld % RING) * Lay::kRowBytes, 16, 8 * Lay::kPixBytes,
-                                                  Lay::kSwizzle);
-                    const uint64_t b0 = bdesc + (uint64_t)(jlo * COUT), b1 = bdesc + (uint64_t)((k0 + 1) * COUT);
+        // The whole warp keeps count and one lane issues: with everything in
+        // one lane's branch each instruction's descriptors went through
+        // vector registers (960x540x64 forward 169 -> 161 us, gradients at
+        // 16x256x192x64 526 -> 514).
+        const bool leader = elect_one();
+        constexpr int ACC = Lay::kAcc;
+        const uint32_t rbase = smem_addr(sm + Lay::kRows);
+        // Weights: [dx][chunk][3 * COUT rows][16 B], K-adjacent chunks 3 * COUT * 16 bytes apart.
+        const uint64_t bdesc = smem_desc(smem_addr(sm + Lay::kW), 3 * COUT * 16, 128);
+        uint32_t ld = 0, tile = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < p.items && ok && !__any_sync(~0u, *abort_flag); it += gridDim.x) {
+            const Item t = item_of(p, it);
+            // Input row r = y0 - 1 + i feeds output rows y = r + 1 - j
+            // (dy = j - 1), j in [jlo, jhi] within the strip; output row
+            // y0 + m is tile `tile + m`.
+            for (int i = 0; i < t.rows + 2 && ok; ++i, ++ld) {
+                const int jlo = i - (t.rows - 1) > 0 ? i - (t.rows - 1) : 0, jhi = i < 2 ? i : 2;
+                ok = __all_sync(~0u, mbar_wait_bounded(&full[ld % RING], (ld / RING) & 1u, p.status));
+                // Block j = 0 starts row y0 + i's accumulator: its slot must be read out.
+                if (ok && jlo == 0) {
+                    const uint32_t tn = tile + i;
+                    ok = __all_sync(~0u, mbar_wait_bounded(&acc_empty[tn % ACC], ((tn / ACC) & 1u) ^ 1u, p.status));
+                }
+                if (!ok) break;
+                tc_fence_after();
+                // The blocks j in [jlo, jhi] as at most two runs with
+                // adjacent accumulators (the ring wraps at most once),
+                // fixed for the row; every step then issues one MMA per
+                // run, its descriptors the row's plus constant offsets.
+                int k0 = jlo;
+                while (k0 < jhi && (tile + i - k0) % ACC != 0) ++k0;
+                const int n0 = k0 - jlo + 1, n1 = jhi - k0;  // blocks in run 0, run 1
+                const uint32_t d0 = tmem + acc_col<COUT, ACC>(tile + i - jlo);
+                const uint32_t d1 = tmem + acc_col<COUT, ACC>(tile + i - k0 - 1);
+                const uint32_t i0 = instr_desc_bf16(n0 * COUT), i1 = instr_desc_bf16(n1 > 0 ? n1 * COUT : 16);
+                const uint64_t a0 = smem_desc(rbase + (ld % RING) * Lay::kRowBytes, 16, 8 * Lay::kPixBytes,
+                                              Lay::kSwizzle);
+                const uint64_t b0 = bdesc + (uint64_t)(jlo * COUT), b1 = bdesc + (uint64_t)((k0 + 1) * COUT);
+                if (leader) {
 #pragma unroll
                     for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
@@ -442,12 +449,13 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                     umma_commit(&empty[ld % RING]);  // the row's only MMAs are these
                     if (jhi == 2) umma_commit(&acc_full[(tile + i - 2) % ACC]);  // row y0 + i - 2 is done
                 }
-                tile += t.rows;
+                __syncwarp();
             }
-            if (!ok) *abort_flag = 1;
-            umma_commit(done);
-            mbar_wait_bounded(done, 0, nullptr);
+            tile += t.rows;
         }
+        if (!ok) *abort_flag = 1;
+        if (leader) umma_commit(done);
+        mbar_wait_bounded(done, 0, nullptr);
         __syncwarp();
     } else {
         // Epilogue: warp w reads lanes 32 (w % 4) .. + 31 of the accumulator,
@@ -624,8 +632,9 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                 float t = 0.f;
 #pragma unroll
                 for (int w = 0; w < 4 * Lay::kTeams; ++w)
-                    t += reinterpret_cast<const float *>(sm + Lay::kStage + (w / 4 * Lay::kTileWarps + threadIdx.x / CW * 4 + w % 4) *
-                                                             kWarpStage)[threadIdx.x % CW];
+                    t += reinterpret_cast<const float *>(
+                        sm + Lay::kStage +
+                        (w / 4 * Lay::kTileWarps + threadIdx.x / CW * 4 + w % 4) * kWarpStage)[threadIdx.x % CW];
                 p.bias_part[(size_t)blockIdx.x * COUT + threadIdx.x] = t;
             }
             if (EPI == EPI_LOSS && threadIdx.x == 0) {
@@ -749,8 +758,8 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
     // The deepest ring of row buffers (3 to 8) that leaves room for two CTAs
     // per SM (228 KB of shared memory, 1 KB of it reserved per CTA).
     constexpr int kBudget = 113 * 1024;
-    constexpr int kFixed = TcLayout<CIN, COUT, OUT_F32, 8, IN_F32>::kBytes - 8 * TcLayout<CIN, COUT, OUT_F32, 8, IN_F32>::kRowBytes;
-    constexpr int kFit = (kBudget - kFixed) / TcLayout<CIN, COUT, OUT_F32, 8, IN_F32>::kRowBytes;
+    using Most = TcLayout<CIN, COUT, OUT_F32, 8, IN_F32>;
+    constexpr int kFit = (kBudget - (Most::kBytes - 8 * Most::kRowBytes)) / Most::kRowBytes;
     constexpr int RING = kFit < 3 ? 3 : (kFit > 8 ? 8 : kFit);
     using Lay = TcLayout<CIN, COUT, OUT_F32, RING, IN_F32>;
     // At least 80 KB, so that no more than two CTAs share an SM's 512
@@ -920,26 +929,28 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
-        if (lane == 0) {
-            const uint32_t ibase = smem_addr(sm + Lay::kIn), obase = smem_addr(sm + Lay::kOut);
-            uint32_t li = 0, lo = 0;  // input row of the step, first output-gradient row of the item
-            bool ok = true, first_item = true;
-            for (int it = blockIdx.x; it < p.items && ok && !*abort_flag; it += gridDim.x) {
-                const Item t = item_of(ip, it);
-                for (int i = 0; i < t.rows + 2 && ok; ++i, ++li) {
-                    ok = mbar_wait_bounded(&in_full[li % RING], (li / RING) & 1u, p.status);
-                    if (ok && i < t.rows)
-                        ok = mbar_wait_bounded(&out_full[(lo + i) % RING], ((lo + i) / RING) & 1u, p.status);
-                    if (!ok) break;
-                    tc_fence_after();
-                    // Blocks b: output-gradient row y0 + i - 2 + b, dy = 2 - b,
-                    // accumulator columns b * COUT on.
-                    const int blo = i < 2 ? 2 - i : 0, bhi = t.rows + 1 - i < 2 ? t.rows + 1 - i : 2;
-                    const uint64_t a0 = smem_desc(ibase + (li % RING) * Lay::kInRow, Lay::kInPix, 8 * Lay::kInPix,
-                                                  Lay::kSwIn);
-                    // Runs of adjacent row buffers; a block's first use starts
-                    // its accumulator, in a run of its own.
-                    const bool fresh = first_item && i < 3;
+        const bool leader = elect_one();
+        const uint32_t ibase = smem_addr(sm + Lay::kIn), obase = smem_addr(sm + Lay::kOut);
+        uint32_t li = 0, lo = 0;  // input row of the step, first output-gradient row of the item
+        bool ok = true, first_item = true;
+        for (int it = blockIdx.x; it < p.items && ok && !__any_sync(~0u, *abort_flag); it += gridDim.x) {
+            const Item t = item_of(ip, it);
+            for (int i = 0; i < t.rows + 2 && ok; ++i, ++li) {
+                ok = __all_sync(~0u, mbar_wait_bounded(&in_full[li % RING], (li / RING) & 1u, p.status));
+                if (ok && i < t.rows)
+                    ok = __all_sync(
+                        ~0u, mbar_wait_bounded(&out_full[(lo + i) % RING], ((lo + i) / RING) & 1u, p.status));
+                if (!ok) break;
+                tc_fence_after();
+                // Blocks b: output-gradient row y0 + i - 2 + b, dy = 2 - b,
+                // accumulator columns b * COUT on.
+                const int blo = i < 2 ? 2 - i : 0, bhi = t.rows + 1 - i < 2 ? t.rows + 1 - i : 2;
+                const uint64_t a0 = smem_desc(ibase + (li % RING) * Lay::kInRow, Lay::kInPix, 8 * Lay::kInPix,
+                                              Lay::kSwIn);
+                // Runs of adjacent row buffers; a block's first use starts
+                // its accumulator, in a run of its own.
+                const bool fresh = first_item && i < 3;
+                if (leader) {
                     for (int b = blo; b <= bhi;) {
                         const uint32_t slot = (lo + i - 2 + b) % RING;
                         const bool start = fresh && b == blo;
@@ -963,12 +974,13 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                     umma_commit(&in_empty[li % RING]);
                     if (blo == 0) umma_commit(&out_empty[(lo + i - 2) % RING]);  // its last use
                 }
-                first_item = false;
-                lo += t.rows;
+                __syncwarp();
             }
-            if (!ok) *abort_flag = 1;
-            umma_commit(done);
+            first_item = false;
+            lo += t.rows;
         }
+        if (!ok) *abort_flag = 1;
+        if (leader) umma_commit(done);
         __syncwarp();
     } else {
         // Epilogue, once: accumulator (mt, dy), lane m = 32 * warp + lane is

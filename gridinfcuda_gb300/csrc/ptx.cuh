@@ -113,6 +113,13 @@ __device__ __forceinline__ void fence_proxy_async_global() {
     asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t yes;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+    return yes != 0;
+}
+
 // Bulk prefetch of global memory into L2: gsrc 16-byte aligned, bytes a
 // multiple of 16, all of it inside an allocation.
 __device__ __forceinline__ void bulk_prefetch_l2(const void *gsrc, uint32_t bytes) {

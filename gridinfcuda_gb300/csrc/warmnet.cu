@@ -329,7 +329,7 @@ ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStr
 // kernels, 941 us so; with the later changes in conv_tc.cu 816, with the
 // programmatic launches, the weights flipped as the data gradient loads them
 // and one copy for loss and status 746, with evenly filled CTAs 536, with the
-// conversion of x inside the first layer 526.
+// conversion of x inside the first layer 526, with the MMA warps converged 514.
 ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo g, cudaStream_t s) {
     const size_t pix = (size_t)g.n * g.h * g.w, ny = pix * n->L;
     ginf_status st = ensure_batch(n, pix);
