@@ -138,6 +138,95 @@ __global__ void k_costs_to_records_pyr(const Tin *__restrict__ src, int W, int H
     }
 }
 
+// The same transform (crec null: without level 1) over XC columns a block, any
+// padded label count, for costs the device reads where they are in host memory.
+// Bound: the link (1001x563x48: 210 GB/s, 516 us for the volume, whether copied
+// or read), which carries whole sectors: a block's runs start and end anywhere
+// in one, so short runs fetch much of the volume twice (32 columns 152 GB/s, 64
+// 175, 128 186), and so do accesses that straddle a line.  Hence runs as long as
+// shared memory allows (two blocks per SM) and a warp access per aligned line,
+// all of a run's in flight at once.
+constexpr int kWideColumns = 256;
+template <typename Tin, typename T>
+__global__ void __launch_bounds__(256) k_costs_to_records_wide(const Tin *__restrict__ src, int W, int H, int L,
+                                                               int Lp, int XC, unsigned char *__restrict__ rec,
+                                                               unsigned char *__restrict__ crec, int cW,
+                                                               uint32_t rec_bytes) {
+    static_assert(sizeof(Tin) == 4, "lines of 32 elements");
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    T *tile = reinterpret_cast<T *>(sm_raw);  // [2][Lp][XC + 1]
+    const int S = XC + 1, x0 = blockIdx.x * XC;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cH = (H + 1) / 2, nn = min(XC, W - x0), cn = min(XC / 2, cW - x0 / 2);
+    constexpr int E = 16 / sizeof(T);
+    const int cpn = Lp / E;                                   // 16-byte chunks per node
+    const int di = 256 / cpn, dc = 256 - di * cpn;            // a block's stride in (node, chunk)
+    const int i00 = threadIdx.x / cpn, c00 = threadIdx.x - i00 * cpn;
+    for (int Y = blockIdx.y; Y < cH; Y += gridDim.y) {
+        const int rows = min(2, H - 2 * Y);
+        for (int u = warp; u < rows * Lp; u += 8) {
+            const int r = u >= Lp, l = u - r * Lp;
+            T *row = tile + (size_t)u * S;
+            if (l >= L) {
+                for (int k = lane; k < nn; k += 32) row[k] = T(0);
+                continue;
+            }
+            const Tin *p = src + (size_t)W * H * l + (size_t)W * (2 * Y + r) + x0;
+            const int k0 = lane - (int)(((uintptr_t)p >> 2) & 31);  // column of the lane in the first line
+            Tin v[kWideColumns / 32 + 1];
+#pragma unroll
+            for (int j = 0; j <= kWideColumns / 32; ++j) {
+                const int k = k0 + 32 * j;
+                if (k >= 0 && k < nn) v[j] = p[k];
+            }
+#pragma unroll
+            for (int j = 0; j <= kWideColumns / 32; ++j) {
+                const int k = k0 + 32 * j;
+                if (k >= 0 && k < nn) row[k] = (T)v[j];
+            }
+        }
+        __syncthreads();
+        for (int r = 0; r < rows; ++r) {
+            unsigned char *out = rec + ((size_t)(2 * Y + r) * W + x0) * rec_bytes;
+            for (int i = i00, c = c00; i < nn;) {
+                alignas(16) T v[E];
+#pragma unroll
+                for (int e = 0; e < E; ++e) v[e] = tile[(size_t)(r * Lp + c * E + e) * S + i];
+                *reinterpret_cast<uint4 *>(out + (size_t)i * rec_bytes + (size_t)c * 16) =
+                    *reinterpret_cast<const uint4 *>(v);
+                i += di;
+                c += dc;
+                if (c >= cpn) {
+                    c -= cpn;
+                    ++i;
+                }
+            }
+        }
+        // Level-1 sums in k_pyramid's order.
+        if (crec) {
+            for (int i = i00, c = c00; i < cn;) {
+                const int dxn = min(2, W - (x0 + 2 * i));
+                alignas(16) T acc[E];
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    acc[e] = T(0);
+                    for (int r = 0; r < rows; ++r)
+                        for (int dx = 0; dx < dxn; ++dx) acc[e] += tile[(size_t)(r * Lp + c * E + e) * S + 2 * i + dx];
+                }
+                *reinterpret_cast<uint4 *>(crec + ((size_t)Y * cW + x0 / 2 + i) * rec_bytes + (size_t)c * 16) =
+                    *reinterpret_cast<const uint4 *>(acc);
+                i += di;
+                c += dc;
+                if (c >= cpn) {
+                    c -= cpn;
+                    ++i;
+                }
+            }
+        }
+        __syncthreads();  // the tiles are refilled for the next row pair
+    }
+}
+
 // k_costs_to_records_pyr for 4-byte elements and a padded label count LP of
 // 16, 32, 64 or 128, over XC columns per block (launched with 32: at 64 the
 // larger tile leaves fewer blocks, and loads in flight, per SM, and the
@@ -813,6 +902,30 @@ RecordFormat make_format(int ctype, int store, int L) {
     } else {                                                                            \
         GINF_DISPATCH_T(f, using M = T; __VA_ARGS__)                                    \
     }
+
+template <typename Tin, typename T>
+cudaError_t launch_wide(const RecordFormat &f, const void *src, int W, int H, unsigned char *rec, unsigned char *crec,
+                        int cW, cudaStream_t s) {
+    auto smem = [&](int xc) { return (size_t)2 * f.Lp * (xc + 1) * sizeof(T); };
+    int xc = kWideColumns;
+    while (xc > 32 && (xc - 32 >= W || smem(xc) > 108 * 1024)) xc -= 32;
+    auto kern = k_costs_to_records_wide<Tin, T>;
+    static SmemLimit limit;
+    const cudaError_t e = limit.ensure(kern, smem(xc));
+    if (e != cudaSuccess) return e;
+    const dim3 grid((W + xc - 1) / xc, (unsigned)std::min((H + 1) / 2, 65535));
+    kern<<<grid, 256, smem(xc), s>>>(static_cast<const Tin *>(src), W, H, f.L, f.Lp, xc, rec, crec, cW, f.rec_bytes);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_costs_from_host(const RecordFormat &f, int cost_type, const void *src, int W, int H,
+                                   unsigned char *rec, unsigned char *crec, int cW, cudaStream_t s) {
+    GINF_DISPATCH_T(f, {
+        return cost_type == CT_F32 ? launch_wide<float, T>(f, src, W, H, rec, crec, cW, s)
+                                   : launch_wide<int, T>(f, src, W, H, rec, crec, cW, s);
+    })
+    return cudaErrorInvalidValue;
+}
 
 cudaError_t launch_costs_to_records(const RecordFormat &f, int cost_type, const void *src, int W, int H,
                                     unsigned char *rec, cudaStream_t s) {

@@ -420,7 +420,10 @@ ginf_status prepare(Call &c, Prepared &P, int levels, bool want_lab2, const int3
     // Level 0 records, with level 1's costs formed on the way when there is
     // a pyramid; then the coarser levels.
     const int nlv = (int)P.lv.size();
-    if (nlv >= 2)
+    if (host_view)
+        GINF_CK(launch_costs_from_host(P.f, g->cost_type, costs_dev, W, H, P.rec,
+                                       nlv >= 2 ? P.rec + P.lv[1].off : nullptr, nlv >= 2 ? P.lv[1].W : 0, s));
+    else if (nlv >= 2)
         GINF_CK(launch_costs_to_records_pyr(P.f, g->cost_type, costs_dev, W, H, P.rec, P.rec + P.lv[1].off,
                                             P.lv[1].W, s));
     else
