@@ -4,6 +4,8 @@
 // (Jacobi and exact Gauss-Seidel wavefront), FP64 energy, stereo costs.
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "ginf_internal.h"
 
 namespace ginf_gpu {
@@ -227,24 +229,27 @@ __global__ void __launch_bounds__(256) k_costs_to_records_wide(const Tin *__rest
     }
 }
 
-// k_costs_to_records_pyr for 4-byte elements and a padded label count LP of
-// 16, 32, 64 or 128, over XC columns per block (launched with 32: at 64 the
-// larger tile leaves fewer blocks, and loads in flight, per SM, and the
-// 1920x1080x64 transform took 0.34 ms against 0.28 ms): the loops are
-// unrolled and the plane pointers advanced instead of recomputed.  A warp's store instruction covers
-// G consecutive 16-byte chunks (G = 8, or 4 at LP = 16) of 32 / G nodes:
-// chunk c of node i reads tile column i at labels 4c..4c+3, bank 4c + i + e
-// (row stride XC + 1), so with G = 8 the 32 lanes hit 32 different banks, and
-// each node's chunks form one contiguous G * 16-byte run in its record.
-// Level-1 sums keep k_pyramid's order (rows, then columns, from zero).
+// Both transforms (crec null: without level 1) for 4-byte elements and a padded
+// label count LP known at compile time, over XC columns per block (32, and 128 at
+// LP = 8: at 64 the larger tile of L = 32 or 64 leaves fewer blocks, and loads in
+// flight, per SM): the loops are unrolled and the plane pointers advanced instead of recomputed.  A warp's store
+// instruction covers G consecutive 16-byte chunks (the largest power of two up
+// to 8 that divides a node's chunks) of 32 / G nodes: chunk c of node i reads
+// tile column i at labels 4c..4c+3, bank 4c + i + e (row stride XC + 1), so with
+// G = 8 the 32 lanes hit 32 different banks, and each node's chunks form one
+// contiguous G * 16-byte run in its record.  Level-1 sums keep k_pyramid's order
+// (rows, then columns, from zero).  Bound: HBM.  us at 1920x1080 with and without
+// level 1, run-time label counts -> here (the bytes' time): L = 8 105, 97 -> 45,
+// 38 (22, 20); L = 24 158, 194 -> 100, 88 (66, 59); L = 48 219, 239 -> 201, 173
+// (132, 117).  L = 8 at 32 columns: 63, 57.
 template <typename Tin, typename T, int LP, int XC>
 __global__ void __launch_bounds__(256) k_costs_to_records_pyr_lp(const Tin *__restrict__ src, int W, int H, int L,
                                                                  unsigned char *__restrict__ rec,
                                                                  unsigned char *__restrict__ crec, int cW,
                                                                  uint32_t rec_bytes) {
-    static_assert(sizeof(T) == 4 && LP % 16 == 0 && XC % 32 == 0, "4-byte elements, whole 16-label groups");
+    static_assert(sizeof(T) == 4 && LP % 8 == 0 && XC % 32 == 0, "4-byte elements, whole chunk pairs");
     constexpr int E = 4, CPN = LP / E;
-    constexpr int G = CPN < 8 ? CPN : 8, NG = 32 / G, CB = CPN / G;
+    constexpr int G = CPN % 8 == 0 ? 8 : (CPN % 4 == 0 ? 4 : 2), NG = 32 / G, CB = CPN / G;
     constexpr int S = XC + 1;  // tile row stride
     extern __shared__ __align__(16) unsigned char sm_raw[];
     T *tile = reinterpret_cast<T *>(sm_raw);  // [2][LP][S]
@@ -295,7 +300,7 @@ __global__ void __launch_bounds__(256) k_costs_to_records_pyr_lp(const Tin *__re
         }
         // Level 1: XC / 2 coarse nodes x CPN chunks, XC * CPN / 64 groups of 32.
 #pragma unroll
-        for (int gi = w; gi < CPN * XC / 64; gi += 8) {
+        for (int gi = crec ? w : CPN * XC / 64; gi < CPN * XC / 64; gi += 8) {
             const int j = (gi / CB) * NG + lane / G, c = (gi % CB) * G + lane % G;
             if (j < cn) {
                 const int dxn = min(2, W - (x0 + 2 * j));
@@ -927,21 +932,6 @@ cudaError_t launch_costs_from_host(const RecordFormat &f, int cost_type, const v
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_costs_to_records(const RecordFormat &f, int cost_type, const void *src, int W, int H,
-                                    unsigned char *rec, cudaStream_t s) {
-    const dim3 grid((W + 31) / 32, (unsigned)std::min(H, 65535)), block(32, 8);
-    GINF_DISPATCH_T(f, {
-        const size_t smem = (size_t)f.Lp * 33 * sizeof(T);
-        if (cost_type == CT_F32)
-            k_costs_to_records<float, T><<<grid, block, smem, s>>>(static_cast<const float *>(src), W, H, f.L, f.Lp,
-                                                                   rec, f.rec_bytes);
-        else
-            k_costs_to_records<int, T><<<grid, block, smem, s>>>(static_cast<const int *>(src), W, H, f.L, f.Lp, rec,
-                                                                 f.rec_bytes);
-    })
-    return cudaGetLastError();
-}
-
 template <typename Tin, typename T, int LP, int XC>
 cudaError_t launch_pyr_lp_t(const Tin *src, int W, int H, int L, unsigned char *rec, unsigned char *crec, int cW,
                             uint32_t rec_bytes, cudaStream_t s) {
@@ -955,8 +945,9 @@ cudaError_t launch_pyr_lp_t(const Tin *src, int W, int H, int L, unsigned char *
     return cudaGetLastError();
 }
 
-// The specialised transform where one exists (4-byte elements, Lp of 16, 32,
-// 64 or 128); `done` false otherwise.
+// The specialised transform where one exists (4-byte elements; Lp of 16, 32, 64
+// or 128, without a change of type every multiple of 8 up to 64 and of 16 up to
+// 128); `done` false otherwise.
 template <typename Tin, typename T>
 cudaError_t launch_pyr_lp(int Lp, const Tin *src, int W, int H, int L, unsigned char *rec, unsigned char *crec, int cW,
                           uint32_t rec_bytes, cudaStream_t s, bool &done) {
@@ -968,10 +959,46 @@ cudaError_t launch_pyr_lp(int Lp, const Tin *src, int W, int H, int L, unsigned 
         case 32: return launch_pyr_lp_t<Tin, T, 32, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
         case 64: return launch_pyr_lp_t<Tin, T, 64, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
         case 128: return launch_pyr_lp_t<Tin, T, 128, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
-        default: done = false;
+        default: break;
         }
+        if constexpr (std::is_same_v<Tin, T>) {
+            switch (Lp) {
+            case 8: return launch_pyr_lp_t<Tin, T, 8, 128>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            case 24: return launch_pyr_lp_t<Tin, T, 24, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            case 40: return launch_pyr_lp_t<Tin, T, 40, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            case 48: return launch_pyr_lp_t<Tin, T, 48, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            case 56: return launch_pyr_lp_t<Tin, T, 56, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            case 80: return launch_pyr_lp_t<Tin, T, 80, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            case 96: return launch_pyr_lp_t<Tin, T, 96, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            case 112: return launch_pyr_lp_t<Tin, T, 112, 32>(src, W, H, L, rec, crec, cW, rec_bytes, s);
+            default: break;
+            }
+        }
+        done = false;
     }
     return cudaSuccess;
+}
+
+cudaError_t launch_costs_to_records(const RecordFormat &f, int cost_type, const void *src, int W, int H,
+                                    unsigned char *rec, cudaStream_t s) {
+    const dim3 grid((W + 31) / 32, (unsigned)std::min(H, 65535)), block(32, 8);
+    GINF_DISPATCH_T(f, {
+        bool done = false;
+        const cudaError_t e0 = cost_type == CT_F32
+                                   ? launch_pyr_lp<float, T>(f.Lp, static_cast<const float *>(src), W, H, f.L, rec,
+                                                             nullptr, 0, f.rec_bytes, s, done)
+                                   : launch_pyr_lp<int, T>(f.Lp, static_cast<const int *>(src), W, H, f.L, rec, nullptr,
+                                                           0, f.rec_bytes, s, done);
+        if (done) return e0;
+        const size_t smem = (size_t)f.Lp * 33 * sizeof(T);
+        if (cost_type == CT_F32)
+            k_costs_to_records<float, T><<<grid, block, smem, s>>>(static_cast<const float *>(src), W, H, f.L, f.Lp,
+                                                                   rec, f.rec_bytes);
+        else
+            k_costs_to_records<int, T><<<grid, block, smem, s>>>(static_cast<const int *>(src), W, H, f.L, f.Lp, rec,
+                                                                 f.rec_bytes);
+    })
+    return cudaGetLastError();
 }
 
 cudaError_t launch_costs_to_records_pyr(const RecordFormat &f, int cost_type, const void *src, int W, int H,

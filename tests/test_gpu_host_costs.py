@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("offset", [0, 1, 31])
 def test_in_place_equals_staged(ginf, dtype, opt, offset):
     import torch
-    for L in (2, 9, 16, 48, 100, 128):
+    for L in (2, 9, 16, 20, 33, 48, 56, 75, 90, 100, 110, 128):  # each compiled transform, and one between
         for W, H, levels in ((3, 4, 1), (31, 5, 3), (33, 4, 2), (97, 3, 1), (255, 5, 2), (257, 6, 3), (513, 3, 1)):
             rs = np.random.RandomState(W + L + offset)
             flat = torch.empty(L * H * W + offset, dtype=torch.float32 if dtype == np.float32 else torch.int32,
