@@ -7,10 +7,11 @@
 // Implicit GEMM.  A tile is M = 128 consecutive pixels of one image row,
 // N = COUT output channels, K = 9 taps x CIN input channels, BF16 operands,
 // FP32 accumulation.  Activations are NHWC BF16.  A CTA owns a strip of
-// tiles going down one 128-pixel column band of an image, so each input row
-// is loaded once (plus one halo row above and below the strip): a row
-// arrives as one TMA tensor copy of 130 pixels x CIN channels (the band plus
-// one pixel either side; pixels and rows outside the image read as zero,
+// tiles going down one column band (up to 128 pixels; a narrower one's last
+// accumulator rows are computed from what the buffer held and not read) of an
+// image, so each input row is loaded once (plus one halo row above and below
+// the strip): a row arrives as one TMA tensor copy of band + 2 pixels x CIN
+// channels (the band plus one pixel either side; pixels and rows outside the image read as zero,
 // which is the convolution's zero padding) into a 1024-byte aligned buffer,
 // swizzled by the copy (128-, 64- or 32-byte swizzle for CIN = 64, 32, 16:
 // one pixel's channels per swizzle row), which is the canonical K-major
@@ -82,7 +83,7 @@ struct ConvTcParams {
     float *bias_part;          // EPI_MASK, EPI_LOSS: [CTA][COUT] sums of the gradient written
     double *loss_part;         // EPI_LOSS: [CTA] sums of squared differences
     int n, h, w;             // images, rows, columns
-    int bands, chunks, rows_per_chunk, items;
+    int band, bands, chunks, rows_per_chunk, items;  // band: pixels of a full one
     int *status;
 };
 
@@ -99,7 +100,7 @@ enum {
 };
 
 constexpr int kTileM = 128;            // pixels per tile (MMA M)
-constexpr int kSlab = kTileM + 2;      // pixels per row copy: the band and one either side
+constexpr int kSlab = kTileM + 2;      // pixels per row copy at most: the band and one either side
 constexpr int kThreadsTc = 192;        // weight gradient: warps 0-3 epilogue, 4 copies, 5 MMA
 constexpr int kCopyWarp = 4, kMmaWarp = 5;
 
@@ -169,12 +170,12 @@ struct Item {
     int img, x0, y0, rows;
 };
 
-// Work item: (image, 128-pixel band, chunk of rows_per_chunk rows), chunks
+// Work item: (image, band of up to 128 pixels, chunk of rows_per_chunk rows), chunks
 // of one band adjacent so that neighbouring CTAs share halo rows in L2.
 __device__ __forceinline__ Item item_of(const ConvTcParams &p, int it) {
     Item r;
     const int chunk = it % p.chunks, rest = it / p.chunks;
-    r.x0 = (rest % p.bands) * kTileM;
+    r.x0 = (rest % p.bands) * p.band;
     r.img = rest / p.bands;
     r.y0 = chunk * p.rows_per_chunk;
     r.rows = min(p.rows_per_chunk, p.h - r.y0);
@@ -200,8 +201,7 @@ struct TcLayout {
     static constexpr int kChunks = CIN / 8;
     static constexpr int kPixBytes = CIN * 2;                          // one pixel: one swizzle row
     static constexpr uint32_t kSwizzle = CIN == 64 ? 2 : (CIN == 32 ? 4 : 6);
-    static constexpr int kCopyBytes = kSlab * kPixBytes;               // what one row's copy writes
-    static constexpr int kRowBytes = (kCopyBytes + 1023) / 1024 * 1024;  // one row buffer, 1024-byte aligned
+    static constexpr int kRowBytes = (kSlab * kPixBytes + 1023) / 1024 * 1024;  // one row buffer, 1024-byte aligned
     static constexpr int kWBytes = 9 * CIN * COUT * 2;      // [tap][chunk][co][16 B]
     static constexpr int kRows = 0;
     static constexpr int kW = kRows + RING * kRowBytes;
@@ -318,10 +318,10 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
         // swizzle would put them (address bits 4-6 xor bits 7-9, as many as a
         // swizzle row's chunks take).  All of a thread's loads are in flight
         // at once, ahead of the wait for the buffer.
-        constexpr int kCopyThreads = Lay::kCopy * 32, kQuads = CIN / 4, kRowQuads = kSlab * kQuads;
-        constexpr int kEach = (kRowQuads + kCopyThreads - 1) / kCopyThreads;
+        constexpr int kCopyThreads = Lay::kCopy * 32, kQuads = CIN / 4;
+        constexpr int kEach = (kSlab * kQuads + kCopyThreads - 1) / kCopyThreads;
         constexpr int kAhead = 1;  // rows the L2 prefetch runs ahead
-        const int t0 = threadIdx.x - Lay::kEpi * 32;
+        const int t0 = threadIdx.x - Lay::kEpi * 32, row_quads = (p.band + 2) * kQuads;
         uint32_t ld = 0;
         bool ok = true;
         for (int it = blockIdx.x; it < p.items && ok && !__any_sync(~0u, *abort_flag); it += gridDim.x) {
@@ -329,13 +329,13 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
             for (int r = t.y0 - 1; r <= t.y0 + t.rows; ++r, ++ld) {
                 const int ra = r + kAhead;
                 if (t0 == 0 && ra >= 0 && ra < p.h && ra <= t.y0 + t.rows) {
-                    const int xl = t.x0 > 0 ? t.x0 - 1 : 0, xr = t.x0 + kTileM + 1 < p.w ? t.x0 + kTileM + 1 : p.w;
+                    const int xl = t.x0 > 0 ? t.x0 - 1 : 0, xr = t.x0 + p.band + 1 < p.w ? t.x0 + p.band + 1 : p.w;
                     bulk_prefetch_l2(p.x + (((size_t)t.img * p.h + ra) * p.w + xl) * CIN,
                                      (uint32_t)((xr - xl) * CIN * 4));
                 }
                 // Quads of the row inside the image: [qlo, qhi).
                 const int left = t.x0 == 0 ? kQuads : 0, right = (p.w - t.x0 + 1) * kQuads;
-                const int qlo = r >= 0 && r < p.h ? left : kRowQuads, qhi = right < kRowQuads ? right : kRowQuads;
+                const int qlo = r >= 0 && r < p.h ? left : row_quads, qhi = right < row_quads ? right : row_quads;
                 const ptrdiff_t row = (((ptrdiff_t)t.img * p.h + r) * p.w + t.x0 - 1) * CIN;  // of quad 0
                 float4 v[kEach];
 #pragma unroll
@@ -352,11 +352,11 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                 }
                 // The rounding kept: the band's own pixels of the strip's own rows, each once.
                 const bool keep = p.x_bf16 && r >= t.y0 && r < t.y0 + t.rows;
-                const int khi = qhi < (kTileM + 1) * kQuads ? qhi : (kTileM + 1) * kQuads;
+                const int khi = qhi < (p.band + 1) * kQuads ? qhi : (p.band + 1) * kQuads;
 #pragma unroll
                 for (int i = 0; i < kEach; ++i) {
                     const int q = t0 + i * kCopyThreads;
-                    if (q >= kRowQuads) break;
+                    if (q >= row_quads) break;
                     const uint2 b = pack_bf16x4(&v[i].x);
                     uint32_t at = (uint32_t)q * 8;
                     at ^= ((at >> 7) & (Lay::kChunks - 1)) << 4;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                         *abort_flag = 1;
                         break;
                     }
-                    mbar_arrive_expect_tx(&full[slot], Lay::kCopyBytes);
+                    mbar_arrive_expect_tx(&full[slot], (uint32_t)(p.band + 2) * Lay::kPixBytes);
                     tma_load_row(smem_addr(sm + Lay::kRows + slot * Lay::kRowBytes), &rows_map, t.x0 - 1, r, t.img,
                                  &full[slot]);
                 }
@@ -516,7 +516,8 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                 // written 512 bytes per instruction (the residual read the
                 // same way).
                 const int x = t.x0 + quarter * 32;
-                const int valid = p.w - x < 32 ? p.w - x : 32;
+                const int ends = t.x0 + p.band < p.w ? t.x0 + p.band : p.w;  // of the band
+                const int valid = ends - x < 32 ? ends - x : 32;
                 const size_t pix = ((size_t)t.img * p.h + t.y0 + j) * p.w + x;
                 // 16-byte chunk q of the warp's block: pixel q / kChunksOut,
                 // chunk q % kChunksOut of its channels, at(q) in the tensor.
@@ -723,16 +724,22 @@ cudaError_t cta_slots(int smem, int *slots) {
 // four rows each (two halo rows per chunk), as many as make the longest CTA
 // shortest -- its items times a chunk's rows with their halo.  False when
 // there is nothing to do or too much to count.  Splitting the rows evenly
-// over the slots and rounding up gave 320 items on 304 slots at 16x256x192
-// (27 rows a chunk), so that the kernels took two chunks' time; now 288 items
-// of 29 rows: gradients at 16x256x192x64 746 -> 536 us.
+// over the slots and rounding up gave 320 items on 304 slots for 16 images of
+// 256x192 (21 rows a chunk), so that the kernels took two chunks' time; now
+// 288 items of 22 rows: gradients there 746 -> 536 us.
+//
+// Bands are as even as whole groups of 16 pixels (the weight gradient's K
+// step) allow: 192 columns are two bands of 96, not 128 and 64, whose CTAs
+// kept unlike SMs busy unlike long (16 images of 192x256 with 64 labels:
+// forward 248 -> 223 us, gradients 602 -> 550; four of 144x300 249 -> 227).
 struct ItemPlan {
-    int bands, rows_per_chunk, chunks, items, grid;
+    int band, bands, rows_per_chunk, chunks, items, grid;
 };
 
 bool plan_items(int n, int h, int w, int slots, ItemPlan &pl) {
     if (n < 1 || h < 1 || w < 1 || slots < 1) return false;
     pl.bands = (w + kTileM - 1) / kTileM;
+    pl.band = ((w + pl.bands - 1) / pl.bands + 15) / 16 * 16;
     const long long strips = (long long)n * pl.bands;
     // Past the first few waves a finer split gains nothing.
     const long long most = (h + 3) / 4 < 2LL * slots ? (h + 3) / 4 : 2LL * slots;
@@ -769,16 +776,17 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
     static TcKernelSetup setup;
     cudaError_t attr_err = setup.ensure(kern, kSmem);
     if (attr_err != cudaSuccess) return attr_err;
-    alignas(64) CUtensorMap map{};
-    if constexpr (!IN_F32) {
-        if (!tensor_map_encoder()) return cudaErrorNotSupported;
-        if (!encode_rows_map(&map, in, CIN, p.n, p.h, p.w, kSlab)) return cudaErrorInvalidValue;
-    }
     int slots = 0;
     cudaError_t e = cta_slots(kSmem, &slots);
     if (e != cudaSuccess) return e;
     ItemPlan pl;
     if (!plan_items(p.n, p.h, p.w, slots, pl)) return cudaErrorInvalidValue;
+    alignas(64) CUtensorMap map{};
+    if constexpr (!IN_F32) {
+        if (!tensor_map_encoder()) return cudaErrorNotSupported;
+        if (!encode_rows_map(&map, in, CIN, p.n, p.h, p.w, pl.band + 2)) return cudaErrorInvalidValue;
+    }
+    p.band = pl.band;
     p.bands = pl.bands;
     p.rows_per_chunk = pl.rows_per_chunk;
     p.chunks = pl.chunks;
@@ -813,7 +821,7 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
 struct WgradParams {
     float *partials;  // [CTA][COUT][9][CIN]
     int n, h, w;
-    int bands, chunks, rows_per_chunk, items;
+    int band, bands, chunks, rows_per_chunk, items;  // band: pixels of a full one
     int *status;
 };
 
@@ -822,8 +830,8 @@ struct WgLayout {
     static constexpr int kInPix = CIN * 2, kOutPix = COUT * 2;  // bytes per pixel = one swizzle row
     static constexpr uint32_t kSwIn = CIN == 64 ? 2 : (CIN == 32 ? 4 : 6);
     static constexpr uint32_t kSwOut = COUT == 64 ? 2 : (COUT == 32 ? 4 : 6);
-    static constexpr int kInCopy = kSlab * kInPix, kInRow = (kInCopy + 1023) / 1024 * 1024;
-    static constexpr int kOutCopy = kTileM * kOutPix, kOutRow = (kOutCopy + 1023) / 1024 * 1024;
+    static constexpr int kInRow = (kSlab * kInPix + 1023) / 1024 * 1024;
+    static constexpr int kOutRow = (kTileM * kOutPix + 1023) / 1024 * 1024;
     static constexpr int kTaps = 128 / CIN;                // taps per M tile
     static constexpr int kMT = (3 + kTaps - 1) / kTaps;    // M tiles per row offset
     static constexpr int kAcc = 3 * kMT;                   // accumulators of COUT columns
@@ -893,6 +901,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
     ip.n = p.n;
     ip.h = p.h;
     ip.w = p.w;
+    ip.band = p.band;
     ip.bands = p.bands;
     ip.chunks = p.chunks;
     ip.rows_per_chunk = p.rows_per_chunk;
@@ -907,7 +916,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                     int slot = (int)(li % RING);
                     ok = mbar_wait_bounded(&in_empty[slot], ((li / RING) & 1u) ^ 1u, p.status);
                     if (!ok) break;
-                    mbar_arrive_expect_tx(&in_full[slot], Lay::kInCopy);
+                    mbar_arrive_expect_tx(&in_full[slot], (uint32_t)(p.band + 2) * Lay::kInPix);
                     tma_load_row(smem_addr(sm + Lay::kIn + slot * Lay::kInRow), &in_map, t.x0 - 1, t.y0 - 1 + i, t.img,
                                  &in_full[slot]);
                     ++li;
@@ -915,7 +924,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                     slot = (int)(lo % RING);
                     ok = mbar_wait_bounded(&out_empty[slot], ((lo / RING) & 1u) ^ 1u, p.status);
                     if (!ok) break;
-                    mbar_arrive_expect_tx(&out_full[slot], Lay::kOutCopy);
+                    mbar_arrive_expect_tx(&out_full[slot], (uint32_t)p.band * Lay::kOutPix);
                     tma_load_row(smem_addr(sm + Lay::kOut + slot * Lay::kOutRow), &out_map, t.x0, t.y0 + i, t.img,
                                  &out_full[slot]);
                     ++lo;
@@ -963,6 +972,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                         for (int mt = 0; mt < Lay::kMT; ++mt)
 #pragma unroll
                             for (int ks = 0; ks < kTileM / 16; ++ks) {
+                                if (ks * 16 >= p.band) break;
                                 // Offsets in 16-byte units: tap block mt starts
                                 // mt * kTaps pixels in, K step ks 16 pixels on.
                                 const uint64_t ao = (uint64_t)((mt * Lay::kTaps + 16 * ks) * Lay::kInPix >> 4);
@@ -1025,16 +1035,17 @@ cudaError_t launch_wgrad_tc(const __nv_bfloat16 *dout, const __nv_bfloat16 *in, 
     static TcKernelSetup setup;
     cudaError_t attr_err = setup.ensure(kern, kSmem);
     if (attr_err != cudaSuccess) return attr_err;
-    alignas(64) CUtensorMap in_map, out_map;
-    if (!encode_rows_map(&in_map, in, CIN, p.n, p.h, p.w, kSlab) ||
-        !encode_rows_map(&out_map, dout, COUT, p.n, p.h, p.w, kTileM))
-        return cudaErrorInvalidValue;
     int slots = 0;
     cudaError_t e = cta_slots(kSmem, &slots);
     if (e != cudaSuccess) return e;
     if (slots > max_parts) slots = max_parts;
     ItemPlan pl;
     if (!plan_items(p.n, p.h, p.w, slots, pl)) return cudaErrorInvalidValue;
+    alignas(64) CUtensorMap in_map, out_map;
+    if (!encode_rows_map(&in_map, in, CIN, p.n, p.h, p.w, pl.band + 2) ||
+        !encode_rows_map(&out_map, dout, COUT, p.n, p.h, p.w, pl.band))
+        return cudaErrorInvalidValue;
+    p.band = pl.band;
     p.bands = pl.bands;
     p.rows_per_chunk = pl.rows_per_chunk;
     p.chunks = pl.chunks;
