@@ -1,7 +1,7 @@
 // batch.cu -- many independent grids solved together: one persistent launch
 // per label bucket walks a work list of (grid, tile) entries, for one
-// half-sweep (the buckets then are parallel branches, each launch starting as
-// the one before it drains) or cooperatively for several with a bounded grid
+// half-sweep (the buckets then are parallel branches, each launch ready as
+// the one before it ends) or cooperatively for several with a bounded grid
 // barrier between them; the whole solve (layout transforms, initialisation,
 // the persistent launches, the labels of the last half-sweep) is captured
 // once into a CUDA graph and replayed.  The tile shape and the
@@ -109,8 +109,7 @@ __global__ void __launch_bounds__(NW * 32) batch_kernel(const BatchLaunch b) {
     __syncthreads();
     const int *bases = b.bases_in_smem ? bases_s : nullptr;
     uint32_t parity = 0;
-    // A launch of one half-sweep starts while the one before it drains.
-    launch_dependents();
+    // Not before the launch of the half-sweep ahead of this one is done.
     grid_dependency_wait();
     for (int it = b.it_begin; it < b.it_end; ++it) {
         int t = blockIdx.x;
@@ -154,7 +153,6 @@ __global__ void __launch_bounds__(kWarpTileWarps * 32) batch_kernel_warp(const B
     __syncthreads();
     const int *bases = b.bases_in_smem ? bases_s : nullptr;
     const int warp = threadIdx.x >> 5;
-    launch_dependents();
     grid_dependency_wait();
     for (int it = b.it_begin; it < b.it_end; ++it) {
         for (int t = blockIdx.x * kWarpTileWarps + warp; t < b.total_tiles; t += gridDim.x * kWarpTileWarps) {
@@ -171,7 +169,6 @@ __global__ void __launch_bounds__(kWarpTileWarps * 32) batch_kernel_warp(const B
 // `wpt` of them per work-list tile.
 constexpr int kBatchLabelWarps = 8;
 __global__ void __launch_bounds__(kBatchLabelWarps * 32) batch_labels(const BatchLaunch b, int wpt) {
-    launch_dependents();
     grid_dependency_wait();
     const int lane = threadIdx.x & 31;
     const long warps = (long)gridDim.x * kBatchLabelWarps, total = (long)b.total_tiles * wpt;
@@ -411,8 +408,8 @@ std::vector<BatchItem> make_items(ginf_batch *b, int tile_nodes) {
 }
 
 // Launches one batch kernel: cooperatively when it runs several half-sweeps
-// (its blocks meet at a grid barrier), else so that it may start while the
-// launch before it drains.
+// (its blocks meet at a grid barrier), else so that it is ready when the launch
+// before it ends.
 template <typename K>
 cudaError_t launch_batch(K kern, LaunchCache &cache, BatchLaunch bl, int warps, size_t slots, uint32_t max_slot,
                          int block_tiles, int num_sms, cudaStream_t s) {

@@ -1056,7 +1056,6 @@ __global__ void __launch_bounds__(NW * 32, 5) sweep_kernel_split(const SweepPara
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
     __shared__ SplitXch<NW> xs;
-    launch_dependents();
     const TableConsts<float> tc = table_consts<float, KIND_QUAD>(p.V, LMIN == LMAX ? LMAX : p.L);
     if (threadIdx.x == 0) {
         mbar_init(&full_bar, NW * 32);
@@ -1081,9 +1080,6 @@ template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, bool DIR
 __device__ __forceinline__ void sweep_body(const SweepParams &p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
-    // The next half-sweep may be launched now; its blocks take SM slots as
-    // these retire and wait below before touching any record.
-    launch_dependents();
     const TableConsts<T> tc = table_consts<T, KIND>(p.V, LMIN == LMAX ? LMAX : p.L);
     if (threadIdx.x == 0) {
         mbar_init(&full_bar, NW * 32);
@@ -1148,9 +1144,15 @@ cudaError_t launch_tiles(K kern, LaunchCache &lc_state, int NW, int nodes, const
     int grid = occ * num_sms;
     const int need = (p.num_tiles + block_tiles - 1) / block_tiles;
     if (grid > need) grid = need;
-    // Programmatic stream serialisation: this launch may begin while the
-    // previous kernel of the stream finishes (the kernel waits for it before
-    // reading records).
+    // Programmatic stream serialisation: the launch is ready when the blocks of
+    // the previous kernel have gone (the kernel waits for its memory before
+    // reading records).  No kernel here lets its successor start earlier:
+    // blocks waiting beside running ones fill the SMs that empty first, and
+    // the half-sweep they then run is that uneven.  us per half-sweep, released
+    // at the start -> at the end: 160x120 L = 16 4.6 -> 2.7, L = 32 7.5 -> 3.6,
+    // L = 64 8.3 -> 5.7; 384x288 7.5 -> 6.5, 14.3 -> 12.4, 24.7 -> 23.9;
+    // 640x480 17.6 -> 16.5, 37.1 -> 33.7, 62.7 -> 62.3; released after their own
+    // wait: 2.9, 3.8, 5.7; 7.3, 14.2, 24.2; 17.2, 36.1, 62.6.
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(grid);
     lc.blockDim = dim3(NW * 32);

@@ -293,7 +293,6 @@ __global__ void __launch_bounds__(64 * SPL, table_blocks(STD, SPL, TI * TN)) swe
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
     __shared__ T mins[sizeof(M) == 2 && STD ? 4 * kTableNodes : 1][kTableMaxGroups];
-    launch_dependents();
     const int L = p.L;
     T *Vs = reinterpret_cast<T *>(smem + (size_t)kTableNodes * p.slot_bytes);
     int odd_table = 0;

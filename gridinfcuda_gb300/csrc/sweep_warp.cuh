@@ -13,7 +13,8 @@
 // accesses per node, L2-resident grids the latency of a half-sweep.  us per
 // half-sweep, block tiles with bulk copies -> this form: 1920x1080 FP32 L = 8
 // 145 -> 106, L = 16 131 -> 119 (4.8 TB/s), L = 24 191 -> 168, L = 32 197 ->
-// 189 (6.1 TB/s); 384x288 L = 16 9.7 -> 7.4, L = 32 14.9 -> 13.4.  At L = 40,
+// 189 (6.1 TB/s); 384x288 L = 16 9.7 -> 7.4, L = 32 14.9 -> 13.4
+// (6.5 and 12.4 since a half-sweep's blocks no longer start beside the last one's).  At L = 40,
 // 48 and 64 it is slower on large grids (1920x1080 258 -> 280, 303 -> 331 and
 // 351 -> 412) for want of registers, hence kWarpTileLabels.  With the lanes of
 // the global accesses laid out as the messages' (a quarter-warp on eight nodes)
@@ -135,7 +136,6 @@ __device__ __forceinline__ void warp_tile(const SweepParams &p, const TableConst
 template <typename T, int LMAX, int LMIN, int MINB>
 __global__ void __launch_bounds__(kWarpTileWarps * 32, MINB) sweep_kernel_warp(const SweepParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    launch_dependents();
     const TableConsts<T> tc = table_consts<T, KIND_LINEAR>(p.V, LMIN == LMAX ? LMAX : p.L);
     const int warp = threadIdx.x >> 5;
     unsigned char *slots = smem + (size_t)warp * 8 * p.slot_bytes;
@@ -152,9 +152,10 @@ cudaError_t launch_warp_kernel(const RecordFormat &f, const SweepParams &p, cuda
 }
 
 // Launches of at most this many tiles at L = 16 take the kernel held to 48
-// registers (40 warps per SM instead of 36): 384x288 7.8 -> 7.4 us, 640x480
-// 18.2 -> 17.4 us, but 800x600 26.3 -> 27.0 us and 1920x1080 119 -> 122 us.
-constexpr long kWarpSmallTiles = 24576;
+// registers (40 warps per SM instead of 36): 240x180 3.9 -> 3.6 us, 384x288
+// (6864 tiles) 6.8 -> 6.5, but 640x480 (19120) 15.8 -> 16.6 and 800x600 24.8 ->
+// 27.1.
+constexpr long kWarpSmallTiles = 12288;
 
 template <typename T, int LM, int LO>
 cudaError_t launch_warp_tiles(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
