@@ -13,8 +13,8 @@
 // accesses per node, L2-resident grids the latency of a half-sweep.  us per
 // half-sweep, block tiles with bulk copies -> this form: 1920x1080 FP32 L = 8
 // 145 -> 106, L = 16 131 -> 119 (4.8 TB/s), L = 24 191 -> 168, L = 32 197 ->
-// 189 (6.1 TB/s); 384x288 L = 16 9.7 -> 7.4, L = 32 14.9 -> 13.4
-// (6.5 and 12.4 since a half-sweep's blocks no longer start beside the last one's).  At L = 40,
+// 189 (6.1 TB/s); 384x288 L = 16 9.7 -> 7.4, L = 32 14.9 -> 13.4 (6.5 and 12.0
+// since a half-sweep's blocks no longer start beside the last one's).  At L = 40,
 // 48 and 64 it is slower on large grids (1920x1080 258 -> 280, 303 -> 331 and
 // 351 -> 412) for want of registers, hence kWarpTileLabels.  With the lanes of
 // the global accesses laid out as the messages' (a quarter-warp on eight nodes)
@@ -25,7 +25,9 @@
 
 namespace ginf_gpu {
 
-constexpr int kWarpTileWarps = 4;  // warps per block, a tile of eight nodes each
+// Warps per block of a batch's launches, a tile of eight nodes each (the batch
+// of twelve grids: two 12.88 ms, four 12.86, eight 12.94).
+constexpr int kWarpTileWarps = 4;
 
 // Tile t of one half-sweep by one warp; `slots` holds the warp's eight slots.
 template <typename T, int LMAX, int LMIN>
@@ -131,40 +133,46 @@ __device__ __forceinline__ void warp_tile(const SweepParams &p, const TableConst
     __syncwarp();
 }
 
-// One half-sweep, a block's warps taking tiles on their own.  MINB: blocks per
-// SM the registers are allocated for (0: no bound).
-template <typename T, int LMAX, int LMIN, int MINB>
-__global__ void __launch_bounds__(kWarpTileWarps * 32, MINB) sweep_kernel_warp(const SweepParams p) {
+// One half-sweep, a block's NW warps taking tiles on their own.  MINB: blocks
+// per SM the registers are allocated for (0: no bound).
+template <typename T, int LMAX, int LMIN, int NW, int MINB>
+__global__ void __launch_bounds__(NW * 32, MINB) sweep_kernel_warp(const SweepParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     const TableConsts<T> tc = table_consts<T, KIND_LINEAR>(p.V, LMIN == LMAX ? LMAX : p.L);
     const int warp = threadIdx.x >> 5;
     unsigned char *slots = smem + (size_t)warp * 8 * p.slot_bytes;
     grid_dependency_wait();
-    for (int t = blockIdx.x * kWarpTileWarps + warp; t < p.num_tiles; t += gridDim.x * kWarpTileWarps)
+    for (int t = blockIdx.x * NW + warp; t < p.num_tiles; t += gridDim.x * NW)
         warp_tile<T, LMAX, LMIN>(p, tc, t, slots);
 }
 
-template <typename T, int LM, int LO, int MINB>
+template <typename T, int LM, int LO, int NW, int MINB = 0>
 cudaError_t launch_warp_kernel(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
     static LaunchCache cache;
-    return launch_tiles(sweep_kernel_warp<T, LM, LO, MINB>, cache, kWarpTileWarps, 8, p, f.slot_bytes, s, num_sms,
-                        (size_t)(kWarpTileWarps - 1) * 8 * f.slot_bytes, kWarpTileWarps);
+    return launch_tiles(sweep_kernel_warp<T, LM, LO, NW, MINB>, cache, NW, 8, p, f.slot_bytes, s, num_sms,
+                        (size_t)(NW - 1) * 8 * f.slot_bytes, NW);
 }
 
-// Launches of at most this many tiles at L = 16 take the kernel held to 48
-// registers (40 warps per SM instead of 36): 240x180 3.9 -> 3.6 us, 384x288
-// (6864 tiles) 6.8 -> 6.5, but 640x480 (19120) 15.8 -> 16.6 and 800x600 24.8 ->
-// 27.1.
-constexpr long kWarpSmallTiles = 12288;
+// Warps per block, us per half-sweep: two at L = 8 (four: 1280x720 55.7 -> 53.2,
+// 1920x1080 115 -> 110, small grids equal), four at L = 24, eight at L = 32 (four:
+// 384x288 12.5 -> 12.0, 1920x1080 197 -> 192).  At L = 16 four up to
+// kWarpTiles4 tiles (800x600, 29900 tiles: 24.8, with two 28.2) and two above
+// it, where the records outgrow the L2 cache (1024x768 44.6 -> 43.6, 1600x900
+// 90.7 -> 76.5, 1920x1080 124 -> 108), and of four those up to kWarpSmallTiles
+// held to 48 registers (40 warps per SM instead of 36: 240x180 3.9 -> 3.6,
+// 384x288, 6864 tiles, 6.8 -> 6.5, but 640x480, 19120, 15.8 -> 16.6).
+constexpr long kWarpSmallTiles = 12288, kWarpTiles4 = 40960;
 
 template <typename T, int LM, int LO>
 cudaError_t launch_warp_tiles(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
     if constexpr (LM == 16) {
         const int n1 = p.W >= 3 ? (p.W - 3) / 2 + 1 : 0;
         const long tiles = p.H >= 3 ? (long)(p.H - 2) * ((n1 + 7) / 8) : 0;
-        if (tiles <= kWarpSmallTiles) return launch_warp_kernel<T, LM, LO, 10>(f, p, s, num_sms);
+        if (tiles <= kWarpSmallTiles) return launch_warp_kernel<T, LM, LO, 4, 10>(f, p, s, num_sms);
+        if (tiles <= kWarpTiles4) return launch_warp_kernel<T, LM, LO, 4>(f, p, s, num_sms);
+        return launch_warp_kernel<T, LM, LO, 2>(f, p, s, num_sms);
     }
-    return launch_warp_kernel<T, LM, LO, 0>(f, p, s, num_sms);
+    return launch_warp_kernel<T, LM, LO, LM == 8 ? 2 : (LM == 32 ? 8 : 4)>(f, p, s, num_sms);
 }
 
 }  // namespace ginf_gpu

@@ -26,6 +26,18 @@ def test_linear_messages_vs_oracle(ginf, orc, dtype):
         assert np.array_equal(mg.view(np.uint32), mw.view(np.uint32)), L
 
 
+@pytest.mark.parametrize("W,H,L", [(390, 290, 16), (401, 263, 13), (760, 560, 16), (1032, 640, 16), (1029, 641, 10),
+                                   (230, 170, 8), (230, 170, 32), (203, 177, 26)])
+def test_warp_half_sweep_block_shapes_vs_oracle(ginf, orc, W, H, L):
+    """Grids on either side of the lines between the warp half-sweep's block
+    shapes (8, 32 labels; at 16 up to 12288, up to 40960 and above of tiles)."""
+    P = synth.random_problem(W, H, L, 77, scale=1.0, trunc=1.7, cost_max=4.0)
+    want, mw = orc.hbp(P.D, P.V, P.model, 1, 3, want_msgs=True)
+    got, mg = ginf.decode_hbp(P.D, P.V, P.model, 1, 3, want_msgs=True)
+    assert np.array_equal(got, want)
+    assert np.array_equal(mg.view(np.uint32), mw.view(np.uint32))
+
+
 @pytest.mark.parametrize("store", [0, 1])
 @pytest.mark.parametrize("norm", [0, 1])
 @pytest.mark.parametrize("trunc", [25.0, 50.0])
