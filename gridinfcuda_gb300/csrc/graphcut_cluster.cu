@@ -27,14 +27,15 @@
 //
 // The global relabel and the final reachability are level-synchronous searches
 // on bit sets, 32 nodes to a word and a word to a thread, with one cluster
-// barrier per level; the few per-pair reductions ride on such barriers.  Every wait inside a round is bounded; one
-// that runs out is recorded and the round ends with all CTAs.
+// barrier per level; the few per-pair reductions ride on such barriers.  Every
+// wait inside a round is bounded; one that runs out is recorded and the round
+// ends with all CTAs.
 //
 // Bound: the latency of a wavefront step with twenty warps on the SM (about
 // 800 cycles, eight per instruction; 400 steps a band, then the bands' lags:
 // 0.33 ms a round of twenty sweeps at 384x288, 16 bands) and the searches'
-// barriers.  384x288x16, one pass from the BP labels, three seeds: 787, - and -
-// ms with one CTA in global memory, 187, 87 and 138 ms here with searches that
+// barriers.  384x288x16, one pass from the BP labels: 787 ms with one CTA in
+// global memory; here, for three seeds, 187, 87 and 138 ms with searches that
 // walked the unreached nodes, 91, 63 and 90 ms with bit sets, 80, 55 and 79 ms
 // with the short step.  Also measured: four diagonals between two waits 137 ms
 // (the lags grow by more than the waits cost), flows formed branch-free and

@@ -168,7 +168,7 @@ ginf_status ginf_decode_hbp(ginf_workspace *ws, const ginf_grid *grid, int32_t n
 /* ICM.  asynchronous == 0: Jacobi sweeps, replacing ginf::decodeIcmSync
  * (src/icm.cc:4-38) and ginf::gpuDecodeIcm (src/gpu/icm.cu:53-83).
  * asynchronous == 1: raster-order Gauss-Seidel, replacing ginf::decodeIcmAsync
- * (src/icm.cc:40-67), run as an exact anti-diagonal wavefront.
+ * (src/icm.cc:40-67), run as an exact wavefront.
  * result (W*H) receives a copy of initial, then interior nodes are updated. */
 ginf_status ginf_decode_icm(ginf_workspace *ws, const ginf_grid *grid, const int32_t *initial,
                             int32_t iters, int32_t asynchronous, int32_t *result,
@@ -182,8 +182,9 @@ ginf_status ginf_decode_icm(ginf_workspace *ws, const ginf_grid *grid, const int
  * change.  int32 grids only (the reference instantiates it for int,
  * graphcut.cc:281).  The results are the reference's bit for bit, including
  * its raster-order pushes and relabels and the state it keeps across label
- * pairs.  result (W*H) receives a copy of initial, then the swaps.  One CTA
- * runs the whole solve; a solve that runs longer than 60 s on the device
+ * pairs.  result (W*H) receives a copy of initial, then the swaps.  One
+ * thread-block cluster runs the whole solve where the grid's state fits its
+ * shared memory, else one CTA; a solve that runs longer than 60 s on the device
  * returns GINF_ERR_TIMEOUT. */
 ginf_status ginf_decode_alpha_beta(ginf_workspace *ws, const ginf_grid *grid, const int32_t *initial,
                                    int32_t iters, int32_t *result, const ginf_options *opt, ginf_stats *stats);
@@ -229,9 +230,10 @@ ginf_status ginf_stereo_costs_u8(int32_t width, int32_t height, int32_t num_labe
  * `iters` half-sweeps, the reference's semantics and stale-belief decode, as
  * ginf_decode_hbp with num_levels == 1).  The reference solves one grid per
  * call (src/include/bp.h:14-26); a batch solves them together in one
- * persistent cooperative launch per label group and `sweeps_per_launch`
- * half-sweeps, walking a work list of (grid, tile) entries, and replays the
- * whole solve from a CUDA graph captured at creation.  Grids: FP32 costs, Potts or
+ * persistent launch per label group and `sweeps_per_launch` half-sweeps
+ * (cooperative for several; the label groups' launches side by side for one),
+ * walking a work list of (grid, tile) entries, and replays the whole solve
+ * from a CUDA graph captured at creation.  Grids: FP32 costs, Potts or
  * truncated-linear smoothness, 2 <= L <= 64, all buffers device memory; the
  * plan keeps the pointers, so later runs see whatever those buffers hold.
  * The tile size and half-sweeps per launch are given in `opt` or chosen by
