@@ -741,16 +741,18 @@ bool plan_items(int n, int h, int w, int slots, ItemPlan &pl) {
     pl.bands = (w + kTileM - 1) / kTileM;
     pl.band = ((w + pl.bands - 1) / pl.bands + 15) / 16 * 16;
     const long long strips = (long long)n * pl.bands;
-    // Past the first few waves a finer split gains nothing.
-    const long long most = (h + 3) / 4 < 2LL * slots ? (h + 3) / 4 : 2LL * slots;
+    // The finest split that is done in k waves of CTAs, for the first few k:
+    // past them the halo rows cost more than the rounding gains.
+    const long long most = (h + 3) / 4, first = (strips + slots - 1) / slots;
     long long best = -1;
-    for (long long c = 1; c <= most; ++c) {
-        const long long rows = (h + c - 1) / c, chunks = (h + rows - 1) / rows;
-        const long long cost = (strips * chunks + slots - 1) / slots * (rows + 2);
-        if (best >= 0 && cost >= best) continue;
-        best = cost;
+    for (long long k = first; k < first + 16; ++k) {
+        const long long c = k * slots / strips < most ? k * slots / strips : most;
+        const long long rows = (h + c - 1) / c;
+        if (best >= 0 && k * (rows + 2) >= best) continue;
+        best = k * (rows + 2);
         pl.rows_per_chunk = (int)rows;
-        pl.chunks = (int)chunks;
+        pl.chunks = (int)((h + rows - 1) / rows);
+        if (c == most) break;
     }
     const long long items = strips * pl.chunks;
     if (items > 0x7fffffffLL) return false;
