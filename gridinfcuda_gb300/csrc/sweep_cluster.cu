@@ -29,8 +29,8 @@
 // against k x (record in + four messages out) / 2 for k single half-sweeps.
 //
 // Measured on GB300 this is slower than one half-sweep per launch (384x288,
-// L = 16, 50 half-sweeps: 0.63 ms at 4 per launch against 0.49 ms; 1920x1080:
-// 10.6 ms against 6.8 ms): at L <= 32 the update is bound by the latency of
+// L = 16, 50 half-sweeps: 0.63 ms at 4 per launch against 0.33 ms; 1920x1080:
+// 10.6 ms against 5.4 ms): at L <= 32 the update is bound by the latency of
 // its sequential scans, not by HBM, and one resident CTA per SM (20 warps),
 // the cluster barriers, the halo's repeated updates and the clusters' GPC
 // packing cost more than the traffic saved.  It is therefore opt-in

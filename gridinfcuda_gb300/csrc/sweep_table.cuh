@@ -14,10 +14,11 @@
 // every thread TI outputs of TN vectors in registers, so that four steps of j
 // read 4 TI entries of V and four of each vector from shared memory for
 // 4 TI TN additions and minima.  Additions and minima go two steps of j to an
-// instruction (add.rn.f32x2, rounded as the scalar one; three-input minimum).  TI and TN follow L so that the block's threads have one
-// group of outputs each or nearly so (launch_table).  The lane-per-message
-// form this replaces read V through the cache once per addition and kept the
-// standard rule's vectors in local memory.
+// instruction (add.rn.f32x2, rounded as the scalar one; three-input minimum).
+// TI and TN follow L so that the block's threads have one group of outputs each
+// or nearly so (launch_table).  The lane-per-message form this replaces read V
+// through the cache once per addition and kept the standard rule's vectors in
+// local memory.
 //
 // Bound: HBM (36 B per updated node and label) for the reference rule up to
 // about 32 labels; above that the latency of a tile's phases with the few
@@ -27,6 +28,8 @@
 //   L           16         32         64          128
 //   reference   52 -> 24   146 -> 37  727 -> 85   - -> 256
 //   standard    127 -> 39  697 -> 75  3866 -> 200 - -> 720
+// (the reference rule at L = 32 33 since launches wait for the last one's blocks
+// to go, sweep_impl.cuh).
 // Also measured for the standard rule at L = 64: four warps of 8 x 4 outputs
 // 237, two of 8 x 8 with the additions paired along i 197 (the reference rule,
 // whose vectors need no subtraction, is faster paired along j).
