@@ -13,8 +13,11 @@
 // So warp j of every CTA runs sweep j, one lane per row, the warps chained by
 // progress counters in shared memory and the bands by mailbox words.
 //
-// What crosses a band's edge travels as one word per column: the flow pushed
-// over the edge, the sender's height after its sweep, and the sweep's number.
+// What crosses a band's edge travels as one 64-bit word per column: the flow
+// pushed over the edge (low half), the sender's height after its sweep and the
+// sweep's number.  It is read and written by scalar 64-bit accesses: the two
+// elements of a vector access are accesses of their own, in no stated order, so
+// a reader could meet a new number beside an old flow.
 // The band below waits for its upper neighbour's word of the same sweep, the
 // band above for its lower neighbour's word of the sweep before; a word is read
 // before its column's next one can be written (which waits, through the other
@@ -105,6 +108,16 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t v;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
     return v;
+}
+
+// A mailbox word's accesses: its own CTA reads it, a neighbour writes it.
+__device__ __forceinline__ uint64_t box_read(uint32_t addr) {
+    uint64_t v;
+    asm volatile("ld.relaxed.cluster.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void box_write(uint32_t addr, uint64_t v) {
+    asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
 }
 
 struct Band {
@@ -351,10 +364,9 @@ __device__ __forceinline__ void sweep(Band &b, int j, int first_tag, int *status
         for (uint32_t n = 1;; ++n) {
             if (seen <= k) seen = *before;
             if (!ok) {
-                asm volatile("ld.relaxed.cluster.shared::cluster.v2.u32 {%0, %1}, [%2];"
-                             : "=r"(w_lo), "=r"(w_hi)
-                             : "r"(box + 8u * k)
-                             : "memory");
+                const uint64_t w = box_read(box + 8u * k);
+                w_lo = (uint32_t)w;
+                w_hi = (uint32_t)(w >> 32);
                 ok = (w_hi ^ want) < (1u << kHeightBits);
             }
             if (__all_sync(~0u, ok && seen > k)) break;
@@ -428,10 +440,7 @@ __device__ __forceinline__ void sweep(Band &b, int j, int first_tag, int *status
             }
         }
         if (e != e_was) ex[k] = e;
-        if (in && edge)
-            asm volatile("st.relaxed.cluster.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(out + 8u * k), "r"(flow),
-                         "r"(tag | (uint32_t)h)
-                         : "memory");
+        if (in && edge) box_write(out + 8u * k, (uint64_t)(tag | (uint32_t)h) << 32 | (uint32_t)flow);
         __threadfence_block();
         __syncwarp();
         if (lane == 0) *mine = k == steps - 1 ? kSweepDone : k;
