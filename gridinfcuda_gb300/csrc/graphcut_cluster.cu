@@ -331,9 +331,10 @@ __device__ __forceinline__ void push_to(int fl, int r, int *res_i, int *ex_q, in
 //
 // A step's latency is the sweeps' rate, and with twenty warps on the SM an
 // instruction of it costs about eight cycles, so what every step does is kept
-// short: a lane meets at most one neighbouring band (bands have two rows or
-// more), with one word in and one out; progress counters end at a value that
-// needs no comparison with the last diagonal.
+// short: a lane meets at most one neighbouring band, with one word in and one
+// out (every band but the last has R >= 2 rows, and the last, which may have one,
+// has none below); progress counters end at a value that needs no comparison
+// with the last diagonal.
 constexpr int kSweepDone = 0x3fffffff;
 template <bool PUSH>
 __device__ __forceinline__ void sweep(Band &b, int j, int first_tag, int *status) {
