@@ -80,6 +80,7 @@ struct ConvTcParams {
     const __nv_bfloat16 *act;  // EPI_MASK: the activations whose ReLU the gradient passes
     const float *target;       // EPI_LOSS: [pixel][COUT]
     float scale;               // EPI_LOSS: 2 / elements
+    int wide_squares;          // EPI_LOSS: square in FP64, not four at a time in FP32 ahead of the FP64 sum
     float *bias_part;          // EPI_MASK, EPI_LOSS: [CTA][COUT] sums of the gradient written
     double *loss_part;         // EPI_LOSS: [CTA] sums of squared differences
     int n, h, w;             // images, rows, columns
@@ -226,13 +227,6 @@ struct TcLayout {
 template <int COUT, int ACC>
 __device__ __forceinline__ uint32_t acc_col(uint32_t t) {
     return (uint32_t)(ACC - 1 - (int)(t % ACC)) * COUT;
-}
-
-// a + b as the unevaluated pair (s, e) (Knuth's TwoSum).
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-    s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
 __device__ __forceinline__ uint2 pack_bf16x4(const float *v) {
@@ -466,8 +460,9 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
         uint32_t tile = 0;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         // EPI_MASK, EPI_LOSS: this lane's four channels (chunk lane % kChunksOut
-        // of a pixel, the same in every pass) and its squares as a float pair.
-        float bsum[4] = {0.f, 0.f, 0.f, 0.f}, loss_hi = 0.f, loss_lo = 0.f;
+        // of a pixel, the same in every pass) and its squares.
+        float bsum[4] = {0.f, 0.f, 0.f, 0.f};
+        double loss = 0.0;
         // The tensor-memory loads are warp-collective: every decision to stop
         // is taken by the whole warp.
         for (int it = blockIdx.x; it < p.items && !__any_sync(~0u, *abort_flag); it += gridDim.x) {
@@ -570,9 +565,12 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                                     const float4 a = xv[i], b = tv[i];
                                     const float d[4] = {(f.x + a.x) - b.x, (f.y + a.y) - b.y, (f.z + a.z) - b.z,
                                                         (f.w + a.w) - b.w};
-                                    float s, e;
-                                    two_sum(loss_hi, d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + d[3] * d[3], s, e);
-                                    two_sum(s, __fadd_rn(e, loss_lo), loss_hi, loss_lo);
+                                    if (p.wide_squares) {
+#pragma unroll
+                                        for (int k = 0; k < 4; ++k) loss += (double)d[k] * (double)d[k];
+                                    } else {
+                                        loss += (double)(d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + d[3] * d[3]);
+                                    }
 #pragma unroll
                                     for (int k = 0; k < 4; ++k) o[k] = p.scale * d[k];
                                 }
@@ -622,7 +620,7 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
                 for (int k = 0; k < 4; ++k) red[4 * lane + k] = bsum[k];
             double *lred = reinterpret_cast<double *>(stage + CW * 4);
             if (EPI == EPI_LOSS) {
-                double l = (double)loss_hi + (double)loss_lo;
+                double l = loss;
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(~0u, l, off);
                 if (lane == 0) *lred = l;
@@ -1111,8 +1109,9 @@ cudaError_t conv_first_tc(int cin, const float *x, __nv_bfloat16 *x_bf16, const 
 // with y = conv + bias + x, per-CTA sums of it per channel in bias_part
 // ([parts][cout]) and of the squared differences in loss_part ([parts]).
 cudaError_t conv_loss_tc(int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias, int nimg, int h,
-                         int wd, const float *x, const float *target, float scale, __nv_bfloat16 *grad,
-                         float *bias_part, double *loss_part, int *parts, int *status, cudaStream_t s) {
+                         int wd, const float *x, const float *target, bool wide_squares, float scale,
+                         __nv_bfloat16 *grad, float *bias_part, double *loss_part, int *parts, int *status,
+                         cudaStream_t s) {
     if (((uintptr_t)in | (uintptr_t)w | (uintptr_t)x | (uintptr_t)target | (uintptr_t)grad) & 15)
         return cudaErrorMisalignedAddress;
     ConvTcParams p{};
@@ -1121,6 +1120,7 @@ cudaError_t conv_loss_tc(int cout, const __nv_bfloat16 *in, const __nv_bfloat16 
     p.res = x;
     p.target = target;
     p.scale = scale;
+    p.wide_squares = wide_squares;
     p.out = grad;
     p.bias_part = bias_part;
     p.loss_part = loss_part;

@@ -35,8 +35,9 @@ cudaError_t conv_fwd_tc(int cin, int cout, bool relu, const __nv_bfloat16 *in, c
                         const float *bias, int nimg, int h, int wd, void *out, const float *res, int *status,
                         cudaStream_t s);
 cudaError_t conv_loss_tc(int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias, int nimg, int h,
-                         int wd, const float *x, const float *target, float scale, __nv_bfloat16 *grad,
-                         float *bias_part, double *loss_part, int *parts, int *status, cudaStream_t s);
+                         int wd, const float *x, const float *target, bool wide_squares, float scale,
+                         __nv_bfloat16 *grad, float *bias_part, double *loss_part, int *parts, int *status,
+                         cudaStream_t s);
 cudaError_t conv_dgrad_tc(int cin, const __nv_bfloat16 *in, const __nv_bfloat16 *w, int nimg, int h, int wd,
                           const __nv_bfloat16 *act, __nv_bfloat16 *grad, float *bias_part, int *parts, int *status,
                           cudaStream_t s);
@@ -334,14 +335,19 @@ ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo 
     const size_t pix = (size_t)g.n * g.h * g.w, ny = pix * n->L;
     ginf_status st = ensure_batch(n, pix);
     if (st != GINF_OK) return st;
-    if ((uintptr_t)target & 15) {  // the kernel reads it 16 bytes at a time
+    // The kernel reads the target 16 bytes at a time.  The loss is an FP64 sum:
+    // of FP32 squares, four at a time, for an aligned target, of single FP64
+    // squares otherwise (16x256x192x64: 531 and 705 us a call; the FP64 unit's
+    // rate shows in the second only).
+    const bool aligned = ((uintptr_t)target & 15) == 0;
+    if (!aligned) {
         GINF_WCK(cudaMemcpyAsync(n->y, target, ny * sizeof(float), cudaMemcpyDeviceToDevice, s));
         target = n->y;
     }
     if ((st = forward_hidden(n, x, g, true, n->status, s)) != GINF_OK) return st;
     int bias_parts = 0;
     GINF_WCK(conv_loss_tc(n->L, n->a[3], n->wbf + n->woff[3], n->params + n->boff[3], g.n, g.h, g.w, x, target,
-                          2.f / (float)ny, n->gb[0], n->bias_part, n->loss_part, &bias_parts, n->status, s));
+                          !aligned, 2.f / (float)ny, n->gb[0], n->bias_part, n->loss_part, &bias_parts, n->status, s));
     int cur = 0;
     for (int l = 3; l >= 0; --l) {
         const int ci = n->cin[l], co = n->cout[l], nw = co * 9 * ci;
