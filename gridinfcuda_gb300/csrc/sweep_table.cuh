@@ -98,8 +98,10 @@ __device__ __forceinline__ void sub4(int *h, const int *a) {
 __device__ __forceinline__ float table_min(float a, float b) { return fminf(a, b); }
 __device__ __forceinline__ int table_min(int a, int b) { return min(a, b); }
 
-// The belief of one node by its four lanes, as belief_part, noting values the
-// fast form does not cover.
+// The belief of one node by its four lanes, as belief_part (in chunks of four
+// labels whatever the store: with FP16 messages' chunks of eight L = 8 took 226 us
+// for six half-sweeps at 640x480, so 209), noting values the fast form does not
+// cover.
 template <typename T, typename M, bool STD>
 __device__ __forceinline__ void table_belief(const SweepParams &p, unsigned char *slot, int L, int dir, T &best,
                                              int &bl, int &odd) {
@@ -131,6 +133,23 @@ __device__ __forceinline__ void table_belief(const SweepParams &p, unsigned char
             }
         }
     }
+}
+
+// The label of a node by its four lanes from its finished belief, in belief_part's
+// chunks.  With a NaN among them the chunks decide the label.
+template <typename T, typename M>
+__device__ __forceinline__ void table_label(const unsigned char *slot, int L, int dir, T &best, int &bl) {
+    constexpr int B = MIO<M, T>::B;
+    best = pos_inf<T>();
+    bl = 0x7fffffff;
+    for (int c = dir * B; c < L; c += 4 * B)
+        for (int i = c; i < c + B && i < L; ++i) {
+            const T v = reinterpret_cast<const T *>(slot)[i];
+            if (bl == 0x7fffffff || v < best) {
+                best = v;
+                bl = i;
+            }
+        }
 }
 
 // The tile's min-convolutions, fast form.  Vs holds V with the steps of j in
@@ -346,6 +365,10 @@ __global__ void __launch_bounds__(64 * SPL, table_blocks(STD, SPL, TI * TN)) swe
         const bool slow = __syncthreads_or(odd | odd_table) != 0;
         if (kF32 && slow) {  // int32 minima have one value
             if constexpr (kF32) {
+                if constexpr (sizeof(M) == 2) {
+                    if (act) table_label<T, M>(slot, L, dir, best, label);
+                    argmin_combine(best, label);
+                }
                 if (act) {
                     if constexpr (STD) message_std_minconv<T, M, kMaxLabels>(p, slot, L, dir);
                     else messages_ref_minconv<T, M, kMaxLabels>(p, slot, L, dir);
