@@ -875,22 +875,28 @@ __device__ __forceinline__ bool tile_finish(const SweepParams &p, const TableCon
 //     +inf outside [0, L), as the single-lane form's missing taps);
 //   - the mean's sum stays sequential in label order: half 0 sums its HL
 //     outputs from zero, half 1 continues from that partial sum;
-//   - the argmin combines the halves' first minima by (value, label).
+//   - the label is the single-lane form's too, NaN beliefs or not: lane dir
+//     scans the chunks dir, dir + 4, ... of all labels, half 1 going on from
+//     half 0, before the lanes combine.  (At L = 128 the halves' labels are
+//     combined instead, and sweep_labels.cu does the same.)
 // Shared words exchanged between the two warps of a group.
 template <int NW>
 struct SplitXch {
     float minh[NW][32];      // lane's minimum of h over its own half
     float sum[NW / 2][32];   // half 0's sequential partial sum of its outputs
     float mean[NW / 2][32];  // the finished mean, from half 1
-    float best[NW][8];       // node's belief minimum over the warp's half
-    int label[NW][8];        // and its first label
+    // Belief minima and their first labels: of half 1's lanes, [NW / 2][32]; at
+    // L = 128 of the nodes by warp, [NW][8].
+    float best[NW / 2 * 32];
+    int label[NW / 2 * 32];
 };
 
 // Belief over labels [base, base + HL) below L of one node by its four lanes
-// of one warp (chunks base + 4 (4 j + dir)); see belief_part.
+// of one warp (chunks base + 4 (4 j + dir)); see belief_part.  With go_on only
+// values below `best` count, not the lane's first.
 template <int HL, bool FULL>
 __device__ __forceinline__ void belief_half(const SweepParams &p, unsigned char *slot, int L, int dir, int base,
-                                            float &best, int &bl) {
+                                            bool go_on, float &best, int &bl) {
     const unsigned char *mb = slot + p.d_bytes;
 #pragma unroll
     for (int j = 0; j < (HL / 4 + 3) / 4; ++j) {
@@ -908,7 +914,7 @@ __device__ __forceinline__ void belief_half(const SweepParams &p, unsigned char 
         store_t<float, 4>(slot + c * sizeof(float), v);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-            if ((FULL || c + kk < L) && (bl == 0x7fffffff || v[kk] < best)) {
+            if ((FULL || c + kk < L) && ((bl == 0x7fffffff && !go_on) || v[kk] < best)) {
                 best = v[kk];
                 bl = c + kk;
             }
@@ -946,17 +952,34 @@ __device__ __forceinline__ bool tile_finish_split(const SweepParams &p, const Ta
     __syncwarp();
     float best = pos_inf<float>();
     int label = 0x7fffffff;
-    if (act) belief_half<HL, LMIN == LMAX>(p, slot, L, dir, base, best, label);
-    argmin_combine(best, label);
-    if (dir == 0) {
-        xs.best[w][k] = best;
-        xs.label[w][k] = label;
-    }
-    __syncthreads();
-    {
-        const float ob = xs.best[w ^ 1][k];
-        const int ol = xs.label[w ^ 1][k];
+    if constexpr (LMIN == LMAX) {
+        if (act) belief_half<HL, true>(p, slot, L, dir, base, false, best, label);
+        argmin_combine(best, label);
+        if (dir == 0) {
+            xs.best[w * 8 + k] = best;
+            xs.label[w * 8 + k] = label;
+        }
+        __syncthreads();
+        const float ob = xs.best[(w ^ 1) * 8 + k];
+        const int ol = xs.label[(w ^ 1) * 8 + k];
         if (ol != 0x7fffffff && (label == 0x7fffffff || ob < best || (!(best < ob) && ol < label))) label = ol;
+    } else {
+        // The half's chunk that is number `turn` modulo four of all labels'.
+        const int turn = hf == 0 ? dir : (dir + HL / 4) & 3;
+        if (act) belief_half<HL, false>(p, slot, L, dir, base, hf == 1, best, label);
+        if (hf == 1) {
+            xs.best[g * 32 + turn * 8 + k] = best;
+            xs.label[g * 32 + turn * 8 + k] = label;
+        }
+        __syncthreads();
+        if (hf == 0) {
+            const float ob = xs.best[g * 32 + lane];
+            if (ob < best) {
+                best = ob;
+                label = xs.label[g * 32 + lane];
+            }
+            argmin_combine(best, label);
+        }
     }
     float h[NH];
     float mloc = pos_inf<float>();

@@ -10,8 +10,8 @@
 // truncated quadratic 347 -> 270 us.
 //
 // The belief's sum and the argmin's lane partition and combine are the
-// half-sweep's (belief_part, and belief_half where the split kernel runs), so
-// the label is the same whatever the costs hold.
+// half-sweep's (belief_part, and the split kernel's halves at 128 labels), so
+// the label is the same whatever the costs hold, NaN included.
 #include <algorithm>
 
 #include "sweep_labels.cuh"
@@ -69,11 +69,10 @@ cudaError_t launch_labels_t(const SweepParams &p, int half, cudaStream_t s) {
 
 cudaError_t launch_sweep_labels(const RecordFormat &f, const SweepParams &p, cudaStream_t s) {
     if (p.W < 3 || p.H < 3) return cudaSuccess;
-    // The half-sweeps that run the split kernel (launch_variant) part their
-    // labels in two halves of the 16-label bucket.
-    const bool split = f.ctype == CT_F32 && f.store == ST_NATIVE && f.L > 64 && p.mode == MODE_STD_QUAD &&
+    // The split kernel (launch_variant) with 128 labels parts them in halves.
+    const bool split = f.ctype == CT_F32 && f.store == ST_NATIVE && f.L == 128 && p.mode == MODE_STD_QUAD &&
                        p.quad_radius <= kQuadWindow;
-    if (split) return launch_labels_t<float, float, true>(p, (f.L + 15) / 16 * 8, s);
+    if (split) return launch_labels_t<float, float, true>(p, 64, s);
     if (f.store == ST_F16) return launch_labels_t<float, __half>(p, 0, s);
     switch (f.ctype) {
         case CT_F32: return launch_labels_t<float, float>(p, 0, s);
