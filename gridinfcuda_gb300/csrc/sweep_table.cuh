@@ -40,8 +40,20 @@
 // only if its table entry is, and NaN only if an operand is NaN or the two
 // are opposite infinities.  So a table with a -0, a -infinity or a NaN, and a
 // tile in which a belief is not above -kTableBig or, for the standard rule's
-// difference, a message not within +-kTableBig, run the sequential form
-// (messages_ref_minconv, message_std_minconv) instead.
+// difference, a message not within +-kTableBig, take the reference's comparison
+// in its order instead.  A hand-made table may well hold a -0.  320x240, six
+// half-sweeps, us: a lane per output or message with V through the cache and the
+// standard rule's vectors in local memory -> eight (four) outputs side by side
+// with V from shared memory (ordinary tables):
+//   L           16         32                64                   128
+//   reference   165 (112)  315 (125)         900 (207)            12520 -> 1655 (500)
+//   standard    254 (131)  1366 -> 274 (171) 10830 -> 1170 (385)  111700 -> 9820 (1090)
+// Where no second figure stands the first form is still the one (as a kernel
+// without V in shared memory it took 175 and 355 us for the reference rule at 16
+// and 32 labels, 1450 at 64, 6250 at 128, and 315, 1190, 5900 and 67300 for the
+// standard one), since the blocked form beside table_convolve costs ordinary
+// tables up to 1 %.  table_convolve itself with these comparisons took 1970 us at
+// 128 labels, but ordinary tables then 1245 us for 1155 (640x480, L = 64).
 #pragma once
 
 #include "sweep_impl.cuh"
@@ -263,6 +275,75 @@ __device__ __forceinline__ void table_convolve(const SweepParams &p, const T *Vs
     }
 }
 
+// Outputs i0 .. i0 + N - 1 of one vector by the reference's comparison in order
+// of j, h(j) the vector; an accumulator starts at infinity, which the first
+// candidate replaces whatever it is.
+template <int N, typename T, typename Fn>
+__device__ __forceinline__ void table_ordered(const T *Vs, int Lp, int L, int i0, Fn h, T *acc) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) acc[i] = pos_inf<T>();
+#pragma unroll 1
+    for (int j = 0; j < L; j += 2) {
+        const bool two = j + 1 < L;
+        const T h0 = h(j), h1 = two ? h(j + 1) : T(0);
+#pragma unroll
+        for (int q = 0; q < N / 2; ++q) {
+            T v[4];  // V(i, j), V(i, j + 1), V(i + 1, j), V(i + 1, j + 1)
+            load_t<T, 4>(reinterpret_cast<const unsigned char *>(Vs + j * Lp + 2 * i0 + 4 * q), v);
+            acc[2 * q] = rmin(acc[2 * q], v[0] + h0);
+            acc[2 * q + 1] = rmin(acc[2 * q + 1], v[2] + h0);
+            if (two) {
+                acc[2 * q] = rmin(acc[2 * q], v[1] + h1);
+                acc[2 * q + 1] = rmin(acc[2 * q + 1], v[3] + h1);
+            }
+        }
+    }
+}
+
+// The lane's part of its node's messages in that form: the standard rule's
+// message towards dir (4-byte messages in place, not yet normalised), the
+// reference rule's outputs 4 dir, 4 dir + 16, ... into the node's first slot.  V
+// is read from shared memory, each entry for a warp at once, and eight (four)
+// outputs run side by side.
+template <typename T, typename M, bool STD>
+__device__ __forceinline__ void table_messages_ordered(const SweepParams &p, const T *Vs, unsigned char *slot, int L,
+                                                       int dir) {
+    if constexpr (STD) {
+        unsigned char *md = slot + p.d_bytes + dir * p.m_bytes;
+        T h[kMaxLabels], o[sizeof(M) == sizeof(T) ? 1 : kMaxLabels];
+        load_h<T, M, kMaxLabels>(slot, md, L, h);
+#pragma unroll 1
+        for (int i = 0; i < L; i += 8) {
+            T r[8];
+            table_ordered<8>(Vs, p.Lp, L, i, [&](int j) { return h[j]; }, r);
+            if constexpr (sizeof(M) == sizeof(T)) {  // normalised later
+                store_t<T, 4>(md + i * sizeof(T), r);
+                store_t<T, 4>(md + (i + 4) * sizeof(T), r + 4);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) o[i + k] = r[k];
+            }
+        }
+        if constexpr (sizeof(M) != sizeof(T)) {
+            normalise(o, L, p.norm_min);
+            store_msg<T, M>(md, o, L);
+        }
+    } else {
+        const T *fr = reinterpret_cast<const T *>(slot);
+#pragma unroll 1
+        for (int i = dir * 4; i < L; i += 16) {
+            T r[4];
+            table_ordered<4>(Vs, p.Lp, L, i, [&](int j) { return fr[j]; }, r);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i + k >= L) r[k] = T(0);
+            unsigned char *out = slot + p.d_bytes + i * sizeof(M);
+            store2<M, T>(out, r[0], r[1]);
+            store2<M, T>(out + 2 * sizeof(M), r[2], r[3]);
+        }
+    }
+}
+
 // Subtracts the mean (summed in label order, as the reference does) or the
 // minimum from one message of the arithmetic type, in place.
 template <typename T>
@@ -312,6 +393,10 @@ template <typename T, typename M, bool STD, int SPL, int TI, int TN>
 __global__ void __launch_bounds__(64 * SPL, table_blocks(STD, SPL, TI * TN)) sweep_kernel_table(const SweepParams p) {
     constexpr int NW = 2 * SPL;
     constexpr bool kF32 = std::is_same<T, float>::value;
+    constexpr bool kNormalise = STD && sizeof(M) == sizeof(T);
+    // Label counts whose ordered form is the blocked one: where a lane per output
+    // was slower beside the table in shared memory than without it (above).
+    constexpr bool kBlocked = kF32 && (STD ? TN > 2 : SPL == 2);
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
     __shared__ T mins[sizeof(M) == 2 && STD ? 4 * kTableNodes : 1][kTableMaxGroups];
@@ -370,17 +455,20 @@ __global__ void __launch_bounds__(64 * SPL, table_blocks(STD, SPL, TI * TN)) swe
                     argmin_combine(best, label);
                 }
                 if (act) {
-                    if constexpr (STD) message_std_minconv<T, M, kMaxLabels>(p, slot, L, dir);
+                    if constexpr (kBlocked) table_messages_ordered<T, M, STD>(p, Vs, slot, L, dir);
+                    else if constexpr (STD) message_std_minconv<T, M, kMaxLabels>(p, slot, L, dir);
                     else messages_ref_minconv<T, M, kMaxLabels>(p, slot, L, dir);
                 }
             }
         } else {
             table_convolve<T, M, STD, TI, TN>(p, Vs, smem, L, mins);
-            if constexpr (STD && sizeof(M) == sizeof(T)) {
+            if constexpr (kNormalise) {
                 __syncthreads();
-                if (act) table_normalise<T>(md, L, p.norm_min);
+                if (!kBlocked && act) table_normalise<T>(md, L, p.norm_min);
             }
         }
+        if constexpr (kNormalise && kBlocked)
+            if (act) table_normalise<T>(md, L, p.norm_min);
         fence_proxy_async_shared();
         __syncthreads();
         if (act) {
