@@ -209,12 +209,17 @@ std::string size_class_key(const ginf_grid &g) {
     return "L" + std::to_string(g.num_labels) + ":s" + std::to_string(s);
 }
 
-// Batch signature: the multiset of (label count, log2 of the node count)
-// buckets, plus the iteration count.
-std::string signature(const std::vector<ginf_grid> &grids, int iters) {
+// Raised when the batch kernels or the way they are launched change so that a
+// choice measured before says nothing about them.
+constexpr int kTuneRevision = 2;
+
+// Batch signature: what was measured (the kernels' revision, the device's SMs),
+// the multiset of (label count, log2 of the node count) buckets, and the
+// iteration count.
+std::string signature(const std::vector<ginf_grid> &grids, int iters, int num_sms) {
     std::map<std::string, int> counts;
     for (const auto &g : grids) counts[size_class_key(g)]++;
-    std::string sig;
+    std::string sig = "r" + std::to_string(kTuneRevision) + ",sm" + std::to_string(num_sms) + ",";
     for (const auto &kv : counts) sig += kv.first + "x" + std::to_string(kv.second) + ",";
     return sig + "it" + std::to_string(iters);
 }
@@ -733,7 +738,7 @@ ginf_status ginf_batch_create(ginf_batch **out, const ginf_grid *grids, int32_t 
     }
     if (st == GINF_OK) {
         TuneChoice c;
-        const std::string sig = signature(b->grids, iters);
+        const std::string sig = signature(b->grids, iters, b->num_sms);
         bool have = false;
         if (opt->tile_nodes != 0 || opt->sweeps_per_launch != 0) {
             // An explicit choice (either knob) is used as given.

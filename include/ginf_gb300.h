@@ -240,7 +240,9 @@ ginf_status ginf_stereo_costs_u8(int32_t width, int32_t height, int32_t num_labe
  * the autotuner, which times the candidates on this batch and caches the
  * winner per mix of (label count, log2 node count) buckets in the JSON file
  * named by $GINF_AUTOTUNE_CACHE (default
- * $XDG_CACHE_HOME or ~/.cache/gridinfcuda_gb300_autotune.json).  A plan
+ * $XDG_CACHE_HOME or ~/.cache/gridinfcuda_gb300_autotune.json).  Choices that
+ * other versions of the batch kernels or devices with another number of SMs
+ * left there are kept but not used.  A plan
  * runs only on the device current at its creation; runs from another device
  * return GINF_ERR_INVALID_ARGUMENT. */
 typedef struct ginf_batch ginf_batch;
