@@ -378,6 +378,12 @@ void make_groups(ginf_batch *b) {
 
 // Nodes per work-list tile: the warp half-sweep's eight, else the plan's.
 int group_tile_nodes(const BatchGroup &grp, int tile_nodes) { return grp.lm <= kWarpTileLabels ? 8 : tile_nodes; }
+// Whether the plan's tile size reaches any group.
+bool tile_size_matters(const ginf_batch *b) {
+    for (const BatchGroup &grp : b->groups)
+        if (grp.lm > kWarpTileLabels) return true;
+    return false;
+}
 
 // Items for a given tile size (8 * NW nodes), in group order, with tile
 // bases counted from each group's start; copied to the device.
@@ -602,6 +608,7 @@ ginf_status capture(ginf_batch *b, const TuneChoice &c) {
         return bfail(GINF_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
     }
     b->choice = c;
+    if (!tile_size_matters(b)) b->choice.tile_nodes = 8;
     b->launches_per_run = launches;
     return GINF_OK;
 }
@@ -615,11 +622,14 @@ ginf_status run_graph(ginf_batch *b, cudaStream_t s) {
     return GINF_OK;
 }
 
-// Times each candidate (tile size x half-sweeps per launch) on the batch.
+// Times each candidate (tile size, where it matters, x half-sweeps per launch)
+// on the batch.
 ginf_status autotune(ginf_batch *b) {
     std::vector<TuneChoice> cands;
     const int spls[3] = {1, 5, 0};
-    for (int tn : {8, 16, 32})
+    std::vector<int> tiles = {8};
+    if (tile_size_matters(b)) tiles = {8, 16, 32};
+    for (int tn : tiles)
         for (int spl : spls) {
             if (spl > 0 && spl >= b->iters) continue;
             TuneChoice c;

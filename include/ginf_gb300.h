@@ -80,7 +80,11 @@ typedef struct ginf_options {
     int32_t normalize;       /* GINF_NORM_*,   default MEAN (F16 uses MIN)  */
     int32_t compute_type;    /* GINF_F32 / GINF_I32 / GINF_F64; -1 = cost_type */
     int32_t tile_nodes;      /* nodes per sweep tile (8, 16 or 32); 0 = default
-                                (16), or the autotuned choice for batches        */
+                                (16), or the autotuned choice for batches.  It
+                                chooses a kernel for Potts / truncated-linear FP32
+                                grids: in a batch above 32 labels, otherwise at 64
+                                and 128 labels (with the FP16 store at 16 and 32
+                                too); the other half-sweeps have one tile size  */
     int32_t sweeps_per_launch; /* batches: half-sweeps per persistent launch;
                                   0 = autotuned.  Single grids: 0 or 1 = one
                                   half-sweep per launch (default); k >= 2 =
@@ -259,8 +263,9 @@ ginf_status ginf_batch_enqueue(ginf_batch *batch, void *stream);
 /* Waits for the batch's stream-ordered replays and reports a device-side
  * error any of them recorded. */
 ginf_status ginf_batch_sync(ginf_batch *batch);
-/* The tile size and half-sweeps per launch in use, and whether this plan
- * measured them (1) or took them from the options or the cache (0). */
+/* The tile size of the grids above 32 labels (8, the one in use, if there are
+ * none) and half-sweeps per launch in use, and whether this plan measured them
+ * (1) or took them from the options or the cache (0). */
 ginf_status ginf_batch_config(const ginf_batch *batch, int32_t *tile_nodes, int32_t *sweeps_per_launch,
                               int32_t *tuned_now);
 ginf_status ginf_batch_destroy(ginf_batch *batch);

@@ -1,5 +1,5 @@
-"""Batch plans: what the autotuner's cache holds, and label buckets with several
-half-sweeps per launch."""
+"""Batch plans: what the autotuner's cache holds, the tile size reported, and
+label buckets with several half-sweeps per launch."""
 import json
 
 import numpy as np
@@ -54,3 +54,17 @@ def test_choices_of_other_kernels_are_measured_anew(ginf, tmp_path, monkeypatch)
     with ginf.Batch(problems, labels, 6) as b:
         second = b.config()
     assert second["tuned_now"] is False and second["tile_nodes"] == first["tile_nodes"]
+
+
+def test_tile_size_reported_is_the_one_in_use(ginf, tmp_path, monkeypatch):
+    """Up to 32 labels a tile is a warp's eight nodes, whatever the options
+    say; a plan with other grids reports theirs."""
+    monkeypatch.setenv("GINF_AUTOTUNE_CACHE", str(tmp_path / "tune.json"))
+    problems, labels = _problems((5, 16, 32))
+    for opt in ({"tile_nodes": 32, "sweeps_per_launch": 1}, {"autotune": -1}, {"autotune": 1}, {}):
+        with ginf.Batch(problems, labels, 6, **opt) as b:
+            assert b.config()["tile_nodes"] == 8, opt
+    problems, labels = _problems((16, 40))
+    for tile in (8, 16, 32):
+        with ginf.Batch(problems, labels, 6, tile_nodes=tile, sweeps_per_launch=1) as b:
+            assert b.config()["tile_nodes"] == tile
