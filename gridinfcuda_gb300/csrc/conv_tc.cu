@@ -44,17 +44,18 @@
 //
 // The first layer reads x in FP32: eight warps take the copying warp's place,
 // round the rows on their way into the buffers and, in training, store the
-// rounding for the weight gradient.  A conversion kernel before a layer that
-// read its output moved x's BF16 through memory twice: 26 + 33 us of a
-// 960x540x64 forward pass, now 42 (180 -> 169 us the call).
+// rounding for the weight gradient: 43 us of a 960x540x64 forward pass, where a
+// conversion kernel before a layer that reads its output, which moves x's BF16
+// through memory twice, took 26 + 33.
 //
 // Programmatic launches: each kernel sets up (barriers, tensor memory, its
 // weights) beside the tail of the one before it and waits before it touches
 // anything else.  A kernel lets its successor start only after its own wait,
 // so what it reads ahead of that wait -- weights and biases -- must have been
-// complete before its predecessor began; the callers see to that.
-// 960x540x64 forward 203 -> 179 us, 16x256x192x64 gradients 816 -> 746 us
-// (with three weight-flipping kernels, a loss kernel and a copy less).
+// complete before its predecessor began; the callers see to that.  Without
+// them a 960x540x64 forward pass takes about 20 us more.
+//
+// 960x540x64 forward: 164 us a call, 141 of them in the four kernels.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -185,8 +186,8 @@ __device__ __forceinline__ Item item_of(const ConvTcParams &p, int it) {
 
 // Warps of a convolution: epilogue, row copies, MMA.  With FP32 input eight
 // warps round the rows on their way to shared memory, and the epilogue has
-// four: eight there 176 us against 169 for a 960x540x64 forward pass (the
-// others: four 543, eight 525, sixteen 542 us at 16x256x192x64 gradients).
+// four: with eight there too a 960x540x64 forward pass took 4 % longer.  The
+// others have eight: with four or sixteen 16x256x192x64 gradients took 3 % longer.
 constexpr int epi_warps(bool in_f32) { return in_f32 ? 4 : 8; }
 constexpr int copy_warps(bool in_f32) { return in_f32 ? 8 : 1; }
 constexpr int conv_threads(bool in_f32) { return (epi_warps(in_f32) + copy_warps(in_f32) + 1) * 32; }
@@ -385,8 +386,8 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
     } else if (warp == Lay::kEpi + Lay::kCopy) {
         // The whole warp keeps count and one lane issues: with everything in
         // one lane's branch each instruction's descriptors went through
-        // vector registers (960x540x64 forward 169 -> 161 us, gradients at
-        // 16x256x192x64 526 -> 514).
+        // vector registers (960x540x64 forward 5 %, 16x256x192x64 gradients 2 %
+        // longer).
         const bool leader = elect_one();
         constexpr int ACC = Lay::kAcc;
         const uint32_t rbase = smem_addr(sm + Lay::kRows);
@@ -718,18 +719,17 @@ cudaError_t cta_slots(int smem, int *slots) {
     return cudaSuccess;
 }
 
-// Work items for `slots` CTAs: each band's rows split into chunks, at least
-// four rows each (two halo rows per chunk), as many as make the longest CTA
-// shortest -- its items times a chunk's rows with their halo.  False when
-// there is nothing to do or too much to count.  Splitting the rows evenly
-// over the slots and rounding up gave 320 items on 304 slots for 16 images of
-// 256x192 (21 rows a chunk), so that the kernels took two chunks' time; now
-// 288 items of 22 rows: gradients there 746 -> 536 us.
+// Work items for `slots` CTAs: each band's rows split into chunks (two halo rows
+// each), at most one per four rows begun, as many as make the longest CTA
+// shortest -- its items times a chunk's rows with their halo.  False when there
+// is nothing to do or too much to count.  16 images of 256x192 on 304 slots are
+// 288 items of 22 rows; an even split of the rows over the slots, rounded up,
+// gives 320 of 21, two chunks' time, and the gradients took 1.4 times as long.
 //
 // Bands are as even as whole groups of 16 pixels (the weight gradient's K
 // step) allow: 192 columns are two bands of 96, not 128 and 64, whose CTAs
-// kept unlike SMs busy unlike long (16 images of 192x256 with 64 labels:
-// forward 248 -> 223 us, gradients 602 -> 550; four of 144x300 249 -> 227).
+// keep unlike SMs busy unlike long (16 images of 192x256 with 64 labels:
+// forward 223 us, 248 with those; gradients 550, 602; four of 144x300 227, 249).
 struct ItemPlan {
     int band, bands, rows_per_chunk, chunks, items, grid;
 };
@@ -816,7 +816,8 @@ cudaError_t launch_conv_tc(const __nv_bfloat16 *in, ConvTcParams p, cudaStream_t
 //
 // Bound: the shared-memory reads of the operands (4 KB of A and COUT x 96
 // bytes of B an MMA).  16x256x192, us a layer (32 -> 64, 32 -> 32, 64 -> 32
-// channels): one MMA per row offset 59, 57, 90; now 46, 35, 56.
+// channels): 33, 23, 38, with evenly filled CTAs; before those 46, 35, 56, and
+// with one MMA per row offset 59, 57, 90.
 
 struct WgradParams {
     float *partials;  // [CTA][COUT][9][CIN]

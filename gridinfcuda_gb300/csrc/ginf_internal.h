@@ -185,6 +185,10 @@ cudaError_t launch_sweep(const RecordFormat &f, const SweepConfig &cfg, SweepPar
 cudaError_t launch_sweep_labels(const RecordFormat &f, const SweepParams &p, cudaStream_t s);
 // Launches of 64-byte-message kernels (L = 32, FP16) with at least this many
 // 16-node tiles store their messages with ordinary stores (see tile_finish).
+// Twenty half-sweeps, bulk copies -> ordinary stores: 1024x576 (18400 tiles)
+// 1316 -> 1062 us, 1920x1080 4300 -> 3390, 3840x2160 16780 -> 13110.  Below the
+// line ordinary stores would win too from 384x288 on (3432 tiles, 315 -> 288 us;
+// 800x600, 14352, 1115 -> 907), not at 160x120 (160 -> 163).
 constexpr long kDirectStoreTiles = 16384;
 
 // Largest L the sweep kernels are compiled for.

@@ -34,15 +34,18 @@
 // wait inside a round is bounded; one that runs out is recorded and the round
 // ends with all CTAs.
 //
-// Bound: the latency of a wavefront step with twenty warps on the SM (about
-// 800 cycles, eight per instruction; 400 steps a band, then the bands' lags:
-// 0.33 ms a round of twenty sweeps at 384x288, 16 bands) and the searches'
-// barriers.  384x288x16, one pass from the BP labels: 787 ms with one CTA in
-// global memory; here, for three seeds, 187, 87 and 138 ms with searches that
-// walked the unreached nodes, 91, 63 and 90 ms with bit sets, 80, 55 and 79 ms
-// with the short step.  Also measured: four diagonals between two waits 137 ms
-// (the lags grow by more than the waits cost), flows formed branch-free and
-// applied by predicated additions 99 ms, no fences in a step 3 % less.
+// Bound: the latency of a wavefront step with twenty warps on the SM, five to a
+// scheduler (ten cycles an instruction, ncu; 0.33 ms a round of twenty sweeps at
+// 384x288: 400 steps a band and the lags of 16 bands), and the searches'
+// barriers.  384x288x16, one pass from the BP labels, three inputs: 80, 55 and
+// 79 ms (one CTA in global memory 787 ms for the first).  Also measured, for the
+// first: searches that walk the unreached nodes instead of bit sets 187 ms before
+// a step was shortened, 91 with bit sets; from there four diagonals between two
+// waits 137 (the lags grow by more than the waits cost), flows formed branch-free
+// and applied by predicated additions 99, no fences in a step 3 % less.
+//
+// Beyond it (state that sixteen bands do not hold, from about 110,000 nodes on;
+// heights or labels that their bits do not) one CTA runs the solve (graphcut.cu).
 #include <cstdint>
 
 #include "ginf_internal.h"

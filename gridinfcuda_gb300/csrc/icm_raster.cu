@@ -23,9 +23,14 @@
 // Bound: the latency of a step -- a shuffle, a table row from shared memory,
 // the additions, the argmin over eight lanes -- times the columns and
 // iterations, plus the strips' lags (2.8 us each).  640x480x32 int32: 0.24 us a
-// step; five iterations 1.18 ms, against 23.0 ms with one launch per
-// anti-diagonal (5590 of them) and 1.98 ms with stores per step and the general
-// argmin (205 instructions a step on one warp, ncu).
+// step (one warp on a scheduler, 5.8 cycles an instruction, ncu); five iterations
+// 1.19 ms, against 23.0 ms with one launch per anti-diagonal (5590 of them) and
+// 1.98 ms with stores per step and the general argmin.
+//
+// A warp a block and the whole table in its shared memory: grids whose strips do
+// not all fit the device at once (128 labels in 4 bytes: 64 KB, three blocks an
+// SM, 1826 rows on 152 SMs; 96 labels twice that) and FP64 grids of more than 64
+// labels keep one launch per anti-diagonal.
 //
 // The sum's order is the reference's and ties go to the lowest label.  Chunks
 // whose costs hold a NaN or a value near -infinity, and tables that do, take

@@ -789,9 +789,8 @@ __device__ __forceinline__ void tile_load(const SweepParams &p, int t, unsigned 
 // allocation), the standard truncated-quadratic update (window radius 8, or
 // 4 for KIND_QUAD4), or every rule.
 // DIRECT (64-byte messages only): the messages leave through ordinary
-// 16-byte stores instead of one bulk copy each, which pays on large launches
-// (the copy engine's per-copy cost dominates 64-byte copies) and not on small,
-// L2-resident ones.
+// 16-byte stores instead of one bulk copy each, whose cost per copy dominates
+// 64-byte copies (kDirectStoreTiles has the figures).
 template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, bool DIRECT = false>
 __device__ __forceinline__ bool tile_finish(const SweepParams &p, const TableConsts<T> &tc, int t,
                                             unsigned char *smem, uint64_t *bar, uint32_t &parity) {

@@ -23,7 +23,7 @@
 // Bound: HBM (36 B per updated node and label) for the reference rule up to
 // about 32 labels; above that the latency of a tile's phases with the few
 // blocks that the table leaves room for, and for the standard rule the issue
-// rate (at L = 64, 13 T additions and minima a second).  Measured, 640x480
+// rate (at L = 64, 12.5 T additions and as many minima a second).  Measured, 640x480
 // FP32, us per half-sweep, lane-per-message form -> this one:
 //   L           16         32         64          128
 //   reference   52 -> 24   146 -> 37  727 -> 85   - -> 256

@@ -65,7 +65,7 @@ struct Geo {
 // eighth partial, 32 neighbouring outputs reading one 128-byte line, and are
 // added in a fixed order.  One thread per output, in order, was a chain of
 // 304 (bias: 768) loads on a few blocks: 16 and 28 us a layer at 16x256x192x64,
-// now about 6 us a layer.
+// now about 7 us a layer.
 //
 // With loss_part, one more block (its warp 0) sums the loss: lane l takes
 // loss_part[l], loss_part[l + 32], ..., then the lanes combine in a fixed
@@ -326,11 +326,9 @@ ginf_status forward(ginf_warmnet *n, const float *x, Geo g, int *status, cudaStr
 // layer's output stays in its kernel: the loss, the BF16 output gradient and
 // its bias sums leave from the epilogue, and each data gradient passes its
 // ReLU and leaves bias sums the same way, so no FP32 gradient is written.
-// 16x256x192x64: 1334 us a call with separate loss, conversion, ReLU and bias
-// kernels, 941 us so; with the later changes in conv_tc.cu 816, with the
-// programmatic launches, the weights flipped as the data gradient loads them
-// and one copy for loss and status 746, with evenly filled CTAs 536, with the
-// conversion of x inside the first layer 526, with the MMA warps converged 514.
+// 16x256x192x64: 519 us a call, 500 of them in its fifteen kernels (34 kernels
+// with separate ones for loss, conversions, ReLU, flipped weights and bias sums
+// took 1335).
 ginf_status gradients(ginf_warmnet *n, const float *x, const float *target, Geo g, cudaStream_t s) {
     const size_t pix = (size_t)g.n * g.h * g.w, ny = pix * n->L;
     ginf_status st = ensure_batch(n, pix);

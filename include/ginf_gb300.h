@@ -172,7 +172,10 @@ ginf_status ginf_decode_hbp(ginf_workspace *ws, const ginf_grid *grid, int32_t n
 /* ICM.  asynchronous == 0: Jacobi sweeps, replacing ginf::decodeIcmSync
  * (src/icm.cc:4-38) and ginf::gpuDecodeIcm (src/gpu/icm.cu:53-83).
  * asynchronous == 1: raster-order Gauss-Seidel, replacing ginf::decodeIcmAsync
- * (src/icm.cc:40-67), run as an exact wavefront.
+ * (src/icm.cc:40-67), run as an exact wavefront: one launch for all iterations,
+ * or, about twenty times slower, one per anti-diagonal and iteration where not
+ * all rows can be resident (1826 rows of 128 labels, more of fewer) and for
+ * FP64 grids of more than 64 labels.
  * result (W*H) receives a copy of initial, then interior nodes are updated. */
 ginf_status ginf_decode_icm(ginf_workspace *ws, const ginf_grid *grid, const int32_t *initial,
                             int32_t iters, int32_t asynchronous, int32_t *result,
@@ -188,8 +191,8 @@ ginf_status ginf_decode_icm(ginf_workspace *ws, const ginf_grid *grid, const int
  * its raster-order pushes and relabels and the state it keeps across label
  * pairs.  result (W*H) receives a copy of initial, then the swaps.  One
  * thread-block cluster runs the whole solve where the grid's state fits its
- * shared memory, else one CTA; a solve that runs longer than 60 s on the device
- * returns GINF_ERR_TIMEOUT. */
+ * shared memory (up to about 110,000 nodes), else one CTA, several times slower;
+ * a solve that runs longer than 60 s on the device returns GINF_ERR_TIMEOUT. */
 ginf_status ginf_decode_alpha_beta(ginf_workspace *ws, const ginf_grid *grid, const int32_t *initial,
                                    int32_t iters, int32_t *result, const ginf_options *opt, ginf_stats *stats);
 
