@@ -398,12 +398,13 @@ __device__ __forceinline__ float min3_f32(float a, float b, float c) {
 }
 
 // The window term of output i at distance k of a quadratic message over
-// h[0, N): min(h[i-k], h[i+k]), or the one that exists at the ends.
+// h[0, N): min(h[i-k], h[i+k]), the one that exists at the ends, +inf where
+// neither does (N = 8 with a window of 8).
 template <int N>
 __device__ __forceinline__ float window_pair(const float *h, int i, int k) {
     const bool lo = i - k >= 0, hi = i + k < N;
     if (lo && hi) return fminf(h[i - k], h[i + k]);
-    return lo ? h[i - k] : h[i + k];
+    return lo ? h[i - k] : (hi ? h[i + k] : pos_inf<float>());
 }
 
 // Outputs c .. c + B - 1 of the windowed quadratic transform over h[0, N)
