@@ -658,17 +658,11 @@ __global__ void __launch_bounds__(conv_threads(IN_F32), 2)
 // pick a split that holds one of these CTAs per SM, not two).
 struct TcKernelSetup {
     SmemLimit smem;
-    std::atomic<bool> carveout[kMaxDevices];
+    Carveout carveout;
     template <typename K>
     cudaError_t ensure(K kern, int bytes) {
-        cudaError_t e = smem.ensure(kern, (size_t)bytes);
-        if (e != cudaSuccess) return e;
-        std::atomic<bool> &c = carveout[current_device()];
-        if (c.load(std::memory_order_acquire)) return cudaSuccess;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-        if (e == cudaSuccess) c.store(true, std::memory_order_release);
-        return e;
+        const cudaError_t e = smem.ensure(kern, (size_t)bytes);
+        return e != cudaSuccess ? e : carveout.ensure(kern, (int)cudaSharedmemCarveoutMaxShared);
     }
 };
 

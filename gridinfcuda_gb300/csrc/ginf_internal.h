@@ -133,6 +133,20 @@ struct SmemLimit {
     }
 };
 
+// The share of an SM's shared memory and L1 cache that a kernel prefers as
+// shared memory, in percent (-1: the driver's choice), set once per device.
+struct Carveout {
+    std::atomic<bool> set[kMaxDevices];
+    template <typename K>
+    cudaError_t ensure(K kern, int percent) {
+        std::atomic<bool> &c = set[current_device()];
+        if (c.load(std::memory_order_acquire)) return cudaSuccess;
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+        if (e == cudaSuccess) c.store(true, std::memory_order_release);
+        return e;
+    }
+};
+
 // Launches a kernel with programmatic stream serialisation: it may begin
 // while the kernel before it in the stream still runs, and waits for that one
 // in grid_dependency_wait().

@@ -535,59 +535,118 @@ __device__ __forceinline__ void message_quad_window(const SweepParams &p, unsign
 // Standard rule, truncated quadratic: O(L) lower envelope of parabolas
 // (Felzenszwalb & Huttenlocher, "Distance Transforms of Sampled Functions",
 // Theory of Computing 8, 2012), then truncation at min(h) + V(0, L-1).
+//
+// Bound: the envelope's stack in local memory, which beside the records' shared
+// memory does not fit the L1 cache (launch_general leaves it room).  So h = from
+// - in is read from the record as it is needed, the stack holds what the outputs
+// take (vertex, its height, left border: 9 bytes a label, with its top in
+// registers), and the outputs go over the incoming message, which nothing reads
+// by then.  1280x720, six half-sweeps, vectors h and o and 16-byte entries in
+// local memory -> here: FP32 L = 48 12900 -> 4460 us, L = 128 83000 -> 28900.
 template <typename T, typename M, int LMAX>
 __device__ void message_std_quad(const SweepParams &p, unsigned char *slot, int L, int dir, T s, T trunc) {
     if constexpr (std::is_same<T, int>::value) {
         return;  // integer grids use the exact O(L^2) rule instead (host side)
     } else {
+        constexpr int B = MIO<M, T>::B;
+        static_assert(LMAX <= 256, "vertices are bytes");
         unsigned char *md = slot + p.d_bytes + dir * p.m_bytes;
-        T h[LMAX], o[LMAX], z[LMAX + 1];
-        int v[LMAX];
-        load_h<T, M, LMAX>(slot, md, L, h);
-        T minh = h[0];
-        for (int i = 1; i < L; ++i) minh = h[i] < minh ? h[i] : minh;
-        if (!(s > T(0))) {
-            for (int i = 0; i < L; ++i) o[i] = minh;
-        } else {
-            int k = 0;
-            v[0] = 0;
-            z[0] = -pos_inf<T>();
-            z[1] = pos_inf<T>();
+        T z[LMAX], hv[LMAX];
+        uint8_t v[LMAX];
+        // The stack's top: its vertex, height, left border and value at zero.
+        int top = 0, vt = 0;
+        T ht = T(0), zt = -pos_inf<T>(), et = T(0), minh = T(0);
+        const bool flat = !(s > T(0));
 #pragma unroll 1
-            for (int q = 1; q < L; ++q) {
-                T sq;
-                for (;;) {
-                    const int pp = v[k];
-                    sq = ((h[q] + s * T(q) * T(q)) - (h[pp] + s * T(pp) * T(pp))) / (T(2) * s * T(q - pp));
-                    if (sq <= z[k] && k > 0) {
-                        --k;
-                        continue;
+        for (int c = 0; c < L; c += B) {
+            T a[B], f[B];
+            MIO<M, T>::load(md + c * sizeof(M), a);
+            load_t<T, B>(slot + c * sizeof(T), f);
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int q = c + k;
+                if (q >= L) break;
+                const T h = f[k] - a[k];
+                minh = q == 0 || h < minh ? h : minh;
+                if (flat) continue;
+                const T eq = h + s * T(q) * T(q);
+                T sq = -pos_inf<T>();
+                if (q > 0) {
+                    for (;;) {
+                        sq = (eq - et) / (T(2) * s * T(q - vt));
+                        if (!(sq <= zt && top > 0)) break;
+                        --top;
+                        vt = v[top];
+                        ht = hv[top];
+                        zt = z[top];
+                        et = ht + s * T(vt) * T(vt);
                     }
-                    break;
+                    // Not even the first parabola lies below: start anew.
+                    if (sq <= zt) sq = -pos_inf<T>();
+                    else ++top;
                 }
-                if (sq <= z[k]) {
-                    v[0] = q;
-                    z[0] = -pos_inf<T>();
-                    z[1] = pos_inf<T>();
-                    continue;
-                }
-                ++k;
-                v[k] = q;
-                z[k] = sq;
-                z[k + 1] = pos_inf<T>();
-            }
-            k = 0;
-#pragma unroll 1
-            for (int q = 0; q < L; ++q) {
-                while (z[k + 1] < T(q)) ++k;
-                const int pp = v[k];
-                o[q] = s * T(q - pp) * T(q - pp) + h[pp];
+                vt = q;
+                ht = h;
+                zt = sq;
+                et = eq;
+                v[top] = (uint8_t)q;
+                hv[top] = h;
+                z[top] = sq;
             }
         }
         const T cap = minh + trunc;
-        for (int i = 0; i < L; ++i) o[i] = rmin(o[i], cap);
-        normalise(o, L, p.norm_min);
-        store_msg<T, M>(md, o, L);
+        // Output q, called for q = 0, 1, ... in turn.
+        int at = 0;
+        T znext = T(0);
+        auto begin = [&] {
+            at = 0;
+            if (flat) return;
+            vt = v[0];
+            ht = hv[0];
+            znext = top > 0 ? z[1] : pos_inf<T>();
+        };
+        auto output = [&](int q) {
+            T o = minh;
+            if (!flat) {
+                while (znext < T(q)) {
+                    ++at;
+                    vt = v[at];
+                    ht = hv[at];
+                    znext = at < top ? z[at + 1] : pos_inf<T>();
+                }
+                o = s * T(q - vt) * T(q - vt) + ht;
+            }
+            return rmin(o, cap);
+        };
+        T val = T(0);
+        begin();
+#pragma unroll 1
+        for (int c = 0; c < L; c += B) {
+            T r[B];
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                r[k] = c + k < L ? output(c + k) : T(0);
+                if (c + k < L) {
+                    if (p.norm_min) val = c + k == 0 ? r[k] : rmin(val, r[k]);
+                    else val += r[k];
+                }
+            }
+            // Messages of the arithmetic type hold the outputs exactly.
+            if constexpr (sizeof(M) == sizeof(T)) MIO<M, T>::store(md + c * sizeof(M), r);
+        }
+        if (!p.norm_min) val = div_labels(val, L);
+        begin();
+#pragma unroll 1
+        for (int c = 0; c < L; c += B) {
+            T r[B];
+            if constexpr (sizeof(M) == sizeof(T)) MIO<M, T>::load(md + c * sizeof(M), r);
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                if constexpr (sizeof(M) != sizeof(T)) r[k] = c + k < L ? output(c + k) : T(0);
+                r[k] = c + k < L ? r[k] - val : T(0);
+            }
+            MIO<M, T>::store(md + c * sizeof(M), r);
+        }
     }
 }
 
@@ -1219,9 +1278,19 @@ template <typename T, typename M>
 cudaError_t launch_table(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms);
 
 // The lower envelope, and FP64 min-convolutions: one kernel per power of two,
-// labels tested against the run-time L.
+// labels tested against the run-time L.  The envelope's stacks want an L1 cache
+// more than the records want blocks: six half-sweeps at 1280x720 with V(0,k) =
+// min(k^2, 200), us, driver's choice -> two fifths of the SM as shared memory:
+// FP32 L = 32 3400 -> 2530, L = 64 9720 -> 8020, L = 128 35000 -> 28900, FP16
+// L = 128 30700 -> 25800, 41x28 FP16 L = 128 890 -> 500 (with four fifths FP32
+// L = 16 took a fifth longer).
 template <typename T, typename M, int LM>
 cudaError_t launch_general(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
+    if constexpr (sizeof(T) == 4) {
+        static Carveout carveout;
+        const cudaError_t e = carveout.ensure(sweep_kernel<T, M, LM, 1, 2, KIND_GENERAL>, 40);
+        if (e != cudaSuccess) return e;
+    }
     return launch_one<T, M, LM, 1, 2, KIND_GENERAL>(p, f.slot_bytes, s, num_sms);
 }
 
