@@ -211,7 +211,7 @@ std::string size_class_key(const ginf_grid &g) {
 
 // Raised when the batch kernels or the way they are launched change so that a
 // choice measured before says nothing about them.
-constexpr int kTuneRevision = 2;
+constexpr int kTuneRevision = 3;
 
 // Batch signature: what was measured (the kernels' revision, the device's SMs),
 // the multiset of (label count, log2 of the node count) buckets, and the
@@ -305,11 +305,11 @@ ginf_status bfail(ginf_status s, const std::string &msg) {
 }  // namespace
 
 // Grids whose label count falls in one bucket (lm = 8, 16, ... 64; exact: L is
-// 16, 32 or 64), solved by one kernel instantiation; items
-// first..first+count-1.
+// 16, 32 or 64; merged: every L between 32 and 64), solved by one kernel
+// instantiation; items first..first+count-1.
 struct BatchGroup {
     int lm = 64;
-    bool exact = true;
+    bool exact = true, merged = false;
     int first = 0, count = 0;
     int total_tiles = 0;
     uint32_t max_slot = 0;
@@ -355,19 +355,43 @@ namespace {
 int label_bucket(int L) { return (L + 7) / 8 * 8; }
 bool label_exact(int L) { return L == 16 || L == 32 || L == 64; }
 
-// Groups the grids by label bucket (once, at creation).
-void make_groups(ginf_batch *b) {
+// The work of a half-sweep, in updated nodes times labels, up to which the label
+// counts between 32 and 64 share a kernel.
+constexpr double kMergeWork = 3e6;
+
+// Groups the grids by label bucket.  A cooperative launch (several half-sweeps)
+// has the device to itself, so every bucket adds its launches' fixed costs; there
+// the buckets between 32 and 64 labels are one while a half-sweep of theirs is
+// short.  us a solve, apart -> together: five grids of 42 to 59 labels, 0.17e6,
+// 14 half-sweeps 280 -> 130; four of 38 to 58, 2.3e6, 12 428 -> 348; three of 36
+// to 60, 8.8e6, 6 488 -> 550.  (Those of up to 32 labels stay apart: warp_tile
+// moves whole vectors of its compiled count, which must be the records'.)
+void make_groups(ginf_batch *b, bool cooperative) {
+    double work = 0.0;
+    int bucket = 0;
+    bool several = false;
+    auto between = [](int L) { return L > 32 && L < 64; };
+    for (const ginf_grid &g : b->grids)
+        if (between(g.num_labels)) {
+            several |= bucket != 0 && bucket != label_bucket(g.num_labels);
+            bucket = label_bucket(g.num_labels);
+            if (g.width > 2 && g.height > 2) work += 0.5 * (g.width - 2) * (g.height - 2) * g.num_labels;
+        }
+    const bool merge = cooperative && several && work <= kMergeWork;
     b->groups.clear();
     b->order.clear();
     for (int lm = 8; lm <= 64; lm += 8)
-        for (int exact = 1; exact >= 0; --exact) {
+        for (int kind = 0; kind < 3; ++kind) {  // exact, merged, other
             BatchGroup grp;
             grp.lm = lm;
-            grp.exact = exact != 0;
+            grp.exact = kind == 0;
+            grp.merged = kind == 1;
             grp.first = (int)b->order.size();
             for (int i = 0; i < b->count; ++i) {
                 const int L = b->grids[i].num_labels;
-                if (label_bucket(L) != lm || label_exact(L) != grp.exact) continue;
+                const bool merged = merge && between(L);
+                if (label_exact(L) != grp.exact || merged != grp.merged || (merged ? 64 : label_bucket(L)) != lm)
+                    continue;
                 b->order.push_back(i);
                 grp.max_slot = std::max(grp.max_slot, b->fmt[i].slot_bytes);
             }
@@ -437,7 +461,9 @@ cudaError_t launch_batch(K kern, LaunchCache &cache, BatchLaunch bl, int warps, 
     const bool one = bl.it_end - bl.it_begin == 1;
     const int need = std::max(1, (bl.total_tiles + block_tiles - 1) / block_tiles);
     int grid = occ * num_sms;
-    if (grid > need && one) grid = need;
+    // No more blocks than tiles: a cooperative launch's others would only meet at
+    // the barrier (one 46-label grid of 40x25, 17 half-sweeps 143 -> 118 us).
+    if (grid > need) grid = need;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(warps * 32);
@@ -481,6 +507,7 @@ cudaError_t launch_group(const BatchGroup &grp, int tile_nodes, const BatchLaunc
         if (grp.lm == 32) return launch_batch_nw<32, 32>(tile_nodes, bl, grp.max_slot, num_sms, s);
         return launch_batch_nw<64, 64>(tile_nodes, bl, grp.max_slot, num_sms, s);
     }
+    if (grp.merged) return launch_batch_nw<64, 33>(tile_nodes, bl, grp.max_slot, num_sms, s);
     switch (grp.lm) {
         case 8: return launch_batch_nw<8, 1>(tile_nodes, bl, grp.max_slot, num_sms, s);
         case 16: return launch_batch_nw<16, 9>(tile_nodes, bl, grp.max_slot, num_sms, s);
@@ -585,6 +612,7 @@ void drop_graph(ginf_batch *b) {
 // here, before the capture, and the graph reads them from there.
 ginf_status capture(ginf_batch *b, const TuneChoice &c) {
     drop_graph(b);
+    make_groups(b, c.sweeps_per_launch != 1 && b->iters > 2);
     const std::vector<BatchItem> items = make_items(b, c.tile_nodes);
     GINF_BCK(cudaMemcpy(b->items_dev, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice));
     GINF_BCK(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
@@ -721,7 +749,7 @@ ginf_status ginf_batch_create(ginf_batch **out, const ginf_grid *grids, int32_t 
     }
     b->arena_bytes = total;
     for (int i = 0; i < count; ++i) b->rec.push_back(b->arena + off[i]);
-    make_groups(b);
+    make_groups(b, false);
     b->items_dev = reinterpret_cast<BatchItem *>(b->arena + items_off);
     b->barrier = reinterpret_cast<unsigned int *>(b->arena + ctl_off);
     b->status = reinterpret_cast<int *>(b->arena + ctl_off + 64);

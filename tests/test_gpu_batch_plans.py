@@ -68,3 +68,39 @@ def test_tile_size_reported_is_the_one_in_use(ginf, tmp_path, monkeypatch):
     for tile in (8, 16, 32):
         with ginf.Batch(problems, labels, 6, tile_nodes=tile, sweeps_per_launch=1) as b:
             assert b.config()["tile_nodes"] == tile
+
+
+@pytest.mark.parametrize("spl", [3, 0])
+@pytest.mark.parametrize("W,H", [(37, 23), (330, 260)])
+def test_groups_of_a_cooperative_launch(ginf, spl, W, H):
+    """Label counts between 32 and 64 in one kernel (the small grids) and apart
+    (the large ones), beside those that always stay apart."""
+    problems, labels = _problems((5, 20, 33, 40, 41, 50, 63, 64), W, H)
+    want = [ginf.decode_hbp(D, V, m, 1, 8).cpu().numpy() for D, V, m in problems]
+    with ginf.Batch(problems, labels, 8, tile_nodes=16, sweeps_per_launch=spl) as b:
+        for _ in range(2):
+            b.run()
+            for (D, _, _), lab, w in zip(problems, labels, want):
+                assert np.array_equal(lab.cpu().numpy(), w), D.shape
+                lab.zero_()
+
+
+def test_time_of_mixed_label_counts_in_cooperative_launches(ginf):
+    """Small grids of four label buckets take at most twice the time of as many
+    grids of one (about the same; with launches for each bucket three times)."""
+    import torch
+    times = []
+    for counts in ((48, 48, 48, 48, 48), (34, 44, 53, 59, 62)):
+        problems, labels = _problems(counts, 60, 50)
+        with ginf.Batch(problems, labels, 15, tile_nodes=16, sweeps_per_launch=0) as b:
+            best = float("inf")
+            for _ in range(6):
+                a, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                torch.cuda.synchronize()
+                a.record()
+                b.run()
+                e.record()
+                torch.cuda.synchronize()
+                best = min(best, a.elapsed_time(e))
+        times.append(best)
+    assert times[1] < 2 * times[0], times
