@@ -923,8 +923,18 @@ cudaError_t launch_wide(const RecordFormat &f, const void *src, int W, int H, un
     return cudaGetLastError();
 }
 
+// Nodes from which on host costs are read by the wide transform: below, its
+// blocks are too few to hide the link's latency, and the device costs' transforms
+// read them.  One level, one half-sweep, device costs' -> wide, us: 40x30 L = 128
+// 96 -> 118, 160x120 L = 64 134 -> 141, 203x151 L = 128 240 -> 225, L = 16
+// 109 -> 107, 640x480 L = 32 462 -> 383.
+constexpr long kWideNodes = 1 << 15;
+
 cudaError_t launch_costs_from_host(const RecordFormat &f, int cost_type, const void *src, int W, int H,
                                    unsigned char *rec, unsigned char *crec, int cW, cudaStream_t s) {
+    if ((long)W * H < kWideNodes)
+        return crec ? launch_costs_to_records_pyr(f, cost_type, src, W, H, rec, crec, cW, s)
+                    : launch_costs_to_records(f, cost_type, src, W, H, rec, s);
     GINF_DISPATCH_T(f, {
         return cost_type == CT_F32 ? launch_wide<float, T>(f, src, W, H, rec, crec, cW, s)
                                    : launch_wide<int, T>(f, src, W, H, rec, crec, cW, s);
