@@ -438,9 +438,9 @@ ginf_status prepare(Call &c, Prepared &P, int levels, bool want_lab2, const int3
     return GINF_OK;
 }
 
-// Truncation radius of a quadratic table, with the comparisons of the
-// device's quad_radius (sweep_impl.cuh): V(0,k) < V(0,L-1) for k <= r on a
-// nondecreasing profile; 9 means "wider than any window".
+// Truncation radius r of a quadratic table: V(0,k) < V(0,L-1) for k <= r on a
+// nondecreasing profile that starts at or below V(0,L-1).  Taps further out are
+// dominated by min(h) + V(0,L-1).  9 means "wider than any window".
 template <typename T>
 int quad_radius_host(const std::vector<unsigned char> &col, int L) {
     const T *v = reinterpret_cast<const T *>(col.data());

@@ -453,25 +453,6 @@ __device__ __forceinline__ void window_outputs(const float *h, int c, const floa
 constexpr int kQuadWindow = 8;
 constexpr int kQuadWindowSmall = 4;
 
-// Truncation radius r of a truncated-quadratic table: V(0,k) < V(0,L-1) for
-// k <= r and V(0,r+1) >= V(0,L-1).  Taps further out are dominated by
-// min(h) + V(0,L-1).  Returns kQuadWindow + 1 when r exceeds the window.
-template <typename T>
-__device__ __forceinline__ int quad_radius(const T *Vt, int L, T trunc) {
-    int r = 0;
-    T prev = __ldg(&Vt[0]);
-    for (int k = 1; k < L && k <= kQuadWindow + 1; ++k) {
-        const T v = __ldg(&Vt[(size_t)L * k]);
-        if (v < prev) return kQuadWindow + 1;  // not a nondecreasing profile: use the lower envelope
-        prev = v;
-        if (!(v < trunc)) break;
-        r = k;
-    }
-    // The profile must also start at its minimum and stay below the cap.
-    if (!(__ldg(&Vt[0]) <= trunc)) return kQuadWindow + 1;
-    return r;
-}
-
 // Standard rule, truncated quadratic, windowed exact form:
 //   out(i) = min( min_{|k| <= r} h(i+k) + V(0,|k|),  min(h) + V(0,L-1) ),
 // which equals the brute-force min_j h(j) + V(i,j) over the whole table
@@ -731,31 +712,29 @@ enum { KIND_LINEAR = 0, KIND_QUAD = 1, KIND_GENERAL = 2, KIND_QUAD4 = 3, KIND_QU
 
 // Constants a launch reads from its smoothness table: slope V(0,1) and
 // truncation V(0,L-1) (bp.cc:35,43), and for the quadratic kernels the taps
-// V(0,k) (+inf beyond the truncation radius) and that radius.
+// V(0,k), +inf beyond the truncation radius.  The loads are independent: the
+// radius is the host's, since finding it here was a chain of loads at the head
+// of every launch (20 half-sweeps of 15x21, L = 16, radius 8: 185 us, so 158).
 template <typename T>
 struct TableConsts {
     T scale, trunc;
     T vtap[kQuadWindow + 1];
     T cpass[kQuadPasses];  // KIND_QUADPASS: increments s (2j-1), +inf beyond the radius
-    int qr;
 };
 
 template <typename T, int KIND>
-__device__ __forceinline__ TableConsts<T> table_consts(const void *V, int L) {
+__device__ __forceinline__ TableConsts<T> table_consts(const void *V, int L, int radius = 0) {
     TableConsts<T> tc;
     const T *Vt = static_cast<const T *>(V);
     tc.scale = __ldg(&Vt[L]);
     tc.trunc = __ldg(&Vt[(size_t)L * (L - 1)]);
-    tc.qr = kQuadWindow + 1;
     if constexpr ((KIND == KIND_QUAD || KIND == KIND_QUAD4) && sizeof(T) == 4) {
-        tc.qr = quad_radius(Vt, L, tc.trunc);
 #pragma unroll
-        for (int k = 0; k <= kQuadWindow; ++k) tc.vtap[k] = k <= tc.qr ? __ldg(&Vt[(size_t)L * k]) : pos_inf<T>();
+        for (int k = 0; k <= kQuadWindow; ++k) tc.vtap[k] = k <= radius ? __ldg(&Vt[(size_t)L * k]) : pos_inf<T>();
     }
     if constexpr (KIND == KIND_QUADPASS && sizeof(T) == 4) {
-        tc.qr = quad_radius(Vt, L, tc.trunc);
 #pragma unroll
-        for (int j = 0; j < kQuadPasses; ++j) tc.cpass[j] = j < tc.qr ? tc.scale * T(2 * j + 1) : pos_inf<T>();
+        for (int j = 0; j < kQuadPasses; ++j) tc.cpass[j] = j < radius ? tc.scale * T(2 * j + 1) : pos_inf<T>();
     }
     return tc;
 }
@@ -1138,7 +1117,7 @@ __global__ void __launch_bounds__(NW * 32, 5) sweep_kernel_split(const SweepPara
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
     __shared__ SplitXch<NW> xs;
-    const TableConsts<float> tc = table_consts<float, KIND_QUAD>(p.V, LMIN == LMAX ? LMAX : p.L);
+    const TableConsts<float> tc = table_consts<float, KIND_QUAD>(p.V, LMIN == LMAX ? LMAX : p.L, p.quad_radius);
     if (threadIdx.x == 0) {
         mbar_init(&full_bar, NW * 32);
         fence_barrier_init();
@@ -1162,7 +1141,7 @@ template <typename T, typename M, int LMAX, int LMIN, int NW, int KIND, bool DIR
 __device__ __forceinline__ void sweep_body(const SweepParams &p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full_bar;
-    const TableConsts<T> tc = table_consts<T, KIND>(p.V, LMIN == LMAX ? LMAX : p.L);
+    const TableConsts<T> tc = table_consts<T, KIND>(p.V, LMIN == LMAX ? LMAX : p.L, p.quad_radius);
     if (threadIdx.x == 0) {
         mbar_init(&full_bar, NW * 32);
         fence_barrier_init();
