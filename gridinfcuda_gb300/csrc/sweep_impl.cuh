@@ -1262,14 +1262,14 @@ cudaError_t launch_table(const RecordFormat &f, const SweepParams &p, cudaStream
 // min(k^2, 200), us, driver's choice -> two fifths of the SM as shared memory:
 // FP32 L = 32 3400 -> 2530, L = 64 9720 -> 8020, L = 128 35000 -> 28900, FP16
 // L = 128 30700 -> 25800, 41x28 FP16 L = 128 890 -> 500 (with four fifths FP32
-// L = 16 took a fifth longer).
+// L = 16 took a fifth longer).  FP64, whose records are larger, four fifths: four
+// half-sweeps of the standard rule's min-convolution, 59x120 L = 32 820 -> 520,
+// L = 48 1720 -> 1200, 320x240 L = 64 12000 -> 11900, though L = 40 3170 -> 3730.
 template <typename T, typename M, int LM>
 cudaError_t launch_general(const RecordFormat &f, const SweepParams &p, cudaStream_t s, int num_sms) {
-    if constexpr (sizeof(T) == 4) {
-        static Carveout carveout;
-        const cudaError_t e = carveout.ensure(sweep_kernel<T, M, LM, 1, 2, KIND_GENERAL>, 40);
-        if (e != cudaSuccess) return e;
-    }
+    static Carveout carveout;
+    const cudaError_t e = carveout.ensure(sweep_kernel<T, M, LM, 1, 2, KIND_GENERAL>, sizeof(T) == 4 ? 40 : 80);
+    if (e != cudaSuccess) return e;
     return launch_one<T, M, LM, 1, 2, KIND_GENERAL>(p, f.slot_bytes, s, num_sms);
 }
 
